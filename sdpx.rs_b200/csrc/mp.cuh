@@ -5,651 +5,892 @@
 // significant first, i32 kind = sign * MPFR kind (2 zero, 3 regular), i32 exponent; a regular
 // value is M * 2^(exponent - 64N) with the top bit of M set.
 //
-// Every operation forms its exact result as a wide integer times a power of two and rounds it
-// once (mp_round):
-//   mp_addsub           aligned exact sum (operands more than 64N + 64 bits apart: the smaller
-//                       one lies below a 2^-64 fraction of an ulp and leaves the larger unchanged)
-//   mp_mul              2N-limb product
-//   mp_recip, mp_div,   the integer quotient floor(2^(128N + 2) / M), floor(M_a 2^(64N + 2) / M_b)
-//   mp_sqrt             or root floor(sqrt(M 2^e)) with its remainder folded into a sticky bit;
+// Everything is a template on N with every loop over words unrolled, so mantissas, products and
+// accumulators live in registers (32-bit words, carries by add.cc / madc chains) instead of
+// run-time-length loops over local memory: an exact product of two 256-bit mantissas is 64
+// multiply-adds.  Every operation forms its exact result (or the exact result's leading words
+// with a sticky bit) and rounds it once:
+//   addsub              aligned sum with a 64-bit guard and a sticky bit (operands more than
+//                       64N + 64 bits apart: the larger one unchanged)
+//   mul                 2N-limb product
+//   recip, divide,      the integer quotient floor(2^(128N + 2) / M), floor(M_a 2^(64N + 2) / M_b)
+//   root                or root floor(sqrt(M 2^e)) with its remainder folded into a sticky bit;
 //                       the quotient or root from a Newton estimate corrected exactly by its
-//                       multiword remainder (the same integers a long division would give)
-//   mp_dot_sub          a - sum x_c y_c (or sum x_c y_c) exact in a two's-complement fixed-point
-//                       accumulator of up to kAccWords words, rounded once -- the exact dot of
-//                       exactdot.rs:53-70; terms spread beyond the accumulator report failure.
+//                       multiword remainder
+//   dot<N, G>           a - sum x_c y_c (or sum x_c y_c) by G lanes, exact in a two's-complement
+//                       fixed-point accumulator and rounded once (the exact dot of
+//                       exactdot.rs:53-70).  Terms whose scales span at most kSpanBits accumulate in
+//                       registers; up to kAccWords words in local memory; wider ones report failure.
+// The arithmetic compiles for the host too (plain C++ in place of the carry chains), where the
+// tests compare it with exact integers.
 #pragma once
 #include <climits>
+#include <cmath>
 #include <cstdint>
+#include <type_traits>
+
+#if defined(__CUDACC__)
+#define MPD_FN __host__ __device__ __forceinline__
+#define MPD_CALL __host__ __device__ __noinline__
+#else
+#define MPD_FN inline
+#define MPD_CALL inline
+#endif
 
 namespace mpd {
 
 constexpr int kMaxN = 8;        // limbs: up to 512-bit values
 constexpr int kAccWords = 40;   // exact-dot accumulator: 2560 bits of spread + width
-constexpr int kWideWords = 2 * kMaxN + 3;
 constexpr int kKindZero = 2, kKindRegular = 3;
 constexpr int kExpMax = (1 << 30) - 1;
 
+template <int N>
 struct Val {
-  unsigned long long m[kMaxN];  // mantissa, top bit of limb N-1 set (unless zero)
-  long long s;                  // scale: value = (-1)^neg M 2^s
+  uint32_t m[2 * N];  // mantissa, top bit set (unless zero), least significant word first
+  long long s;        // scale: value = (-1)^neg M 2^s
   bool neg, zero;
 };
 
-__device__ __forceinline__ Val mp_load(const unsigned char* p, int N) {
-  Val v;
-  const unsigned long long* l = reinterpret_cast<const unsigned long long*>(p);
-  const int kind = *reinterpret_cast<const int*>(p + 8 * N);
-  const int ex = *reinterpret_cast<const int*>(p + 8 * N + 4);
-  v.zero = (kind == kKindZero || kind == -kKindZero);
-  v.neg = kind < 0;
-#pragma unroll
-  for (int q = 0; q < kMaxN; ++q) v.m[q] = (q < N && !v.zero) ? l[q] : 0ull;
-  v.s = (long long)ex - 64LL * N;
-  return v;
+// ---- word arithmetic ----
+
+MPD_FN uint32_t funnel_l(uint32_t lo, uint32_t hi, int r) {  // high word of (hi:lo) << r, 0 <= r < 32
+#if defined(__CUDA_ARCH__)
+  return __funnelshift_l(lo, hi, r);
+#else
+  return r ? (hi << r) | (lo >> (32 - r)) : hi;
+#endif
+}
+MPD_FN uint32_t funnel_r(uint32_t lo, uint32_t hi, int r) {  // low word of (hi:lo) >> r, 0 <= r < 32
+#if defined(__CUDA_ARCH__)
+  return __funnelshift_r(lo, hi, r);
+#else
+  return r ? (lo >> r) | (hi << (32 - r)) : lo;
+#endif
+}
+MPD_FN int clz32(uint32_t v) {
+#if defined(__CUDA_ARCH__)
+  return __clz((int)v);
+#else
+  return v ? __builtin_clz(v) : 32;
+#endif
 }
 
-// Store v (zeros as +0); an exponent outside the MPFR range sets bit 4 (non-finite) of *status.
-__device__ __forceinline__ void mp_store(unsigned char* p, int N, const Val& v, uint32_t* status) {
-  unsigned long long* l = reinterpret_cast<unsigned long long*>(p);
-  int* kind = reinterpret_cast<int*>(p + 8 * N);
-  const long long ex = v.s + 64LL * N;
-  if (v.zero || ex > kExpMax || ex < -kExpMax) {
-    if (!v.zero && status) atomicOr(status, 4u);
-    for (int q = 0; q < N; ++q) l[q] = 0ull;
-    kind[0] = kKindZero;
-    kind[1] = 0;
-    return;
+// a[0..K) += b[0..K) + c; the carry out.  (The asm blocks below write their outputs last: operands
+// of equal value may share a register with an output.)
+template <int K>
+MPD_FN uint32_t add_words(uint32_t* a, const uint32_t* b, uint32_t c) {
+#if defined(__CUDA_ARCH__)
+  constexpr int K4 = K / 4 * 4;
+#pragma unroll
+  for (int i = 0; i < K4; i += 4)
+    asm("{\n\t.reg .u32 t0, t1, t2, t3;\n\t"
+        "add.cc.u32 t0, %13, 0xffffffff;\n\t"
+        "addc.cc.u32 t0, %5, %9;\n\t"
+        "addc.cc.u32 t1, %6, %10;\n\t"
+        "addc.cc.u32 t2, %7, %11;\n\t"
+        "addc.cc.u32 t3, %8, %12;\n\t"
+        "addc.u32 %4, 0, 0;\n\t"
+        "mov.u32 %0, t0;\n\tmov.u32 %1, t1;\n\tmov.u32 %2, t2;\n\tmov.u32 %3, t3;\n\t}"
+        : "=r"(a[i]), "=r"(a[i + 1]), "=r"(a[i + 2]), "=r"(a[i + 3]), "=r"(c)
+        : "r"(a[i]), "r"(a[i + 1]), "r"(a[i + 2]), "r"(a[i + 3]), "r"(b[i]), "r"(b[i + 1]), "r"(b[i + 2]),
+          "r"(b[i + 3]), "r"(c));
+#pragma unroll
+  for (int i = K4; i < K; ++i)
+    asm("{\n\t.reg .u32 t0;\n\t"
+        "add.cc.u32 t0, %4, 0xffffffff;\n\t"
+        "addc.cc.u32 t0, %2, %3;\n\t"
+        "addc.u32 %1, 0, 0;\n\t"
+        "mov.u32 %0, t0;\n\t}"
+        : "=r"(a[i]), "=r"(c)
+        : "r"(a[i]), "r"(b[i]), "r"(c));
+#else
+  for (int i = 0; i < K; ++i) {
+    const uint64_t t = (uint64_t)a[i] + b[i] + c;
+    a[i] = (uint32_t)t;
+    c = (uint32_t)(t >> 32);
   }
-  for (int q = 0; q < N; ++q) l[q] = v.m[q];
-  kind[0] = v.neg ? -kKindRegular : kKindRegular;
-  kind[1] = (int)ex;
+#endif
+  return c;
+}
+// a[0..K) -= b[0..K); the borrow out.
+template <int K>
+MPD_FN uint32_t sub_words(uint32_t* a, const uint32_t* b) {
+  uint32_t t[K];
+#pragma unroll
+  for (int i = 0; i < K; ++i) t[i] = ~b[i];
+  return 1u - add_words<K>(a, t, 1u);
+}
+// a[0..K) += x (one word); the carry out.
+template <int K>
+MPD_FN uint32_t add_word(uint32_t* a, uint32_t x) {
+  uint32_t z[K];
+#pragma unroll
+  for (int i = 0; i < K; ++i) z[i] = 0u;
+  z[0] = x;
+  return add_words<K>(a, z, 0u);
+}
+// a[0..K) = -a.
+template <int K>
+MPD_FN void neg_words(uint32_t* a) {
+  uint32_t z[K];
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    a[i] = ~a[i];
+    z[i] = 0u;
+  }
+  add_words<K>(a, z, 1u);
+}
+template <int K>
+MPD_FN bool is_zero(const uint32_t* a) {
+  uint32_t o = 0;
+#pragma unroll
+  for (int i = 0; i < K; ++i) o |= a[i];
+  return o == 0;
+}
+// sign of a - b over K words
+template <int K>
+MPD_FN int cmp_words(const uint32_t* a, const uint32_t* b) {
+  int r = 0;
+#pragma unroll
+  for (int i = 0; i < K; ++i) r = a[i] == b[i] ? r : (a[i] > b[i] ? 1 : -1);
+  return r;
 }
 
-__device__ __forceinline__ Val mp_zero() {
-  Val v;
+// One link of a multiply-accumulate chain: the P 64-bit words (acc[2i+1] : acc[2i]) += a[2i] * b,
+// carry in and out in c.
+template <int P>
+MPD_FN void mac_link(uint32_t* acc, const uint32_t* a, uint32_t b, uint32_t& c) {
+#if defined(__CUDA_ARCH__)
+  if constexpr (P == 4) {
+    asm("{\n\t.reg .u32 t0, t1, t2, t3, t4, t5, t6, t7;\n\t"
+        "add.cc.u32 t0, %22, 0xffffffff;\n\t"
+        "madc.lo.cc.u32 t0, %17, %21, %9;\n\t"
+        "madc.hi.cc.u32 t1, %17, %21, %10;\n\t"
+        "madc.lo.cc.u32 t2, %18, %21, %11;\n\t"
+        "madc.hi.cc.u32 t3, %18, %21, %12;\n\t"
+        "madc.lo.cc.u32 t4, %19, %21, %13;\n\t"
+        "madc.hi.cc.u32 t5, %19, %21, %14;\n\t"
+        "madc.lo.cc.u32 t6, %20, %21, %15;\n\t"
+        "madc.hi.cc.u32 t7, %20, %21, %16;\n\t"
+        "addc.u32 %8, 0, 0;\n\t"
+        "mov.u32 %0, t0;\n\tmov.u32 %1, t1;\n\tmov.u32 %2, t2;\n\tmov.u32 %3, t3;\n\t"
+        "mov.u32 %4, t4;\n\tmov.u32 %5, t5;\n\tmov.u32 %6, t6;\n\tmov.u32 %7, t7;\n\t}"
+        : "=r"(acc[0]), "=r"(acc[1]), "=r"(acc[2]), "=r"(acc[3]), "=r"(acc[4]), "=r"(acc[5]), "=r"(acc[6]),
+          "=r"(acc[7]), "=r"(c)
+        : "r"(acc[0]), "r"(acc[1]), "r"(acc[2]), "r"(acc[3]), "r"(acc[4]), "r"(acc[5]), "r"(acc[6]), "r"(acc[7]),
+          "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(a[6]), "r"(b), "r"(c));
+  } else if constexpr (P == 2) {
+    asm("{\n\t.reg .u32 t0, t1, t2, t3;\n\t"
+        "add.cc.u32 t0, %12, 0xffffffff;\n\t"
+        "madc.lo.cc.u32 t0, %9, %11, %5;\n\t"
+        "madc.hi.cc.u32 t1, %9, %11, %6;\n\t"
+        "madc.lo.cc.u32 t2, %10, %11, %7;\n\t"
+        "madc.hi.cc.u32 t3, %10, %11, %8;\n\t"
+        "addc.u32 %4, 0, 0;\n\t"
+        "mov.u32 %0, t0;\n\tmov.u32 %1, t1;\n\tmov.u32 %2, t2;\n\tmov.u32 %3, t3;\n\t}"
+        : "=r"(acc[0]), "=r"(acc[1]), "=r"(acc[2]), "=r"(acc[3]), "=r"(c)
+        : "r"(acc[0]), "r"(acc[1]), "r"(acc[2]), "r"(acc[3]), "r"(a[0]), "r"(a[2]), "r"(b), "r"(c));
+  } else {
+    asm("{\n\t.reg .u32 t0, t1;\n\t"
+        "add.cc.u32 t0, %7, 0xffffffff;\n\t"
+        "madc.lo.cc.u32 t0, %5, %6, %3;\n\t"
+        "madc.hi.cc.u32 t1, %5, %6, %4;\n\t"
+        "addc.u32 %2, 0, 0;\n\t"
+        "mov.u32 %0, t0;\n\tmov.u32 %1, t1;\n\t}"
+        : "=r"(acc[0]), "=r"(acc[1]), "=r"(c)
+        : "r"(acc[0]), "r"(acc[1]), "r"(a[0]), "r"(b), "r"(c));
+  }
+#else
+  for (int i = 0; i < P; ++i) {
+    const unsigned __int128 t = (unsigned __int128)((uint64_t)a[2 * i] * b) +
+                                (((uint64_t)acc[2 * i + 1] << 32) | acc[2 * i]) + c;
+    acc[2 * i] = (uint32_t)t;
+    acc[2 * i + 1] = (uint32_t)(t >> 32);
+    c = (uint32_t)(t >> 64);
+  }
+#endif
+}
+// The 2N words at acc += sum_i a[2i] b 2^(64 i); the carry out.
+template <int N>
+MPD_FN uint32_t mac_chain(uint32_t* acc, const uint32_t* a, uint32_t b) {
+  uint32_t c = 0;
+  constexpr int N4 = N / 4 * 4;
 #pragma unroll
-  for (int q = 0; q < kMaxN; ++q) v.m[q] = 0ull;
+  for (int i = 0; i < N4; i += 4) mac_link<4>(acc + 2 * i, a + 2 * i, b, c);
+  if constexpr ((N & 3) >= 2) mac_link<2>(acc + 2 * N4, a + 2 * N4, b, c);
+  if constexpr (N & 1) mac_link<1>(acc + 2 * (N - 1), a + 2 * (N - 1), b, c);
+  return c;
+}
+
+// P (4N words) = a * b (2N words each).  The products a_i b_j with i + j even and with i + j odd
+// are summed in two accumulators (the second one word up), so that every chain adds aligned
+// 64-bit products with one running carry.
+template <int N>
+MPD_FN void mul_words(uint32_t* P, const uint32_t* a, const uint32_t* b) {
+  constexpr int W = 2 * N;
+  uint32_t O[2 * W];
+#pragma unroll
+  for (int i = 0; i < W; i += 2) {
+    const uint64_t e = (uint64_t)a[i] * b[0], o = (uint64_t)a[i + 1] * b[0];
+    P[i] = (uint32_t)e;
+    P[i + 1] = (uint32_t)(e >> 32);
+    O[i] = (uint32_t)o;
+    O[i + 1] = (uint32_t)(o >> 32);
+  }
+#pragma unroll
+  for (int i = W; i < 2 * W; ++i) P[i] = O[i] = 0u;
+#pragma unroll
+  for (int j = 1; j < W; ++j) {
+    if (j & 1) {
+      const uint32_t c = mac_chain<N>(P + j + 1, a + 1, b[j]);
+      if (j + 1 + W < 2 * W) P[j + 1 + W] += c;
+      O[j - 1 + W] += mac_chain<N>(O + j - 1, a, b[j]);
+    } else {
+      P[j + W] += mac_chain<N>(P + j, a, b[j]);
+      O[j + W] += mac_chain<N>(O + j, a + 1, b[j]);
+    }
+  }
+  add_words<2 * W - 1>(P + 1, O, 0u);
+}
+
+// ---- rounding ----
+
+template <int N>
+MPD_FN Val<N> zero_val() {
+  Val<N> v;
+#pragma unroll
+  for (int q = 0; q < 2 * N; ++q) v.m[q] = 0u;
   v.s = 0;
   v.neg = false;
   v.zero = true;
   return v;
 }
-
-// Round S (W little-endian words, magnitude) * 2^scale to N limbs, ties to even.
-__device__ inline Val mp_round(const unsigned long long* S, int W, bool neg, long long scale, int N) {
-  int top = -1;
-  for (int w = W - 1; w >= 0; --w)
-    if (S[w]) {
-      top = w;
-      break;
-    }
-  if (top < 0) return mp_zero();
-  const int bitlen = top * 64 + 64 - __clzll(S[top]);
-  int shift = bitlen - 64 * N;
-  auto window = [&](int start) -> unsigned long long {  // bits [start, start + 64) of S
-    const int word = (start >= 0) ? start / 64 : -((-start + 63) / 64);
-    const int off = start - 64 * word;
-    const unsigned long long lo = (word >= 0 && word < W) ? S[word] : 0ull;
-    const unsigned long long hi = (word + 1 >= 0 && word + 1 < W) ? S[word + 1] : 0ull;
-    return (lo >> off) | (off ? (hi << (64 - off)) : 0ull);
-  };
-  Val v;
+template <int N>
+MPD_FN Val<N> one_val() {
+  Val<N> v = zero_val<N>();
   v.zero = false;
-  v.neg = neg;
-#pragma unroll
-  for (int q = 0; q < kMaxN; ++q) v.m[q] = q < N ? window(shift + 64 * q) : 0ull;
-  if (shift > 0) {
-    const int rb = shift - 1;
-    const bool round_bit = (S[rb / 64] >> (rb % 64)) & 1ull;
-    bool sticky = false;
-    for (int w = 0; w < rb / 64; ++w) sticky = sticky || (S[w] != 0);
-    if (rb % 64) sticky = sticky || ((S[rb / 64] & ((1ull << (rb % 64)) - 1)) != 0);
-    if (round_bit && (sticky || (v.m[0] & 1ull))) {
-      bool carry = true;
-      for (int q = 0; q < N && carry; ++q) {
-        v.m[q] += 1;
-        carry = (v.m[q] == 0);
-      }
-      if (carry) {
-        v.m[N - 1] = 1ull << 63;
-        shift += 1;
-      }
-    }
-  }
-  v.s = scale + shift;
+  v.m[2 * N - 1] = 1u << 31;
+  v.s = 1 - 64LL * N;
   return v;
 }
 
-// dst += src << sh (bits) over W words (two's complement); src has n words.
-__device__ __forceinline__ void add_shifted(unsigned long long* dst, int W, const unsigned long long* src, int n,
-                                            long long sh) {
-  const int q = (int)(sh >> 6), r = (int)(sh & 63);
-  unsigned long long carry = 0;
-  for (int i = 0; i <= n && q + i < W; ++i) {
-    const unsigned long long lo = i < n ? src[i] : 0ull;
-    const unsigned long long prev = (i > 0 && i - 1 < n) ? src[i - 1] : 0ull;
-    const unsigned long long part = r ? ((lo << r) | (prev >> (64 - r))) : lo;
-    const unsigned long long a = dst[q + i];
-    const unsigned long long t = a + part;
-    const unsigned long long c1 = t < a;
-    const unsigned long long t2 = t + carry;
-    const unsigned long long c2 = t2 < t;
-    dst[q + i] = t2;
-    carry = c1 + c2;
+template <int K, int W>
+struct ShiftStage {  // shift S left by W words while its top W words are zero, then by W/2, ...
+  static MPD_FN void run(uint32_t* S, int& sh) {
+    if (W < K) {
+      uint32_t o = 0;
+#pragma unroll
+      for (int i = 0; i < W && i < K; ++i) o |= S[K - 1 - i];
+      if (o == 0) {
+#pragma unroll
+        for (int i = K - 1; i >= 0; --i) S[i] = i >= W ? S[i >= W ? i - W : 0] : 0u;
+        sh += 32 * W;
+      }
+    }
+    ShiftStage<K, W / 2>::run(S, sh);
   }
-  for (int i = q + n + 1; i < W && carry; ++i) {
-    dst[i] += carry;
-    carry = dst[i] == 0;
-  }
-}
-// dst -= src << sh (two's complement over W words)
-__device__ __forceinline__ void sub_shifted(unsigned long long* dst, int W, const unsigned long long* src, int n,
-                                            long long sh) {
-  const int q = (int)(sh >> 6), r = (int)(sh & 63);
-  unsigned long long borrow = 0;
-  for (int i = 0; i <= n && q + i < W; ++i) {
-    const unsigned long long lo = i < n ? src[i] : 0ull;
-    const unsigned long long prev = (i > 0 && i - 1 < n) ? src[i - 1] : 0ull;
-    const unsigned long long part = r ? ((lo << r) | (prev >> (64 - r))) : lo;
-    const unsigned long long a = dst[q + i];
-    const unsigned long long t = a - part;
-    const unsigned long long b1 = a < part;
-    const unsigned long long t2 = t - borrow;
-    const unsigned long long b2 = t < borrow;
-    dst[q + i] = t2;
-    borrow = b1 + b2;
-  }
-  for (int i = q + n + 1; i < W && borrow; ++i) {
-    const unsigned long long a = dst[i];
-    dst[i] = a - borrow;
-    borrow = a < borrow;
-  }
+};
+template <int K>
+struct ShiftStage<K, 0> {
+  static MPD_FN void run(uint32_t*, int&) {}
+};
+
+// Shift the nonzero S (K <= 64 words) left until its top bit is set; the bits shifted.
+template <int K>
+MPD_FN int normalize(uint32_t* S) {
+  int sh = 0;
+  if (S[K - 1] == 0) ShiftStage<K, 32>::run(S, sh);
+  const int c = clz32(S[K - 1]) & 31;
+#pragma unroll
+  for (int i = K - 1; i > 0; --i) S[i] = funnel_l(S[i - 1], S[i], c);
+  S[0] <<= c;
+  return sh + c;
 }
 
-// a + sign * b, exact then rounded (sign = -1: subtraction).
-__device__ inline Val mp_addsub(const Val& a, const Val& b, int sign, int N) {
-  Val bb = b;
-  if (sign < 0) bb.neg = !bb.neg;
-  if (bb.zero) {
-    if (a.zero) {  // (+0) + (-0) = +0 under round to nearest
-      Val z = mp_zero();
-      z.neg = a.neg && bb.neg;
-      return z;
+// S (K > 2N words, top bit set) * 2^scale rounded to N limbs, ties to even.
+template <int N, int K>
+MPD_FN Val<N> round_top(const uint32_t* S, bool neg, long long scale) {
+  Val<N> v;
+  v.zero = false;
+  v.neg = neg;
+#pragma unroll
+  for (int q = 0; q < 2 * N; ++q) v.m[q] = S[K - 2 * N + q];
+  uint32_t sticky = S[K - 2 * N - 1] << 1;
+#pragma unroll
+  for (int i = 0; i < K - 2 * N - 1; ++i) sticky |= S[i];
+  long long s = scale + 32 * (K - 2 * N);
+  if ((S[K - 2 * N - 1] >> 31) && (sticky || (v.m[0] & 1u))) {
+    if (add_word<2 * N>(v.m, 1u)) {  // carried out: the mantissa wrapped to zero
+      v.m[2 * N - 1] = 1u << 31;
+      s += 1;
     }
-    return a;
   }
-  if (a.zero) return bb;
-  const long long gap = 64LL * N + 64;
-  const long long d = a.s - bb.s;
+  v.s = s;
+  return v;
+}
+
+// ---- elements ----
+
+template <int N>
+MPD_FN Val<N> load(const unsigned char* p) {
+  Val<N> v;
+  const unsigned long long* l = reinterpret_cast<const unsigned long long*>(p);
+  unsigned long long w[N + 1];
+#pragma unroll
+  for (int q = 0; q <= N; ++q) w[q] = l[q];
+  const int kind = (int)(uint32_t)w[N], ex = (int)(uint32_t)(w[N] >> 32);
+  v.zero = (kind == kKindZero || kind == -kKindZero);
+  v.neg = kind < 0;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    v.m[2 * q] = v.zero ? 0u : (uint32_t)w[q];
+    v.m[2 * q + 1] = v.zero ? 0u : (uint32_t)(w[q] >> 32);
+  }
+  v.s = (long long)ex - 64LL * N;
+  return v;
+}
+
+// The scale and kind of an element alone: false for a zero.
+template <int N>
+MPD_FN bool load_scale(const unsigned char* p, long long* s) {
+  const unsigned long long w = reinterpret_cast<const unsigned long long*>(p)[N];
+  const int kind = (int)(uint32_t)w;
+  *s = (long long)(int)(uint32_t)(w >> 32) - 64LL * N;
+  return kind != kKindZero && kind != -kKindZero;
+}
+
+// Store v (zeros as +0); an exponent outside the MPFR range sets bit 4 (non-finite) of *status.
+template <int N>
+MPD_FN void store(unsigned char* p, const Val<N>& v, uint32_t* status) {
+  unsigned long long* l = reinterpret_cast<unsigned long long*>(p);
+  const long long ex = v.s + 64LL * N;
+  const bool out = !v.zero && (ex > kExpMax || ex < -kExpMax);
+#if defined(__CUDA_ARCH__)
+  if (out && status) atomicOr(status, 4u);
+#else
+  if (out && status) *status |= 4u;
+#endif
+  const bool z = v.zero || out;
+#pragma unroll
+  for (int q = 0; q < N; ++q)
+    l[q] = z ? 0ull : ((unsigned long long)v.m[2 * q + 1] << 32) | (unsigned long long)v.m[2 * q];
+  const uint32_t kind = z ? (uint32_t)kKindZero : (uint32_t)(v.neg ? -kKindRegular : kKindRegular);
+  l[N] = ((unsigned long long)(z ? 0u : (uint32_t)(int)ex) << 32) | kind;
+}
+
+// ---- sums and products ----
+
+// B >>= d bits over K words (d <= 32 K); bits shifted out are or-ed into the result's last bit.
+template <int K, int W>
+struct DropStage {
+  static MPD_FN void run(uint32_t* B, int ws, uint32_t& lost) {
+    if (ws & W) {
+#pragma unroll
+      for (int i = 0; i < W && i < K; ++i) lost |= B[i];
+#pragma unroll
+      for (int i = 0; i < K; ++i) B[i] = i + W < K ? B[i + W < K ? i + W : 0] : 0u;
+    }
+    DropStage<K, (2 * W <= K ? 2 * W : 0)>::run(B, ws, lost);
+  }
+};
+template <int K>
+struct DropStage<K, 0> {
+  static MPD_FN void run(uint32_t*, int, uint32_t&) {}
+};
+template <int K>
+MPD_FN void shift_right_sticky(uint32_t* B, int d) {
+  uint32_t lost = 0;
+  DropStage<K, 1>::run(B, d >> 5, lost);
+  const int r = d & 31;
+  lost |= B[0] & ((1u << r) - 1u);
+#pragma unroll
+  for (int i = 0; i < K - 1; ++i) B[i] = funnel_r(B[i], B[i + 1], r);
+  B[K - 1] >>= r;
+  B[0] |= lost ? 1u : 0u;
+}
+
+// a + sign * b, the exact sum rounded once (sign = -1: subtraction).  The smaller operand is
+// aligned with 64 guard bits below the larger one's last bit and a sticky bit at the lowest of
+// them: two operands within 64 bits of each other are summed exactly, and for the others the sum
+// loses at most one leading bit, so the guard and the sticky bit decide the rounding.
+template <int N>
+MPD_CALL Val<N> addsub(Val<N> a, Val<N> b, int sign) {
+  if (sign < 0) b.neg = !b.neg;
+  if (b.zero) return a.zero ? zero_val<N>() : a;
+  if (a.zero) return b;
+  constexpr long long gap = 64LL * N + 64;
+  const long long d = a.s - b.s;
   if (d > gap) return a;
-  if (d < -gap) return bb;
-  const long long lo = a.s < bb.s ? a.s : bb.s;
-  const int W = 2 * N + 3;
-  unsigned long long A[kWideWords] = {}, B[kWideWords] = {};
-  add_shifted(A, W, a.m, N, a.s - lo);
-  add_shifted(B, W, bb.m, N, bb.s - lo);
-  bool neg;
-  if (a.neg == bb.neg) {
-    add_shifted(A, W, B, W, 0);
-    neg = a.neg;
+  if (d < -gap) return b;
+  constexpr int K = 2 * N + 2;
+  const bool swap = d < 0;
+  uint32_t A[K], B[K];
+  A[0] = A[1] = B[0] = B[1] = 0u;
+#pragma unroll
+  for (int q = 0; q < 2 * N; ++q) {
+    A[q + 2] = swap ? b.m[q] : a.m[q];
+    B[q + 2] = swap ? a.m[q] : b.m[q];
+  }
+  long long s = (swap ? b.s : a.s) - 64;
+  bool neg = swap ? b.neg : a.neg;
+  shift_right_sticky<K>(B, (int)(swap ? -d : d));
+  if (a.neg == b.neg) {
+    if (add_words<K>(A, B, 0u)) {
+      const uint32_t low = A[0] & 1u;
+#pragma unroll
+      for (int i = 0; i < K - 1; ++i) A[i] = funnel_r(A[i], A[i + 1], 1);
+      A[K - 1] = (A[K - 1] >> 1) | (1u << 31);
+      A[0] |= low;
+      s += 1;
+    }
   } else {
-    int cmp = 0;
-    for (int w = W - 1; w >= 0 && !cmp; --w) cmp = A[w] > B[w] ? 1 : (A[w] < B[w] ? -1 : 0);
-    if (cmp == 0) return mp_zero();
-    if (cmp > 0) {
-      sub_shifted(A, W, B, W, 0);
-      neg = a.neg;
-    } else {
-      sub_shifted(B, W, A, W, 0);
-      for (int w = 0; w < W; ++w) A[w] = B[w];
-      neg = bb.neg;
+    if (sub_words<K>(A, B)) {  // equal scales, the second mantissa larger
+      neg_words<K>(A);
+      neg = !neg;
+    }
+    if (!(A[K - 1] >> 31)) {
+      if (is_zero<K>(A)) return zero_val<N>();
+      s -= normalize<K>(A);
     }
   }
-  return mp_round(A, W, neg, lo, N);
+  return round_top<N, K>(A, neg, s);
 }
 
-__device__ inline Val mp_mul(const Val& a, const Val& b, int N) {
-  if (a.zero || b.zero) {
-    Val z = mp_zero();
-    z.neg = a.neg != b.neg;
-    return z;
-  }
-  unsigned long long P[2 * kMaxN + 1] = {};
-  for (int i = 0; i < N; ++i) {
-    unsigned long long carry = 0;
-    for (int j = 0; j < N; ++j) {
-      const unsigned long long lo = a.m[i] * b.m[j], hi = __umul64hi(a.m[i], b.m[j]);
-      const unsigned long long t = P[i + j] + lo;
-      const unsigned long long c1 = t < lo;
-      const unsigned long long t2 = t + carry;
-      const unsigned long long c2 = t2 < t;
-      P[i + j] = t2;
-      carry = hi + c1 + c2;
-    }
-    P[i + N] += carry;
-  }
-  return mp_round(P, 2 * N, a.neg != b.neg, a.s + b.s, N);
+template <int N>
+MPD_FN Val<N> mul(const Val<N>& a, const Val<N>& b) {
+  if (a.zero || b.zero) return zero_val<N>();
+  uint32_t P[4 * N];
+  mul_words<N>(P, a.m, b.m);
+  const int c = 1 - (int)(P[4 * N - 1] >> 31);  // the top bit is at most one place down
+#pragma unroll
+  for (int i = 4 * N - 1; i > 0; --i) P[i] = funnel_l(P[i - 1], P[i], c);
+  P[0] <<= c;
+  return round_top<N, 4 * N>(P, a.neg != b.neg, a.s + b.s - c);
 }
 
 // sign of a - b: -1, 0, 1.
-__device__ inline int mp_cmp(const Val& a, const Val& b, int N) {
+template <int N>
+MPD_FN int cmp(const Val<N>& a, const Val<N>& b) {
   if (a.zero && b.zero) return 0;
-  const Val d = mp_addsub(a, b, -1, N);
-  return d.zero ? 0 : (d.neg ? -1 : 1);
+  if (a.zero) return b.neg ? 1 : -1;
+  if (b.zero) return a.neg ? -1 : 1;
+  if (a.neg != b.neg) return a.neg ? -1 : 1;
+  int c = a.s != b.s ? (a.s > b.s ? 1 : -1) : cmp_words<2 * N>(a.m, b.m);
+  return a.neg ? -c : c;
 }
 
-// a - sum_c x[c] y[c] (a given) or sum_c x[c] y[c] (a null), the exact value rounded once.
-// x_c at x + c * xs, y_c at y + c * ys (element strides).  *ok = false when the terms do not
-// fit the accumulator.
-__device__ inline Val mp_dot_sub(const Val* a, const unsigned char* x, long xs, const unsigned char* y, long ys,
-                                 int count, int N, bool* ok) {
-  const long esz = 8L * N + 8;
-  long long lo = LLONG_MAX, hi = LLONG_MIN;
-  for (int c = 0; c < count; ++c) {
-    const Val xv = mp_load(x + c * xs * esz, N), yv = mp_load(y + c * ys * esz, N);
+// ---- Newton estimates and the correctly rounded reciprocal, quotient and square root ----
+
+// A value as (double in [0.5, 1), binary exponent): v = f 2^e, f its leading 53 bits.
+template <int N>
+MPD_FN double frac_exp(const Val<N>& v, long long* e) {
+  const unsigned long long top = ((unsigned long long)v.m[2 * N - 1] << 32) | v.m[2 * N - 2];
+  *e = v.s + 64LL * N;
+  const double f = (double)(top >> 11) * 0x1p-53;
+  return v.neg ? -f : f;
+}
+
+// f 2^e as a value (f a finite double).
+template <int N>
+MPD_FN Val<N> from_double(double f, long long e) {
+  Val<N> v = zero_val<N>();
+  if (f == 0.0) return v;
+  int fe = 0;
+  const double m = frexp(fabs(f), &fe);  // in [0.5, 1)
+  const unsigned long long top = (unsigned long long)(m * 0x1p64);  // exact: 53 significant bits
+  v.zero = false;
+  v.neg = f < 0;
+  v.m[2 * N - 1] = (uint32_t)(top >> 32);
+  v.m[2 * N - 2] = (uint32_t)top;
+  v.s = e + fe - 64LL * N;
+  return v;
+}
+
+// 1 / x and 1 / sqrt(x) by Newton's iteration from an FP64 seed (quadratic convergence: four
+// steps carry 53 bits past 512): accurate to a few units in the last place, not correctly
+// rounded -- the Jacobi rotation parameters, whose orthogonality they bound, and the estimates
+// that the correctly rounded operations correct.
+template <int N>
+MPD_CALL Val<N> recip_approx(Val<N> x) {
+  long long e;
+  const double f = frac_exp<N>(x, &e);
+  Val<N> y = from_double<N>(1.0 / f, -e);
+  const Val<N> two = from_double<N>(0.5, 2);
+  constexpr int steps = N <= 2 ? 2 : (N <= 4 ? 3 : 4);
+#pragma unroll 1
+  for (int k = 0; k < steps; ++k) y = mul<N>(y, addsub<N>(two, mul<N>(x, y), -1));
+  return y;
+}
+template <int N>
+MPD_CALL Val<N> rsqrt_approx(Val<N> x) {  // x > 0
+  long long e;
+  const double f = frac_exp<N>(x, &e);
+  // x = f 2^e: 1/sqrt(x) = (1/sqrt(f 2^(e mod 2))) 2^(-(e - e mod 2) / 2)
+  const long long odd = e & 1;
+  Val<N> y = from_double<N>(1.0 / sqrt(f * (odd ? 2.0 : 1.0)), -((e - odd) / 2));
+  const Val<N> three = from_double<N>(0.75, 2);
+  constexpr int steps = N <= 2 ? 2 : (N <= 4 ? 3 : 4);
+#pragma unroll 1
+  for (int k = 0; k < steps; ++k) {
+    Val<N> t = addsub<N>(three, mul<N>(x, mul<N>(y, y)), -1);
+    t.s -= 1;  // / 2
+    y = mul<N>(y, t);
+  }
+  return y;
+}
+
+// Q (2N + 1 words) = floor(v 2^sh) for a positive v whose integer is at most 64N + 31 bits wide.
+template <int N>
+MPD_FN void to_words(const Val<N>& v, long long sh, uint32_t* Q) {
+  const int t = (int)(v.s + sh) & 31;  // Q = M_v 2^t: the estimates below have 0 <= t < 32
+  Q[2 * N] = funnel_l(v.m[2 * N - 1], 0u, t);
+#pragma unroll
+  for (int i = 2 * N - 1; i > 0; --i) Q[i] = funnel_l(v.m[i - 1], v.m[i], t);
+  Q[0] = v.m[0] << t;
+}
+
+// R -= Q M modulo 2^(32 (2N + 2)), Q 2N + 1 words with a small top word, M 2N words: remainders of
+// the estimates below stay within a few M, so their low 2N + 2 words are the whole remainder.
+template <int N>
+MPD_FN void sub_product(uint32_t* R, const uint32_t* Q, const uint32_t* M) {
+  uint32_t P[4 * N];
+  mul_words<N>(P, Q, M);
+  uint32_t T[2 * N + 2];
+#pragma unroll
+  for (int i = 0; i < 2 * N + 2; ++i) T[i] = i < 4 * N ? P[i < 4 * N ? i : 0] : 0u;
+  const uint64_t t0 = (uint64_t)Q[2 * N] * M[0];
+  const uint32_t up[2] = {(uint32_t)t0, (uint32_t)(t0 >> 32) + Q[2 * N] * M[1]};
+  add_words<2>(T + 2 * N, up, 0u);
+  sub_words<2 * N + 2>(R, T);
+}
+
+// Step Q until R = X - Q M lies in [0, M) (R 2N + 2 words, two's complement).
+template <int N>
+MPD_FN void fix_quotient(uint32_t* Q, uint32_t* R, const uint32_t* M) {
+  uint32_t D[2 * N + 2];
+#pragma unroll
+  for (int i = 0; i < 2 * N + 2; ++i) D[i] = i < 2 * N ? M[i < 2 * N ? i : 0] : 0u;
+#pragma unroll 1
+  for (int it = 0; it < 4096 && (R[2 * N + 1] >> 31); ++it) {
+    uint32_t one[2 * N + 1] = {1u};
+    sub_words<2 * N + 1>(Q, one);
+    add_words<2 * N + 2>(R, D, 0u);
+  }
+#pragma unroll 1
+  for (int it = 0; it < 4096 && cmp_words<2 * N + 2>(R, D) >= 0; ++it) {
+    add_word<2 * N + 1>(Q, 1u);
+    sub_words<2 * N + 2>(R, D);
+  }
+}
+// (Q + sticky) 2^scale rounded, sticky below Q's last bit.
+template <int N>
+MPD_FN Val<N> round_quotient(const uint32_t* Q, bool sticky, bool neg, long long scale) {
+  constexpr int K = 2 * N + 2;
+  uint32_t S[K];
+  S[0] = sticky ? 1u : 0u;
+#pragma unroll
+  for (int i = 0; i < 2 * N + 1; ++i) S[i + 1] = Q[i];
+  const int sh = normalize<K>(S);
+  return round_top<N, K>(S, neg, scale - 32 - sh);
+}
+
+// 1 / d: Q = floor(2^K / M_d), K = 128N + 2, remainder sticky.
+template <int N>
+MPD_CALL Val<N> recip(Val<N> d) {
+  constexpr long long K = 128LL * N + 2;
+  Val<N> m = d;  // M_d 2^-64N in [1/2, 1)
+  m.neg = false;
+  m.s = -64LL * N;
+  const Val<N> y = recip_approx<N>(m);  // ~ 2^64N / M_d
+  uint32_t Q[2 * N + 1], R[2 * N + 2];
+  to_words<N>(y, K - 64LL * N, Q);  // ~ 2^K / M_d
+#pragma unroll
+  for (int i = 0; i < 2 * N + 2; ++i) R[i] = 0u;  // 2^K vanishes modulo 2^(64N + 64)
+  sub_product<N>(R, Q, d.m);
+  fix_quotient<N>(Q, R, d.m);
+  return round_quotient<N>(Q, !is_zero<2 * N + 2>(R), d.neg, -K - d.s);
+}
+
+// a / b: Q = floor(M_a 2^K / M_b), K = 64N + 2, remainder sticky.  b must be nonzero.
+template <int N>
+MPD_CALL Val<N> divide(Val<N> a, Val<N> b) {
+  if (a.zero) return zero_val<N>();
+  constexpr long long K = 64LL * N + 2;
+  Val<N> an = a, bn = b;
+  an.neg = bn.neg = false;
+  an.s = bn.s = -64LL * N;
+  const Val<N> q = mul<N>(an, recip_approx<N>(bn));  // ~ M_a / M_b
+  uint32_t Q[2 * N + 1], R[2 * N + 2];
+  to_words<N>(q, K, Q);
+#pragma unroll
+  for (int i = 0; i < 2 * N; ++i) R[i] = 0u;  // M_a 2^K modulo 2^(64N + 64)
+  R[2 * N] = a.m[0] << 2;
+  R[2 * N + 1] = funnel_l(a.m[0], a.m[1], 2);
+  sub_product<N>(R, Q, b.m);
+  fix_quotient<N>(Q, R, b.m);
+  return round_quotient<N>(Q, !is_zero<2 * N + 2>(R), a.neg != b.neg, a.s - b.s - K);
+}
+
+// sqrt(a), a >= 0: Y = floor(sqrt(M 2^e)), the radicand 2 (64N + 2) bits wide (e even with s - e),
+// remainder sticky.
+template <int N>
+MPD_CALL Val<N> root(Val<N> a) {
+  if (a.zero) return a;
+  long long e = 64LL * N + 4;
+  if ((a.s - e) & 1) e += 1;
+  Val<N> x = a;  // M 2^e
+  x.neg = false;
+  x.s = e;
+  const Val<N> y = mul<N>(x, rsqrt_approx<N>(x));  // ~ sqrt(M 2^e)
+  uint32_t Y[2 * N + 1], R[2 * N + 2], D[2 * N + 2];
+  to_words<N>(y, 0, Y);
+  {  // R = M 2^e - Y^2 modulo 2^(64N + 64)
+    const int r = (int)(e - 64LL * N);
+#pragma unroll
+    for (int i = 0; i < 2 * N; ++i) R[i] = 0u;
+    R[2 * N] = a.m[0] << r;
+    R[2 * N + 1] = funnel_l(a.m[0], a.m[1], r);
+    sub_product<N>(R, Y, Y);  // Y (Y mod 2^64N), the rest of Y^2 follows
+    const uint64_t t0 = (uint64_t)Y[2 * N] * Y[0];
+    const uint32_t up[2] = {(uint32_t)t0, (uint32_t)(t0 >> 32) + Y[2 * N] * Y[1]};
+    sub_words<2>(R + 2 * N, up);
+  }
+  // 0 <= R <= 2Y: while negative Y -= 1, R += 2Y + 1 (new Y); while R > 2Y, R -= 2Y + 1, Y += 1
+  auto twice = [&]() {  // D = 2Y + 1
+    D[0] = (Y[0] << 1) | 1u;
+#pragma unroll
+    for (int i = 1; i < 2 * N + 1; ++i) D[i] = funnel_l(Y[i - 1], Y[i], 1);
+    D[2 * N + 1] = Y[2 * N] >> 31;
+  };
+#pragma unroll 1
+  for (int it = 0; it < 4096 && (R[2 * N + 1] >> 31); ++it) {
+    uint32_t one[2 * N + 1] = {1u};
+    sub_words<2 * N + 1>(Y, one);
+    twice();
+    add_words<2 * N + 2>(R, D, 0u);
+  }
+#pragma unroll 1
+  for (int it = 0; it < 4096; ++it) {
+    twice();
+    if (cmp_words<2 * N + 2>(R, D) < 0) break;
+    sub_words<2 * N + 2>(R, D);
+    add_word<2 * N + 1>(Y, 1u);
+  }
+  return round_quotient<N>(Y, !is_zero<2 * N + 2>(R), false, (a.s - e) / 2);
+}
+
+// ---- exact dots ----
+
+// Register accumulator: terms of 128N bits whose scales span at most kSpanBits, 72 bits of room
+// for the count and the sign.
+template <int N>
+struct Acc {
+  static constexpr int W = 4 * N + 12;
+  uint32_t w[W];
+};
+constexpr int kSpanBits = 12 * 32 - 72;
+
+template <int N, int Q>
+struct PlaceStage {  // T <<= q words, q's bits from Q up
+  static MPD_FN void run(uint32_t* T, int q) {
+    if (q & Q) {
+#pragma unroll
+      for (int i = Acc<N>::W - 1; i >= 0; --i) T[i] = i >= Q ? T[i >= Q ? i - Q : 0] : 0u;
+    }
+    PlaceStage<N, (Q < 8 ? 2 * Q : 0)>::run(T, q);
+  }
+};
+template <int N>
+struct PlaceStage<N, 0> {
+  static MPD_FN void run(uint32_t*, int) {}
+};
+
+// acc += (-1)^neg P 2^sh, P 4N words, 0 <= sh < 512, the shifted P within the accumulator.
+template <int N>
+MPD_FN void acc_add(Acc<N>& acc, const uint32_t* P, int sh, bool neg) {
+  constexpr int W = Acc<N>::W;
+  uint32_t T[W];
+  const int r = sh & 31;
+  T[0] = P[0] << r;
+#pragma unroll
+  for (int i = 1; i < 4 * N; ++i) T[i] = funnel_l(P[i - 1], P[i], r);
+  T[4 * N] = funnel_l(P[4 * N - 1], 0u, r);
+#pragma unroll
+  for (int i = 4 * N + 1; i < W; ++i) T[i] = 0u;
+  PlaceStage<N, 1>::run(T, sh >> 5);
+  const uint32_t mask = neg ? 0xffffffffu : 0u;
+#pragma unroll
+  for (int i = 0; i < W; ++i) T[i] ^= mask;
+  add_words<W>(acc.w, T, mask & 1u);
+}
+
+// acc += v's mantissa 2^sh with v's sign, 0 <= sh <= kSpanBits + 64N: placed like a product's upper
+// half when it sits that high.
+template <int N>
+MPD_FN void acc_add_value(Acc<N>& acc, const Val<N>& v, long long sh) {
+  const bool high = sh >= 64LL * N;
+  uint32_t P[4 * N];
+#pragma unroll
+  for (int i = 0; i < 2 * N; ++i) {
+    P[i] = high ? 0u : v.m[i];
+    P[2 * N + i] = high ? v.m[i] : 0u;
+  }
+  acc_add<N>(acc, P, (int)(high ? sh - 64LL * N : sh), v.neg);
+}
+
+// acc 2^lo rounded once (acc two's complement, destroyed).
+template <int N>
+MPD_FN Val<N> acc_round(Acc<N>& acc, long long lo) {
+  constexpr int W = Acc<N>::W;
+  const bool neg = acc.w[W - 1] >> 31;
+  if (neg) neg_words<W>(acc.w);
+  if (is_zero<W>(acc.w)) return zero_val<N>();
+  const int sh = normalize<W>(acc.w);
+  return round_top<N, W>(acc.w, neg, lo - sh);
+}
+
+#if defined(__CUDACC__)
+
+// The terms of dot() that span more than kSpanBits: the accumulator in local memory.
+template <int N, int G>
+__device__ __noinline__ Val<N> dot_wide(const Val<N>* a, const unsigned char* x, long xs, const unsigned char* y,
+                                        long ys, int count, int sub, unsigned mask, long long lo, int W) {
+  constexpr long esz = 8L * N + 8;
+  uint32_t acc[2 * kAccWords];
+  for (int w = 0; w < 2 * W; ++w) acc[w] = 0u;
+  auto add = [&](const uint32_t* P, int words, long long sh, bool neg) {  // acc += (-1)^neg P 2^sh
+    const int q = (int)(sh >> 5), r = (int)(sh & 31);
+    const uint32_t m = neg ? 0xffffffffu : 0u;
+    uint32_t c = neg ? 1u : 0u, prev = 0u;
+    for (int i = 0; q + i < 2 * W; ++i) {
+      const uint32_t cur = i < words ? P[i] : 0u;
+      const uint64_t t = (uint64_t)acc[q + i] + (funnel_l(prev, cur, r) ^ m) + c;
+      acc[q + i] = (uint32_t)t;
+      c = (uint32_t)(t >> 32);
+      prev = cur;
+    }
+  };
+  if (sub == 0 && a && !a->zero) add(a->m, 2 * N, a->s - lo, a->neg);
+#pragma unroll 1
+  for (int c = sub; c < count; c += G) {
+    const Val<N> xv = load<N>(x + c * xs * esz), yv = load<N>(y + c * ys * esz);
     if (xv.zero || yv.zero) continue;
-    const long long s = xv.s + yv.s;
+    uint32_t P[4 * N];
+    mul_words<N>(P, xv.m, yv.m);
+    add(P, 4 * N, xv.s + yv.s - lo, (xv.neg != yv.neg) != (a != nullptr));
+  }
+  for (int o = G / 2; o > 0; o >>= 1) {
+    uint32_t c = 0;
+    for (int w = 0; w < 2 * W; ++w) {
+      const uint64_t t = (uint64_t)acc[w] + __shfl_xor_sync(mask, acc[w], o) + c;
+      acc[w] = (uint32_t)t;
+      c = (uint32_t)(t >> 32);
+    }
+  }
+  const bool neg = acc[2 * W - 1] >> 31;
+  if (neg) {
+    uint32_t c = 1;
+    for (int w = 0; w < 2 * W; ++w) {
+      acc[w] = ~acc[w] + c;
+      c = (c && acc[w] == 0) ? 1u : 0u;
+    }
+  }
+  int top = 2 * W - 1;
+  while (top >= 0 && acc[top] == 0) --top;
+  if (top < 0) return zero_val<N>();
+  uint32_t S[2 * N + 2];  // the leading 2N + 1 words and a sticky word
+  uint32_t low = 0;
+#pragma unroll
+  for (int i = 0; i < 2 * N + 1; ++i) {
+    const int w = top - (2 * N) + i;
+    S[i + 1] = w >= 0 ? acc[w] : 0u;
+  }
+  for (int w = top - 2 * N - 1; w >= 0; --w) low |= acc[w];
+  S[0] = low ? 1u : 0u;
+  const int sh = normalize<2 * N + 2>(S);
+  return round_top<N, 2 * N + 2>(S, neg, lo + 32LL * (top - 2 * N - 1) - sh);
+}
+
+// a - sum_c x[c] y[c] (a given) or sum_c x[c] y[c] (a null), the exact value rounded once, by the
+// aligned group of G lanes (a power of two; every lane of the group calls with the same
+// arguments and gets the result): each lane accumulates the terms c = lane, lane + G, ... exactly in one frame
+// (the group's lowest scale), and the partial accumulators are summed exactly by a butterfly.
+// x_c at x + c * xs, y_c at y + c * ys (element strides).  *ok = false when the terms do not fit
+// kAccWords words.
+template <int N, int G>
+__device__ __noinline__ Val<N> dot(const Val<N>* a, const unsigned char* x, long xs, const unsigned char* y, long ys,
+                                   int count, bool* ok) {
+  constexpr long esz = 8L * N + 8;
+  const int lane = threadIdx.x & 31, sub = lane & (G - 1);
+  const unsigned mask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (lane & ~(G - 1));
+  long long lo = LLONG_MAX, hi = LLONG_MIN;
+#pragma unroll 1
+  for (int c = sub; c < count; c += G) {
+    long long sx, sy;
+    const bool lx = load_scale<N>(x + c * xs * esz, &sx), ly = load_scale<N>(y + c * ys * esz, &sy);
+    if (!lx || !ly) continue;
+    const long long s = sx + sy;
     lo = s < lo ? s : lo;
     hi = s > hi ? s : hi;
+  }
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) {
+    const long long l2 = __shfl_xor_sync(mask, lo, o), h2 = __shfl_xor_sync(mask, hi, o);
+    lo = l2 < lo ? l2 : lo;
+    hi = h2 > hi ? h2 : hi;
   }
   if (a && !a->zero) {  // the addend's top bit sits where a product term's would at scale s - 64N
     lo = a->s < lo ? a->s : lo;
     hi = (a->s - 64LL * N) > hi ? (a->s - 64LL * N) : hi;
   }
-  if (lo == LLONG_MAX) return mp_zero();
-  const long long span = hi - lo + 128LL * N + 72;  // largest term's width + log2(count) + sign
-  const int W = (int)((span + 63) / 64) + 1;
-  if (W > kAccWords) {
-    *ok = false;
-    return mp_zero();
+  if (lo == LLONG_MAX) return zero_val<N>();
+  if (hi - lo > kSpanBits) {
+    const long long span = hi - lo + 128LL * N + 72;  // largest term's width + log2(count) + sign
+    const long long W = (span + 63) / 64 + 1;
+    if (W > kAccWords) {
+      *ok = false;
+      return zero_val<N>();
+    }
+    return dot_wide<N, G>(a, x, xs, y, ys, count, sub, mask, lo, (int)W);
   }
-  unsigned long long acc[kAccWords];
-  for (int w = 0; w < W; ++w) acc[w] = 0ull;
-  if (a && !a->zero) {
-    if (a->neg)
-      sub_shifted(acc, W, a->m, N, a->s - lo);
-    else
-      add_shifted(acc, W, a->m, N, a->s - lo);
-  }
-  for (int c = 0; c < count; ++c) {
-    const Val xv = mp_load(x + c * xs * esz, N), yv = mp_load(y + c * ys * esz, N);
+  Acc<N> acc;
+#pragma unroll
+  for (int w = 0; w < Acc<N>::W; ++w) acc.w[w] = 0u;
+  uint32_t P[4 * N];
+  if (sub == 0 && a && !a->zero) acc_add_value<N>(acc, *a, a->s - lo);
+#pragma unroll 1
+  for (int c = sub; c < count; c += G) {
+    const Val<N> xv = load<N>(x + c * xs * esz), yv = load<N>(y + c * ys * esz);
     if (xv.zero || yv.zero) continue;
-    unsigned long long P[2 * kMaxN] = {};
-    for (int i = 0; i < N; ++i) {
-      unsigned long long carry = 0;
-      for (int j = 0; j < N; ++j) {
-        const unsigned long long plo = xv.m[i] * yv.m[j], phi = __umul64hi(xv.m[i], yv.m[j]);
-        const unsigned long long t = P[i + j] + plo;
-        const unsigned long long c1 = t < plo;
-        const unsigned long long t2 = t + carry;
-        const unsigned long long c2 = t2 < t;
-        P[i + j] = t2;
-        carry = phi + c1 + c2;
-      }
-      P[i + N] += carry;
-    }
-    const bool term_neg = (xv.neg != yv.neg) != (a != nullptr);  // a - sum: products subtract
-    if (term_neg)
-      sub_shifted(acc, W, P, 2 * N, xv.s + yv.s - lo);
-    else
-      add_shifted(acc, W, P, 2 * N, xv.s + yv.s - lo);
-  }
-  const bool neg = (acc[W - 1] >> 63) != 0;
-  if (neg) {  // magnitude of a two's-complement value
-    unsigned long long carry = 1;
-    for (int w = 0; w < W; ++w) {
-      acc[w] = ~acc[w] + carry;
-      carry = (carry && acc[w] == 0) ? 1ull : 0ull;
-    }
-  }
-  return mp_round(acc, W, neg, lo, N);
-}
-
-// A value as (double in [0.5, 1), binary exponent): v = f 2^e.
-__device__ __forceinline__ double frac_exp(const Val& v, int N, long long* e) {
-  const double top = (double)(v.m[N - 1] >> 11) * 0x1p-53;  // the top 53 bits, in [0.5, 1)
-  *e = v.s + 64LL * N;
-  return v.neg ? -top : top;
-}
-
-// f 2^e as a Val (f a finite nonzero double).
-__device__ inline Val from_double(double f, long long e, int N) {
-  Val v = mp_zero();
-  if (f == 0.0) return v;
-  int fe = 0;
-  const double m = frexp(fabs(f), &fe);  // m in [0.5, 1)
-  v.zero = false;
-  v.neg = f < 0;
-  v.m[N - 1] = (unsigned long long)(m * 0x1p64);  // exact: 53 significant bits
-  v.s = e + fe - 64LL * N;
-  return v;
-}
-
-// mp_dot_sub computed by a whole warp (every lane calls it with the same arguments; every lane
-// gets the result): the lanes take the terms c = lane, lane + 32, ..., each accumulates its
-// terms exactly in the same fixed-point frame (the warp-wide lowest scale), the partial
-// accumulators are added exactly by a shuffle tree, and lane 0 rounds once -- the bits of
-// mp_dot_sub, about thirty times faster for long dots.
-__device__ inline Val mp_dot_sub_warp(const Val* a, const unsigned char* x, long xs, const unsigned char* y, long ys,
-                                      int count, int N, bool* ok) {
-  const long esz = 8L * N + 8;
-  const int lane = threadIdx.x & 31;
-  long long lo = LLONG_MAX, hi = LLONG_MIN;
-  for (int c = lane; c < count; c += 32) {
-    const Val xv = mp_load(x + c * xs * esz, N), yv = mp_load(y + c * ys * esz, N);
-    if (xv.zero || yv.zero) continue;
-    const long long s = xv.s + yv.s;
-    lo = s < lo ? s : lo;
-    hi = s > hi ? s : hi;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const long long l2 = __shfl_xor_sync(0xffffffffu, lo, o), h2 = __shfl_xor_sync(0xffffffffu, hi, o);
-    lo = l2 < lo ? l2 : lo;
-    hi = h2 > hi ? h2 : hi;
-  }
-  if (a && !a->zero) {
-    lo = a->s < lo ? a->s : lo;
-    hi = (a->s - 64LL * N) > hi ? (a->s - 64LL * N) : hi;
-  }
-  if (lo == LLONG_MAX) return mp_zero();
-  const long long span = hi - lo + 128LL * N + 72;
-  const int W = (int)((span + 63) / 64) + 1;
-  if (W > kAccWords) {
-    *ok = false;
-    return mp_zero();
-  }
-  unsigned long long acc[kAccWords];
-  for (int w = 0; w < W; ++w) acc[w] = 0ull;
-  if (lane == 0 && a && !a->zero) {
-    if (a->neg)
-      sub_shifted(acc, W, a->m, N, a->s - lo);
-    else
-      add_shifted(acc, W, a->m, N, a->s - lo);
-  }
-  for (int c = lane; c < count; c += 32) {
-    const Val xv = mp_load(x + c * xs * esz, N), yv = mp_load(y + c * ys * esz, N);
-    if (xv.zero || yv.zero) continue;
-    unsigned long long P[2 * kMaxN] = {};
-    for (int i = 0; i < N; ++i) {
-      unsigned long long carry = 0;
-      for (int j = 0; j < N; ++j) {
-        const unsigned long long plo = xv.m[i] * yv.m[j], phi = __umul64hi(xv.m[i], yv.m[j]);
-        const unsigned long long t = P[i + j] + plo;
-        const unsigned long long c1 = t < plo;
-        const unsigned long long t2 = t + carry;
-        const unsigned long long c2 = t2 < t;
-        P[i + j] = t2;
-        carry = phi + c1 + c2;
-      }
-      P[i + N] += carry;
-    }
-    const bool term_neg = (xv.neg != yv.neg) != (a != nullptr);
-    if (term_neg)
-      sub_shifted(acc, W, P, 2 * N, xv.s + yv.s - lo);
-    else
-      add_shifted(acc, W, P, 2 * N, xv.s + yv.s - lo);
-  }
-  for (int o = 16; o > 0; o >>= 1) {  // exact two's-complement sum of the partial accumulators
-    unsigned long long carry = 0;
-    for (int w = 0; w < W; ++w) {
-      const unsigned long long b = __shfl_down_sync(0xffffffffu, acc[w], o);
-      const unsigned long long t = acc[w] + b;
-      const unsigned long long c1 = t < b;
-      const unsigned long long t2 = t + carry;
-      const unsigned long long c2 = t2 < t;
-      acc[w] = t2;
-      carry = c1 + c2;
-    }
-  }
-  Val r = mp_zero();
-  if (lane == 0) {
-    const bool neg = (acc[W - 1] >> 63) != 0;
-    if (neg) {
-      unsigned long long carry = 1;
-      for (int w = 0; w < W; ++w) {
-        acc[w] = ~acc[w] + carry;
-        carry = (carry && acc[w] == 0) ? 1ull : 0ull;
-      }
-    }
-    r = mp_round(acc, W, neg, lo, N);
+    mul_words<N>(P, xv.m, yv.m);
+    acc_add<N>(acc, P, (int)(xv.s + yv.s - lo), (xv.neg != yv.neg) != (a != nullptr));
   }
 #pragma unroll
-  for (int q = 0; q < kMaxN; ++q) r.m[q] = __shfl_sync(0xffffffffu, r.m[q], 0);
-  r.s = __shfl_sync(0xffffffffu, r.s, 0);
-  r.neg = __shfl_sync(0xffffffffu, (int)r.neg, 0) != 0;
-  r.zero = __shfl_sync(0xffffffffu, (int)r.zero, 0) != 0;
-  return r;
+  for (int o = G / 2; o > 0; o >>= 1) {
+    uint32_t t[Acc<N>::W];
+#pragma unroll
+    for (int w = 0; w < Acc<N>::W; ++w) t[w] = __shfl_xor_sync(mask, acc.w[w], o);
+    add_words<Acc<N>::W>(acc.w, t, 0u);
+  }
+  return acc_round<N>(acc, lo);
 }
 
-// 1 / x and 1 / sqrt(x) by Newton's iteration from an FP64 seed (quadratic convergence: four
-// steps carry 53 bits past 512): accurate to a few units in the last place, not correctly
-// rounded -- used only for the Jacobi rotation parameters, whose orthogonality they bound.
-__device__ inline Val mp_recip_approx(const Val& x, int N) {
-  long long e;
-  const double f = frac_exp(x, N, &e);
-  Val y = from_double(1.0 / f, -e, N);
-  const Val two = from_double(0.5, 2, N);
-  const int steps = N <= 2 ? 2 : (N <= 4 ? 3 : 4);
-  for (int k = 0; k < steps; ++k) y = mp_mul(y, mp_addsub(two, mp_mul(x, y, N), -1, N), N);
-  return y;
-}
-__device__ inline Val mp_rsqrt_approx(const Val& x, int N) {  // x > 0
-  long long e;
-  const double f = frac_exp(x, N, &e);
-  // x = f 2^e: 1/sqrt(x) = (1/sqrt(f 2^(e mod 2))) 2^(-(e - e mod 2) / 2)
-  const long long odd = e & 1;
-  Val y = from_double(1.0 / sqrt(f * (odd ? 2.0 : 1.0)), -((e - odd) / 2), N);
-  const Val three = from_double(0.75, 2, N);
-  const int steps = N <= 2 ? 2 : (N <= 4 ? 3 : 4);
-  for (int k = 0; k < steps; ++k) {
-    Val t = mp_addsub(three, mp_mul(x, mp_mul(y, y, N), N), -1, N);
-    t.s -= 1;  // / 2
-    y = mp_mul(y, t, N);
+// f(std::integral_constant<int, N>) for a run-time limb count 1..kMaxN (a kernel per limb count).
+template <class F>
+inline void by_limbs(int N, F&& f) {
+  switch (N) {
+    case 1: f(std::integral_constant<int, 1>()); break;
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 3: f(std::integral_constant<int, 3>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    case 5: f(std::integral_constant<int, 5>()); break;
+    case 6: f(std::integral_constant<int, 6>()); break;
+    case 7: f(std::integral_constant<int, 7>()); break;
+    case 8: f(std::integral_constant<int, 8>()); break;
+    default: break;
   }
-  return y;
 }
 
-
-// ---- correctly rounded reciprocal, quotient and square root ----
-// Each forms the exact integer quotient (or root) and remainder that a binary long division (or
-// digit-by-digit root) would give, from a Newton estimate in MpFloat arithmetic corrected exactly:
-// the remainder of the estimate is computed in multiword integers and the estimate stepped by
-// one until 0 <= remainder < divisor (a few steps: the estimate is within a few units); the
-// remainder then becomes the sticky bit of one rounding to 64N bits, ties to even.
-constexpr int kQW = kMaxN + 2;      // quotient / root words (N + 1 used)
-constexpr int kRW = 2 * kMaxN + 4;  // remainder words, two's complement
-
-// P = A (na words) * B (nb words), na + nb words.
-__device__ inline void mul_words(const unsigned long long* A, int na, const unsigned long long* B, int nb,
-                                 unsigned long long* P) {
-  for (int i = 0; i < na + nb; ++i) P[i] = 0ull;
-  for (int i = 0; i < na; ++i) {
-    unsigned long long carry = 0;
-    for (int j = 0; j < nb; ++j) {
-      const unsigned long long lo = A[i] * B[j], hi = __umul64hi(A[i], B[j]);
-      const unsigned long long t = P[i + j] + lo;
-      const unsigned long long c1 = t < lo;
-      const unsigned long long t2 = t + carry;
-      const unsigned long long c2 = t2 < t;
-      P[i + j] = t2;
-      carry = hi + c1 + c2;
-    }
-    P[i + nb] = carry;
-  }
-}
-// R += M (M n words, zero-extended; R W words, two's complement); R -= M.
-__device__ inline void addw(unsigned long long* R, int W, const unsigned long long* M, int n) {
-  unsigned long long carry = 0;
-  for (int w = 0; w < W; ++w) {
-    const unsigned long long m = w < n ? M[w] : 0ull;
-    const unsigned long long t = R[w] + m;
-    const unsigned long long c1 = t < m;
-    const unsigned long long t2 = t + carry;
-    carry = c1 + (t2 < t);
-    R[w] = t2;
-  }
-}
-__device__ inline void subw(unsigned long long* R, int W, const unsigned long long* M, int n) {
-  unsigned long long borrow = 0;
-  for (int w = 0; w < W; ++w) {
-    const unsigned long long m = w < n ? M[w] : 0ull;
-    const unsigned long long t = R[w] - m;
-    const unsigned long long b1 = R[w] < m;
-    const unsigned long long t2 = t - borrow;
-    borrow = b1 + (t < borrow);
-    R[w] = t2;
-  }
-}
-// Non-negative R (W words) against M (n words): -1, 0, 1.
-__device__ inline int cmpw(const unsigned long long* R, int W, const unsigned long long* M, int n) {
-  for (int w = W - 1; w >= 0; --w) {
-    const unsigned long long m = w < n ? M[w] : 0ull;
-    if (R[w] != m) return R[w] > m ? 1 : -1;
-  }
-  return 0;
-}
-__device__ inline void incw(unsigned long long* Q, int W) {
-  for (int w = 0; w < W; ++w)
-    if (++Q[w] != 0ull) break;
-}
-__device__ inline void decw(unsigned long long* Q, int W) {
-  for (int w = 0; w < W; ++w)
-    if (Q[w]-- != 0ull) break;
-}
-// floor(mantissa(v) 2^(s_v + sh)) into Q (QW words); v > 0.
-__device__ inline void to_int_words(const Val& v, int N, long long sh, unsigned long long* Q, int QW) {
-  for (int w = 0; w < QW; ++w) Q[w] = 0ull;
-  const long long t = v.s + sh;  // Q = M_v 2^t
-  if (t >= 0) {
-    const int q = (int)(t >> 6), r = (int)(t & 63);
-    for (int i = 0; i <= N; ++i) {
-      const unsigned long long lo = i < N ? v.m[i] : 0ull, prev = i > 0 ? v.m[i - 1] : 0ull;
-      if (q + i < QW) Q[q + i] = r ? ((lo << r) | (prev >> (64 - r))) : lo;
-    }
-  } else {
-    const long long u = -t;
-    const int q = (int)(u >> 6), r = (int)(u & 63);
-    for (int w = 0; w < QW; ++w) {
-      const int i = w + q;
-      const unsigned long long lo = i < N ? v.m[i] : 0ull, hi = (i + 1) < N ? v.m[i + 1] : 0ull;
-      Q[w] = r ? ((lo >> r) | (hi << (64 - r))) : lo;
-    }
-  }
-}
-// Step Q until R = X - Q D lies in [0, D) (D n words; R kRW words, two's complement).
-__device__ inline void fix_quotient(unsigned long long* Q, int QW, unsigned long long* R, const unsigned long long* D,
-                                    int n) {
-  for (int it = 0; it < 4096 && (R[kRW - 1] >> 63); ++it) {
-    decw(Q, QW);
-    addw(R, kRW, D, n);
-  }
-  for (int it = 0; it < 4096 && cmpw(R, kRW, D, n) >= 0; ++it) {
-    incw(Q, QW);
-    subw(R, kRW, D, n);
-  }
-}
-__device__ inline Val round_with_sticky(const unsigned long long* Q, int QW, const unsigned long long* R, bool neg,
-                                        long long scale, int N) {
-  bool sticky = false;
-  for (int w = 0; w < kRW; ++w) sticky = sticky || R[w];
-  unsigned long long S[kQW + 1];
-  unsigned long long carry = sticky ? 1ull : 0ull;
-  for (int w = 0; w <= QW; ++w) {  // S = 2 Q + sticky
-    const unsigned long long q = w < QW ? Q[w] : 0ull;
-    S[w] = (q << 1) | carry;
-    carry = q >> 63;
-  }
-  return mp_round(S, QW + 1, neg, scale, N);
-}
-
-// 1 / d: Q = floor(2^K / M_d), K = 128N + 2, remainder sticky.
-__device__ inline Val mp_recip(const Val& d, int N) {
-  const int K = 128 * N + 2, QW = N + 1;
-  Val m = d;  // M_d 2^-64N in [1/2, 1)
-  m.neg = false;
-  m.s = -64LL * N;
-  const Val y = mp_recip_approx(m, N);  // ~ 2^64N / M_d
-  unsigned long long Q[kQW], R[kRW], P[kRW];
-  to_int_words(y, N, K - 64LL * N, Q, QW);  // ~ 2^K / M_d
-  mul_words(Q, QW, d.m, N, P);               // QW + N words
-  for (int w = 0; w < kRW; ++w) R[w] = 0ull;
-  R[K >> 6] = 1ull << (K & 63);
-  subw(R, kRW, P, QW + N);
-  fix_quotient(Q, QW, R, d.m, N);
-  return round_with_sticky(Q, QW, R, d.neg, -(long long)K - d.s - 1, N);
-}
-
-// a / b: Q = floor(M_a 2^K / M_b), K = 64N + 2, remainder sticky.  b must be nonzero.
-__device__ inline Val mp_div(const Val& a, const Val& b, int N) {
-  if (a.zero) {
-    Val z = mp_zero();
-    z.neg = a.neg != b.neg;
-    return z;
-  }
-  const int K = 64 * N + 2, QW = N + 1;
-  Val an = a, bn = b;
-  an.neg = bn.neg = false;
-  an.s = bn.s = -64LL * N;
-  const Val q = mp_mul(an, mp_recip_approx(bn, N), N);  // ~ M_a / M_b
-  unsigned long long Q[kQW], R[kRW], P[kRW];
-  to_int_words(q, N, K, Q, QW);
-  mul_words(Q, QW, b.m, N, P);
-  for (int w = 0; w < kRW; ++w) R[w] = 0ull;
-  for (int w = 0; w < N; ++w) {  // M_a 2^K: K = 64 N + 2
-    R[w + N] |= a.m[w] << 2;
-    R[w + N + 1] |= a.m[w] >> 62;
-  }
-  subw(R, kRW, P, QW + N);
-  fix_quotient(Q, QW, R, b.m, N);
-  return round_with_sticky(Q, QW, R, a.neg != b.neg, a.s - b.s - K - 1, N);
-}
-
-// sqrt(a), a >= 0: Y = floor(sqrt(M 2^e)), the radicand 2 (64N + 2) bits wide (e even with s - e),
-// remainder sticky.
-__device__ inline Val mp_sqrt(const Val& a, int N) {
-  if (a.zero) return a;
-  const int RB = 64 * N + 2, QW = N + 1;
-  long long e = 2LL * RB - 64LL * N;
-  if ((a.s - e) & 1) e += 1;
-  Val x = a;  // M 2^e
-  x.neg = false;
-  x.s = e;
-  const Val y = mp_mul(x, mp_rsqrt_approx(x, N), N);  // ~ sqrt(M 2^e)
-  unsigned long long Y[kQW], R[kRW], P[kRW], T[kQW + 1];
-  to_int_words(y, N, 0, Y, QW);
-  mul_words(Y, QW, Y, QW, P);  // Y^2, 2 QW words
-  for (int w = 0; w < kRW; ++w) R[w] = 0ull;
-  {
-    const int q = (int)(e >> 6), r = (int)(e & 63);  // X = M 2^e
-    for (int i = 0; i <= N; ++i) {
-      const unsigned long long lo = i < N ? a.m[i] : 0ull, prev = i > 0 ? a.m[i - 1] : 0ull;
-      R[q + i] |= r ? ((lo << r) | (prev >> (64 - r))) : lo;
-    }
-  }
-  subw(R, kRW, P, 2 * QW);
-  // 0 <= R = X - Y^2 <= 2Y: while negative Y -= 1, R += 2Y + 1 (new Y); while R > 2Y, R -= 2Y + 1, Y += 1
-  for (int it = 0; it < 4096 && (R[kRW - 1] >> 63); ++it) {
-    decw(Y, QW);
-    unsigned long long c = 1;
-    for (int w = 0; w <= QW; ++w) {  // T = 2Y + 1
-      const unsigned long long v = w < QW ? Y[w] : 0ull, pv = w > 0 ? Y[w - 1] : 0ull;
-      T[w] = (v << 1) | (pv >> 63) | c;
-      c = 0;
-    }
-    addw(R, kRW, T, QW + 1);
-  }
-  for (int it = 0; it < 4096; ++it) {
-    unsigned long long c = 1;
-    for (int w = 0; w <= QW; ++w) {  // T = 2Y + 1
-      const unsigned long long v = w < QW ? Y[w] : 0ull, pv = w > 0 ? Y[w - 1] : 0ull;
-      T[w] = (v << 1) | (pv >> 63) | c;
-      c = 0;
-    }
-    if (cmpw(R, kRW, T, QW + 1) < 0) break;
-    subw(R, kRW, T, QW + 1);
-    incw(Y, QW);
-  }
-  return round_with_sticky(Y, QW, R, false, (a.s - e) / 2 - 1, N);
-}
+#endif  // __CUDACC__
 
 }  // namespace mpd

@@ -10,9 +10,9 @@
 //                                      MpFloat arithmetic: the reference's MPFR right SVD
 //                                      (mpfr_svd.rs, Golub-Kahan + dqds + inverse iteration) is
 //                                      replaced by a method whose rotations of disjoint column
-//                                      pairs run in parallel, one warp per pair (its column sums
-//                                      exact dots over the lanes); singular values
-//                                      are the final column norms, sorted descending
+//                                      pairs run in parallel (their column sums exact dots);
+//                                      singular values are the final column norms, sorted
+//                                      descending
 //   lambda = sigma, Lambda^-1/2 = 1 / sqrt(sigma)
 //   R = L1 V Lambda^-1/2,  Rinv = Lambda^1/2 (L1^-T V)',  G = R R' (upper)
 // V is unique up to the signs of its columns (and rotations within clusters of equal singular
@@ -31,82 +31,140 @@ namespace {
 
 using mpd::Val;
 
-constexpr int kNtThreads = 512;  // 16 warps: up to 16 rotations of a round at once
-constexpr int kNtWarps = kNtThreads / 32;
+// Up to 4 limbs 16 warps (128 registers a thread hold a dot's accumulator, operands and product);
+// above, 8 warps.
+template <int N>
+constexpr int kNtThreads = N <= 4 ? 512 : 256;
 constexpr int kNtMaxSweeps = 80;
+constexpr int kNtMax = 64;  // block order
+constexpr int kPairs = kNtMax / 2;
 
 __device__ __forceinline__ void named_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
-// a + b and a * b, rounded once
-__device__ __forceinline__ Val add(const Val& a, const Val& b, int N) { return mpd::mp_addsub(a, b, 1, N); }
-__device__ __forceinline__ Val sub(const Val& a, const Val& b, int N) { return mpd::mp_addsub(a, b, -1, N); }
-__device__ __forceinline__ Val mul(const Val& a, const Val& b, int N) { return mpd::mp_mul(a, b, N); }
-
 // Exact-dot Cholesky (lower, in place, column-major ld n) by a group of `nt` threads that
 // synchronise on named barrier `bar`: the group's first warp forms each pivot (its dot split over
-// the lanes), the group the column below it.
-__device__ void chol_group(unsigned char* L, int n, int N, int t, int nt, int bar, unsigned char* sd,
+// the lanes), then eight lanes take a row's dot and one thread a row its difference and quotient.
+template <int N>
+__device__ void chol_group(unsigned char* L, int n, int t, int nt, int bar, unsigned char* sd, unsigned char* sdot,
                            volatile int* fail, uint32_t* status) {
-  const long esz = 8L * N + 8;
+  constexpr int esz = 8 * N + 8, G = 8;
   auto at = [&](int i, int k) { return L + ((long)i + (long)k * n) * esz; };
+  bool ok = true;
   for (int j = 0; j < n; ++j) {
     if (t < 32) {  // the group's first warp forms the pivot's dot, its lane 0 the rest
-      bool ok = true;
-      const Val dot = mpd::mp_dot_sub_warp(nullptr, at(j, 0), n, at(j, 0), n, j, N, &ok);
+      const Val<N> dot = mpd::dot<N, 32>(nullptr, at(j, 0), n, at(j, 0), n, j, &ok);
       if (t == 0) {
-        const Val d = sub(mpd::mp_load(at(j, j), N), dot, N);
-        if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
+        const Val<N> d = mpd::addsub<N>(mpd::load<N>(at(j, j)), dot, -1);
         if (d.zero || d.neg) {
           *fail = 1;
         } else {
-          const Val r = mpd::mp_sqrt(d, N);
-          mpd::mp_store(at(j, j), N, r, status);
-          mpd::mp_store(sd, N, r, status);
+          const Val<N> r = mpd::root<N>(d);
+          mpd::store<N>(at(j, j), r, status);
+          mpd::store<N>(sd, r, status);
         }
+      }
+    } else {
+      for (int i = j + 1 + (t - 32) / G; i < n; i += (nt - 32) / G) {  // group-uniform
+        const Val<N> dot = mpd::dot<N, G>(nullptr, at(i, 0), n, at(j, 0), n, j, &ok);
+        if ((t & (G - 1)) == 0) mpd::store<N>(sdot + i * esz, dot, status);
       }
     }
     named_sync(bar, nt);
-    if (*fail) return;
-    const Val r = mpd::mp_load(sd, N);
-    for (int i = j + 1 + t; i < n; i += nt) {
-      bool ok = true;
-      const Val dot = mpd::mp_dot_sub(nullptr, at(i, 0), n, at(j, 0), n, j, N, &ok);
-      if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
-      mpd::mp_store(at(i, j), N, mpd::mp_div(sub(mpd::mp_load(at(i, j), N), dot, N), r, N), status);
+    if (*fail) break;
+    if (t < n - 1 - j) {
+      const int i = j + 1 + t;
+      const Val<N> d = mpd::addsub<N>(mpd::load<N>(at(i, j)), mpd::load<N>(sdot + i * esz), -1);
+      mpd::store<N>(at(i, j), mpd::divide<N>(d, mpd::load<N>(sd)), status);
     }
     named_sync(bar, nt);
   }
+  if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
+}
+
+// The rotation of a pair of columns with x'x = aa, y'y = bb, x'y = gg: false when the pair is
+// orthogonal to working accuracy (|gamma| <= 2^-(64N-8) sqrt(ab)), else c and sn:
+// zeta = (b - a) / (2 g), t = sign(zeta) / (|zeta| + sqrt(1 + zeta^2)), c = 1/sqrt(1+t^2), sn = c t.
+template <int N>
+__device__ __noinline__ bool rotation(const Val<N>& aa, const Val<N>& bb, const Val<N>& gg, Val<N>& c, Val<N>& sn) {
+  if (gg.zero || aa.zero || bb.zero) return false;
+  {
+    Val<N> ab = mpd::mul<N>(aa, bb);
+    ab.s -= 2LL * (64 * N - 8);
+    if (mpd::cmp<N>(mpd::mul<N>(gg, gg), ab) <= 0) return false;
+  }
+  const Val<N> one = mpd::one_val<N>();
+  Val<N> g2 = gg;
+  g2.s += 1;
+  Val<N> zeta = mpd::mul<N>(mpd::addsub<N>(bb, aa, -1), mpd::recip_approx<N>(g2));
+  Val<N> t;
+  if (zeta.zero) {
+    t = one;
+  } else if (zeta.s + 64LL * N > 32LL * N + 8) {  // |zeta| > 2^(32N+8): t = 1 / (2 zeta)
+    Val<N> z2 = zeta;
+    z2.s += 1;
+    t = mpd::recip_approx<N>(z2);
+  } else {
+    Val<N> az = zeta;
+    az.neg = false;
+    const Val<N> w = mpd::addsub<N>(one, mpd::mul<N>(zeta, zeta), 1);
+    const Val<N> sq = mpd::mul<N>(w, mpd::rsqrt_approx<N>(w));
+    t = mpd::recip_approx<N>(mpd::addsub<N>(az, sq, 1));
+    t.neg = zeta.neg;
+  }
+  c = mpd::rsqrt_approx<N>(mpd::addsub<N>(one, mpd::mul<N>(t, t), 1));
+  sn = mpd::mul<N>(c, t);
+  return true;
+}
+
+// Columns of a round-robin round r over mm positions: pair k holds positions k and mm - 1 - k
+// (position 0 fixed, the others rotating).  False when the pair holds the padding column.
+__device__ __forceinline__ bool round_pair(int k, int r, int mm, int n, int* p, int* q) {
+  const int pb = mm - 1 - k;
+  *p = k == 0 ? 0 : 1 + (k - 1 + r) % (mm - 1);
+  *q = 1 + (pb - 1 + r) % (mm - 1);
+  return *p < n && *q < n;
 }
 
 // One CTA per block (see the file comment).  Work: five n x n matrices per block at element
 // 5 * mat (L1, L2, the Jacobi matrix A, V, X), two n-vectors at element 2 * vec (sigma, sqrt sigma).
-__global__ void __launch_bounds__(kNtThreads) k_mp_nt_scale(const MpNtBlock* __restrict__ blocks, int N,
-                                                            const unsigned char* __restrict__ s,
-                                                            const unsigned char* __restrict__ z,
-                                                            const unsigned char* __restrict__ frac,
-                                                            unsigned char* __restrict__ work,
-                                                            unsigned char* __restrict__ wvec,
-                                                            unsigned char* __restrict__ lam,
-                                                            unsigned char* __restrict__ lisqrt,
-                                                            unsigned char* __restrict__ R,
-                                                            unsigned char* __restrict__ Rinv,
-                                                            unsigned char* __restrict__ G, int* __restrict__ bstatus,
-                                                            uint32_t* __restrict__ status) {
-  __shared__ __align__(8) unsigned char sd[2][8 * mpd::kMaxN + 8];
+// Bound by the chain of the Jacobi rounds.  A round is three phases: the 3 n / 2 column sums (exact
+// dots, eight lanes each); the rotations, one lane a pair -- the chain of some fifty MpFloat
+// operations runs once for all pairs of the round, on one warp -- while the other warps apply the
+// previous round's rotations to V, which no dot reads; and the rotations of A, one thread an entry
+// pair.  (With a warp a pair and the whole round on it, every lane repeats that chain, and four
+// warps a scheduler repeat it against one another.)
+template <int N>
+__global__ void __launch_bounds__(kNtThreads<N>) k_mp_nt_scale(const MpNtBlock* __restrict__ blocks,
+                                                               const unsigned char* __restrict__ s,
+                                                               const unsigned char* __restrict__ z,
+                                                               const unsigned char* __restrict__ frac,
+                                                               unsigned char* __restrict__ work,
+                                                               unsigned char* __restrict__ wvec,
+                                                               unsigned char* __restrict__ lam,
+                                                               unsigned char* __restrict__ lisqrt,
+                                                               unsigned char* __restrict__ R,
+                                                               unsigned char* __restrict__ Rinv,
+                                                               unsigned char* __restrict__ G, int* __restrict__ bstatus,
+                                                               uint32_t* __restrict__ status) {
+  constexpr int T = kNtThreads<N>, esz = 8 * N + 8, LG = 8;
+  __shared__ __align__(8) unsigned char sd[2][esz];
+  __shared__ __align__(8) unsigned char ssum[3 * kPairs * esz];        // column sums (Cholesky: dots of both halves)
+  __shared__ __align__(8) unsigned char srot[2][2 * kPairs * esz];     // c and sn of this round and the last
+  __shared__ int spair[2][2 * kPairs];                                 // their columns; first -1: not rotated
   __shared__ volatile int fail[2];
   __shared__ int rotated;
-  __shared__ int perm[64];
+  __shared__ int perm[kNtMax];
+  static_assert(3 * kPairs >= kNtMax, "Cholesky staging");
   const MpNtBlock B = blocks[blockIdx.x];
-  const int n = B.n, nn = n * n, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const long esz = 8L * N + 8;
+  const int n = B.n, nn = n * n, tid = threadIdx.x;
   auto el = [&](unsigned char* base, long e) { return base + e * esz; };
   unsigned char* L1 = work + 5 * B.mat * esz;
-  unsigned char* L2 = L1 + nn * esz;
-  unsigned char* A = L2 + nn * esz;
-  unsigned char* V = A + nn * esz;
-  unsigned char* X = V + nn * esz;
+  unsigned char* L2 = L1 + (long)nn * esz;
+  unsigned char* A = L2 + (long)nn * esz;
+  unsigned char* V = A + (long)nn * esz;
+  unsigned char* X = V + (long)nn * esz;
   unsigned char* sig = wvec + 2 * B.vec * esz;
   unsigned char* root = sig + n * esz;
   if (tid == 0) {
@@ -114,38 +172,39 @@ __global__ void __launch_bounds__(kNtThreads) k_mp_nt_scale(const MpNtBlock* __r
     bstatus[blockIdx.x] = 0;
   }
   // S and Z, lower triangles (svec upper column order: (i, j), j <= i, at i (i + 1) / 2 + j)
-  const Val fv = mpd::mp_load(frac, N);
-  for (int e = tid; e < nn; e += kNtThreads) {
+  const Val<N> fv = mpd::load<N>(frac);
+  for (int e = tid; e < nn; e += T) {
     const int i = e % n, j = e / n;
-    Val sv = mpd::mp_zero(), zv = mpd::mp_zero();
+    Val<N> sv = mpd::zero_val<N>(), zv = sv;
     if (i >= j) {
       const long t = (long)i * (i + 1) / 2 + j;
-      sv = mpd::mp_load(s + (B.svec + t) * esz, N);
-      zv = mpd::mp_load(z + (B.svec + t) * esz, N);
+      sv = mpd::load<N>(s + (B.svec + t) * esz);
+      zv = mpd::load<N>(z + (B.svec + t) * esz);
       if (i != j) {
-        sv = mul(sv, fv, N);
-        zv = mul(zv, fv, N);
+        sv = mpd::mul<N>(sv, fv);
+        zv = mpd::mul<N>(zv, fv);
       }
     }
-    mpd::mp_store(el(L1, e), N, sv, status);
-    mpd::mp_store(el(L2, e), N, zv, status);
+    mpd::store<N>(el(L1, e), sv, status);
+    mpd::store<N>(el(L2, e), zv, status);
   }
   __syncthreads();
-  if (tid < kNtThreads / 2)
-    chol_group(L1, n, N, tid, kNtThreads / 2, 1, sd[0], &fail[0], status);
+  if (tid < T / 2)
+    chol_group<N>(L1, n, tid, T / 2, 1, sd[0], ssum, &fail[0], status);
   else
-    chol_group(L2, n, N, tid - kNtThreads / 2, kNtThreads / 2, 2, sd[1], &fail[1], status);
+    chol_group<N>(L2, n, tid - T / 2, T / 2, 2, sd[1], srot[0], &fail[1], status);
   __syncthreads();
   // a failed block's outputs are zeros
   auto zero_outputs = [&]() {
-    for (int e = tid; e < nn; e += kNtThreads) {
-      mpd::mp_store(el(R, B.mat + e), N, mpd::mp_zero(), status);
-      mpd::mp_store(el(Rinv, B.mat + e), N, mpd::mp_zero(), status);
-      mpd::mp_store(el(G, B.mat + e), N, mpd::mp_zero(), status);
+    const Val<N> zv = mpd::zero_val<N>();
+    for (int e = tid; e < nn; e += T) {
+      mpd::store<N>(el(R, B.mat + e), zv, status);
+      mpd::store<N>(el(Rinv, B.mat + e), zv, status);
+      mpd::store<N>(el(G, B.mat + e), zv, status);
     }
-    for (int r = tid; r < n; r += kNtThreads) {
-      mpd::mp_store(el(lam, B.vec + r), N, mpd::mp_zero(), status);
-      mpd::mp_store(el(lisqrt, B.vec + r), N, mpd::mp_zero(), status);
+    for (int r = tid; r < n; r += T) {
+      mpd::store<N>(el(lam, B.vec + r), zv, status);
+      mpd::store<N>(el(lisqrt, B.vec + r), zv, status);
     }
   };
   if (fail[0] || fail[1]) {
@@ -153,157 +212,143 @@ __global__ void __launch_bounds__(kNtThreads) k_mp_nt_scale(const MpNtBlock* __r
     zero_outputs();
     return;
   }
+  bool ok = true;
   // A = M = L2' L1 (entry (i, j): rows k >= max(i, j)), V = I
-  Val one = mpd::mp_zero();
-  one.zero = false;
-  one.m[N - 1] = 1ull << 63;
-  one.s = 1 - 64LL * N;
-  for (int e = tid; e < nn; e += kNtThreads) {
+  for (int e = tid; e < nn; e += T) {
     const int i = e % n, j = e / n, k0 = i > j ? i : j;
-    bool ok = true;
-    const Val m = mpd::mp_dot_sub(nullptr, el(L2, k0 + (long)i * n), 1, el(L1, k0 + (long)j * n), 1, n - k0, N, &ok);
-    if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
-    mpd::mp_store(el(A, e), N, m, status);
-    mpd::mp_store(el(V, e), N, i == j ? one : mpd::mp_zero(), status);
+    const Val<N> m = mpd::dot<N, 1>(nullptr, el(L2, k0 + (long)i * n), 1, el(L1, k0 + (long)j * n), 1, n - k0, &ok);
+    mpd::store<N>(el(A, e), m, status);
+    mpd::store<N>(el(V, e), i == j ? mpd::one_val<N>() : mpd::zero_val<N>(), status);
   }
-  // One-sided Jacobi: sweeps of round-robin rounds (position 0 fixed, the others rotating), the
-  // disjoint pairs of a round one per warp.  A pair rotates while |gamma| > 2^-(64N-8) sqrt(ab).
-  const int mm = n + (n & 1);
+  // rotate the rows of M2's columns (p, q) of the pairs stored in buffer `buf`, threads t of nt
+  const int mm = n + (n & 1), P = mm / 2;
+  auto rotate = [&](unsigned char* M2, int buf, int t, int nt) {
+    for (int e = t; e < P * n; e += nt) {
+      const int k = e / n, i = e % n, p = spair[buf][2 * k], q = spair[buf][2 * k + 1];
+      if (p < 0) continue;
+      const Val<N> c = mpd::load<N>(srot[buf] + 2 * k * esz), sn = mpd::load<N>(srot[buf] + (2 * k + 1) * esz);
+      unsigned char* xp = el(M2, i + (long)p * n);
+      unsigned char* xq = el(M2, i + (long)q * n);
+      const Val<N> vp = mpd::load<N>(xp), vq = mpd::load<N>(xq);
+      mpd::store<N>(xp, mpd::addsub<N>(mpd::mul<N>(c, vp), mpd::mul<N>(sn, vq), -1), status);
+      mpd::store<N>(xq, mpd::addsub<N>(mpd::mul<N>(sn, vp), mpd::mul<N>(c, vq), 1), status);
+    }
+  };
+  // One-sided Jacobi: sweeps of round-robin rounds until one without a rotation.
+  int cur = 0;
+  if (tid < 2 * kPairs) spair[0][tid] = spair[1][tid] = -1;
   bool converged = n <= 1;
   for (int sweep = 0; sweep < kNtMaxSweeps && !converged; ++sweep) {
     __syncthreads();
     if (tid == 0) rotated = 0;
-    for (int r = 0; r < mm - 1; ++r) {
+    for (int r = 0; r < mm - 1; ++r, cur ^= 1) {
+      __syncthreads();  // A is rotated
+      for (int d = tid / LG; d < 3 * P; d += T / LG) {  // group-uniform
+        int p, q;
+        if (!round_pair(d / 3, r, mm, n, &p, &q)) continue;
+        const int x = d % 3 == 1 ? q : p, y = d % 3 == 0 ? p : q;  // (p, p), (q, q), (p, q)
+        const Val<N> v = mpd::dot<N, LG>(nullptr, el(A, (long)x * n), 1, el(A, (long)y * n), 1, n, &ok);
+        if ((tid & (LG - 1)) == 0) mpd::store<N>(ssum + d * esz, v, status);
+      }
       __syncthreads();
-      for (int k = warp; k < mm / 2; k += kNtWarps) {
-        const int pa = k, pb = mm - 1 - k;
-        const int p = pa == 0 ? 0 : 1 + (pa - 1 + r) % (mm - 1);
-        const int q = pb == 0 ? 0 : 1 + (pb - 1 + r) % (mm - 1);
-        if (p >= n || q >= n) continue;
-        // the three column sums as exact dots over the warp (every lane gets the same bits)
-        bool okd = true;
-        const Val aa = mpd::mp_dot_sub_warp(nullptr, el(A, (long)p * n), 1, el(A, (long)p * n), 1, n, N, &okd);
-        const Val bb = mpd::mp_dot_sub_warp(nullptr, el(A, (long)q * n), 1, el(A, (long)q * n), 1, n, N, &okd);
-        const Val gg = mpd::mp_dot_sub_warp(nullptr, el(A, (long)p * n), 1, el(A, (long)q * n), 1, n, N, &okd);
-        if (!okd && lane == 0) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
-        bool rot = !gg.zero && !aa.zero && !bb.zero;
-        if (rot) {
-          Val ab = mul(aa, bb, N);
-          ab.s -= 2LL * (64 * N - 8);
-          rot = mpd::mp_cmp(mul(gg, gg, N), ab, N) > 0;
-        }
-        if (!rot) continue;  // warp-uniform: every lane holds the same sums
-        // zeta = (b - a) / (2 g), t = sign(zeta) / (|zeta| + sqrt(1 + zeta^2)), c = 1/sqrt(1+t^2)
-        Val g2 = gg;
-        g2.s += 1;
-        Val zeta = mul(sub(bb, aa, N), mpd::mp_recip_approx(g2, N), N);
-        Val t;
-        if (zeta.zero) {
-          t = one;
-        } else if (zeta.s + 64LL * N > 32LL * N + 8) {  // |zeta| > 2^(32N+8): t = 1 / (2 zeta)
-          Val z2 = zeta;
-          z2.s += 1;
-          t = mpd::mp_recip_approx(z2, N);
-        } else {
-          Val az = zeta;
-          az.neg = false;
-          const Val w = add(one, mul(zeta, zeta, N), N);
-          const Val sq = mul(w, mpd::mp_rsqrt_approx(w, N), N);
-          t = mpd::mp_recip_approx(add(az, sq, N), N);
-          t.neg = zeta.neg;
-        }
-        const Val c = mpd::mp_rsqrt_approx(add(one, mul(t, t, N), N), N);
-        const Val sn = mul(c, t, N);
-        for (int i = lane; i < n; i += 32) {
-          unsigned char* M2[2] = {A, V};
-          for (int w = 0; w < 2; ++w) {
-            unsigned char* xp = el(M2[w], i + (long)p * n);
-            unsigned char* xq = el(M2[w], i + (long)q * n);
-            const Val vp = mpd::mp_load(xp, N), vq = mpd::mp_load(xq, N);
-            mpd::mp_store(xp, N, sub(mul(c, vp, N), mul(sn, vq, N), N), status);
-            mpd::mp_store(xq, N, add(mul(sn, vp, N), mul(c, vq, N), N), status);
+      if (tid < 32) {
+        if (tid < P) {
+          int p, q;
+          Val<N> c, sn;
+          bool rot = round_pair(tid, r, mm, n, &p, &q);
+          if (rot)
+            rot = rotation<N>(mpd::load<N>(ssum + 3 * tid * esz), mpd::load<N>(ssum + (3 * tid + 1) * esz),
+                              mpd::load<N>(ssum + (3 * tid + 2) * esz), c, sn);
+          spair[cur][2 * tid] = rot ? p : -1;
+          spair[cur][2 * tid + 1] = q;
+          if (rot) {
+            mpd::store<N>(srot[cur] + 2 * tid * esz, c, status);
+            mpd::store<N>(srot[cur] + (2 * tid + 1) * esz, sn, status);
+            atomicAdd(&rotated, 1);
           }
         }
-        if (lane == 0) atomicAdd(&rotated, 1);
+      } else {
+        rotate(V, cur ^ 1, tid - 32, T - 32);  // the last round's rotations
       }
+      __syncthreads();
+      rotate(A, cur, tid, T);
     }
     __syncthreads();
     converged = rotated == 0;
   }
+  rotate(V, cur ^ 1, tid, T);  // the last round of the last sweep (none rotated once converged)
+  if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
   if (!converged) {
     if (tid == 0) bstatus[blockIdx.x] = SDPXG_ST_SVD_UNCONVERGED;
     zero_outputs();
     return;
   }
+  __syncthreads();
   // singular values: column norms (exact sums of squares, correctly rounded roots), descending
-  for (int j = tid; j < n; j += kNtThreads) {
-    bool ok = true;
-    const Val ss = mpd::mp_dot_sub(nullptr, el(A, (long)j * n), 1, el(A, (long)j * n), 1, n, N, &ok);
-    if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
-    mpd::mp_store(el(sig, j), N, mpd::mp_sqrt(ss, N), status);
+  for (int j = tid / LG; j < n; j += T / LG) {
+    const Val<N> ss = mpd::dot<N, LG>(nullptr, el(A, (long)j * n), 1, el(A, (long)j * n), 1, n, &ok);
+    if ((tid & (LG - 1)) == 0) mpd::store<N>(el(sig, j), mpd::root<N>(ss), status);
   }
   __syncthreads();
-  for (int j = tid; j < n; j += kNtThreads) {
-    const Val sj = mpd::mp_load(el(sig, j), N);
+  for (int j = tid; j < n; j += T) {
+    const Val<N> sj = mpd::load<N>(el(sig, j));
     int rank = 0;
     for (int k = 0; k < n; ++k) {
       if (k == j) continue;
-      const int c = mpd::mp_cmp(mpd::mp_load(el(sig, k), N), sj, N);
+      const int c = mpd::cmp<N>(mpd::load<N>(el(sig, k)), sj);
       rank += (c > 0 || (c == 0 && k < j)) ? 1 : 0;
     }
     perm[rank] = j;
   }
   __syncthreads();
-  for (int r = tid; r < n; r += kNtThreads) {
-    const Val sg = mpd::mp_load(el(sig, perm[r]), N);
-    const Val rt = mpd::mp_sqrt(sg, N);
-    mpd::mp_store(el(lam, B.vec + r), N, sg, status);
-    mpd::mp_store(el(root, r), N, rt, status);
-    mpd::mp_store(el(lisqrt, B.vec + r), N, mpd::mp_recip(rt, N), status);
+  for (int r = tid; r < n; r += T) {
+    const Val<N> sg = mpd::load<N>(el(sig, perm[r]));
+    const Val<N> rt = mpd::root<N>(sg);
+    mpd::store<N>(el(lam, B.vec + r), sg, status);
+    mpd::store<N>(el(root, r), rt, status);
+    mpd::store<N>(el(lisqrt, B.vec + r), mpd::recip<N>(rt), status);
   }
   __syncthreads();
-  // R = L1 V Lambda^-1/2 (row i of L1 has entries k <= i); X = L1^-T V (back substitution)
-  for (int e = tid; e < nn; e += kNtThreads) {
+  // R = L1 V Lambda^-1/2 (row i of L1 has entries k <= i); X = L1^-T V (back substitution, eight
+  // lanes a column)
+  for (int e = tid; e < nn; e += T) {
     const int i = e % n, r = e / n;
-    bool ok = true;
-    const Val d = mpd::mp_dot_sub(nullptr, el(L1, i), n, el(V, (long)perm[r] * n), 1, i + 1, N, &ok);
-    if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
-    mpd::mp_store(el(R, B.mat + e), N, mul(d, mpd::mp_load(el(lisqrt, B.vec + r), N), N), status);
+    const Val<N> d = mpd::dot<N, 1>(nullptr, el(L1, i), n, el(V, (long)perm[r] * n), 1, i + 1, &ok);
+    mpd::store<N>(el(R, B.mat + e), mpd::mul<N>(d, mpd::load<N>(el(lisqrt, B.vec + r))), status);
   }
-  for (int r = tid; r < n; r += kNtThreads) {
-    for (int i = n - 1; i >= 0; --i) {
-      bool ok = true;
-      const Val b = mpd::mp_load(el(V, i + (long)perm[r] * n), N);
-      const Val d = mpd::mp_dot_sub(&b, el(L1, i + 1 + (long)i * n), 1, el(X, i + 1 + (long)r * n), 1, n - 1 - i, N,
-                                    &ok);
-      if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
-      mpd::mp_store(el(X, i + (long)r * n), N, mpd::mp_div(d, mpd::mp_load(el(L1, i + (long)i * n), N), N), status);
+  {
+    const unsigned gmask = 0xffu << (tid & 24);
+    for (int r = tid / LG; r < n; r += T / LG) {
+      for (int i = n - 1; i >= 0; --i) {
+        const Val<N> b = mpd::load<N>(el(V, i + (long)perm[r] * n));
+        const Val<N> d = mpd::dot<N, LG>(&b, el(L1, i + 1 + (long)i * n), 1, el(X, i + 1 + (long)r * n), 1, n - 1 - i,
+                                         &ok);
+        if ((tid & (LG - 1)) == 0)
+          mpd::store<N>(el(X, i + (long)r * n), mpd::divide<N>(d, mpd::load<N>(el(L1, i + (long)i * n))), status);
+        __syncwarp(gmask);  // x_i visible to the group's next dot
+      }
     }
   }
   __syncthreads();
   // Rinv(r, j) = sqrt(sigma_r) X(j, r); G = R R' (upper: exact dots of rows of R)
-  for (int e = tid; e < nn; e += kNtThreads) {
+  for (int e = tid; e < nn; e += T) {
     const int r = e % n, j = e / n;
-    mpd::mp_store(el(Rinv, B.mat + e), N,
-                  mul(mpd::mp_load(el(X, j + (long)r * n), N), mpd::mp_load(el(root, r), N), N), status);
-    Val g = mpd::mp_zero();
-    if (r <= j) {
-      bool ok = true;
-      g = mpd::mp_dot_sub(nullptr, el(R, B.mat + r), n, el(R, B.mat + j), n, n, N, &ok);
-      if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
-    }
-    mpd::mp_store(el(G, B.mat + e), N, g, status);
+    mpd::store<N>(el(Rinv, B.mat + e),
+                  mpd::mul<N>(mpd::load<N>(el(X, j + (long)r * n)), mpd::load<N>(el(root, r))), status);
+    Val<N> g = mpd::zero_val<N>();
+    if (r <= j) g = mpd::dot<N, 1>(nullptr, el(R, B.mat + r), n, el(R, B.mat + j), n, n, &ok);
+    mpd::store<N>(el(G, B.mat + e), g, status);
   }
+  if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
 }
 
 // The working-precision 1/sqrt 2 (FloatConst::FRAC_1_SQRT_2): sqrt(1/2) rounded once.
-__global__ void k_mp_frac_sqrt2(int N, unsigned char* out, uint32_t* status) {
+template <int N>
+__global__ void k_mp_frac_sqrt2(unsigned char* out, uint32_t* status) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  Val h = mpd::mp_zero();
-  h.zero = false;
-  h.m[N - 1] = 1ull << 63;
-  h.s = -64LL * N;  // 2^63 2^(64(N-1)) 2^-64N = 1/2
-  mpd::mp_store(out, N, mpd::mp_sqrt(h, N), status);
+  Val<N> h = mpd::one_val<N>();
+  h.s -= 1;  // 1/2
+  mpd::store<N>(out, mpd::root<N>(h), status);
 }
 
 }  // namespace
@@ -314,9 +359,12 @@ void mp_launch_nt_scale(const MpNtBlock* blocks, int nblk, int N, const unsigned
                         uint32_t* status, cudaStream_t st) {
   if (N < 1 || N > mpd::kMaxN) throw std::invalid_argument("MPFR NT scaling: limbs must be in 1..8");
   if (nblk <= 0) return;
-  ++g_launches, k_mp_frac_sqrt2<<<1, 32, 0, st>>>(N, frac, status);
-  ++g_launches, k_mp_nt_scale<<<nblk, kNtThreads, 0, st>>>(blocks, N, s, z, frac, work, wvec, lam, lisqrt, R, Rinv,
-                                                           G, bstatus, status);
+  mpd::by_limbs(N, [&](auto l) {
+    constexpr int L = l();
+    ++g_launches, k_mp_frac_sqrt2<L><<<1, 32, 0, st>>>(frac, status);
+    ++g_launches, k_mp_nt_scale<L><<<nblk, kNtThreads<L>, 0, st>>>(blocks, s, z, frac, work, wvec, lam, lisqrt, R,
+                                                                   Rinv, G, bstatus, status);
+  });
   check(cudaGetLastError(), "k_mp_nt_scale");
 }
 

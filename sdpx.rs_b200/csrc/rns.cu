@@ -1894,7 +1894,7 @@ extern "C" int32_t sdpxg_mp_step_length(sdpxg_ctx* ctx, uint32_t limbs, uint64_t
     if (!orders || !d || !Rx || !lisqrt || !alpha_max || !alpha || !path) throw std::invalid_argument("null pointer");
     std::vector<MpStepBlock> desc;
     std::vector<int> slot;
-    long tri = 0, sq = 0, lin = 0, fw = 0;
+    long tri = 0, sq = 0, lin = 0;
     for (uint64_t b = 0; b < nblocks; ++b) {
       if (orders[b] > 64) throw std::invalid_argument("sdpxg_mp_step_length: block orders must be at most 64");
       const long n = (long)orders[b];
@@ -1905,7 +1905,6 @@ extern "C" int32_t sdpxg_mp_step_length(sdpxg_ctx* ctx, uint32_t limbs, uint64_t
       tri += n * (n + 1) / 2;
       sq += n * n;
       lin += n;
-      fw += n * n + 2 * n;
     }
     const size_t esz = 8 * (size_t)N + 8;
     cudaStream_t st = E->st;
@@ -1913,7 +1912,6 @@ extern "C" int32_t sdpxg_mp_step_length(sdpxg_ctx* ctx, uint32_t limbs, uint64_t
     DevBuf<MpStepBlock> dd(std::max<size_t>(desc.size(), 1));
     DevBuf<unsigned char> dD(tri * esz + esz), dR(sq * esz + esz), dL(lin * esz + esz), dX(sq * esz + esz),
         dY(sq * esz + esz), dwork(2 * sq * esz + esz), dconst(2 * esz), dal(std::max<size_t>(desc.size(), 1) * esz);
-    DevBuf<double> dfw(fw + 1);
     DevBuf<int> dpath(std::max<size_t>(desc.size(), 1));
     DevBuf<uint32_t> stw(1);
     check(cudaMemsetAsync(stw.p, 0, sizeof(uint32_t), st), "memset");
@@ -1933,7 +1931,7 @@ extern "C" int32_t sdpxg_mp_step_length(sdpxg_ctx* ctx, uint32_t limbs, uint64_t
                                         dY.p + b.mat * esz, &hs);
       if (rc) return rc;
     }
-    mp_launch_step_bound(dd, (int)desc.size(), N, dY, dL, dconst, dwork, dfw, dal, dpath, stw, st);
+    mp_launch_step_bound(dd, (int)desc.size(), N, dY, dL, dconst, dwork, dal, dpath, stw, st);
     std::vector<unsigned char> hal(desc.size() * esz);
     std::vector<int> hpath(desc.size());
     uint32_t hs = 0;
