@@ -295,11 +295,11 @@ struct ShiftStage<K, 0> {
   static MPD_FN void run(uint32_t*, int&) {}
 };
 
-// Shift the nonzero S (K <= 64 words) left until its top bit is set; the bits shifted.
+// Shift the nonzero S (K <= 128 words) left until its top bit is set; the bits shifted.
 template <int K>
 MPD_FN int normalize(uint32_t* S) {
   int sh = 0;
-  if (S[K - 1] == 0) ShiftStage<K, 32>::run(S, sh);
+  if (S[K - 1] == 0) ShiftStage<K, (K > 64 ? 64 : 32)>::run(S, sh);
   const int c = clz32(S[K - 1]) & 31;
 #pragma unroll
   for (int i = K - 1; i > 0; --i) S[i] = funnel_l(S[i - 1], S[i], c);

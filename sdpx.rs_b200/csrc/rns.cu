@@ -9,24 +9,27 @@
 // INT8 tensor-core form (the default, RNS_FORM_INT8):
 //   k_rns_scan       per row of op(A) / column of op(B): lowest set-bit exponent lo and the
 //                    width `bits` of the aligned integers (rns_blas.rs:2164-2183 alignment)
-//   k_rns_pow2       2^s mod p for every prime and every bit position an entry can reach
+//   k_rns_factors    2^(s + 64) mod p for every prime and every alignment shift s, plain and times
+//                    the prime's CRT weight (kept with the prime set)
 //   k_rns8_residues  every entry as the integer M * 2^(e - 64N - lo) reduced to symmetric
-//                    residues modulo L primes below 2^15, each split into two signed-byte
+//                    residues modulo L primes below 2^15 (the mantissa's 32-bit words against
+//                    2^(32 i) mod p and two Montgomery steps), each split into two signed-byte
 //                    digits r = lo + 256 hi, written as K-major byte planes
 //                    (rns_blas.rs:929-986 panel residues)
 //   k_i8_mod_gemm    per prime, the four digit products on tcgen05.mma kind::i8 with INT32
 //                    accumulators in TMEM, recombined and reduced modulo the prime in the
 //                    epilogue; K beyond 2^16 in chunks whose residues are added
 //                    (rns_blas.rs:447-580 per-prime integer products)
-//   k_rns_crt        Garner's mixed-radix CRT back to the signed integer, then one rounding to
-//                    64N bits, ties to even (rns_blas.rs:1873-2125 CRT and pack,
-//                    exactdot.rs:1316-1392 from_scaled_integer)
+//   k_rns_crt        the residues, two primes at a time, against multiples of the prime product's
+//                    cofactors back to the signed integer, then one rounding to 64N bits, ties to
+//                    even (rns_blas.rs:1873-2125 CRT and pack, exactdot.rs:1316-1392
+//                    from_scaled_integer)
 // FP64 form (RNS_FORM_FP64, the plain form on CUDA cores):
 //   k_rns_residues   residues modulo primes below 2^21 as doubles
 //   k_rns_gemm       one exact FP64 product per prime: symmetric residues keep |r| < 2^20, so
 //                    8192 products sum exactly below 2^53; partial sums are reduced modulo the
 //                    prime every 8192 terms
-//   k_rns_crt        as above.
+//   k_rns_crt_f64    the same reconstruction prime by prime.
 // The number of primes L follows the needed width 2*(64N) + spreads + log2(k) + 2 bits, the
 // same bound as the reference's Plan (rns_blas.rs:2202-2208); the reference's own primes are
 // 18-26 bits wide, the INT8 form uses 15-bit primes so that a residue is two signed bytes.
@@ -47,6 +50,7 @@
 #include "../../include/sdpx_b200.h"
 #include "engine.cuh"
 #include "i8_gemm.cuh"
+#include "mp.cuh"
 #include "mp_ldl.cuh"
 
 using namespace sdpxg;
@@ -231,76 +235,122 @@ k_rns_gemm(const double* __restrict__ RA, const double* __restrict__ RB, double*
     }
 }
 
-// 2^s mod p_t for s < S (row t of the table).
-extern "C" __global__ void k_rns_pow2(int L, const int* __restrict__ primes, int S, uint32_t* __restrict__ out) {
-  const int t = blockIdx.y, s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= L || s >= S) return;
-  out[(size_t)t * S + s] = pow2mod(s, (uint32_t)primes[t]);
+// Per prime p < 2^15 of the INT8 form: c[i] = 2^(32 i) mod p, p, p^-1 mod 2^32 (16-byte rows).
+struct ResiduePrime {
+  uint32_t c[2 * RNS_MAXN];
+  uint32_t p, ninv, pad[2];
+};
+
+// x 2^-32 modulo p (Montgomery): x - t p with t = x p^-1 mod 2^32 is a multiple of 2^32.  The
+// result lies in (-p, x >> 32].
+__device__ __forceinline__ int redc(unsigned long long x, uint32_t p, uint32_t ninv) {
+  return (int)(uint32_t)(x >> 32) - (int)__umulhi((uint32_t)x * ninv, p);
 }
 
-// (M 2^shift) mod p for the mantissa M = sum_q limbs[q] 2^(64q): Horner over the limbs with
-// 2^32 and 2^64 mod p from the power table's row (row[s] = 2^s mod p, s < S, S > 64), each
-// step one Barrett reduction, then one product with row[shift].
-__device__ __forceinline__ uint32_t residue_of(const unsigned long long* limbs, int N, const uint32_t* row,
-                                               int shift, uint32_t p, unsigned long long mu) {
-  const unsigned long long c32 = row[32], c64 = row[64];
-  unsigned long long r = 0;
+// (sum_i w_i 2^(32 i)) f 2^-64 mod p in [0, p), i < NW <= 32: the words against the table of
+// 2^(32 i) mod p in one 64-bit sum (below 2^52), one Montgomery step, the factor, another one.
+// With f = 2^(shift + 64) mod p it is the residue of the words shifted by `shift`.
+template <int NW>
+__device__ __forceinline__ int residue_words(const uint32_t* w, const uint32_t* c, uint32_t p, uint32_t ninv,
+                                             uint32_t f) {
+  unsigned long long acc = 0;
 #pragma unroll
-  for (int q = RNS_MAXN - 1; q >= 0; --q) {
-    if (q < N) {
-      const unsigned long long v = limbs[q];
-      const unsigned long long lm = modb((v >> 32) * c32 + (v & 0xFFFFFFFFull), p, mu);
-      r = modb(r * c64 + lm, p, mu);
-    }
-  }
-  return modb(r * row[shift], p, mu);
+  for (int i = 0; i < NW; ++i) acc += (unsigned long long)w[i] * c[i];
+  const uint32_t x = (uint32_t)(redc(acc, p, ninv) + (int)p);  // in (0, 2^20 + p]
+  const int r = redc((unsigned long long)x * f, p, ninv);      // in (-p, 8]
+  return r < 0 ? r + (int)p : r;
+}
+
+// Factor table of the residues: row t, entry s: 2^(s + 64) mod p_t; row L + t: times w_t (the CRT
+// weight of p_t, which the left operand of a product carries so that the product's residues are
+// the CRT's coefficients).
+extern "C" __global__ void k_rns_factors(int L, const uint32_t* __restrict__ primes, const uint32_t* __restrict__ wt,
+                                         int S, uint32_t* __restrict__ out) {
+  const int t = blockIdx.y, s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= L || s >= S) return;
+  const uint32_t p = primes[t], v = pow2mod(s + 64, p);
+  out[(size_t)t * S + s] = v;
+  out[(size_t)(L + t) * S + s] = (uint32_t)((unsigned long long)v * wt[t] % p);
 }
 
 // INT8 form: symmetric residues modulo L primes below 2^15 of every entry of a view, each split
 // into signed-byte digits r = lo + 256 hi (|hi| <= 64), written to K-major byte planes: digit d
 // of prime t for line x (a row of op(A) or a column of op(B)) and inner index y at
 // out[((2t + d) * Rpad + x) * Kld + y].  Lines >= nlines and y >= len (the padding) get zeros.
-// One thread per (x, y), y fastest: the plane writes are coalesced.  The residue of
-// M * 2^shift is (M mod p)(2^shift mod p) mod p, M mod p by Horner over the 64-bit limbs
-// (residue_of: three power-table reads per prime).
-extern "C" __global__ void k_rns8_residues(const unsigned char* __restrict__ X, int N, int nlines, int len,
-                                           long sx, long sy, const int* __restrict__ lo, int L,
-                                           const int* __restrict__ primes, const unsigned long long* __restrict__ mu,
-                                           const uint32_t* __restrict__ pow2, int S, int8_t* __restrict__ out,
-                                           int Rpad, int Kld) {
+// Bound by the integer multiply-adds: 2N of them per entry and prime plus two Montgomery steps
+// (about 30 instructions at 4 limbs, where a Horner scheme of 64-bit Barrett steps took 225).  A
+// thread holds E consecutive entries of a line in registers for all its primes, so that a prime's
+// table row is read once for E entries and the digits are written E bytes at a time.  grid.y
+// splits the primes when the entries alone leave SMs idle.  2000 x 2000 entries of 256 bits (42 primes):
+// 2127 us before, 505 us so.  NW: words of the mantissa, rounded up.
+template <int NW, int E>
+__global__ void __launch_bounds__(256) k_rns8_residues(const unsigned char* __restrict__ X, int N, int nlines,
+                                                       int len, long sx, long sy, const int* __restrict__ lo, int L,
+                                                       const ResiduePrime* __restrict__ rp,
+                                                       const uint32_t* __restrict__ factor, int S,
+                                                       int8_t* __restrict__ out, int Rpad, int Kld) {
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long)Rpad * Kld) return;
-  const int y = (int)(idx % Kld), x = (int)(idx / Kld);
+  const int per = Kld / E;  // Kld is a multiple of 128
+  if (idx >= (long)Rpad * per) return;
+  const int y = (int)(idx % per) * E, x = (int)(idx / per);
   const size_t plane = (size_t)Rpad * Kld;
   int8_t* o = out + (size_t)x * Kld + y;
-  bool live = x < nlines && y < len;
-  bool neg = false;
-  int shift = 0;
-  unsigned long long limbs[RNS_MAXN];
-  if (live) {
-    const unsigned char* e = X + ((long)x * sx + (long)y * sy) * (8L * N + 8);
-    const int kind = elem_kind(e, N);
-    live = abs(kind) == MP_REGULAR;
-    if (live) {
-      neg = kind < 0;
-      shift = elem_exp(e, N) - 64 * N - lo[x];
-      const unsigned long long* lp = reinterpret_cast<const unsigned long long*>(e);
+  uint32_t w[E][NW];
+  int shift[E];
+  bool neg[E];
 #pragma unroll
-      for (int q = 0; q < RNS_MAXN; ++q) limbs[q] = q < N ? lp[q] : 0ull;
+  for (int e = 0; e < E; ++e) {
+    shift[e] = 0;
+    neg[e] = false;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) w[e][i] = 0u;
+    if (x < nlines && y + e < len) {
+      const unsigned char* el = X + ((long)x * sx + (long)(y + e) * sy) * (8L * N + 8);
+      const int kind = elem_kind(el, N);
+      if (abs(kind) == MP_REGULAR) {
+        neg[e] = kind < 0;
+        shift[e] = elem_exp(el, N) - 64 * N - lo[x];
+        const unsigned long long* lp = reinterpret_cast<const unsigned long long*>(el);
+#pragma unroll
+        for (int q = 0; q < NW / 2; ++q) {
+          const unsigned long long v = q < N ? lp[q] : 0ull;
+          w[e][2 * q] = (uint32_t)v;
+          w[e][2 * q + 1] = (uint32_t)(v >> 32);
+        }
+      }
     }
   }
-  for (int t = 0; t < L; ++t) {
-    int dlo = 0, dhi = 0;
-    if (live) {
-      const int p = primes[t];
-      int r = (int)residue_of(limbs, N, pow2 + (size_t)t * S, shift, (uint32_t)p, mu[t]);
-      if (r > p / 2) r -= p;
-      if (neg) r = -r;
-      dlo = ((r + 128) & 255) - 128;
-      dhi = (r - dlo) >> 8;
+  const int per_t = (L + gridDim.y - 1) / gridDim.y, t0 = blockIdx.y * per_t, t1 = min(L, t0 + per_t);
+#pragma unroll 1
+  for (int t = t0; t < t1; ++t) {
+    uint32_t c[NW];
+    const uint4* row = reinterpret_cast<const uint4*>(rp[t].c);
+#pragma unroll
+    for (int i = 0; i < NW / 4; ++i) {
+      const uint4 v = __ldg(row + i);
+      c[4 * i] = v.x;
+      c[4 * i + 1] = v.y;
+      c[4 * i + 2] = v.z;
+      c[4 * i + 3] = v.w;
     }
-    o[(size_t)(2 * t) * plane] = (int8_t)dlo;
-    o[(size_t)(2 * t + 1) * plane] = (int8_t)dhi;
+    const uint2 pn = __ldg(reinterpret_cast<const uint2*>(&rp[t].p));
+    uint32_t blo = 0, bhi = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      int r = residue_words<NW>(w[e], c, pn.x, pn.y, __ldg(factor + (size_t)t * S + shift[e]));
+      if (r > (int)(pn.x >> 1)) r -= (int)pn.x;
+      if (neg[e]) r = -r;
+      blo |= ((uint32_t)r & 255u) << (8 * e);
+      bhi |= ((uint32_t)((r + 128) >> 8) & 255u) << (8 * e);
+    }
+    int8_t* d = o + (size_t)(2 * t) * plane;
+    if (E == 4) {
+      *reinterpret_cast<uint32_t*>(d) = blo;
+      *reinterpret_cast<uint32_t*>(d + plane) = bhi;
+    } else {
+      *reinterpret_cast<uint16_t*>(d) = (uint16_t)blo;
+      *reinterpret_cast<uint16_t*>(d + plane) = (uint16_t)bhi;
+    }
   }
 }
 
@@ -350,17 +400,19 @@ __device__ __forceinline__ unsigned long long word_at(const unsigned long long (
 }
 
 // CRT of the L residues of every output, then one rounding to 64N bits (ties to even).
-// Residues are read as R (double: the FP64 form's exact integers, possibly negative; int: the
-// INT8 form's residues in [0, p)).  With M = prod p_t, M_t = M / p_t and w_t = M_t^-1 mod p_t:
-// c_t = r_t w_t mod p_t, S = sum_t c_t M_t (exact, WW words), f = sum_t c_t / p_t in FP64, and
-// the signed integer is X = S - rint(f) M.  The prime set covers more than twice the largest |X|
-// plus a margin (|X| < M / 4), so S / M = f sits within 1/4 of an integer and FP64's error
-// (below L^2 2^-53) cannot move rint(f); X is then exact.  L products of a table row with one
-// small factor per output, instead of Garner's L^2 / 2 modular steps.  S lives in registers: the
-// kernel is instantiated for the smallest word count WM >= WW (launch_crt).
-template <typename R, int WM>
-__global__ void __launch_bounds__(128) k_rns_crt(const R* __restrict__ RC, long planeC, int m, int n, int L, int WW,
-                                                 const uint32_t* __restrict__ primes,
+// With M = prod p_t, M_t = M / p_t and w_t = M_t^-1 mod p_t: c_t = r_t w_t mod p_t,
+// S = sum_t c_t M_t (exact), f = sum_t c_t / p_t, and the signed integer is X = S - rint(f) M.  The
+// prime set covers more than twice the largest |X| plus a margin (|X| < M / 4), so S / M = f
+// sits within 1/4 of an integer and the error of f in floating point (below L^2 2^-24 in FP32)
+// cannot move rint(f); X is then exact.
+//
+// FP64 form (exact integers |r| < 2^53 of either sign, primes below 2^21): S in 32-bit digits, one
+// 64-bit accumulator each (c < 2^21 times a 32-bit digit is below 2^53, so up to 2^11 primes sum
+// without overflow), carried once after the loop; S lives in registers: the kernel is instantiated
+// for the smallest word count WM >= WW (launch_crt_f64).
+template <int WM>
+__global__ void __launch_bounds__(128) k_rns_crt_f64(const double* __restrict__ RC, long planeC, int m, int n, int L,
+                                                 int WW, const uint32_t* __restrict__ primes,
                                                  const uint32_t* __restrict__ wt, const double* __restrict__ pinv,
                                                  const unsigned long long* __restrict__ mu,
                                                  const unsigned long long* __restrict__ MT,
@@ -384,8 +436,6 @@ __global__ void __launch_bounds__(128) k_rns_crt(const R* __restrict__ RC, long 
     write_zero();
     return;
   }
-  // S accumulates in 32-bit digits, one 64-bit accumulator each (c < 2^21 times a 32-bit digit
-  // is below 2^53, so up to 2^11 primes sum without overflow), carried once after the loop
   unsigned long long acc[2 * WM];
 #pragma unroll
   for (int w = 0; w < 2 * WM; ++w) acc[w] = 0ull;
@@ -394,11 +444,9 @@ __global__ void __launch_bounds__(128) k_rns_crt(const R* __restrict__ RC, long 
     const uint32_t p = primes[t];
     const double pi = pinv[t];
     long long r = (long long)RC[t * planeC + idx];
-    if (!std::is_same<R, int>::value) {  // the FP64 form's exact integers (|r| < 2^53, any sign)
-      r -= (long long)floor((double)r * pi) * (long long)p;  // within one multiple of p
-      if (r < 0) r += p;
-      if (r >= (long long)p) r -= p;
-    }  // the INT8 form's residues are in [0, p) already
+    r -= (long long)floor((double)r * pi) * (long long)p;  // within one multiple of p
+    if (r < 0) r += p;
+    if (r >= (long long)p) r -= p;
     const unsigned long long c = modb((unsigned long long)r * wt[t], p, mu[t]);
     f += (double)c * pi;
     const uint32_t* row = reinterpret_cast<const uint32_t*>(MT + (size_t)t * WW);  // 32-bit digits of M_t
@@ -507,36 +555,186 @@ __global__ void __launch_bounds__(128) k_rns_crt(const R* __restrict__ RC, long 
   *oexp = (int)exponent;
 }
 
-// The CRT kernel for WW words, instantiated with the smallest register width that holds them.
-template <typename R>
-void launch_crt(unsigned blocks, cudaStream_t st, const R* RC, long planeC, int m, int n, int L, int WW,
-                const uint32_t* primes, const uint32_t* wt, const double* pinv, const unsigned long long* mu,
-                const unsigned long long* MT,
-                const unsigned long long* Mbig, const int* loA, const int* loB, int N, int upper_only,
-                unsigned char* C, uint32_t* status) {
-  if (WW <= 8)
-    k_rns_crt<R, 8><<<blocks, 128, 0, st>>>(RC, planeC, m, n, L, WW, primes, wt, pinv, mu, MT, Mbig, loA, loB, N,
-                                            upper_only, C, status);
-  else if (WW <= 16)
-    k_rns_crt<R, 16><<<blocks, 128, 0, st>>>(RC, planeC, m, n, L, WW, primes, wt, pinv, mu, MT, Mbig, loA, loB, N,
-                                             upper_only, C, status);
-  else if (WW <= 32)
-    k_rns_crt<R, 32><<<blocks, 128, 0, st>>>(RC, planeC, m, n, L, WW, primes, wt, pinv, mu, MT, Mbig, loA, loB, N,
-                                             upper_only, C, status);
+void launch_crt_f64(unsigned blocks, cudaStream_t st, const double* RC, long planeC, int m, int n, int L, int WW,
+                    const uint32_t* primes, const uint32_t* wt, const double* pinv, const unsigned long long* mu,
+                    const unsigned long long* MT, const unsigned long long* Mbig, const int* loA, const int* loB,
+                    int N, int upper_only, unsigned char* C, uint32_t* status) {
+  if (WW <= 16)
+    k_rns_crt_f64<16><<<blocks, 128, 0, st>>>(RC, planeC, m, n, L, WW, primes, wt, pinv, mu, MT, Mbig, loA, loB, N,
+                                              upper_only, C, status);
   else
-    k_rns_crt<R, RNS_MAXW><<<blocks, 128, 0, st>>>(RC, planeC, m, n, L, WW, primes, wt, pinv, mu, MT, Mbig, loA, loB,
-                                                   N, upper_only, C, status);
+    k_rns_crt_f64<RNS_MAXW><<<blocks, 128, 0, st>>>(RC, planeC, m, n, L, WW, primes, wt, pinv, mu, MT, Mbig, loA, loB,
+                                                    N, upper_only, C, status);
+}
+
+// INT8 form: one entry of a pair's table row.  Primes are taken two at a time:
+// c_1 M/p_1 + c_2 M/p_2 = (c_1 p_2 + c_2 p_1) M/(p_1 p_2), so a pair costs one 31-bit coefficient
+// against one row of M/(p_1 p_2) in digits of kCrtBits bits: 31 + 26 bits leave room for 2^7
+// pairs in a 64-bit accumulator.
+constexpr int kCrtBits = 26;
+struct CrtPair {
+  uint32_t p1, p2;  // an odd set's last prime has p2 = 1 and no second residue
+  float inv;        // 1 / (p1 p2)
+  uint32_t w1, w2;  // CRT weights, for residues that do not carry them
+  uint32_t pad;
+  unsigned long long mu1, mu2;  // Barrett constants of p1, p2
+};
+
+// The INT8 form's CRT: residues in [0, p) per output, already times w_t unless `weights`.  Bound by
+// the multiply-adds of the coefficients with the table rows (D a pair, one thread an output), D the
+// number of digits rounded up to the instantiated widths (launch_crt).  Then the carried words,
+// S - rint(f) M, its magnitude shifted up to the top of the K words, and one rounding at the bit
+// below the N leading limbs.  2000 x 2000 outputs of 256 bits: 2166 us with one prime a step in 32-bit
+// digits, 803 us so.
+template <int D>
+__global__ void __launch_bounds__(128) k_rns_crt(const int* __restrict__ RC, long planeC, int m, int n, int L,
+                                                 const CrtPair* __restrict__ pairs, const uint32_t* __restrict__ rows,
+                                                 const uint32_t* __restrict__ Mbig, int weights,
+                                                 const int* __restrict__ loA, const int* __restrict__ loB, int N,
+                                                 int upper_only, unsigned char* __restrict__ C,
+                                                 uint32_t* __restrict__ status) {
+  constexpr int K = (kCrtBits * D + 31) / 32;  // words of S
+  const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (long)m * n) return;
+  const int i = (int)(idx % m), j = (int)(idx / m);
+  unsigned long long* ol = reinterpret_cast<unsigned long long*>(C + idx * (8L * N + 8));
+  auto write_zero = [&]() {
+    for (int q = 0; q < N; ++q) ol[q] = 0ull;
+    ol[N] = (unsigned long long)MP_ZERO;
+  };
+  if (upper_only && i > j) {
+    write_zero();
+    return;
+  }
+  unsigned long long acc[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) acc[d] = 0ull;
+  float f = 0.f;
+  const int np = (L + 1) >> 1;
+#pragma unroll 1
+  for (int t = 0; t < np; ++t) {
+    const CrtPair pr = pairs[t];
+    uint32_t c1 = (uint32_t)RC[2 * t * planeC + idx];
+    uint32_t c2 = 2 * t + 1 < L ? (uint32_t)RC[(2 * t + 1) * planeC + idx] : 0u;
+    if (weights) {
+      c1 = modb((unsigned long long)c1 * pr.w1, pr.p1, pr.mu1);
+      if (c2) c2 = modb((unsigned long long)c2 * pr.w2, pr.p2, pr.mu2);
+    }
+    const uint32_t c = c1 * pr.p2 + c2 * pr.p1;
+    f = fmaf((float)c, pr.inv, f);
+    const uint4* row = reinterpret_cast<const uint4*>(rows + (size_t)t * D);
+#pragma unroll
+    for (int d = 0; d < D; d += 4) {
+      const uint4 v = __ldg(row + d / 4);
+      acc[d] += (unsigned long long)c * v.x;
+      acc[d + 1] += (unsigned long long)c * v.y;
+      acc[d + 2] += (unsigned long long)c * v.z;
+      acc[d + 3] += (unsigned long long)c * v.w;
+    }
+  }
+  uint32_t S[K];
+#pragma unroll
+  for (int w = 0; w < K; ++w) S[w] = 0u;
+  {
+    unsigned long long carry = 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      const unsigned long long v = acc[d] + carry;
+      const uint32_t dig = (uint32_t)v & ((1u << kCrtBits) - 1u);
+      carry = v >> kCrtBits;
+      const int w = kCrtBits * d / 32, off = kCrtBits * d % 32;
+      S[w] |= dig << off;
+      if (off + kCrtBits > 32) S[w + 1] |= dig >> (32 - off);
+    }
+  }
+  {  // S -= k M (two's complement over K words; |X| < M / 4 fits with room for the sign)
+    const uint32_t k = (uint32_t)__float2int_rn(f);
+    long long carry = 0;
+#pragma unroll
+    for (int w = 0; w < K; ++w) {
+      const long long v = (long long)S[w] - (long long)((unsigned long long)k * __ldg(Mbig + w)) + carry;
+      S[w] = (uint32_t)v;
+      carry = v >> 32;
+    }
+  }
+  const bool neg = S[K - 1] >> 31;
+  if (neg) mpd::neg_words<K>(S);
+  if (mpd::is_zero<K>(S)) {
+    write_zero();
+    return;
+  }
+  const int sh = mpd::normalize<K>(S);
+  const int low = K - 2 * N;  // words below the mantissa
+  int wrapped = 0;
+  if (low > 0) {  // round at the mantissa's last bit, ties to even
+    uint32_t last = 0, half = 0, sticky = 0, up[K];
+#pragma unroll
+    for (int w = 0; w < K; ++w) {
+      last = w == low ? S[w] : last;
+      half = w == low - 1 ? S[w] : half;
+      sticky |= w < low - 1 ? S[w] : 0u;
+    }
+    const bool inc = (half >> 31) && ((half << 1) || sticky || (last & 1u));
+#pragma unroll
+    for (int w = 0; w < K; ++w) {
+      S[w] = w < low ? 0u : S[w];
+      up[w] = (inc && w == low) ? 1u : 0u;
+    }
+    if (mpd::add_words<K>(S, up, 0u)) {  // carried out: the mantissa wrapped to zero
+      S[K - 1] = 1u << 31;
+      wrapped = 1;
+    }
+  }
+  const long long exponent = (long long)loA[i] + loB[j] + 32 * K - sh + wrapped;
+  if (exponent > MP_EXP_MAX || exponent < -MP_EXP_MAX) {
+    atomicOr(status, SDPXG_ST_NONFINITE);
+    write_zero();
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < RNS_MAXN; ++q) {  // limb N - 1 - q
+    const int h = K - 1 - 2 * q;
+    const unsigned long long v = ((unsigned long long)(h >= 0 ? S[h >= 0 ? h : 0] : 0u) << 32) |
+                                 (h >= 1 ? S[h >= 1 ? h - 1 : 0] : 0u);
+    if (q < N) ol[N - 1 - q] = v;
+  }
+  ol[N] = ((unsigned long long)(uint32_t)(int)exponent << 32) |
+          (uint32_t)(neg ? -MP_REGULAR : MP_REGULAR);
+}
+
+// Digits of a CRT table row as instantiated, for at least d of them.
+constexpr int kCrtMaxDigits = 152;  // 256 primes below 2^15
+int crt_digits(int d) {
+  for (int w : {8, 12, 16, 20, 24, 28, 32, 36, 40, 44, 52, 64, 96, kCrtMaxDigits})
+    if (d <= w) return w;
+  throw std::runtime_error("CRT: prime set too large");
+}
+void launch_crt(cudaStream_t st, int digits, const int* RC, long planeC, int m, int n, int L, const CrtPair* pairs,
+                const uint32_t* rows, const uint32_t* Mbig, int weights, const int* loA, const int* loB, int N,
+                int upper_only, unsigned char* C, uint32_t* status) {
+  const unsigned blocks = (unsigned)(((long)m * n + 127) / 128);
+  ++g_launches;
+  switch (digits) {
+#define CRT_CASE(D)                                                                                              \
+  case D:                                                                                                        \
+    k_rns_crt<D><<<blocks, 128, 0, st>>>(RC, planeC, m, n, L, pairs, rows, Mbig, weights, loA, loB, N, upper_only, \
+                                         C, status);                                                             \
+    break;
+    CRT_CASE(8) CRT_CASE(12) CRT_CASE(16) CRT_CASE(20) CRT_CASE(24) CRT_CASE(28) CRT_CASE(32) CRT_CASE(36)
+    CRT_CASE(40) CRT_CASE(44) CRT_CASE(52) CRT_CASE(64) CRT_CASE(96) CRT_CASE(kCrtMaxDigits)
+#undef CRT_CASE
+    default: throw std::runtime_error("CRT: unknown table width");
+  }
 }
 
 // ---- exact forms of small factors (rns_blas.rs:2990-3194 diag_congruence, 4025-4174
 // svec_quadratic, 4175-4277 symmetric_bilinear) ----
 // Residues in [0, p_t) of a flat array of MpFloat<N> aligned at one exponent lo (the class's
 // lowest set bit): entry e is (-1)^s M_e 2^(exp_e - 64N - lo); out[t * count + e].  absval drops
-// the signs.  The residue is computed as in k_rns8_residues (residue_of).
+// the signs.  The residue is computed as in k_rns8_residues (residue_words).
 extern "C" __global__ void k_rns_class_residues(const unsigned char* __restrict__ X, int N, int count, int lo,
-                                                int absval, int L, const int* __restrict__ primes,
-                                                const unsigned long long* __restrict__ mu,
-                                                const uint32_t* __restrict__ pow2, int S, int* __restrict__ out) {
+                                                int absval, int L, const ResiduePrime* __restrict__ rp,
+                                                const uint32_t* __restrict__ factor, int S, int* __restrict__ out) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= count) return;
   const unsigned char* x = X + (size_t)e * (8 * N + 8);
@@ -547,13 +745,13 @@ extern "C" __global__ void k_rns_class_residues(const unsigned char* __restrict_
   }
   const bool neg = kind < 0 && !absval;
   const int shift = elem_exp(x, N) - 64 * N - lo;
-  const unsigned long long* lp = reinterpret_cast<const unsigned long long*>(x);
-  unsigned long long limbs[RNS_MAXN];
+  const uint32_t* lp = reinterpret_cast<const uint32_t*>(x);
+  uint32_t w[2 * RNS_MAXN];
 #pragma unroll
-  for (int q = 0; q < RNS_MAXN; ++q) limbs[q] = q < N ? lp[q] : 0ull;
+  for (int q = 0; q < 2 * RNS_MAXN; ++q) w[q] = q < 2 * N ? lp[q] : 0u;
   for (int t = 0; t < L; ++t) {
-    const int p = primes[t];
-    int r = (int)residue_of(limbs, N, pow2 + (size_t)t * S, shift, (uint32_t)p, mu[t]);
+    const int p = (int)rp[t].p;
+    int r = residue_words<2 * RNS_MAXN>(w, rp[t].c, rp[t].p, rp[t].ninv, factor[(size_t)t * S + shift]);
     if (neg && r) r = p - r;
     out[(size_t)t * count + e] = r;
   }
@@ -643,6 +841,12 @@ struct PrimeTables {
   std::vector<double> pinv;
   std::vector<unsigned long long> mu;  // floor((2^64 - 1) / p_t), the Barrett constants
   std::vector<unsigned long long> M, MT;  // M = prod p_t; MT row t = M / p_t (WW words each)
+  // INT8 form (primes below 2^15): residue constants; prime pairs, rows of M / (p_1 p_2) in `digits`
+  // digits of kCrtBits bits, M in 32-bit words
+  std::vector<ResiduePrime> rp;
+  std::vector<CrtPair> pairs;
+  std::vector<uint32_t> rows, M32;
+  int digits = 0;
 };
 
 // The largest RNS_MAXL primes below 2^bits, descending.
@@ -718,6 +922,51 @@ PrimeTables make_tables(const std::vector<uint32_t>& ps, int L) {
     T.pinv[t] = 1.0 / (double)p;
     T.mu[t] = ~0ull / p;
   }
+  if (ps[0] >= (1u << 15)) return T;
+  T.rp.resize(L);
+  for (int t = 0; t < L; ++t) {
+    ResiduePrime& r = T.rp[t];
+    const uint32_t p = T.primes[t];
+    for (int i = 0; i < 2 * RNS_MAXN; ++i) r.c[i] = (uint32_t)powmod64(2, 32ull * i, p);
+    r.p = p;
+    uint32_t inv = p;  // p p = 1 mod 8; each step doubles the correct bits
+    for (int k = 0; k < 4; ++k) inv *= 2u - p * inv;
+    r.ninv = inv;
+    r.pad[0] = r.pad[1] = 0;
+  }
+  T.digits = crt_digits((int)((log2m + 10) / kCrtBits) + 1);
+  const int np = (L + 1) / 2;
+  T.pairs.resize(np);
+  T.rows.assign((size_t)np * T.digits, 0u);
+  T.M32.assign(((size_t)kCrtBits * T.digits + 31) / 32, 0u);
+  for (size_t w = 0; w < T.M32.size() && w < 2 * T.M.size(); ++w) T.M32[w] = (uint32_t)(T.M[w / 2] >> (32 * (w % 2)));
+  for (int j = 0; j < np; ++j) {
+    CrtPair& c = T.pairs[j];
+    const int t1 = 2 * j, t2 = 2 * j + 1;
+    c.p1 = T.primes[t1];
+    c.p2 = t2 < L ? T.primes[t2] : 1u;
+    c.inv = (float)(1.0 / ((double)c.p1 * c.p2));
+    c.w1 = T.wt[t1];
+    c.w2 = t2 < L ? T.wt[t2] : 0u;
+    c.pad = 0;
+    c.mu1 = T.mu[t1];
+    c.mu2 = t2 < L ? T.mu[t2] : 0ull;
+    std::vector<unsigned long long> x(T.MT.begin() + (size_t)t1 * T.WW, T.MT.begin() + (size_t)(t1 + 1) * T.WW);
+    if (t2 < L) {  // M / p1 / p2
+      unsigned __int128 rem = 0;
+      for (int w = T.WW - 1; w >= 0; --w) {
+        rem = (rem << 64) | x[w];
+        x[w] = (unsigned long long)(rem / c.p2);
+        rem %= c.p2;
+      }
+    }
+    for (int d = 0; d < T.digits; ++d) {
+      const int w = kCrtBits * d / 64, off = kCrtBits * d % 64;
+      unsigned long long v = w < T.WW ? x[w] >> off : 0ull;
+      if (off + kCrtBits > 64 && w + 1 < T.WW) v |= x[w + 1] << (64 - off);
+      T.rows[(size_t)j * T.digits + d] = (uint32_t)v & ((1u << kCrtBits) - 1u);
+    }
+  }
   return T;
 }
 
@@ -733,7 +982,11 @@ struct DevTables {
   DevBuf<unsigned long long> mu;
   DevBuf<int> iprimes;
   DevBuf<unsigned long long> M, MT;
+  DevBuf<ResiduePrime> rp;
+  DevBuf<CrtPair> pairs;
+  DevBuf<uint32_t> rows, M32, fac;
   int L = -1;
+  int S = 0;  // shifts covered by the factor table (0: none for this L)
   std::map<int, PrimeTables> host;
   const PrimeTables& get(int bits, int L_, cudaStream_t st) {
     auto it = host.find(L_);
@@ -751,16 +1004,55 @@ struct DevTables {
       iprimes.upload(ip.data(), L_, st);
       M.upload(T.M.data(), T.WW, st);
       MT.upload(T.MT.data(), T.MT.size(), st);
+      if (T.digits) {
+        grow(rp, L_); grow(pairs, T.pairs.size()); grow(rows, T.rows.size()); grow(M32, T.M32.size());
+        rp.upload(T.rp.data(), L_, st);
+        pairs.upload(T.pairs.data(), T.pairs.size(), st);
+        rows.upload(T.rows.data(), T.rows.size(), st);
+        M32.upload(T.M32.data(), T.M32.size(), st);
+      }
       L = L_;
+      S = 0;
     }
     return T;
+  }
+  // The residue factors 2^(s + 64) mod p_t for every shift s < need (built once per prime set; rows
+  // t: plain, L + t: times w_t).
+  void factors(int need, cudaStream_t st) {
+    if (need <= S && S > 0) return;
+    S = (std::max(need, 1) + 255) / 256 * 256;
+    grow(fac, 2 * (size_t)L * S);
+    ++g_launches, k_rns_factors<<<dim3(S / 256, L), 256, 0, st>>>(L, primes, wt, S, fac);
+  }
+  // Digit planes of a view (k_rns8_residues); weighted: the residues carry the CRT weights.
+  void planes(cudaStream_t st, const unsigned char* X, int N, int nlines, int len, long sx, long sy, const int* lo,
+              bool weighted, int8_t* out, int Rpad, int Kld) const {
+    const uint32_t* f = fac.p + (weighted ? (size_t)L * S : 0);
+    auto launch = [&](auto kernel, int E) {
+      const long blocks = ((long)Rpad * (Kld / E) + 255) / 256;
+      // two blocks per SM or more; at least four primes a block, so that loading the entries stays small
+      const int split = (int)std::min<long>(std::max<long>(1, 296 / blocks), std::max(1, L / 4));
+      ++g_launches, kernel<<<dim3((unsigned)blocks, split), 256, 0, st>>>(X, N, nlines, len, sx, sy, lo, L, rp, f, S,
+                                                                          out, Rpad, Kld);
+    };
+    if (N <= 2) launch(k_rns8_residues<4, 4>, 4);
+    else if (N <= 4) launch(k_rns8_residues<8, 4>, 4);
+    else if (N <= 6) launch(k_rns8_residues<12, 4>, 4);
+    else if (N <= 8) launch(k_rns8_residues<16, 4>, 4);
+    else launch(k_rns8_residues<32, 2>, 2);
+  }
+  // CRT of m x n outputs (INT8 form); weights: the residues do not carry the weights yet.
+  void crt(cudaStream_t st, const int* RC, long plane, int m, int n, bool weights, const int* loA, const int* loB,
+           int N, int upper_only, unsigned char* C, uint32_t* status) const {
+    launch_crt(st, host.at(L).digits, RC, plane, m, n, L, pairs, rows, M32, weights ? 1 : 0, loA, loB, N, upper_only, C,
+               status);
   }
 };
 
 struct RnsWorkspace {
   DevBuf<unsigned char> a, b, c;  // staging of the host entry point
   DevBuf<int> loA, loB, bitsA, bitsB, maxbits, err;
-  DevBuf<uint32_t> status, pow2;
+  DevBuf<uint32_t> status;
   DevTables t21, t15;
   DevBuf<double> RA, RB, RC;  // FP64 form
   DevBuf<int8_t> PA, PB;      // INT8 form: digit planes
@@ -828,15 +1120,11 @@ int32_t rns_product(RnsWorkspace& ws, cudaStream_t st, int form, int N, char ta,
     const int Kld = (int)((std::max<uint64_t>(k, 1) + 127) / 128 * 128);
     grow(ws.RC8, (size_t)L * planeC);
     if (k) {
-      const int S = 64 * N + std::max(hb[0], hb[1]) + 1;
-      grow(ws.pow2, (size_t)L * S);
-      ++g_launches, k_rns_pow2<<<dim3((S + 255) / 256, L), 256, 0, st>>>(L, DT.iprimes, S, ws.pow2);
+      DT.factors(std::max(hb[0], hb[1]) - 64 * N + 1, st);
       grow(ws.PA, (size_t)L * 2 * Mpad * Kld);
       grow(ws.PB, (size_t)L * 2 * Npad * Kld);
-      ++g_launches, k_rns8_residues<<<(unsigned)(((long)Mpad * Kld + 255) / 256), 256, 0, st>>>(
-          dA, N, (int)m, (int)k, asx, asy, ws.loA, L, DT.iprimes, DT.mu, ws.pow2, S, ws.PA, Mpad, Kld);
-      ++g_launches, k_rns8_residues<<<(unsigned)(((long)Npad * Kld + 255) / 256), 256, 0, st>>>(
-          dB, N, (int)n, (int)k, bsx, bsy, ws.loB, L, DT.iprimes, DT.mu, ws.pow2, S, ws.PB, Npad, Kld);
+      DT.planes(st, dA, N, (int)m, (int)k, asx, asy, ws.loA, true, ws.PA, Mpad, Kld);
+      DT.planes(st, dB, N, (int)n, (int)k, bsx, bsy, ws.loB, false, ws.PB, Npad, Kld);
       check(cudaMemsetAsync(ws.err.p, 0, sizeof(int), st), "memset");
       for (int k0 = 0; k0 < Kld; k0 += kI8Chunk) {
         I8GemmArgs ga;
@@ -850,9 +1138,7 @@ int32_t rns_product(RnsWorkspace& ws, cudaStream_t st, int form, int N, char ta,
     } else {
       check(cudaMemsetAsync(ws.RC8.p, 0, (size_t)L * planeC * sizeof(int), st), "memset");
     }
-    ++g_launches, launch_crt<int>((unsigned)((m * n + 127) / 128), st, 
-        ws.RC8, planeC, (int)m, (int)n, L, T.WW, DT.primes, DT.wt, DT.pinv, DT.mu, DT.MT, DT.M, ws.loA, ws.loB, N,
-        upper_only ? 1 : 0, dC, ws.status);
+    DT.crt(st, ws.RC8, planeC, (int)m, (int)n, false, ws.loA, ws.loB, N, upper_only ? 1 : 0, dC, ws.status);
   } else {
     const long planeA = (long)(m * std::max<uint64_t>(k, 1)), planeB = (long)(std::max<uint64_t>(k, 1) * n);
     grow(ws.RA, (size_t)L * planeA);
@@ -869,7 +1155,7 @@ int32_t rns_product(RnsWorkspace& ws, cudaStream_t st, int form, int N, char ta,
     } else {
       check(cudaMemsetAsync(ws.RC.p, 0, (size_t)L * planeC * sizeof(double), st), "memset");
     }
-    ++g_launches, launch_crt<double>((unsigned)((m * n + 127) / 128), st, 
+    ++g_launches, launch_crt_f64((unsigned)((m * n + 127) / 128), st,
         ws.RC, planeC, (int)m, (int)n, L, T.WW, DT.primes, DT.wt, DT.pinv, DT.mu, DT.MT, DT.M, ws.loA, ws.loB, N,
         upper_only ? 1 : 0, dC, ws.status);
   }
@@ -939,22 +1225,18 @@ int32_t rns_congruence(RnsWorkspace& ws, cudaStream_t st, int N, char ta, uint64
     return 2;
   }
   DevTables& DT = ws.t15;
-  const PrimeTables& T = DT.get(15, L, st);
+  DT.get(15, L, st);
   const int Mpad = (int)((m + 127) / 128 * 128), Kpad = (int)((k + 127) / 128 * 128);
   const long planeT = (long)(k * m), planeC = (long)(m * m);
   grow(ws.RT8, (size_t)L * planeT);
   grow(ws.RC8, (size_t)L * planeC);
-  const int S = 64 * N + std::max(hb[0], bits_x) + 1;
-  grow(ws.pow2, (size_t)L * S);
-  ++g_launches, k_rns_pow2<<<dim3((S + 255) / 256, L), 256, 0, st>>>(L, DT.iprimes, S, ws.pow2);
+  DT.factors(std::max(hb[0], bits_x) - 64 * N + 1, st);
   grow(ws.PA, (size_t)L * 2 * Mpad * Kpad);  // A~ (rows of op(A)), used by both products
   grow(ws.PB, (size_t)L * 2 * (size_t)std::max(Kpad, Mpad) * Kpad);
-  ++g_launches, k_rns8_residues<<<(unsigned)(((long)Mpad * Kpad + 255) / 256), 256, 0, st>>>(
-      dA, N, (int)m, (int)k, asx, asy, ws.loA, L, DT.iprimes, DT.mu, ws.pow2, S, ws.PA, Mpad, Kpad);
+  DT.planes(st, dA, N, (int)m, (int)k, asx, asy, ws.loA, false, ws.PA, Mpad, Kpad);
   ++g_launches, k_fill_int<<<(unsigned)((k + 255) / 256), 256, 0, st>>>(ws.loX, (int)k, (int)lo_x);
-  // X~ by rows (line r: entries (r, c)): the left operand of T = X~ A~'
-  ++g_launches, k_rns8_residues<<<(unsigned)(((long)Kpad * Kpad + 255) / 256), 256, 0, st>>>(
-      dX, N, (int)k, (int)k, 1, (long)ldx, ws.loX, L, DT.iprimes, DT.mu, ws.pow2, S, ws.PB, Kpad, Kpad);
+  // X~ by rows (line r: entries (r, c)): the left operand of T = X~ A~'; it carries the CRT weights
+  DT.planes(st, dX, N, (int)k, (int)k, 1, (long)ldx, ws.loX, true, ws.PB, Kpad, Kpad);
   check(cudaMemsetAsync(ws.err.p, 0, sizeof(int), st), "memset");
   for (int k0 = 0; k0 < Kpad; k0 += kI8Chunk) {  // T (k x m) = X~ A~'
     I8GemmArgs ga;
@@ -974,9 +1256,7 @@ int32_t rns_congruence(RnsWorkspace& ws, cudaStream_t st, int N, char ta, uint64
     launch_i8_gemm(2, ws.PA, ws.PB, ga, st);
   }
   ++g_launches, k_add_const_int<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(ws.loA, (int)m, (int)lo_x, ws.loB2);
-  ++g_launches, launch_crt<int>((unsigned)((m * m + 127) / 128), st, 
-      ws.RC8, planeC, (int)m, (int)m, L, T.WW, DT.primes, DT.wt, DT.pinv, DT.mu, DT.MT, DT.M, ws.loA, ws.loB2, N,
-      upper_only ? 1 : 0, dC, ws.status);
+  DT.crt(st, ws.RC8, planeC, (int)m, (int)m, false, ws.loA, ws.loB2, N, upper_only ? 1 : 0, dC, ws.status);
   check(cudaGetLastError(), "congruence launch");
   int herr = 0;
   copy_d2h(&hs, ws.status.p, sizeof(uint32_t), st);
@@ -1028,14 +1308,12 @@ int ceil_log2(uint64_t v) {
 }
 
 // CRT of `count` outputs (residues ws.RC8[t * count + o]) at exponent `lo` into dOut.
-void crt_vector(RnsWorkspace& ws, cudaStream_t st, DevTables& DT, const PrimeTables& T, int N, int L, int count,
-                int lo, unsigned char* dOut) {
+void crt_vector(RnsWorkspace& ws, cudaStream_t st, DevTables& DT, int N, int count, int lo,
+                unsigned char* dOut) {
   grow(ws.loA, count); grow(ws.loB, 1);
   ++g_launches, k_fill_int<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(ws.loA, count, lo);
   ++g_launches, k_fill_int<<<1, 32, 0, st>>>(ws.loB, 1, 0);
-  ++g_launches, launch_crt<int>((unsigned)((count + 127) / 128), st, 
-      ws.RC8, count, count, 1, L, T.WW, DT.primes, DT.wt, DT.pinv, DT.mu, DT.MT, DT.M, ws.loA, ws.loB, N, 0, dOut,
-      ws.status);
+  DT.crt(st, ws.RC8, count, count, 1, true, ws.loA, ws.loB, N, 0, dOut, ws.status);
 }
 
 // The residue tables of the classes: class c's residues at ws.cres + off[c] * L (count[c] per prime).
@@ -1047,13 +1325,11 @@ void class_residues(RnsWorkspace& ws, cudaStream_t st, DevTables& DT, int N, int
     total += (size_t)std::max(count[c], 1);
   }
   grow(ws.cres, total * L);
-  const int S = 64 * N + maxbits + 1;
-  grow(ws.pow2, (size_t)L * S);
-  ++g_launches, k_rns_pow2<<<dim3((S + 255) / 256, L), 256, 0, st>>>(L, DT.iprimes, S, ws.pow2);
+  DT.factors(maxbits - 64 * N + 1, st);
   for (int c = 0; c < n; ++c)
     if (count[c])
       ++g_launches, k_rns_class_residues<<<(unsigned)((count[c] + 127) / 128), 128, 0, st>>>(
-          arr[c], N, count[c], lo[c], absval[c], L, DT.iprimes, DT.mu, ws.pow2, S, ws.cres.p + off[c] * L);
+          arr[c], N, count[c], lo[c], absval[c], L, DT.rp, DT.fac, DT.S, ws.cres.p + off[c] * L);
 }
 
 // v[k] = sum_{i <= j} c_ij x_tri(j)+i q_ik q_jk (c_ii = 1, c_ij = sqrt2), k < kmax, each rounded
@@ -1077,14 +1353,14 @@ int32_t rns_svec_quadratic(RnsWorkspace& ws, cudaStream_t st, int N, int h, int 
     return 2;
   }
   DevTables& DT = ws.t15;
-  const PrimeTables& T = DT.get(15, L, st);
+  DT.get(15, L, st);
   size_t off[3];
   const int absv[3] = {abs_q, 0, 0};
   class_residues(ws, st, DT, N, L, arr, count, lo, absv, 3, std::max(bits[0], std::max(bits[1], bits[2])), off);
   grow(ws.RC8, (size_t)L * kmax);
   ++g_launches, k_rns_svec_quadratic<<<dim3((unsigned)((kmax + 63) / 64), (unsigned)L), 64, 0, st>>>(
       h, kmax, ws.cres.p + off[1] * L, ws.cres.p + off[0] * L, ws.cres.p + off[2] * L, L, DT.iprimes, ws.RC8);
-  crt_vector(ws, st, DT, T, N, L, kmax, 2 * lo[0] + lo[1] + lo[2], dOut);
+  crt_vector(ws, st, DT, N, kmax, 2 * lo[0] + lo[1] + lo[2], dOut);
   check(cudaGetLastError(), "svec_quadratic launch");
   copy_d2h(&hs, ws.status.p, sizeof(uint32_t), st);
   check(cudaStreamSynchronize(st), "sync");
@@ -1112,14 +1388,14 @@ int32_t rns_bilinear(RnsWorkspace& ws, cudaStream_t st, int N, int h, int cols, 
     return 2;
   }
   DevTables& DT = ws.t15;
-  const PrimeTables& T = DT.get(15, L, st);
+  DT.get(15, L, st);
   size_t off[2];
   const int absv[2] = {0, 0};
   class_residues(ws, st, DT, N, L, arr, count, lo, absv, 2, std::max(bits[0], bits[1]), off);
   grow(ws.RC8, (size_t)L * np);
   ++g_launches, k_rns_bilinear<<<dim3((unsigned)((np + 63) / 64), (unsigned)L), 64, 0, st>>>(
       h, cols, ws.cres.p + off[1] * L, ws.cres.p + off[0] * L, dPairs, np, L, DT.iprimes, ws.RC8);
-  crt_vector(ws, st, DT, T, N, L, np, 2 * lo[0] + lo[1], dOut);
+  crt_vector(ws, st, DT, N, np, 2 * lo[0] + lo[1], dOut);
   check(cudaGetLastError(), "symmetric_bilinear launch");
   copy_d2h(&hs, ws.status.p, sizeof(uint32_t), st);
   check(cudaStreamSynchronize(st), "sync");
@@ -1163,18 +1439,16 @@ int32_t rns_diag_congruence(RnsWorkspace& ws, cudaStream_t st, int N, uint64_t m
     return 2;
   }
   DevTables& DT = ws.t15;
-  const PrimeTables& T = DT.get(15, L, st);
+  DT.get(15, L, st);
   const int Mpad = (int)((m + 127) / 128 * 128), Kpad = (int)((k + 127) / 128 * 128);
   const long planeC = (long)(m * m);
   grow(ws.RC8, (size_t)L * planeC);
   size_t off[1];
   const int absv[1] = {0};
   class_residues(ws, st, DT, N, L, arr, count, &lo_d, absv, 1, std::max(hb[0], bits_d), off);
-  const int S = 64 * N + std::max(hb[0], bits_d) + 1;  // the table class_residues just built
   grow(ws.PA, (size_t)L * 2 * Mpad * Kpad);
   grow(ws.PB, (size_t)L * 2 * Mpad * Kpad);
-  ++g_launches, k_rns8_residues<<<(unsigned)(((long)Mpad * Kpad + 255) / 256), 256, 0, st>>>(
-      dA, N, (int)m, (int)k, (long)lda, 1, ws.loA, L, DT.iprimes, DT.mu, ws.pow2, S, ws.PA, Mpad, Kpad);
+  DT.planes(st, dA, N, (int)m, (int)k, (long)lda, 1, ws.loA, false, ws.PA, Mpad, Kpad);
   ++g_launches, k_rns8_scale_planes<<<(unsigned)(((long)Mpad * Kpad + 255) / 256), 256, 0, st>>>(
       ws.PA, ws.cres.p + off[0] * L, (int)k, L, DT.iprimes, ws.PB, Mpad, Kpad);
   check(cudaMemsetAsync(ws.err.p, 0, sizeof(int), st), "memset");
@@ -1186,9 +1460,7 @@ int32_t rns_diag_congruence(RnsWorkspace& ws, cudaStream_t st, int N, uint64_t m
     launch_i8_gemm(2, ws.PA, ws.PB, ga, st);
   }
   ++g_launches, k_add_const_int<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(ws.loA, (int)m, lo_d, ws.loB2);
-  ++g_launches, launch_crt<int>((unsigned)((m * m + 127) / 128), st, 
-      ws.RC8, planeC, (int)m, (int)m, L, T.WW, DT.primes, DT.wt, DT.pinv, DT.mu, DT.MT, DT.M, ws.loA, ws.loB2, N,
-      upper_only ? 1 : 0, dC, ws.status);
+  DT.crt(st, ws.RC8, planeC, (int)m, (int)m, true, ws.loA, ws.loB2, N, upper_only ? 1 : 0, dC, ws.status);
   check(cudaGetLastError(), "diag_congruence launch");
   int herr = 0;
   copy_d2h(&hs, ws.status.p, sizeof(uint32_t), st);
