@@ -3,7 +3,7 @@
 //
 // Factorisation H + eps I = U'U (upper), right-looking over 64 x 64 tiles
 // (kkt/ldl/dense_block.rs:334-365 potrf_dynamic, 370-388 potrf_tile, 515-594 tiled_potrf):
-//   k_potrf_diag   factor the diagonal tile with the dynamic pivot rule; store Dinv = U_kk^-1
+//   k_potrf_diag   factor the diagonal tile with the dynamic pivot rule; store Dinv = U_kk^-T
 //   k_trsm_panel   U[k, j] = U_kk^-T H[k, j] for the tiles right of the diagonal
 //   k_syrk_update  H[i, j] -= U[k, i]' U[k, j] on the upper trailing tiles
 // Inverse X = U^-1, recursive over tile groups: with U = [U11 U12; 0 U22],
@@ -20,7 +20,7 @@
 
 // F = Hsave + eps I (copy), diag0 = diag(F).
 extern "C" __global__ void k_shifted_copy(const double* __restrict__ Hs, double* __restrict__ F,
-                                          int m, double eps, double* __restrict__ diag0) {
+                                          long ldf, int m, double eps, double* __restrict__ diag0) {
   long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   long total = (long)m * m;
   for (; idx < total; idx += (long)gridDim.x * blockDim.x) {
@@ -30,7 +30,7 @@ extern "C" __global__ void k_shifted_copy(const double* __restrict__ Hs, double*
       v += eps;
       diag0[i] = v;
     }
-    F[idx] = v;
+    F[i + j * ldf] = v;
   }
 }
 
@@ -82,10 +82,10 @@ __device__ __forceinline__ void potrf_pivot(double d, const double* diag, int nb
   info[2] = 1.0 / r;
 }
 
-// Diagonal tile: lagged upper Cholesky with the dynamic pivot rule, then Dinv = U^-1.
+// Diagonal tile: lagged upper Cholesky with the dynamic pivot rule, then Dinv = U^-T.
 // Dynamic shared memory: two CH_NB x CH_LD tiles.
 extern "C" __global__ void __launch_bounds__(1024)
-k_potrf_diag(double* __restrict__ H, int m, int kb, double eps, double delta, int dynamic,
+k_potrf_diag(double* __restrict__ H, long ld, int m, int kb, double eps, double delta, int dynamic,
              const double* __restrict__ diag0, double* __restrict__ Dinv,
              uint32_t* __restrict__ status) {
   extern __shared__ double pd_sm[];
@@ -108,7 +108,7 @@ k_potrf_diag(double* __restrict__ H, int m, int kb, double eps, double delta, in
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       int i = tx + 32 * p, j = ty + 32 * q;
-      a[p][q] = (i <= j && j < nb) ? H[(k0 + i) + (long)(k0 + j) * m] : 0.0;
+      a[p][q] = (i <= j && j < nb) ? H[(k0 + i) + (long)(k0 + j) * ld] : 0.0;
       mm[p][q] = (i == j) ? 1.0 : 0.0;
       if (i == 0 && j < nb) rowbuf[0][j] = a[p][q];
       if (i == 0) mrowbuf[0][j] = (j == 0) ? 1.0 : 0.0;
@@ -157,9 +157,9 @@ k_potrf_diag(double* __restrict__ H, int m, int kb, double eps, double delta, in
   __syncthreads();
   for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
     int i = e % nb, j = e / nb;
-    if (i <= j) H[(k0 + i) + (long)(k0 + j) * m] = A[i + j * CH_LD];
+    if (i <= j) H[(k0 + i) + (long)(k0 + j) * ld] = A[i + j * CH_LD];
   }
-  // Dinv = U^-1 = L^-T D^-1/2: Dinv[c][i] = M[i][c] / sqrt(d_i) (upper, zero elsewhere)
+  // Dinv = U^-T = D^-1/2 L^-1: Dinv[i][c] = M[i][c] / sqrt(d_i) (lower, zero elsewhere)
   double* D = Dinv + (long)kb * CH_NB * CH_NB;
 #pragma unroll
   for (int p = 0; p < 2; ++p)
@@ -167,13 +167,13 @@ k_potrf_diag(double* __restrict__ H, int m, int kb, double eps, double delta, in
     for (int q = 0; q < 2; ++q) {
       const int i = tx + 32 * p, c = ty + 32 * q;
       const bool live = (i >= c && i < nb);
-      D[c + i * CH_NB] = live ? mm[p][q] / root[i] : 0.0;
+      D[i + c * CH_NB] = live ? mm[p][q] / root[i] : 0.0;
     }
 }
 
 // ------------------------------------------------------------------------------------
 extern "C" __global__ void __launch_bounds__(SDPXG_THREADS)
-k_trsm_panel(double* __restrict__ H, int m, int kb, const double* __restrict__ Dinv) {
+k_trsm_panel(double* __restrict__ H, long ld, int m, int kb, const double* __restrict__ Dinv) {
   extern __shared__ double sm[];
   double* D = sm;                 // CH_NB x CH_LD
   double* P = D + CH_NB * CH_LD;  // CH_NB x CH_LD
@@ -182,10 +182,10 @@ k_trsm_panel(double* __restrict__ H, int m, int kb, const double* __restrict__ D
   const int c0 = cb * CH_NB, nc = min(CH_NB, m - c0);
   const double* Dg = Dinv + (long)kb * CH_NB * CH_NB;
   for (int e = threadIdx.x; e < CH_NB * CH_NB; e += blockDim.x)
-    D[(e % CH_NB) + (e / CH_NB) * CH_LD] = Dg[e];
+    D[(e / CH_NB) + (e % CH_NB) * CH_LD] = Dg[e];  // U_kk^-1 from its transpose
   for (int e = threadIdx.x; e < nb * nc; e += blockDim.x) {
     int i = e % nb, c = e / nb;
-    P[i + c * CH_LD] = H[(k0 + i) + (long)(c0 + c) * m];
+    P[i + c * CH_LD] = H[(k0 + i) + (long)(c0 + c) * ld];
   }
   for (int e = threadIdx.x; e < CH_NB * CH_NB; e += blockDim.x) {  // zero the ragged edge
     int i = e % CH_NB, c = e / CH_NB;
@@ -215,7 +215,7 @@ k_trsm_panel(double* __restrict__ H, int m, int kb, const double* __restrict__ D
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       int i = tx + 16 * a, c = ty + 16 * b;
-      if (i < nb && c < nc) H[(k0 + i) + (long)(c0 + c) * m] = acc[a][b];
+      if (i < nb && c < nc) H[(k0 + i) + (long)(c0 + c) * ld] = acc[a][b];
     }
 }
 
@@ -223,7 +223,7 @@ k_trsm_panel(double* __restrict__ H, int m, int kb, const double* __restrict__ D
 // Trailing update on upper tiles; blockIdx.x enumerates (ib <= jb) over the T x T trailing
 // tile grid in column order.
 extern "C" __global__ void __launch_bounds__(SDPXG_THREADS)
-k_syrk_update(double* __restrict__ H, int m, int kb) {
+k_syrk_update(double* __restrict__ H, long ld, int m, int kb) {
   extern __shared__ double syrk_sm[];
   double (*Ui)[CH_NB + 2] = reinterpret_cast<double (*)[CH_NB + 2]>(syrk_sm);
   double (*Uj)[CH_NB + 2] = reinterpret_cast<double (*)[CH_NB + 2]>(syrk_sm + CH_NB * (CH_NB + 2));
@@ -239,8 +239,8 @@ k_syrk_update(double* __restrict__ H, int m, int kb) {
   const int j0 = jb * CH_NB, nj = min(CH_NB, m - j0);
   for (int e = threadIdx.x; e < CH_NB * CH_NB; e += blockDim.x) {
     int l = e % CH_NB, c = e / CH_NB;
-    Ui[l][c] = (l < nb && c < ni) ? H[(k0 + l) + (long)(i0 + c) * m] : 0.0;
-    Uj[l][c] = (l < nb && c < nj) ? H[(k0 + l) + (long)(j0 + c) * m] : 0.0;
+    Ui[l][c] = (l < nb && c < ni) ? H[(k0 + l) + (long)(i0 + c) * ld] : 0.0;
+    Uj[l][c] = (l < nb && c < nj) ? H[(k0 + l) + (long)(j0 + c) * ld] : 0.0;
   }
   __syncthreads();
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
@@ -265,12 +265,12 @@ k_syrk_update(double* __restrict__ H, int m, int kb) {
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       int r = tx + 16 * a, c = ty + 16 * b;
-      if (r < ni && c < nj && (ib < jb || r <= c)) H[(i0 + r) + (long)(j0 + c) * m] -= acc[a][b];
+      if (r < ni && c < nj && (ib < jb || r <= c)) H[(i0 + r) + (long)(j0 + c) * ld] -= acc[a][b];
     }
 }
 
 // ------------------------------------------------------------------------------------
-// Inverse of the factor.  Diagonal tiles: X_ii = Dinv_i (stored in Uinv and, transposed, UinvT).
+// Inverse of the factor.  Diagonal tiles: X_ii = Dinv_i' (stored in Uinv and, transposed, UinvT).
 extern "C" __global__ void k_trtri_diag(int m, const double* __restrict__ Dinv,
                                         double* __restrict__ Uinv, double* __restrict__ UinvT) {
   const int ib = blockIdx.x;
@@ -278,9 +278,9 @@ extern "C" __global__ void k_trtri_diag(int m, const double* __restrict__ Dinv,
   const double* D = Dinv + (long)ib * CH_NB * CH_NB;
   for (int e = threadIdx.x; e < ni * ni; e += blockDim.x) {
     int r = e % ni, c = e / ni;
-    double v = D[r + c * CH_NB];  // zero below the diagonal
-    Uinv[(i0 + r) + (long)(i0 + c) * m] = v;
-    UinvT[(i0 + c) + (long)(i0 + r) * m] = v;
+    double v = D[r + c * CH_NB];  // U^-T(r, c), zero above the diagonal
+    UinvT[(i0 + r) + (long)(i0 + c) * m] = v;
+    Uinv[(i0 + c) + (long)(i0 + r) * m] = v;
   }
 }
 
@@ -304,7 +304,7 @@ __device__ __forceinline__ void cp_async_wait() {
 // masked or out of range) while the tensor cores work on the current one.
 // Dynamic shared memory: two stages of two tiles.
 extern "C" __global__ void __launch_bounds__(SDPXG_THREADS)
-k_trinv_level(const double* __restrict__ F, double* __restrict__ Uinv, double* __restrict__ UinvT,
+k_trinv_level(const double* __restrict__ F, long ldf, double* __restrict__ Uinv, double* __restrict__ UinvT,
               double* __restrict__ Tmp, int n, int level, int phase) {
   extern __shared__ double tl_sm[];
   const int g = 1 << level, h = g >> 1;
@@ -318,6 +318,7 @@ k_trinv_level(const double* __restrict__ F, double* __restrict__ Uinv, double* _
   const double* A;
   const double* B;
   int ar, ac, br, bc, K;
+  const long lda = phase == 0 ? ldf : n;
   if (phase == 0) {
     A = F; ar = L0; ac = R0; B = Uinv; br = R0; bc = R0; K = Rn;
   } else {
@@ -335,7 +336,7 @@ k_trinv_level(const double* __restrict__ F, double* __restrict__ Uinv, double* _
       const int r = e % CH_NB, k = e / CH_NB;
       const int gr = ar + tm * CH_NB + r, gc = ac + k0 + k;
       const bool in = (tm * CH_NB + r < Ln) && (k0 + k < K) && !(phase == 1 && gr > gc);
-      cp_async8(As + r + k * TI_LD, in ? A + gr + (long)gc * n : A, in);
+      cp_async8(As + r + k * TI_LD, in ? A + gr + gc * lda : A, in);
       const int hr = br + k0 + r, hc = bc + tn * CH_NB + k;
       const bool inb = (k0 + r < K) && (tn * CH_NB + k < Rn) && !(phase == 0 && hr > hc);
       cp_async8(Bs + r + k * TI_LD, inb ? B + hr + (long)hc * n : B, inb);

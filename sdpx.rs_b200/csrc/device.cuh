@@ -221,9 +221,9 @@ __global__ void k_op_adjoint_partial(const BlockDesc*, const int*, const int*, c
                                      long, int);
 __global__ void k_op_adjoint_gather(int, const int*, const int*, const int*, const int*,
                                     const double*, long, double, double, double*, long);
-__global__ void k_potrf_diag(double*, int, int, double, double, int, const double*, double*,
+__global__ void k_potrf_diag(double*, long, int, int, double, double, int, const double*, double*,
                              uint32_t*);
-__global__ void k_trsm_panel(double*, int, int, const double*);
+__global__ void k_trsm_panel(double*, long, int, int, const double*);
 __global__ void k_gram_basis(const BlockDesc*, const int*, const int*, const int*, const long*,
                              const double*, const double*, double*);
 __global__ void k_gram_schur(const BlockDesc*, const int*, const int*, const int*, const long*,
@@ -233,13 +233,13 @@ __global__ void k_gram_forward(const BlockDesc*, const int*, const int*, const i
                                const double*, double, double, double*, double*, unsigned*);
 __global__ void k_gram_adjoint(const BlockDesc*, const int*, const int*, const int*, const int*,
                                const long*, const double*, const double*, const double*, double*);
-__global__ void k_chol_dataflow(double*, int, int, const unsigned*, int, int*, double, double, int,
+__global__ void k_chol_dataflow(double*, long, int, int, const unsigned*, int, int*, double, double, int,
                                 const double*, double*, uint32_t*);
-__global__ void k_syrk_update(double*, int, int);
+__global__ void k_syrk_update(double*, long, int, int);
 __global__ void k_trtri_diag(int, const double*, double*, double*);
-__global__ void k_trinv_level(const double*, double*, double*, double*, int, int, int);
+__global__ void k_trinv_level(const double*, long, double*, double*, double*, int, int, int);
 __global__ void k_tri_colgemv(const double*, int, int, const double*, double*);
-__global__ void k_shifted_copy(const double*, double*, int, double, double*);
+__global__ void k_shifted_copy(const double*, double*, long, int, double, double*);
 __global__ void k_strided_diag(const double*, long, int, double, double*);
 __global__ void k_transpose_block(const double*, long, int, int, double*, long);
 __global__ void k_symv_cols(const double*, int, const double*, const double*, double*);

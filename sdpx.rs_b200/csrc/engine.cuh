@@ -41,8 +41,9 @@ constexpr size_t kSmemTrsm = 2 * 64 * 65 * sizeof(double);
 constexpr size_t kSmemSyrk = 2 * 64 * 66 * sizeof(double);
 constexpr size_t kSmemTrtri = 2 * 64 * 65 * sizeof(double);
 constexpr size_t kSmemTrinv = 4 * 64 * 68 * sizeof(double);  // k_trinv_level: 2 stages x 2 tiles
-constexpr size_t kSmemDf = (3 * 64 * 68 + 2 * 8 * 64) * sizeof(double);  // k_chol_dataflow
+constexpr size_t kSmemDf = (4 * 64 * 68 + 2 * 64) * sizeof(double);  // k_chol_dataflow
 constexpr size_t kSmemGram = 3 * kMatD * sizeof(double);                 // k_gram_basis/adjoint
+constexpr int kDfThreads = 320;    // k_chol_dataflow: 8 MMA warps, one loading, one publishing
 constexpr int kDfMaxTiles = 256;  // dataflow schedule up to m = 16384 (nt^3/6 items)
 
 // Rank-one test of one PSD column block: svec v (upper, column order, off-diagonal x sqrt2) of
@@ -89,25 +90,24 @@ inline bool rank_one_column(const double* v, int n, double* u, double* sigma) {
   return true;
 }
 
-// Work list of the dataflow Cholesky (k_chol_dataflow): POTRF(k), TRSM(k, j), GEMM(k, i, j) of
-// the right-looking tiled algorithm in a topological order with one step of look-ahead: the
-// update of tile row k + 1, POTRF(k + 1) and its TRSM row come before the rest of step k's
-// trailing update.  Encoded type << 30 | k << 20 | i << 10 | j.
+// Work list of the dataflow Cholesky (k_chol_dataflow), tile row by tile row after the chain
+// (ticket 0: every POTRF(k), TRSM(k, k+1) and the update of tile (k+1, k+1) by row k):
+//   PRE(i, i) (i >= 2): the sums of rows < i - 1 of the diagonal tile; PRE(i, i+1) (i >= 1): the sums
+//   of rows < i of the tile right of it; FULL(i, j >= i + 2): the whole tile U(i, j).
+// The PRE items of a row come first: the chain waits for them.
+// Encoded type << 30 | k << 20 | i << 10 | j with k the number of rows an item sums over.
+enum : unsigned { kCholFull = 1u, kCholPre = 2u, kCholChain = 3u };
 inline std::vector<unsigned> chol_schedule(int nt) {
   auto code = [](unsigned type, int k, int i, int j) {
     return (type << 30) | ((unsigned)k << 20) | ((unsigned)i << 10) | (unsigned)j;
   };
   std::vector<unsigned> it;
   if (nt <= 0) return it;
-  // ticket 0: the critical-path chain (every POTRF(k), TRSM(k, k+1) and GEMM(k, k+1, k+1))
-  it.push_back(code(3u, 0, 0, 0));
-  // then step by step the rest of each step: the TRSM row beyond k + 1, and the trailing
-  // updates row by row (rows k + 1 and k + 2 first feed the chain's next two steps)
-  for (int k = 0; k + 1 < nt; ++k) {
-    for (int j = k + 2; j < nt; ++j) it.push_back(code(1u, k, k, j));
-    for (int i = k + 1; i < nt; ++i)
-      for (int j = i; j < nt; ++j)
-        if (!(i == k + 1 && j == k + 1)) it.push_back(code(2u, k, i, j));
+  it.push_back(code(kCholChain, 0, 0, 0));
+  for (int i = 0; i < nt; ++i) {
+    if (i >= 2) it.push_back(code(kCholPre, i - 1, i, i));
+    if (i >= 1 && i + 1 < nt) it.push_back(code(kCholPre, i, i, i + 1));
+    for (int j = i + 2; j < nt; ++j) it.push_back(code(kCholFull, i, i, j));
   }
   return it;
 }
@@ -117,24 +117,22 @@ inline std::vector<unsigned> chol_schedule(int nt) {
 // which k_chol_dataflow cannot deadlock (the chain, ticket 0, only waits on items that precede
 // every item waiting on it) -- and that every tile ends factored.  False on any violation.
 inline bool chol_schedule_valid(const std::vector<unsigned>& it, int nt) {
-  std::vector<int> upd((size_t)nt * nt, 0), fin((size_t)nt * nt, 0);
-  auto U = [&](int i, int j) -> int& { return upd[(size_t)i * nt + j]; };
-  auto Fn = [&](int i, int j) -> int& { return fin[(size_t)i * nt + j]; };
+  std::vector<int> prog(nt, 0), pre_d(nt, 0), pre_o(nt, 0);  // the kernel's progress words
   bool chain = false;
-  int step = 0;          // next chain step
+  int step = 0;            // next chain step
   bool diag_done = false;  // the chain's POTRF of `step` is done, its TRSM is pending
   auto advance = [&]() {
     while (chain && step < nt) {
       const int s = step;
       if (!diag_done) {
-        if (s > 0 && (U(s, s) != s - 1 || !Fn(s - 1, s))) return;  // GEMM(s-1, s, s) inputs
-        U(s, s) = s;
-        Fn(s, s) = 1;
+        if (prog[s] != s || (s >= 2 && !pre_d[s])) return;  // U(s-1, s) is the chain's own
+        prog[s] = s + 1;
         diag_done = true;
       }
       if (s + 1 < nt) {
-        if (U(s, s + 1) != s) return;  // TRSM(s, s+1) input
-        Fn(s, s + 1) = 1;
+        if (s >= 1 && !pre_o[s]) return;
+        if (prog[s + 1] != s) return;
+        prog[s + 1] = s + 1;
       }
       diag_done = false;
       ++step;
@@ -142,32 +140,34 @@ inline bool chol_schedule_valid(const std::vector<unsigned>& it, int nt) {
   };
   for (size_t t = 0; t < it.size(); ++t) {
     const unsigned c = it[t];
-    const int type = (int)(c >> 30), k = (int)((c >> 20) & 1023u);
-    const int i = (int)((c >> 10) & 1023u), j = (int)(c & 1023u);
+    const unsigned type = c >> 30;
+    const int k = (int)((c >> 20) & 1023u), i = (int)((c >> 10) & 1023u), j = (int)(c & 1023u);
     if (k >= nt || i >= nt || j >= nt) return false;
-    if (type == 3) {
+    if (type == kCholChain) {
       if (t != 0 || chain) return false;
       chain = true;
       advance();
       continue;
     }
     advance();
-    if (type == 1) {
-      if (i != k || j <= k + 1 || !Fn(k, k) || U(k, j) != k) return false;
-      Fn(k, j) = 1;
-    } else if (type == 2) {
-      if (i <= k || j < i || (i == k + 1 && j == k + 1) || !Fn(k, i) || !Fn(k, j) || U(i, j) != k)
-        return false;
-      U(i, j) = k + 1;
+    if (prog[i] < k || prog[j] < k) return false;  // the rows an item sums over are final
+    if (type == kCholFull) {
+      if (k != i || j < i + 2 || prog[i] != i + 1 || prog[j] != i) return false;
+      prog[j] = i + 1;
+    } else if (type == kCholPre && i == j) {
+      if (i < 2 || k != i - 1 || pre_d[i]) return false;
+      pre_d[i] = 1;
+    } else if (type == kCholPre) {
+      if (i < 1 || j != i + 1 || k != i || pre_o[i]) return false;
+      pre_o[i] = 1;
     } else {
       return false;
     }
   }
   advance();
   if (!chain || step != nt) return false;
-  for (int i = 0; i < nt; ++i)
-    for (int j = i; j < nt; ++j)
-      if (!Fn(i, j) || U(i, j) != i) return false;
+  for (int j = 0; j < nt; ++j)
+    if (prog[j] != j + 1) return false;
   return true;
 }
 constexpr int kNB = 64;
@@ -735,7 +735,7 @@ class Engine {
     adj_part_.alloc(std::max<size_t>((size_t)ncol_ * 2, 1));
     nchol = (n + kNB - 1) / kNB;
     Hsave_.alloc((size_t)n * n);
-    F_.alloc((size_t)n * n);
+    F_.alloc((size_t)factor_ld(n) * n);
     Dinv_.alloc((size_t)std::max(nchol, 1) * kNB * kNB);
     diag0_.alloc(std::max(n, 1));
     tri_y_.alloc(std::max(n, 1));
@@ -1042,6 +1042,7 @@ class Engine {
   // and its transpose, a GEMM scratch, and the dataflow work list.
   struct FactorBufs {
     int n = 0, nchol = 0, df_items = 0, df_grid = 0;
+    long ldf = 0;  // leading dimension of F: even, so that tile columns start on 16 bytes
     const double* H = nullptr;
     double *F = nullptr, *Dinv = nullptr, *diag0 = nullptr, *Uinv = nullptr, *UinvT = nullptr, *Tmp = nullptr;
     const unsigned* df_list = nullptr;
@@ -1065,7 +1066,7 @@ class Engine {
     if (!chol_schedule_valid(items, nt)) throw CudaError("invalid Cholesky work list");
     list.alloc(items.size());
     list.upload(items.data(), items.size(), st);
-    sync.alloc(2 + 2 * (size_t)nt * nt);
+    sync.alloc(2 + 3 * (size_t)nt);
     int sms = 0;
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "SM count");
     // one CTA per SM: the chain CTA (the critical path) then has its SM to itself; the
@@ -1074,9 +1075,10 @@ class Engine {
     *grid_out = std::max(1, std::min(sms, *items_out));
   }
 
+  static long factor_ld(int rows) { return rows + (rows & 1); }
   FactorBufs full_bufs() {
     FactorBufs b;
-    b.n = n; b.nchol = nchol; b.df_items = df_items_; b.df_grid = df_grid_;
+    b.n = n; b.nchol = nchol; b.df_items = df_items_; b.df_grid = df_grid_; b.ldf = factor_ld(n);
     b.H = Hsave_; b.F = F_; b.Dinv = Dinv_; b.diag0 = diag0_; b.Uinv = Uinv_; b.UinvT = UinvT_; b.Tmp = Tmp_;
     b.df_list = df_list_; b.df_sync = df_sync_;
     return b;
@@ -1085,7 +1087,7 @@ class Engine {
   void setup_sub(SubFactor& s, int ns) {
     const int nt = (ns + kNB - 1) / kNB;
     s.H.alloc((size_t)ns * ns);
-    s.F.alloc((size_t)ns * ns);
+    s.F.alloc((size_t)factor_ld(ns) * ns);
     s.Dinv.alloc((size_t)nt * kNB * kNB);
     s.diag0.alloc(ns);
     s.Uinv.alloc((size_t)ns * ns);
@@ -1094,6 +1096,7 @@ class Engine {
     s.b = FactorBufs();
     s.b.n = ns;
     s.b.nchol = nt;
+    s.b.ldf = factor_ld(ns);
     make_schedule(nt, s.df_list, s.df_sync, &s.b.df_items, &s.b.df_grid);
     s.b.H = s.H; s.b.F = s.F; s.b.Dinv = s.Dinv; s.b.diag0 = s.diag0; s.b.Uinv = s.Uinv;
     s.b.UinvT = s.UinvT; s.b.Tmp = s.Tmp; s.b.df_list = s.df_list; s.b.df_sync = s.df_sync;
@@ -1110,23 +1113,23 @@ class Engine {
   // original diagonal is taken from there (+ eps) instead of from H.
   void launch_chol(const FactorBufs& b, double eps, bool dynamic, double dyn_eps, double dyn_delta,
                    const double* diag_src = nullptr, long diag_stride = 0) {
-    ++g_launches, k_shifted_copy<<<1184, 256, 0, st>>>(b.H, b.F, b.n, eps, b.diag0);
+    ++g_launches, k_shifted_copy<<<1184, 256, 0, st>>>(b.H, b.F, b.ldf, b.n, eps, b.diag0);
     if (diag_src)
       ++g_launches, k_strided_diag<<<(b.n + 255) / 256, 256, 0, st>>>(diag_src, diag_stride, b.n, eps, b.diag0);
     if (b.df_items > 0) {  // one persistent launch over the whole tile schedule
-      check(cudaMemsetAsync(b.df_sync, 0, (2 + 2 * (size_t)b.nchol * b.nchol) * sizeof(int), st),
+      check(cudaMemsetAsync(b.df_sync, 0, (2 + 3 * (size_t)b.nchol) * sizeof(int), st),
             "dataflow sync reset");
-      ++g_launches, k_chol_dataflow<<<b.df_grid, 256, kSmemDf, st>>>(
-          b.F, b.n, b.nchol, b.df_list, b.df_items, b.df_sync, dyn_eps, dyn_delta, dynamic ? 1 : 0, b.diag0,
+      ++g_launches, k_chol_dataflow<<<b.df_grid, kDfThreads, kSmemDf, st>>>(
+          b.F, b.ldf, b.n, b.nchol, b.df_list, b.df_items, b.df_sync, dyn_eps, dyn_delta, dynamic ? 1 : 0, b.diag0,
           b.Dinv, status_);
     }
     for (int kb = 0; b.df_items == 0 && kb < b.nchol; ++kb) {
-      ++g_launches, k_potrf_diag<<<1, 1024, kSmemTrtri, st>>>(b.F, b.n, kb, dyn_eps, dyn_delta, dynamic ? 1 : 0,
+      ++g_launches, k_potrf_diag<<<1, 1024, kSmemTrtri, st>>>(b.F, b.ldf, b.n, kb, dyn_eps, dyn_delta, dynamic ? 1 : 0,
                                                               b.diag0, b.Dinv, status_);
       int rest = b.nchol - kb - 1;
       if (rest > 0) {
-        ++g_launches, k_trsm_panel<<<rest, SDPXG_THREADS, kSmemTrsm, st>>>(b.F, b.n, kb, b.Dinv);
-        ++g_launches, k_syrk_update<<<rest * (rest + 1) / 2, SDPXG_THREADS, kSmemSyrk, st>>>(b.F, b.n, kb);
+        ++g_launches, k_trsm_panel<<<rest, SDPXG_THREADS, kSmemTrsm, st>>>(b.F, b.ldf, b.n, kb, b.Dinv);
+        ++g_launches, k_syrk_update<<<rest * (rest + 1) / 2, SDPXG_THREADS, kSmemSyrk, st>>>(b.F, b.ldf, b.n, kb);
       }
     }
     launched("factor");
@@ -1138,7 +1141,7 @@ class Engine {
       const int g = 1 << level, h = g >> 1;
       dim3 grid(h, h, (b.nchol + g - 1) / g);
       for (int phase = 0; phase < 2; ++phase)
-        ++g_launches, k_trinv_level<<<grid, SDPXG_THREADS, kSmemTrinv, st>>>(b.F, b.Uinv, b.UinvT, b.Tmp, b.n,
+        ++g_launches, k_trinv_level<<<grid, SDPXG_THREADS, kSmemTrinv, st>>>(b.F, b.ldf, b.Uinv, b.UinvT, b.Tmp, b.n,
                                                                              level, phase);
     }
     launched("trinv");
@@ -1182,7 +1185,7 @@ class Engine {
   bool factor_split(double eps, bool dynamic, double dyn_eps, double dyn_delta) {
     prepare_split();
     const int n1 = split_n1(), n2 = n - n1;
-    const long ldn = n;
+    const long ldn = n, ldf = factor_ld(n);
     clear_status();
     check(cudaMemsetAsync(oz_status_word(), 0, sizeof(uint32_t), st), "memset");
     // phase timers: the dataflow launches under KT_FACTOR, the diagonal-block inverses under
@@ -1199,13 +1202,13 @@ class Engine {
     tbegin(KT_TRINV);
     launch_trinv(sub1_.b);
     tend(KT_TRINV);
-    double* U12 = F_.p + (long)n1 * ldn;  // F[0:n1, n1:n]
+    double* U12 = F_.p + (long)n1 * ldf;  // F[0:n1, n1:n]
     tbegin(KT_SPLIT);
     // U12 = X11' H12: rows of the left operand are the columns of X11, rows of the right
     // operand the columns of H12
-    ozaki_gemm(oz, st, n1, n2, n1, sub1_.Uinv, n1, 1, Hsave_.p + (long)n1 * ldn, ldn, 1, 1.0, 0.0, U12, ldn, 0);
+    ozaki_gemm(oz, st, n1, n2, n1, sub1_.Uinv, n1, 1, Hsave_.p + (long)n1 * ldn, ldn, 1, 1.0, 0.0, U12, ldf, 0);
     // S = H22 - U12' U12 (full, exactly symmetric: the integer product of an operand with itself)
-    ozaki_gemm(oz, st, n2, n2, n1, U12, ldn, 1, U12, ldn, 1, -1.0, 1.0, sub2_.H, n2, 0);
+    ozaki_gemm(oz, st, n2, n2, n1, U12, ldf, 1, U12, ldf, 1, -1.0, 1.0, sub2_.H, n2, 0);
     tend(KT_SPLIT);
     // the pivot rule's original diagonal is that of H22 + eps I, as in the plain form
     tbegin(KT_FACTOR);
@@ -1216,11 +1219,9 @@ class Engine {
     tend(KT_TRINV);
     tbegin(KT_SPLIT);
     // X12 = -(X11 U12) X22
-    ozaki_gemm(oz, st, n1, n2, n1, sub1_.Uinv, 1, n1, U12, ldn, 1, 1.0, 0.0, Tmp_, n1, 0);
+    ozaki_gemm(oz, st, n1, n2, n1, sub1_.Uinv, 1, n1, U12, ldf, 1, 1.0, 0.0, Tmp_, n1, 0);
     ozaki_gemm(oz, st, n1, n2, n2, Tmp_, 1, n1, sub2_.Uinv, n2, 1, -1.0, 0.0, Uinv_.p + (long)n1 * ldn, ldn, 0);
-    // assemble U, X and X'
-    copy_block(F_, ldn, sub1_.F, n1, n1, n1);
-    copy_block(F_.p + (long)n1 * ldn + n1, ldn, sub2_.F, n2, n2, n2);
+    // assemble X and X' (the diagonal blocks of U stay in their own storage: nothing reads them)
     copy_block(Uinv_, ldn, sub1_.Uinv, n1, n1, n1);
     copy_block(Uinv_.p + (long)n1 * ldn + n1, ldn, sub2_.Uinv, n2, n2, n2);
     copy_block(UinvT_, ldn, sub1_.UinvT, n1, n1, n1);
@@ -1311,7 +1312,6 @@ class Engine {
   const double* uinv() const { return Uinv_.p; }
   const double* uinvT() const { return UinvT_.p; }
   bool factored() const { return factor_ok_; }
-  double* F() { return F_.p; }
   const BlockDesc* blocks() const { return blocks_.p; }
 
  private:
