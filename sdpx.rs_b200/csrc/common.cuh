@@ -53,6 +53,17 @@ struct RefineParams {
   int max_iter, guard_max;
 };
 
+// What a fused norm-and-control kernel of the refined solve does (k_refine).
+enum RefineKind { REFINE_HEAD = 0, REFINE_STEP = 1, REFINE_OUTER_INIT = 2, REFINE_OUTER_STEP = 3 };
+struct RefineOp {
+  int kind, rows, reset;    // reset: HEAD starts a new KKT solve
+  long n;                   // STEP: entries of the two copies below
+  double* x;                // STEP: x <- cand when the candidate is kept
+  const double* cand;
+  double* e;                // STEP: e <- e2 when the loop goes on
+  const double* e2;
+};
+
 // One reduction of a batched launch (k_reduce_batch): op over x (and y) of length n.
 struct RedReq {
   int op;

@@ -7,6 +7,8 @@
 //   lambda_inv_circ_op 757-780, affine_ds 455-460, step_length_psd_component 1180-1231,
 //   admits 1168-1178, margins ~590-606; and the binary64 factored Hs / Hs^-1 application
 //   of kkt/condensed/psd.rs:1968-2002.
+#include <cooperative_groups.h>
+
 #include "eig.cuh"
 
 namespace {
@@ -175,14 +177,6 @@ extern "C" __global__ void k_ginv_from_rinv(const BlockDesc* __restrict__ blocks
   }
 }
 
-// ---------------------------------------------------------------------------------------
-// Congruences on svec vectors.  mode:
-//   0  W x     = svec(R' X R)          1  W' x     = svec(R X R')
-//   2  Winv x  = svec(Rinv' X Rinv)    3  Winv' x  = svec(Rinv X Rinv')
-//   4  Hs x    = W'(W x)  (two congruences through R, never the squared G)
-//   5  Hs^-1 x = Winv(Winv' x)
-// grid = (blocks, columns); column c of x / y starts at c * ld.
-// ---------------------------------------------------------------------------------------
 __device__ void cta_congruence(double* Y, double* T, const double* X, const double* B,
                                bool outer_t, int n) {
   // outer_t: Y = B X B'  else Y = B' X B
@@ -198,35 +192,126 @@ __device__ void cta_congruence(double* Y, double* T, const double* X, const doub
   __syncthreads();
 }
 
-extern "C" __global__ void __launch_bounds__(SDPXG_CONE_THREADS)
+// ---------------------------------------------------------------------------------------
+// Congruences on svec vectors.  mode:
+//   0  W x     = svec(R' X R)          1  W' x     = svec(R X R')
+//   2  Winv x  = svec(Rinv' X Rinv)    3  Winv' x  = svec(Rinv X Rinv')
+//   4  Hs x    = W'(W x)  (two congruences through R, never the squared G)
+//   5  Hs^-1 x = Winv(Winv' x)
+// plus `base` when it is given (y = op(x) + base).  grid.y: columns; column c of x / y / base
+// starts at c * ld.
+//
+// One cluster of four CTAs per block.  A 64^3 product is 2.1 us of one SM's FP64 pipe and an
+// operator of two congruences has four of them, so one CTA per block was bound by its own pipe
+// (about 10 us at n = 60); the 8-wide tile columns J and 7 - J go to CTA J (equal work on the upper
+// triangle), which forms T = X op(B) for its columns and the upper tiles of op(B)' T.  Between the
+// two congruences each CTA reads the others' columns through distributed shared memory.
+// ---------------------------------------------------------------------------------------
+namespace {
+
+constexpr int kCongCtas = 4;
+constexpr int kCongThreads = 256;
+
+// T (16 columns: tile columns J0 and J1 of CTA `rank`) = X op(B), op(B) = B' (outer_t) or B: warp w
+// forms row tile w of both tile columns, its four accumulation chains in flight together.
+__device__ __forceinline__ void slab_times(double* T, const double* X, const double* B, bool outer_t, int n, int J0,
+                                           int J1) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = lane >> 2, q = lane & 3;
+  const int nt = (n + 7) >> 3, ks = (n + 3) >> 2;
+  if (w >= nt || J0 >= nt) return;
+  const bool two = J1 < nt;
+  double c[4][2] = {};
+  for (int k0 = 0; k0 < ks; k0 += 2) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int k = ((k0 + u) << 2) + q;
+      if (k0 + u < ks) {
+        const double a = SM(X, 8 * w + r, k);
+        dmma_m8n8k4(c[u][0], c[u][1], a, outer_t ? SM(B, 8 * J0 + r, k) : SM(B, k, 8 * J0 + r));
+        if (two) dmma_m8n8k4(c[2 + u][0], c[2 + u][1], a, outer_t ? SM(B, 8 * J1 + r, k) : SM(B, k, 8 * J1 + r));
+      }
+    }
+  }
+  SM(T, 8 * w + r, 2 * q) = c[0][0] + c[1][0];
+  SM(T, 8 * w + r, 2 * q + 1) = c[0][1] + c[1][1];
+  SM(T, 8 * w + r, 8 + 2 * q) = c[2][0] + c[3][0];
+  SM(T, 8 * w + r, 8 + 2 * q + 1) = c[2][1] + c[3][1];
+}
+
+// Y (the same 16 columns, upper tiles only) = op(B)' T, op(B)' = B (outer_t) or B'.
+__device__ __forceinline__ void slab_close(double* Y, const double* T, const double* B, bool outer_t, int n, int J0,
+                                           int J1) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = lane >> 2, q = lane & 3;
+  const int nt = (n + 7) >> 3, ks = (n + 3) >> 2;
+  const int n1 = J1 < nt ? J1 + 1 : 0, n0 = J0 < nt ? J0 + 1 : 0;
+  for (int t = w; t < n1 + n0; t += kCongThreads / 32) {
+    const int I = t < n1 ? t : t - n1, s = t < n1 ? 8 : 0;
+    double c[4][2] = {};
+    for (int k0 = 0; k0 < ks; k0 += 4) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int k = ((k0 + u) << 2) + q;
+        if (k0 + u < ks)
+          dmma_m8n8k4(c[u][0], c[u][1], outer_t ? SM(B, 8 * I + r, k) : SM(B, k, 8 * I + r), SM(T, k, s + r));
+      }
+    }
+    SM(Y, 8 * I + r, s + 2 * q) = (c[0][0] + c[1][0]) + (c[2][0] + c[3][0]);
+    SM(Y, 8 * I + r, s + 2 * q + 1) = (c[0][1] + c[1][1]) + (c[2][1] + c[3][1]);
+  }
+}
+
+}  // namespace
+
+extern "C" __global__ void __cluster_dims__(kCongCtas, 1, 1) __launch_bounds__(kCongThreads)
 k_congruence(const BlockDesc* __restrict__ blocks, int mode, const double* __restrict__ R,
-             const double* __restrict__ Rinv, const double* __restrict__ x, double* __restrict__ y,
-             long ld) {
+             const double* __restrict__ Rinv, const double* __restrict__ x, const double* __restrict__ base,
+             double* __restrict__ y, long ld) {
+  namespace cg = cooperative_groups;
   extern __shared__ double smem[];
-  const BlockDesc bd = blocks[blockIdx.x];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), J0 = rank, J1 = 7 - rank;
+  const BlockDesc bd = blocks[blockIdx.x / kCongCtas];
   const int n = bd.n;
-  const long coff = (long)blockIdx.y * ld;
+  const long off = (long)blockIdx.y * ld + bd.svec_off;
   double* B = smem;
   double* X = B + kMat;
   double* T = X + kMat;
-  double* Y = T + kMat;
+  double* Y = T + 16 * SDPXG_LD;
   const bool use_r = (mode == 0 || mode == 1 || mode == 4);
   cta_load_mat(B, (use_r ? R : Rinv) + bd.mat_off, n);
-  cta_load_smat(X, x + coff + bd.svec_off, n);
+  cta_load_smat(X, x + off, n);
   __syncthreads();
-  if (mode <= 3) {
-    cta_congruence(Y, T, X, B, mode == 1 || mode == 3, n);
-  } else {
-    // first stage: W x (R' X R) for Hs, Winv' x (Rinv X Rinv') for Hs^-1
-    cta_congruence(Y, T, X, B, mode == 5, n);
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-      int i = e % n, j = e / n;
-      SM(X, i, j) = 0.5 * (SM(Y, i, j) + SM(Y, j, i));
+  // W x (R' X R) first for Hs, Winv' x (Rinv X Rinv') first for Hs^-1
+  bool outer_t = mode == 1 || mode == 3 || mode == 5;
+  slab_times(T, X, B, outer_t, n, J0, J1);
+  __syncthreads();
+  slab_close(Y, T, B, outer_t, n, J0, J1);
+  if (mode >= 4) {
+    cluster.sync();  // every CTA's columns are in its Y, and nobody reads X any more
+    for (int e = threadIdx.x; e < SDPXG_NMAX * SDPXG_NMAX; e += kCongThreads) {
+      const int i = e & 63, j = e >> 6, J = j >> 3;
+      if (i > j || j >= n) continue;
+      const double* Yr = cluster.map_shared_rank(Y, J < kCongCtas ? J : 7 - J);
+      const double v = SM(Yr, i, (J < kCongCtas ? 0 : 8) + (j & 7));
+      SM(X, i, j) = v;
+      SM(X, j, i) = v;
     }
+    cluster.sync();  // everyone has read Y
+    outer_t = !outer_t;
+    slab_times(T, X, B, outer_t, n, J0, J1);
     __syncthreads();
-    cta_congruence(Y, T, X, B, mode == 4, n);
+    slab_close(Y, T, B, outer_t, n, J0, J1);
   }
-  cta_store_svec(y + coff + bd.svec_off, Y, n);
+  __syncthreads();
+  for (int c = threadIdx.x >> 5; c < 16; c += kCongThreads / 32) {  // svec: one warp a column
+    const int j = (c < 8 ? J0 : J1) * 8 + (c & 7);
+    if (j >= n) continue;
+    for (int i = threadIdx.x & 31; i <= j; i += 32) {
+      const double v = (i == j) ? SM(Y, i, c) : SM(Y, i, c) * SDPXG_SQRT2;
+      const long o = off + tri_idx(i, j);
+      y[o] = base ? v + base[o] : v;
+    }
+  }
 }
 
 // x = svec((Y Z + Z Y) / 2) per block.

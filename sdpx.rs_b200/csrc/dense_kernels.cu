@@ -447,6 +447,10 @@ k_coldot_seg(const double* __restrict__ A, int n, int tri, const double* __restr
   }
   double t = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
   t = warp_sum(t);
+  if (s1 - s0 == 1) {  // one segment: nothing to combine
+    if (lane == 0) out[c] = (rbase ? rbase[c] : 0.0) + alpha * t;
+    return;
+  }
   unsigned ticket = 0;
   if (lane == 0) {
     partial[(long)sg * n + c] = t;

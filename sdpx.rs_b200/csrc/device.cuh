@@ -197,7 +197,7 @@ __global__ void k_nt_factor(const BlockDesc*, const double*, const double*, doub
 __global__ void k_nt_svd(const BlockDesc*, double*, double*, double*, double*, double*, uint32_t*);
 __global__ void k_identity_scaling(const BlockDesc*, double*, double*, double*, double*, double*);
 __global__ void k_ginv_from_rinv(const BlockDesc*, const double*, double*);
-__global__ void k_congruence(const BlockDesc*, int, const double*, const double*, const double*,
+__global__ void k_congruence(const BlockDesc*, int, const double*, const double*, const double*, const double*,
                              double*, long);
 __global__ void k_circ_op(const BlockDesc*, const double*, const double*, double*);
 __global__ void k_lam_inv_circ(const BlockDesc*, const double*, const double*, double*);
@@ -215,12 +215,12 @@ __global__ void k_schur_gather(int, const int*, const int*, const int*, const in
 __global__ void k_add_upper_csc(int, const int*, const int*, const double*, double*);
 __global__ void k_op_forward(const BlockDesc*, const int*, const int*, const int*, const long*,
                              const double*, const int*, const int*, const double*, long, double,
-                             double, double*, long);
+                             double, const double*, double*, long);
 __global__ void k_op_adjoint_partial(const BlockDesc*, const int*, const int*, const int*,
                                      const long*, const double*, const double*, long, double*,
                                      long, int);
 __global__ void k_op_adjoint_gather(int, const int*, const int*, const int*, const int*,
-                                    const double*, long, double, double, double*, long);
+                                    const double*, long, double, double, const double*, double*, long);
 __global__ void k_potrf_diag(double*, long, int, int, double, double, int, const double*, double*,
                              uint32_t*);
 __global__ void k_trsm_panel(double*, long, int, int, const double*);
@@ -230,7 +230,7 @@ __global__ void k_gram_schur(const BlockDesc*, const int*, const int*, const int
                              const long*, const double*, const double*, double*);
 __global__ void k_gram_forward(const BlockDesc*, const int*, const int*, const int*, const int*,
                                const int*, const long*, const double*, const double*,
-                               const double*, double, double, double*, double*, unsigned*);
+                               const double*, double, double, const double*, double*, double*, unsigned*);
 __global__ void k_gram_adjoint(const BlockDesc*, const int*, const int*, const int*, const int*,
                                const long*, const double*, const double*, const double*, double*);
 __global__ void k_chol_dataflow(double*, long, int, int, const unsigned*, int, int*, double, double, int,
@@ -252,19 +252,14 @@ __global__ void k_reduce_final(int, int, const double*, double*);
 __global__ void k_reduce_fused(int, long, const double*, const double*, double*, unsigned*, double*);
 __global__ void k_reduce_batch(RedBatch, double*, unsigned*, double*, int);
 __global__ void k_lincomb_batch(LinBatch);
-__global__ void k_refine_head(const double*, const double*, const double*, const double*,
-                              const double*, int, RefineCtl*, RefineParams, cudaGraphConditionalHandle);
-__global__ void k_refine_step(const double*, RefineCtl*, RefineParams, cudaGraphConditionalHandle);
-__global__ void k_refine_outer_init(const double*, const double*, const double*, const double*,
-                                    RefineCtl*, RefineParams, cudaGraphConditionalHandle);
-__global__ void k_refine_outer_step(const double*, const double*, RefineCtl*, RefineParams,
-                                    cudaGraphConditionalHandle);
-__global__ void k_refine_copy(const int*, long, double*, const double*, const int*, long, double*,
-                              const double*);
+__global__ void k_refine(RedBatch, double*, unsigned*, int, RefineOp, RefineCtl*, RefineParams,
+                         cudaGraphConditionalHandle);
+__global__ void k_refine_keep(const RefineCtl*, long, double*, const double*, double*, const double*, long, double*,
+                              const double*, double*, const double*);
 __global__ void k_diag_absmax(const double*, int, double*);
 __global__ void k_nn_scale(int, const int*, const double*, const double*, double*, double*, uint32_t*);
 __global__ void k_nn_identity(int, double*, double*);
-__global__ void k_nn_cone(int, const int*, int, const double*, const double*, double*, long);
+__global__ void k_nn_cone(int, const int*, int, const double*, const double*, const double*, double*, long);
 __global__ void k_nn_circ(int, const int*, const double*, const double*, double*);
 __global__ void k_nn_lam_inv(int, const int*, const double*, const double*, double*);
 __global__ void k_nn_affine_ds(int, const int*, const double*, double*);
@@ -272,7 +267,8 @@ __global__ void k_nn_shift(int, const int*, double*, double);
 __global__ void k_nn_step(int, const int*, const double*, const double*, const double*, const double*,
                           double, int, double*);
 __global__ void k_nn_margins(int, const int*, const double*, double*);
-__global__ void k_nn_forward(int, int, const int*, const double*, const double*, double, double, double*);
+__global__ void k_nn_forward(int, int, const int*, const double*, const double*, double, double, const double*,
+                             double*);
 __global__ void k_nn_adjoint(int, int, const int*, const double*, const double*, double, double*);
 __global__ void k_nn_schur(int, int, const double*, const double*, double*);
 __global__ void k_ms_basis(const BlockDesc*, const MsDesc*, const double*, const double*, double*);
@@ -280,11 +276,11 @@ __global__ void k_ms_gram(const BlockDesc*, const MsDesc*, const double*, double
 __global__ void k_ms_schur(const MsDesc*, const int*, const int*, const long*, const double*, const int*,
                            const double*, double*);
 __global__ void k_ms_forward(const BlockDesc*, const MsDesc*, const int*, const int*, const double*,
-                             const double*, const double*, double, double, double*);
+                             const double*, const double*, double, double, const double*, double*);
 __global__ void k_ms_adjoint(const BlockDesc*, const MsDesc*, const int*, const int*, const double*, const int*,
                              const double*, const double*, double*);
 __global__ void k_csr_spmv(int, const int*, const int*, const double*, const double*, double,
-                           double, double*);
+                           double, const double*, double*);
 }
 
 // Kernel launches issued by this library in this process (every launch site increments it).
@@ -309,7 +305,7 @@ class Reducer {
     if (n > 0 && !x) throw std::invalid_argument("null device buffer: reduction input");
     int s = count_++;
     if (n > 0) {
-      ++g_launches, k_reduce_fused<<<kBlocks, 256, 0, st>>>(op, n, x, y, partial_.p + (size_t)s * kBlocks,
+      ++g_launches, k_reduce_fused<<<blocks_for(n), 256, 0, st>>>(op, n, x, y, partial_.p + (size_t)s * kBlocks,
                                                           counters_.p + s, slots_.p + s);
     } else {  // an empty input: the operation's identity (1 for the finite test, 0 otherwise)
       copy_h2d(slots_.p + s, &id_[op], sizeof(double), st);
@@ -324,18 +320,26 @@ class Reducer {
     if (count_ + k > kSlots) throw CudaError("reducer slots exhausted");
     RedBatch b{};
     int i = 0;
+    long most = 0;
     for (const RedReq& q : reqs) {
       if (q.n > 0 && !q.x) throw std::invalid_argument("null device buffer: reduction input");
       b.r[i++] = q;
+      most = std::max(most, q.n);
     }
     const int first = count_;
     count_ += k;
-    ++g_launches, k_reduce_batch<<<dim3(kBlocks, k), 256, 0, st>>>(b, partial_.p, counters_.p, slots_.p, first);
+    ++g_launches, k_reduce_batch<<<dim3(blocks_for(most), k), 256, 0, st>>>(b, partial_.p, counters_.p, slots_.p, first);
     return first;
   }
   int count() const { return count_; }
-  // Device address of a slot (read by the control kernels of the device-driven solves).
-  const double* slot(int s) const { return slots_.p + s; }
+  // Blocks of a reduction of n entries: four entries a thread or more.  A block's partial costs a
+  // fence, a ticket and a place in the fold, so 148 blocks for a few hundred entries took 7 us
+  // where one block takes 3.
+  static int blocks_for(long n) { return (int)std::min<long>(kBlocks, std::max<long>(1, (n + 1023) / 1024)); }
+  // Scratch of a fused reduction (k_refine): partials and a ticket of `rows` slots nobody else uses
+  // while the kernel runs (stream order).
+  double* partials() { return partial_.p; }
+  unsigned* ticket() { return counters_.p; }
   // Slots queued by a replayed captured segment (its reductions ran inside the graph).
   void set_count(int c) { count_ = c; }
   const PinnedBuf<double>& fetch(cudaStream_t st) {

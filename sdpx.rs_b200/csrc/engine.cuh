@@ -32,7 +32,7 @@ namespace sdpxg {
 constexpr int kMatD = SDPXG_LD * SDPXG_NMAX;
 constexpr size_t kSmemNtFactor = (3 * kMatD + 2 * SDPXG_CHOL_SCRATCH) * sizeof(double);
 constexpr size_t kSmemNt = (5 * kMatD + 2 * SDPXG_NMAX) * sizeof(double) + (SDPXG_NMAX + 1) * sizeof(int);
-constexpr size_t kSmemCong = 4 * kMatD * sizeof(double);
+constexpr size_t kSmemCong = (2 * kMatD + 2 * 16 * SDPXG_LD) * sizeof(double);
 constexpr size_t kSmemCirc = 2 * kMatD * sizeof(double);
 constexpr size_t kSmemStep = (4 * kMatD + SDPXG_CHOL_SCRATCH + 4 * SDPXG_NMAX + 32) * sizeof(double);
 constexpr size_t kSmemMarg = (kMatD + 5 * SDPXG_NMAX + 32) * sizeof(double);
@@ -273,6 +273,8 @@ class Engine {
     for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second.exec);
     for (auto& kv : programs_) cudaGraphExecDestroy(kv.second.exec);
     for (auto& e : ev_) if (e) cudaEventDestroy(e);
+    for (auto& e : branch_ev_) if (e) cudaEventDestroy(e);
+    if (branch_) cudaStreamDestroy(branch_);
     if (st) cudaStreamDestroy(st);
   }
 
@@ -346,6 +348,34 @@ class Engine {
     if (kernels) *kernels = k;
     return g;
   }
+  // While a run is being captured: f's launches go to a branch of their own, beside what the main
+  // stream captures up to join().  Outside a capture f simply runs first.
+  template <typename F>
+  void fork(F&& f) {
+    forked_ = false;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    check(cudaStreamIsCapturing(st, &cs), "capture status");
+    if (cs != cudaStreamCaptureStatusActive) {
+      f();
+      return;
+    }
+    check(cudaEventRecord(branch_ev_[0], st), "fork");
+    check(cudaStreamWaitEvent(branch_, branch_ev_[0], 0), "fork");
+    std::swap(st, branch_);
+    try {
+      f();
+    } catch (...) {
+      std::swap(st, branch_);
+      throw;
+    }
+    std::swap(st, branch_);
+    check(cudaEventRecord(branch_ev_[1], branch_), "join");
+    forked_ = true;
+  }
+  void join() {
+    if (forked_) check(cudaStreamWaitEvent(st, branch_ev_[1], 0), "join");
+    forked_ = false;
+  }
   // Instantiated graphs with device-side control flow (the refined KKT solve), keyed like the
   // segments and dropped with them.  Kernel counts: fixed per launch, per inner and per outer
   // refinement step.
@@ -380,6 +410,8 @@ class Engine {
     device = dev;
     check(cudaSetDevice(device), "cudaSetDevice");
     check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream");
+    check(cudaStreamCreateWithFlags(&branch_, cudaStreamNonBlocking), "branch stream");
+    for (auto& e : branch_ev_) check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "branch event");
     set_smem(reinterpret_cast<const void*>(k_nt_factor), kSmemNtFactor);
     set_smem(reinterpret_cast<const void*>(k_nt_svd), kSmemNt);
     set_smem(reinterpret_cast<const void*>(k_congruence), kSmemCong);
@@ -710,12 +742,12 @@ class Engine {
     c2b_loc_.alloc(std::max<size_t>(c2b_loc.size(), 1)); c2b_loc_.upload(c2b_loc.data(), c2b_loc.size(), st);
     wblk_.alloc(std::max(nwork_, 1)); wblk_.upload(wblk.data(), wblk.size(), st);
     wloc_.alloc(std::max(nwork_, 1)); wloc_.upload(wloc.data(), wloc.size(), st);
-    {  // 64-row tiles of every block for the forward product
+    {  // 32-row tiles of every block for the forward product
       std::vector<int> fb, fr;
       for (int j = 0; j < nblk; ++j) {
         if (gram[j]) continue;  // Gram and matrix-valued sampled blocks have their own operators
         int tn = hblocks[j].n * (hblocks[j].n + 1) / 2;
-        for (int r0 = 0; r0 < tn; r0 += 64) {
+        for (int r0 = 0; r0 < tn; r0 += 32) {
           fb.push_back(j);
           fr.push_back(r0);
         }
@@ -822,18 +854,18 @@ class Engine {
     check(cudaStreamSynchronize(st), "scaling sync");
   }
 
-  // y = op(x) for cone operator `mode`, ncols columns with stride ld.
-  void cone_apply(int mode, const double* x, double* y, int ncols = 1, long ld = 0) {
+  // y = op(x) (+ base) for cone operator `mode`, ncols columns with stride ld.
+  void cone_apply(int mode, const double* x, double* y, int ncols = 1, long ld = 0, const double* base = nullptr) {
     need(x, "cone_apply x");
     need(y, "cone_apply y");
     if (!nblk && !nnn_) return;
     tbegin(KT_CONE);
     if (nblk)
-      ++g_launches, k_congruence<<<dim3(nblk, ncols), SDPXG_CONE_THREADS, kSmemCong, st>>>(
-          blocks_, mode, R_, Rinv_, x, y, ld ? ld : m);
+      ++g_launches, k_congruence<<<dim3(4 * nblk, ncols), 256, kSmemCong, st>>>(blocks_, mode, R_, Rinv_, x, base, y,
+                                                                               ld ? ld : m);
     if (nnn_)
       ++g_launches, k_nn_cone<<<dim3((nnn_ + 255) / 256, ncols), 256, 0, st>>>(nnn_, nn_idx_, mode, nnw_, x,
-                                                                               y, ld ? ld : m);
+                                                                               base, y, ld ? ld : m);
     launched("k_congruence");
     tend(KT_CONE);
   }
@@ -911,36 +943,38 @@ class Engine {
   }
 
   // ---- constraint operator ----
-  // y = alpha * A x + beta * y   (rows m)
-  void A_forward(const double* x, double alpha, double beta, double* y) {
+  // y = alpha * A x + beta * base   (rows m; base null: y itself)
+  void A_forward(const double* x, double alpha, double beta, double* y, const double* base = nullptr) {
+    if (!base) base = y;
     need(x, "A_forward x");
     need(y, "A_forward y");
     if (nnn_) {
       ++g_launches, k_nn_forward<<<(nnn_ + 255) / 256, 256, 0, st>>>(nnn_, n, nn_idx_, Ann_, x, alpha, beta,
-                                                                     y);
+                                                                     base, y);
       launched("k_nn_forward");
     }
     if (!nblk) return;
     if (nftile_) {
-      ++g_launches, k_op_forward<<<dim3(nftile_, 1), 256, 0, st>>>(
+      ++g_launches, k_op_forward<<<dim3(nftile_, 1), 512, 0, st>>>(
           blocks_, kcount_, col_ptr_, col_idx_, acol_off_, acol_, ftile_blk_, ftile_r0_, x, n, alpha,
-          beta, y, m);
+          beta, base, y, m);
       launched("k_op_forward");
     }
     if (nms_) {
       ++g_launches, k_ms_forward<<<dim3(nms_, (ms_tnmax_ + 255) / 256), 256, 0, st>>>(
-          blocks_, ms_desc_, col_ptr_, col_idx_, ms_w_, ms_q_, x, alpha, beta, y);
+          blocks_, ms_desc_, col_ptr_, col_idx_, ms_w_, ms_q_, x, alpha, beta, base, y);
       launched("k_ms_forward");
     }
     if (ngblk_) {
       ++g_launches, k_gram_forward<<<ngitem_, 256, 0, st>>>(
           blocks_, gitem_blk_, gitem_c0_, kcount_, col_ptr_, col_idx_, gu_off_, gsig_, gU_, x,
-          alpha, beta, y, gf_part_, gf_cnt_);
+          alpha, beta, base, y, gf_part_, gf_cnt_);
       launched("k_gram_forward");
     }
   }
-  // y = alpha * A' z + beta * y   (length n)
-  void A_adjoint(const double* z, double alpha, double beta, double* y) {
+  // y = alpha * A' z + beta * base   (length n; base null: y itself)
+  void A_adjoint(const double* z, double alpha, double beta, double* y, const double* base = nullptr) {
+    if (!base) base = y;
     need(z, "A_adjoint z");
     need(y, "A_adjoint y");
     if (nwork_) {
@@ -961,7 +995,7 @@ class Engine {
     }
     if (n) {
       ++g_launches, k_op_adjoint_gather<<<dim3((n + 255) / 256, 1), 256, 0, st>>>(
-          n, c2b_ptr_, c2b_blk_, c2b_loc_, col_ptr_, adj_part_, ncol_, alpha, beta, y, n);
+          n, c2b_ptr_, c2b_blk_, c2b_loc_, col_ptr_, adj_part_, ncol_, alpha, beta, base, y, n);
       launched("k_op_adjoint_gather");
     }
     if (n && nnn_) {
@@ -969,16 +1003,17 @@ class Engine {
       launched("k_nn_adjoint");
     }
   }
-  // y = alpha * P x + beta * y  (P symmetric)
-  void P_mult(const double* x, double alpha, double beta, double* y) {
+  // y = alpha * P x + beta * base  (P symmetric; base null: y itself)
+  void P_mult(const double* x, double alpha, double beta, double* y, const double* base = nullptr) {
+    if (!base) base = y;
     need(x, "P_mult x");
     need(y, "P_mult y");
     if (!n) return;
     if (p_nnz_ == 0) {
-      lincomb(n, 0.0, nullptr, beta, beta == 0.0 ? nullptr : y, 0.0, nullptr, y);
+      lincomb(n, 0.0, nullptr, beta, beta == 0.0 ? nullptr : base, 0.0, nullptr, y);
       return;
     }
-    ++g_launches, k_csr_spmv<<<(n + 255) / 256, 256, 0, st>>>(n, prp_, pci_, pv_, x, alpha, beta, y);
+    ++g_launches, k_csr_spmv<<<(n + 255) / 256, 256, 0, st>>>(n, prp_, pci_, pv_, x, alpha, beta, base, y);
     launched("k_csr_spmv");
   }
   bool has_P() const { return p_nnz_ > 0; }
@@ -1244,8 +1279,8 @@ class Engine {
     if (!oz.status.p) oz.status.alloc(1);
     return oz.status.p;
   }
-  // x = F^-1 r = U^-1 (U^-T r) through the explicit inverse: two coalesced GEMVs.
-  void trisolve(const double* r, double* x) {
+  // x = F^-1 r (+ base) = U^-1 (U^-T r) through the explicit inverse: two coalesced GEMVs.
+  void trisolve(const double* r, double* x, const double* base = nullptr) {
     need(r, "trisolve r");
     need(x, "trisolve x");
     tbegin(KT_TRISOLVE);
@@ -1253,7 +1288,7 @@ class Engine {
     const dim3 grid((n + 7) / 8, (n + 255) / 256);
     ++g_launches, k_coldot_seg<<<grid, 256, 0, st>>>(Uinv_, n, 1, r, nullptr, 1.0, tri_y_, gv_part_,
                                                      gv_cnt_);
-    ++g_launches, k_coldot_seg<<<grid, 256, 0, st>>>(UinvT_, n, 2, tri_y_, nullptr, 1.0, x, gv_part_,
+    ++g_launches, k_coldot_seg<<<grid, 256, 0, st>>>(UinvT_, n, 2, tri_y_, base, 1.0, x, gv_part_,
                                                      gv_cnt_);
     launched("trisolve");
     tend(KT_TRISOLVE);
@@ -1362,6 +1397,9 @@ class Engine {
   int df_items_ = 0, df_grid_ = 0;
   SubFactor sub1_, sub2_;  // diagonal blocks of the split form
   cudaEvent_t ev_[2 * KT_N] = {};
+  cudaStream_t branch_ = nullptr;  // fork(): used while capturing only
+  cudaEvent_t branch_ev_[2] = {};
+  bool forked_ = false;
   struct GraphEntry {
     cudaGraphExec_t exec;
     int red_count;

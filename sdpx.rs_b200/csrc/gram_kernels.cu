@@ -118,7 +118,7 @@ k_gram_schur(const BlockDesc* __restrict__ blocks, const int* __restrict__ tiles
     }
 }
 
-// y_j = alpha svec(U_j diag(sigma x_cols) U_j') + beta y_j, K = k_j split in 64-column chunks.
+// y_j = alpha svec(U_j diag(sigma x_cols) U_j') + beta base_j, K = k_j split in 64-column chunks.
 // One CTA per (Gram block, chunk) item (the items of a block are consecutive, chunk order):
 // it stages its 64 columns of U (coalesced, column t at Us[t * GR_LD + row], zero padded) and
 // their weights d_t = sigma_t x[col_t], forms the upper 8 x 8 tiles of U_c diag(d) U_c' on the
@@ -132,7 +132,7 @@ k_gram_forward(const BlockDesc* __restrict__ blocks, const int* __restrict__ ite
                const int* __restrict__ col_ptr, const int* __restrict__ col_idx,
                const long* __restrict__ gu_off, const double* __restrict__ gsig,
                const double* __restrict__ U, const double* __restrict__ x, double alpha,
-               double beta, double* __restrict__ y, double* __restrict__ part,
+               double beta, const double* base, double* y, double* __restrict__ part,
                unsigned* __restrict__ cnt) {
   __shared__ __align__(16) double Us[GR_KCH * GR_LD];
   __shared__ double d[GR_KCH];
@@ -188,7 +188,7 @@ k_gram_forward(const BlockDesc* __restrict__ blocks, const int* __restrict__ ite
       v += __ldcg(P0 + (size_t)c * (SDPXG_NMAX * SDPXG_NMAX) + col * SDPXG_NMAX + row);
     const long idx = bd.svec_off + (long)col * (col + 1) / 2 + row;
     const double s2 = (row == col) ? v : v * SDPXG_SQRT2;
-    y[idx] = alpha * s2 + ((beta == 0.0) ? 0.0 : beta * y[idx]);
+    y[idx] = alpha * s2 + ((beta == 0.0) ? 0.0 : beta * base[idx]);
   }
 }
 

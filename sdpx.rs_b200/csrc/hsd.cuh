@@ -154,6 +154,8 @@ class HsdSolver {
   bool reduced_solve(const double* r, double* x);
   void reduced_first(const double* r, double* x);
   bool reduced_refine(const double* r, double* x, double normb, double norme);
+  void reduced_pass(const double* r, double* x);
+  void condense(const double* bx, const double* bz);
   void condense_first(const double* bx, const double* bz, double* x);
   void recover(const double* bz, const double* x, double* z);
   bool solve_raw(const double* bx, const double* bz, double* x, double* z);
@@ -245,9 +247,12 @@ enum : int { SEG_RS_HEAD = 1, SEG_RS_STEP = 2, SEG_RAW_HEAD = 3, SEG_RAW_TAIL = 
 // Queues |r|max, |e|max and finite(x).
 inline void HsdSolver::reduced_first(const double* r, double* x) {
   const int n = n_;
+  reduced_pass(r, x);
+  E.red.add_batch(st(), {{RED_MAXABS, n, r, nullptr}, {RED_MAXABS, n, en_, nullptr}, {RED_FINITE, n, x, nullptr}});
+}
+inline void HsdSolver::reduced_pass(const double* r, double* x) {
   E.trisolve(r, x);
   E.schur_residual(r, x, en_);
-  E.red.add_batch(st(), {{RED_MAXABS, n, r, nullptr}, {RED_MAXABS, n, en_, nullptr}, {RED_FINITE, n, x, nullptr}});
 }
 
 // Stationary refinement of the reduced system against the unshifted Schur complement, from the
@@ -260,8 +265,7 @@ inline bool HsdSolver::reduced_refine(const double* r, double* x, double normb, 
     double previous = norme;
     times.inner_refinements++;
     E.segment(SEG_RS_STEP, {r, x}, [&] {
-      E.trisolve(en_, dxn_);
-      E.lincomb(n, 1.0, x, 1.0, dxn_, 0.0, nullptr, candn_);
+      E.trisolve(en_, candn_, x);
       E.schur_residual(r, candn_, e2n_);
       E.red.add(st(), RED_MAXABS, n, e2n_, nullptr);
     });
@@ -292,26 +296,25 @@ inline bool HsdSolver::reduced_solve(const double* r, double* x) {
 }
 
 // Condense: xhat = bx + A' Hs^-1 bz (kkt/condensed/mod.rs:2416-2507), then the first pass.
+inline void HsdSolver::condense(const double* bx, const double* bz) {
+  E.cone_apply(CM_HINV, bz, tm_);         // Hs^-1 bz
+  E.A_adjoint(tm_, 1.0, 1.0, xhat_, bx);  // bx + A' Hs^-1 bz
+}
 inline void HsdSolver::condense_first(const double* bx, const double* bz, double* x) {
-  E.cone_apply(CM_HINV, bz, tm_);     // Hs^-1 bz
-  E.copy(xhat_, bx, n_);
-  E.A_adjoint(tm_, 1.0, 1.0, xhat_);  // bx + A' Hs^-1 bz
+  condense(bx, bz);
   reduced_first(xhat_, x);
 }
 
 // Recover z = Hs^-1 (A x - bz) (kkt/condensed/mod.rs:2511-2604).
 inline void HsdSolver::recover(const double* bz, const double* x, double* z) {
-  E.lincomb(m_, -1.0, bz, 0.0, nullptr, 0.0, nullptr, tm_);
-  E.A_forward(x, 1.0, 1.0, tm_);  // A x - bz
+  E.A_forward(x, 1.0, -1.0, tm_, bz);  // A x - bz
   E.cone_apply(CM_HINV, tm_, z);
 }
 
 // Condense, reduced solve, recover (kkt/condensed/mod.rs:2416-2622).
 inline bool HsdSolver::solve_raw(const double* bx, const double* bz, double* x, double* z) {
   if (!st_.ir_enable) {
-    E.cone_apply(CM_HINV, bz, tm_);
-    E.copy(xhat_, bx, n_);
-    E.A_adjoint(tm_, 1.0, 1.0, xhat_);
+    condense(bx, bz);
     E.trisolve(xhat_, x);
     recover(bz, x, z);
     return true;
@@ -325,14 +328,20 @@ inline bool HsdSolver::solve_raw(const double* bx, const double* bz, double* x, 
 }
 
 // e = b - [P A'; A -Hs] [x; z] against the unshifted original operator.
+// The two halves are independent: while a graph is captured the second one goes to its branch.
 inline void HsdSolver::residual_full(const double* bx, const double* bz, const double* x,
                                      const double* z, double* ex, double* ez) {
-  E.P_mult(x, -1.0, 0.0, wn_);
-  E.lincomb(n_, 1.0, bx, 1.0, wn_, 0.0, nullptr, ex);
-  E.A_adjoint(z, -1.0, 1.0, ex);
-  E.cone_apply(CM_HS, z, wm3_);
-  E.lincomb(m_, 1.0, bz, 1.0, wm3_, 0.0, nullptr, ez);
-  E.A_forward(x, -1.0, 1.0, ez);
+  E.fork([&] {
+    E.cone_apply(CM_HS, z, ez, 1, 0, bz);
+    E.A_forward(x, -1.0, 1.0, ez);
+  });
+  if (E.has_P()) {
+    E.P_mult(x, -1.0, 1.0, ex, bx);
+    E.A_adjoint(z, -1.0, 1.0, ex);
+  } else {
+    E.A_adjoint(z, -1.0, 1.0, ex, bx);
+  }
+  E.join();
 }
 
 // Solve with outer refinement on the original operator (kkt/condensed/kkt.rs:275-318,
@@ -425,11 +434,12 @@ inline bool HsdSolver::kkt_solve(const double* bx, const double* bz, double* x, 
 }
 
 // Graph of one refined KKT solve (kkt_solve's steps, in its order):
-//   head run (finite bx, bz; condense; first reduced pass) -> k_refine_head
-//   WHILE inner: [trisolve e, candidate, reduced residual] -> k_refine_step -> keep candidate
-//   tail run (recover; full residual; norms) -> k_refine_outer_init
-//   WHILE outer: [condense (ex, ez); first pass] -> k_refine_head -> WHILE inner (on cx)
-//                -> [recover; candidate (x, z); full residual] -> k_refine_outer_step -> keep
+//   head run (condense; first reduced pass) -> HEAD
+//   WHILE inner: [candidate x + F^-1 e, reduced residual] -> STEP (keeps the candidate)
+//   tail run (recover; full residual) -> OUTER_INIT
+//   WHILE outer: [condense (ex, ez); first pass] -> HEAD -> WHILE inner (on cx)
+//                -> [recover; candidate (x, z); full residual] -> OUTER_STEP -> keep
+// with HEAD, STEP, ... the norms and the control of that point in one kernel (k_refine).
 // Runs are captured once from the same Engine calls as the host-driven path; the graph is cached
 // per (bx, bz, x, z, refinement settings) and replayed.
 inline bool HsdSolver::kkt_solve_graph(const double* bx, const double* bz, double* x, double* z) {
@@ -445,10 +455,6 @@ inline bool HsdSolver::kkt_solve_graph(const double* bx, const double* bz, doubl
     if (E.red.count() != 0) throw CudaError("a captured program must start with an empty reducer");
     const uint64_t launches0 = g_launches;  // capture counts launches that do not run
     RefineCtl* c = ctl_.p;
-    const int* accept = &c->accept;
-    const int* cont = &c->cont;
-    const int* oaccept = &c->oaccept;
-    const int* ocont = &c->ocont;
     cudaGraph_t G = nullptr;
     std::vector<cudaGraph_t> runs;  // captured runs, destroyed once cloned into G
     Engine::Program built;
@@ -461,16 +467,31 @@ inline bool HsdSolver::kkt_solve_graph(const double* bx, const double* bz, doubl
         check(cudaGraphAddChildGraphNode(&nd, g, d.data(), d.size(), run), "child node");
         return nd;
       };
-      auto kernel = [&](cudaGraph_t g, cudaGraphNode_t dep, const void* fn, void** args,
-                        unsigned grid) {
+      auto kernel = [&](cudaGraph_t g, cudaGraphNode_t dep, const void* fn, void** args, dim3 grid) {
         cudaKernelNodeParams kp{};
         kp.func = const_cast<void*>(fn);
-        kp.gridDim = dim3(grid);
-        kp.blockDim = dim3(grid > 1 ? 256 : 32);
+        kp.gridDim = grid;
+        kp.blockDim = dim3(256);
         kp.kernelParams = args;
         cudaGraphNode_t nd;
         check(cudaGraphAddKernelNode(&nd, g, &dep, 1, &kp), "kernel node");
         return nd;
+      };
+      // the norms and the control of one point
+      auto control = [&](cudaGraph_t g, cudaGraphNode_t dep, std::initializer_list<RedReq> reqs, RefineOp op,
+                         cudaGraphConditionalHandle h) {
+        RedBatch b{};
+        long most = 0;
+        op.rows = 0;
+        for (const RedReq& q : reqs) {
+          b.r[op.rows++] = q;
+          most = std::max(most, q.n);
+        }
+        double* partial = E.red.partials();
+        unsigned* ticket = E.red.ticket();
+        int pitch = Reducer::kBlocks;
+        void* args[] = {&b, &partial, &ticket, &pitch, &op, &c, &prm, &h};
+        return kernel(g, dep, (const void*)k_refine, args, dim3(Reducer::blocks_for(most), op.rows));
       };
       auto loop = [&](cudaGraph_t g, cudaGraphNode_t dep, cudaGraphConditionalHandle h,
                       cudaGraph_t* body) {
@@ -491,121 +512,83 @@ inline bool HsdSolver::kkt_solve_graph(const double* bx, const double* bz, doubl
         runs.push_back(g);
         return g;
       };
-      const unsigned cgrid = (unsigned)std::min<long>((2L * std::max(n, m) + 255) / 256, 592);
+      const unsigned cgrid = (unsigned)std::min<long>(((long)n + m + 255) / 256, 592);
       // inner refinement loop on (r, xx): body of a WHILE node
       uint64_t k_step = 0;
-      auto inner = [&](cudaGraph_t body, const double* r, double* xx,
-                       cudaGraphConditionalHandle h) {
-        int se = 0;
+      auto inner = [&](cudaGraph_t body, const double* r, double* xx, cudaGraphConditionalHandle h) {
         cudaGraph_t g = run(&k_step, [&] {
-          E.trisolve(en_, dxn_);
-          E.lincomb(n, 1.0, xx, 1.0, dxn_, 0.0, nullptr, candn_);
+          E.trisolve(en_, candn_, xx);
           E.schur_residual(r, candn_, e2n_);
-          se = E.red.add(st(), RED_MAXABS, n, e2n_, nullptr);
         });
         cudaGraphNode_t a = child(body, {}, g);
-        const double* p_se = E.red.slot(se);
-        void* sa[] = {&p_se, &c, &prm, &h};
-        cudaGraphNode_t b = kernel(body, a, (const void*)k_refine_step, sa, 1);
-        long nn = n;
-        double* d1 = xx;
-        const double* s1 = candn_.p;
-        double* d2 = en_.p;
-        const double* s2 = e2n_.p;
-        void* ca[] = {&accept, &nn, &d1, &s1, &cont, &nn, &d2, &s2};
-        kernel(body, b, (const void*)k_refine_copy, ca, cgrid);
+        control(body, a, {{RED_MAXABS, n, e2n_, nullptr}}, RefineOp{REFINE_STEP, 0, 0, n, xx, candn_, en_, e2n_}, h);
       };
       // head
-      int h0 = 0, h1 = 0, hb = 0;
       uint64_t k_head = 0;
       cudaGraph_t g_head = run(&k_head, [&] {
-        h0 = E.red.add_batch(st(), {{RED_FINITE, n, bx, nullptr}, {RED_FINITE, m, bz, nullptr}});
-        h1 = h0 + 1;
-        hb = E.red.count();
-        condense_first(bx, bz, x);
+        condense(bx, bz);
+        reduced_pass(xhat_, x);
       });
       cudaGraphNode_t nh = child(G, {}, g_head);
       cudaGraphConditionalHandle hin;
       check(cudaGraphConditionalHandleCreate(&hin, G, 0, 0), "conditional handle");
-      {
-        const double *a0 = E.red.slot(h0), *a1 = E.red.slot(h1), *a2 = E.red.slot(hb),
-                     *a3 = E.red.slot(hb + 1), *a4 = E.red.slot(hb + 2);
-        int reset = 1;
-        void* args[] = {&a0, &a1, &a2, &a3, &a4, &reset, &c, &prm, &hin};
-        nh = kernel(G, nh, (const void*)k_refine_head, args, 1);
-      }
+      nh = control(G, nh,
+                   {{RED_MAXABS, n, xhat_, nullptr}, {RED_MAXABS, n, en_, nullptr}, {RED_FINITE, n, x, nullptr},
+                    {RED_FINITE, n, bx, nullptr}, {RED_FINITE, m, bz, nullptr}},
+                   RefineOp{REFINE_HEAD, 0, 1, 0, nullptr, nullptr, nullptr, nullptr}, hin);
       cudaGraph_t body1;
       cudaGraphNode_t w1 = loop(G, nh, hin, &body1);
       inner(body1, xhat_, x, hin);
       // tail
-      int t0 = 0;
       uint64_t k_tail = 0;
       cudaGraph_t g_tail = run(&k_tail, [&] {
         recover(bz, x, z);
         residual_full(bx, bz, x, z, ex_, ez_);
-        t0 = E.red.add_batch(st(), {{RED_MAXABS, n, bx, nullptr}, {RED_MAXABS, m, bz, nullptr},
-                                    {RED_MAXABS, n, ex_, nullptr}, {RED_MAXABS, m, ez_, nullptr}});
       });
       cudaGraphNode_t nt = child(G, {w1}, g_tail);
       cudaGraphConditionalHandle hout;
       check(cudaGraphConditionalHandleCreate(&hout, G, 0, 0), "conditional handle");
-      {
-        const double *a0 = E.red.slot(t0), *a1 = E.red.slot(t0 + 1), *a2 = E.red.slot(t0 + 2),
-                     *a3 = E.red.slot(t0 + 3);
-        void* args[] = {&a0, &a1, &a2, &a3, &c, &prm, &hout};
-        nt = kernel(G, nt, (const void*)k_refine_outer_init, args, 1);
-      }
+      nt = control(G, nt,
+                   {{RED_MAXABS, n, bx, nullptr}, {RED_MAXABS, m, bz, nullptr}, {RED_MAXABS, n, ex_, nullptr},
+                    {RED_MAXABS, m, ez_, nullptr}},
+                   RefineOp{REFINE_OUTER_INIT, 0, 0, 0, nullptr, nullptr, nullptr, nullptr}, hout);
       cudaGraph_t body2;
       loop(G, nt, hout, &body2);
       // outer body: correction (cx, cz) = K^-1 (ex, ez), candidate, full residual
-      int ob = 0;
       uint64_t k_ohead = 0;
       cudaGraph_t g_oh = run(&k_ohead, [&] {
-        ob = E.red.count();
-        condense_first(ex_, ez_, cx_);
+        condense(ex_, ez_);
+        reduced_pass(xhat_, cx_);
       });
       cudaGraphNode_t no = child(body2, {}, g_oh);
       cudaGraphConditionalHandle hin2;
       check(cudaGraphConditionalHandleCreate(&hin2, body2, 0, 0), "conditional handle");
-      {
-        const double* nul = nullptr;
-        const double *a2 = E.red.slot(ob), *a3 = E.red.slot(ob + 1), *a4 = E.red.slot(ob + 2);
-        int reset = 0;
-        void* args[] = {&nul, &nul, &a2, &a3, &a4, &reset, &c, &prm, &hin2};
-        no = kernel(body2, no, (const void*)k_refine_head, args, 1);
-      }
+      no = control(body2, no,
+                   {{RED_MAXABS, n, xhat_, nullptr}, {RED_MAXABS, n, en_, nullptr}, {RED_FINITE, n, cx_, nullptr}},
+                   RefineOp{REFINE_HEAD, 0, 0, 0, nullptr, nullptr, nullptr, nullptr}, hin2);
       cudaGraph_t body3;
       cudaGraphNode_t w3 = loop(body2, no, hin2, &body3);
       inner(body3, xhat_, cx_, hin2);
-      int u0 = 0;
       uint64_t k_otail = 0;
       cudaGraph_t g_ot = run(&k_otail, [&] {
         recover(ez_, cx_, cz_);
         E.lincomb_batch({LinReq{n, 1.0, 1.0, 0.0, x, cx_, nullptr, candx_},
                          LinReq{m, 1.0, 1.0, 0.0, z, cz_, nullptr, candz_}});
         residual_full(bx, bz, candx_, candz_, ex2_, ez2_);
-        u0 = E.red.add_batch(st(), {{RED_MAXABS, n, ex2_, nullptr}, {RED_MAXABS, m, ez2_, nullptr}});
       });
       cudaGraphNode_t nq = child(body2, {w3}, g_ot);
-      {
-        const double *a0 = E.red.slot(u0), *a1 = E.red.slot(u0 + 1);
-        void* args[] = {&a0, &a1, &c, &prm, &hout};
-        nq = kernel(body2, nq, (const void*)k_refine_outer_step, args, 1);
-      }
+      nq = control(body2, nq, {{RED_MAXABS, n, ex2_, nullptr}, {RED_MAXABS, m, ez2_, nullptr}},
+                   RefineOp{REFINE_OUTER_STEP, 0, 0, 0, nullptr, nullptr, nullptr, nullptr}, hout);
       {
         long nn = n, mm = m;
-        double *d1 = x, *d2 = z;
-        const double *s1 = candx_.p, *s2 = candz_.p;
-        void* args[] = {&oaccept, &nn, &d1, &s1, &oaccept, &mm, &d2, &s2};
-        nq = kernel(body2, nq, (const void*)k_refine_copy, args, cgrid);
-        double *e1 = ex_.p, *e2 = ez_.p;
-        const double *f1 = ex2_.p, *f2 = ez2_.p;
-        void* args2[] = {&ocont, &nn, &e1, &f1, &ocont, &mm, &e2, &f2};
-        kernel(body2, nq, (const void*)k_refine_copy, args2, cgrid);
+        double *d1 = x, *d2 = z, *e1 = ex_.p, *e2 = ez_.p;
+        const double *s1 = candx_.p, *s2 = candz_.p, *f1 = ex2_.p, *f2 = ez2_.p;
+        void* args[] = {&c, &nn, &d1, &s1, &e1, &f1, &mm, &d2, &s2, &e2, &f2};
+        kernel(body2, nq, (const void*)k_refine_keep, args, dim3(cgrid));
       }
       check(cudaGraphInstantiate(&built.exec, G, 0), "cudaGraphInstantiate");
       built.fixed = k_head + 1 + k_tail + 1;
-      built.per_inner = k_step + 2;
+      built.per_inner = k_step + 1;
       built.per_outer = k_ohead + 1 + k_otail + 1 + 2;
     } catch (...) {
       for (cudaGraph_t g : runs) cudaGraphDestroy(g);

@@ -31,7 +31,7 @@ extern "C" __global__ void k_nn_identity(int cnt, double* __restrict__ w, double
 // y = op(x) on the orthant rows; modes as k_congruence: 0 W, 1 W', 2 W^-1, 3 W^-T, 4 Hs, 5 Hs^-1.
 extern "C" __global__ void k_nn_cone(int cnt, const int* __restrict__ idx, int mode,
                                      const double* __restrict__ w, const double* __restrict__ x,
-                                     double* __restrict__ y, long ld) {
+                                     const double* __restrict__ base, double* __restrict__ y, long ld) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cnt) return;
   const long r = idx[i] + (long)blockIdx.y * ld;
@@ -43,7 +43,7 @@ extern "C" __global__ void k_nn_cone(int cnt, const int* __restrict__ idx, int m
     case 4: v = (wi * wi) * xi; break;
     default: v = xi / (wi * wi); break;
   }
-  y[r] = v;
+  y[r] = base ? v + base[r] : v;
 }
 
 // x = y o z (elementwise Jordan product of the orthant)
@@ -147,13 +147,13 @@ extern "C" __global__ void k_nn_margins(int cnt, const int* __restrict__ idx,
 // y[idx[i]] = alpha (A_nn x)_i + beta y[idx[i]]: one thread per orthant row (coalesced over i).
 extern "C" __global__ void k_nn_forward(int cnt, int n, const int* __restrict__ idx,
                                         const double* __restrict__ Ann, const double* __restrict__ x,
-                                        double alpha, double beta, double* __restrict__ y) {
+                                        double alpha, double beta, const double* base, double* y) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cnt) return;
   double acc = 0.0;
   for (int j = 0; j < n; ++j) acc = fma(Ann[i + (long)j * cnt], x[j], acc);
   const int r = idx[i];
-  y[r] = alpha * acc + ((beta == 0.0) ? 0.0 : beta * y[r]);
+  y[r] = alpha * acc + ((beta == 0.0) ? 0.0 : beta * base[r]);
 }
 
 // y[j] += alpha (A_nn' z)_j: one warp per column j (contiguous), fixed-order warp reduction.

@@ -2,8 +2,8 @@
 // with inner refinement against the unshifted Schur complement, recover, outer refinement against
 // the original operator: kkt/condensed/kkt.rs:275-318 with kkt/refinement.rs:118-191) runs as ONE
 // CUDA graph whose two refinement loops are WHILE conditional nodes.  After each straight run of
-// the graph a single thread reads the run's reduction slots, applies the reference's stopping
-// rule (tolerance abstol + reltol |b|, stop when the residual ratio falls below stop_ratio,
+// the graph one kernel reduces the run's norms and one thread of its last block applies the
+// reference's stopping rule (tolerance abstol + reltol |b|, stop when the residual ratio falls below stop_ratio,
 // keep the candidate only when it improved, at most max_iter steps) and sets the loop's
 // condition.  Every loop also stops once `guard` body executions have run, so no condition can
 // stay set.  The arithmetic is the host driver's, operation for operation, so the graph's
@@ -17,40 +17,34 @@ __device__ __forceinline__ void ctl_set(cudaGraphConditionalHandle h, bool go) {
   cudaGraphSetConditional(h, go ? 1u : 0u);
 }
 
-// Start of a reduced solve: slots |r|max, |e|max, finite(x) of the first pass (and, at the head
-// of a KKT solve, finite(bx), finite(bz)).  reset != 0 starts a new KKT solve.
-extern "C" __global__ void k_refine_head(const double* fin_bx, const double* fin_bz,
-                                         const double* nr, const double* ne, const double* fin_x,
-                                         int reset, RefineCtl* c, RefineParams p,
-                                         cudaGraphConditionalHandle h) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// Start of a reduced solve: |r|max, |e|max, finite(x) of the first pass (and, at the head of a KKT
+// solve, finite(bx), finite(bz)).  reset != 0 starts a new KKT solve.
+__device__ void refine_head(const double* v, int rows, int reset, RefineCtl* c, const RefineParams& p,
+                            cudaGraphConditionalHandle h) {
   if (reset) {
     RefineCtl z{};
     z.ok = 1;
     *c = z;
   }
   bool ok = c->ok != 0;
-  if (fin_bx && *fin_bx != 1.0) ok = false;
-  if (fin_bz && *fin_bz != 1.0) ok = false;
-  if (*fin_x != 1.0 || !isfinite(*ne)) ok = false;
+  for (int k = 3; k < rows; ++k)
+    if (v[k] != 1.0) ok = false;
+  if (v[2] != 1.0 || !isfinite(v[1])) ok = false;
   c->ok = ok ? 1 : 0;
-  c->normb = *nr;
-  c->norme = *ne;
+  c->normb = v[0];
+  c->norme = v[1];
   c->tol = p.abstol + p.reltol * c->normb;
   c->it = 0;
   c->accept = c->cont = 0;
   ctl_set(h, ok && !(c->norme <= c->tol) && p.max_iter > 0);
 }
 
-// After one inner step: slot |e2|max of the candidate's reduced residual.
-extern "C" __global__ void k_refine_step(const double* ne2, RefineCtl* c, RefineParams p,
-                                         cudaGraphConditionalHandle h) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// After one inner step: |e2|max of the candidate's reduced residual.
+__device__ void refine_step(double e, RefineCtl* c, const RefineParams& p, cudaGraphConditionalHandle h) {
   c->inner_steps++;
   c->guard++;
   bool go = false;
   int acc = 0;
-  const double e = *ne2;
   if (!isfinite(e)) {
     c->ok = 0;
   } else {
@@ -73,13 +67,11 @@ extern "C" __global__ void k_refine_step(const double* ne2, RefineCtl* c, Refine
   ctl_set(h, go);
 }
 
-// After recover + full residual: slots |bx|, |bz|, |ex|, |ez|.
-extern "C" __global__ void k_refine_outer_init(const double* nbx, const double* nbz,
-                                               const double* nex, const double* nez, RefineCtl* c,
-                                               RefineParams p, cudaGraphConditionalHandle h) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  c->onormb = host_max(*nbx, *nbz);
-  const double e = host_max(*nex, *nez);
+// After recover + full residual: |bx|, |bz|, |ex|, |ez|.
+__device__ void refine_outer_init(const double* v, RefineCtl* c, const RefineParams& p,
+                                  cudaGraphConditionalHandle h) {
+  c->onormb = host_max(v[0], v[1]);
+  const double e = host_max(v[2], v[3]);
   c->onorme = e;
   c->oit = 0;
   c->oaccept = c->ocont = 0;
@@ -93,17 +85,15 @@ extern "C" __global__ void k_refine_outer_init(const double* nbx, const double* 
   ctl_set(h, go);
 }
 
-// After one outer correction: slots |ex2|, |ez2| of the candidate's full residual.
-extern "C" __global__ void k_refine_outer_step(const double* nex2, const double* nez2,
-                                               RefineCtl* c, RefineParams p,
-                                               cudaGraphConditionalHandle h) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// After one outer correction: |ex2|, |ez2| of the candidate's full residual.
+__device__ void refine_outer_step(const double* v, RefineCtl* c, const RefineParams& p,
+                                  cudaGraphConditionalHandle h) {
   c->outer_steps++;
   c->guard++;
   bool go = false;
   int acc = 0;
   if (c->ok) {  // the correction's own solve passed its checks
-    const double e = host_max(*nex2, *nez2);
+    const double e = host_max(v[0], v[1]);
     if (!isfinite(e)) {
       c->ok = 0;
     } else {
@@ -127,17 +117,86 @@ extern "C" __global__ void k_refine_outer_step(const double* nex2, const double*
   ctl_set(h, go);
 }
 
-// d1 = s1 (n1 entries) when *f1 is set, d2 = s2 (n2 entries) when *f2 is set.
-extern "C" __global__ void k_refine_copy(const int* f1, long n1, double* d1, const double* s1,
-                                         const int* f2, long n2, double* d2, const double* s2) {
-  const bool a = *f1 != 0, b = *f2 != 0;
+// The norms of one control point and the control itself in one launch: grid row r is request r
+// (largest magnitude or all finite, both independent of the order of combination), the block that
+// arrives last folds every row, one thread of it applies the stopping rule and sets the loop's
+// condition, and after an inner step the block keeps the candidate and its residual (n entries).
+// A graph node costs about 3 us here whatever it computes, and a refined solve of a small system is
+// little else: norms, control and copy were three nodes each time.
+extern "C" __global__ void __launch_bounds__(256)
+k_refine(RedBatch b, double* __restrict__ partial, unsigned* __restrict__ ticket, int pitch, RefineOp op,
+         RefineCtl* c, RefineParams p, cudaGraphConditionalHandle h) {
+  __shared__ double red[8];
+  __shared__ double val[kRedBatchMax];
+  __shared__ int last, keep[2];
+  const RedReq q = b.r[blockIdx.y];
+  const bool fin = q.op == 3;  // RED_FINITE, else RED_MAXABS
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double acc = fin ? 1.0 : 0.0;
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < q.n; i += (long)gridDim.x * blockDim.x) {
+    const double v = q.x[i];
+    acc = fin ? fmin(acc, isfinite(v) ? 1.0 : 0.0) : fmax(acc, fabs(v));
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const double v = __shfl_xor_sync(0xffffffffu, acc, o);
+    acc = fin ? fmin(acc, v) : fmax(acc, v);
+  }
+  if (lane == 0) red[warp] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) acc = fin ? fmin(acc, red[w]) : fmax(acc, red[w]);
+    partial[blockIdx.y * pitch + blockIdx.x] = acc;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int r = warp; r < op.rows; r += 8) {
+    const bool f = b.r[r].op == 3;
+    double v = f ? 1.0 : 0.0;
+    for (int k = lane; k < (int)gridDim.x; k += 32) {
+      const double u = __ldcg(partial + r * pitch + k);
+      v = f ? fmin(v, u) : fmax(v, u);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double u = __shfl_xor_sync(0xffffffffu, v, o);
+      v = f ? fmin(v, u) : fmax(v, u);
+    }
+    if (lane == 0) val[r] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *ticket = 0u;
+    if (op.kind == REFINE_HEAD) refine_head(val, op.rows, op.reset, c, p, h);
+    else if (op.kind == REFINE_STEP) refine_step(val[0], c, p, h);
+    else if (op.kind == REFINE_OUTER_INIT) refine_outer_init(val, c, p, h);
+    else refine_outer_step(val, c, p, h);
+    keep[0] = op.kind == REFINE_STEP && c->accept;
+    keep[1] = op.kind == REFINE_STEP && c->cont;
+  }
+  __syncthreads();
+  if (keep[0])
+    for (long i = threadIdx.x; i < op.n; i += blockDim.x) op.x[i] = op.cand[i];
+  if (keep[1])
+    for (long i = threadIdx.x; i < op.n; i += blockDim.x) op.e[i] = op.e2[i];
+}
+
+// After an outer step: x1 <- y1 (n entries) and x2 <- y2 (m) when the candidate is kept, e1 <- f1 and
+// e2 <- f2 when the loop goes on.
+extern "C" __global__ void k_refine_keep(const RefineCtl* c, long n, double* x1, const double* y1, double* e1,
+                                         const double* f1, long m, double* x2, const double* y2, double* e2,
+                                         const double* f2) {
+  const bool a = c->oaccept != 0, b = c->ocont != 0;
   if (!a && !b) return;
   const long stride = (long)gridDim.x * blockDim.x;
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n1 + n2; i += stride) {
-    if (i < n1) {
-      if (a) d1[i] = s1[i];
-    } else if (b) {
-      d2[i - n1] = s2[i - n1];
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n + m; i += stride) {
+    if (i < n) {
+      if (a) x1[i] = y1[i];
+      if (b) e1[i] = f1[i];
+    } else {
+      if (a) x2[i - n] = y2[i - n];
+      if (b) e2[i - n] = f2[i - n];
     }
   }
 }

@@ -71,7 +71,7 @@ extern "C" __global__ void k_ms_forward(const BlockDesc* __restrict__ blocks, co
                                         const int* __restrict__ col_ptr, const int* __restrict__ col_idx,
                                         const double* __restrict__ w, const double* __restrict__ Q,
                                         const double* __restrict__ x, double alpha, double beta,
-                                        double* __restrict__ y) {
+                                        const double* base, double* y) {
   const MsDesc d = ms[blockIdx.x];
   const BlockDesc bd = blocks[d.j];
   const int n = bd.n, tn = n * (n + 1) / 2, c0 = col_ptr[d.j];
@@ -92,8 +92,8 @@ extern "C" __global__ void k_ms_forward(const BlockDesc* __restrict__ blocks, co
   }
   double v = (bi == bj) ? acc : 0.5 * acc;
   if (row != col) v *= SDPXG_SQRT2;
-  double* out = y + bd.svec_off + e;
-  *out = beta == 0.0 ? alpha * v : fma(alpha, v, beta * *out);
+  const int o = bd.svec_off + e;
+  y[o] = beta == 0.0 ? alpha * v : fma(alpha, v, beta * base[o]);
 }
 
 // p[col_ptr[j] + t] = w_t q_k' Z_rs q_k for the block's primitive t = (s, r, k): one thread each.

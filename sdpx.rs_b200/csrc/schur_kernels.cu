@@ -142,17 +142,20 @@ extern "C" __global__ void k_add_upper_csc(int n, const int* __restrict__ colptr
   }
 }
 
-// y[rows of block j] = alpha * Acol_j x[cols_j] + beta * y   (one CTA per block, thread/row)
-// One CTA per 64-row tile of a block (tile list ftile_blk / ftile_r0): 64 rows x 4 column
-// groups; the four partial sums are combined in a fixed order (deterministic).
-extern "C" __global__ void __launch_bounds__(256)
+// y[rows of block j] = alpha * Acol_j x[cols_j] + beta * base.  One CTA per 32-row tile of a block
+// (tile list ftile_blk / ftile_r0): one row a lane, the columns dealt to 16 warps, four loads in
+// flight a thread; the partial sums are combined in a fixed order (deterministic).  Bound by the
+// memory round trips of a thread's columns: at 200 columns 13 of them (64 rows and four column
+// groups a CTA had 50).
+#define FWD_GROUPS 16
+extern "C" __global__ void __launch_bounds__(32 * FWD_GROUPS)
 k_op_forward(const BlockDesc* __restrict__ blocks, const int* __restrict__ kcount,
              const int* __restrict__ col_ptr, const int* __restrict__ col_idx,
              const long* __restrict__ acol_off, const double* __restrict__ Acol,
              const int* __restrict__ ftile_blk, const int* __restrict__ ftile_r0,
-             const double* __restrict__ x, long ldx, double alpha, double beta,
-             double* __restrict__ y, long ldy) {
-  __shared__ double part[4][64];
+             const double* __restrict__ x, long ldx, double alpha, double beta, const double* base,
+             double* y, long ldy) {
+  __shared__ double part[FWD_GROUPS][32];
   const int j = ftile_blk[blockIdx.x], r0 = ftile_r0[blockIdx.x];
   const BlockDesc bd = blocks[j];
   const int tn = bd.n * (bd.n + 1) / 2;
@@ -160,22 +163,30 @@ k_op_forward(const BlockDesc* __restrict__ blocks, const int* __restrict__ kcoun
   const double* A = Acol + acol_off[j];
   const int* cols = col_idx + col_ptr[j];
   const double* xc = x + (long)blockIdx.y * ldx;
-  double* yc = y + (long)blockIdx.y * ldy;
-  const int rr = threadIdx.x & 63, g = threadIdx.x >> 6;
+  const int rr = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int r = r0 + rr;
-  double acc = 0.0;
-  if (r < tn)
-    for (int t = g; t < k; t += 4) acc = fma(A[(long)t * tn + r], xc[cols[t]], acc);
-  part[g][rr] = acc;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  if (r < tn) {
+    int t = g;
+    for (; t + 3 * FWD_GROUPS < k; t += 4 * FWD_GROUPS)
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        acc[u] = fma(A[(long)(t + u * FWD_GROUPS) * tn + r], xc[cols[t + u * FWD_GROUPS]], acc[u]);
+    for (; t < k; t += FWD_GROUPS) acc[0] = fma(A[(long)t * tn + r], xc[cols[t]], acc[0]);
+  }
+  part[g][rr] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
   __syncthreads();
   if (g == 0 && r < tn) {
-    double s = ((part[0][rr] + part[1][rr]) + part[2][rr]) + part[3][rr];
-    double prev = (beta == 0.0) ? 0.0 : beta * yc[bd.svec_off + r];
-    yc[bd.svec_off + r] = alpha * s + prev;
+    double s = 0.0;
+#pragma unroll
+    for (int u = 0; u < FWD_GROUPS; ++u) s += part[u][rr];
+    const long o = (long)blockIdx.y * ldy + bd.svec_off + r;
+    y[o] = alpha * s + ((beta == 0.0) ? 0.0 : beta * base[o]);
   }
 }
 
-// Per-block partial adjoint p[acol column] = Acol_j[:, t] . z_j  (one warp per column)
+// Per-block partial adjoint p[acol column] = Acol_j[:, t] . z_j  (one warp per column, eight loads
+// in flight a lane)
 extern "C" __global__ void k_op_adjoint_partial(const BlockDesc* __restrict__ blocks,
                                                 const int* __restrict__ wblk,
                                                 const int* __restrict__ wloc,
@@ -192,26 +203,32 @@ extern "C" __global__ void k_op_adjoint_partial(const BlockDesc* __restrict__ bl
   const int tn = bd.n * (bd.n + 1) / 2;
   const double* A = Acol + acol_off[j] + (long)t * tn;
   const double* zc = z + (long)blockIdx.y * ldz + bd.svec_off;
-  double acc = 0.0;
-  for (int r = lane; r < tn; r += 32) acc = fma(A[r], zc[r], acc);
+  double a8[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  int r = lane;
+  for (; r + 7 * 32 < tn; r += 8 * 32)
+#pragma unroll
+    for (int u = 0; u < 8; ++u) a8[u] = fma(A[r + 32 * u], zc[r + 32 * u], a8[u]);
+#pragma unroll
+  for (int u = 0; u < 7; ++u)
+    if (r + 32 * u < tn) a8[u] = fma(A[r + 32 * u], zc[r + 32 * u], a8[u]);
+  double acc = ((a8[0] + a8[1]) + (a8[2] + a8[3])) + ((a8[4] + a8[5]) + (a8[6] + a8[7]));
   acc = warp_sum(acc);
   if (lane == 0) p[(long)blockIdx.y * ldp + col_ptr[j] + t] = acc;
 }
 
-// y[i] = alpha * sum over (block, t) of constraint i of p[...] + beta * y[i]  (cone order)
+// y[i] = alpha * sum over (block, t) of constraint i of p[...] + beta * base[i]  (cone order)
 extern "C" __global__ void k_op_adjoint_gather(int n, const int* __restrict__ c2b_ptr,
                                                const int* __restrict__ c2b_blk,
                                                const int* __restrict__ c2b_loc,
                                                const int* __restrict__ col_ptr,
                                                const double* __restrict__ p, long ldp,
-                                               double alpha, double beta, double* __restrict__ y,
+                                               double alpha, double beta, const double* base, double* y,
                                                long ldy) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double* pc = p + (long)blockIdx.y * ldp;
   double acc = 0.0;
   for (int q = c2b_ptr[i]; q < c2b_ptr[i + 1]; ++q) acc += pc[col_ptr[c2b_blk[q]] + c2b_loc[q]];
-  double* yc = y + (long)blockIdx.y * ldy;
-  double prev = (beta == 0.0) ? 0.0 : beta * yc[i];
-  yc[i] = alpha * acc + prev;
+  const long o = (long)blockIdx.y * ldy + i;
+  y[o] = alpha * acc + ((beta == 0.0) ? 0.0 : beta * base[o]);
 }

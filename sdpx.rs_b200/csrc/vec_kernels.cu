@@ -155,10 +155,10 @@ extern "C" __global__ void k_diag_absmax(const double* __restrict__ H, int m,
 extern "C" __global__ void k_csr_spmv(int n, const int* __restrict__ rowptr,
                                       const int* __restrict__ colidx,
                                       const double* __restrict__ val, const double* __restrict__ x,
-                                      double alpha, double beta, double* __restrict__ y) {
+                                      double alpha, double beta, const double* base, double* y) {
   int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   double acc = 0.0;
   for (int p = rowptr[r]; p < rowptr[r + 1]; ++p) acc = fma(val[p], x[colidx[p]], acc);
-  y[r] = alpha * acc + (beta == 0.0 ? 0.0 : beta * y[r]);
+  y[r] = alpha * acc + (beta == 0.0 ? 0.0 : beta * base[r]);
 }
