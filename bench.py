@@ -181,8 +181,8 @@ def fp64_gemm_peak():
 def schur_model(prob, gram=False):
     """Algorithmic work per launch of the timed phases (flop or bytes).
 
-    factor: m^3/3 (Cholesky of the m x m Schur complement); trinv: m^3/3 (inverse of the
-    triangular factor); assemble: sum_j 4 k_j n_j^3 + k_j^2 n_j (n_j + 1) in the ordinary form,
+    factor: 2 m^3/3 (Cholesky of the m x m Schur complement and the inverse of its factor, one
+    launch; trinv, a launch of its own only for m > 16384: m^3/3); assemble: sum_j 4 k_j n_j^3 + k_j^2 n_j (n_j + 1) in the ordinary form,
     sum_j 8 n_j^3 + 3 k_j^2 in the rank-one Gram form; scale: 20 n_j^3 per block; trisolve and
     symv: 8 m^2 bytes (two triangles, or the full matrix once).
     """
@@ -201,7 +201,7 @@ def schur_model(prob, gram=False):
         assemble = sum(8.0 * d ** 3 + 3.0 * kj * kj for kj, d in zip(k, orders))
     else:
         assemble = sum(4.0 * kj * d ** 3 + 2.0 * kj * kj * d * (d + 1) / 2 for kj, d in zip(k, orders))
-    return {"n": n, "factor_flops": n ** 3 / 3.0, "trisolve_bytes": 8.0 * n * n,
+    return {"n": n, "factor_flops": 2.0 * n ** 3 / 3.0, "trisolve_bytes": 8.0 * n * n,
             "symv_bytes": 8.0 * n * n, "assemble_flops": assemble,
             "scale_flops": sum(20.0 * d ** 3 for d in orders)}
 
@@ -591,7 +591,7 @@ def run_ours(args, world, rank, local):
                 "note": "INT8 pipe; peak = cuBLASLt INT8 GEMM 8192^3 (torch._int_mm) measured in this run"}
     elif dom in ("factor", "trinv", "assemble", "scale", "cone", "step"):
         fp64 = fp64_gemm_peak()
-        flops = {"factor": half_flops, "trinv": half_flops,
+        flops = {"factor": 2.0 * half_flops, "trinv": half_flops,
                  "assemble": model["assemble_flops"], "scale": model["scale_flops"]}.get(dom)
         if flops is None:
             flops = sum(4.0 * d ** 3 for _, d in prob.cones)
@@ -600,7 +600,7 @@ def run_ours(args, world, rank, local):
                 "frac": achieved / fp64, "traffic": traffic_from_profile(dom),
                 "kernel": "k_chol_dataflow" if dom == "factor" else dom, "launch_ms": per * 1e3,
                 "note": "FP64 pipe; the split form factors two diagonal halves of order ~m/2 "
-                        "(n^3/3 flop per launch); peak = cuBLAS DGEMM 8192^3 measured in this run "
+                        "(2 n^3/3 flop per launch: factor and inverse); peak = cuBLAS DGEMM 8192^3 measured in this run "
                         "(FP64 is not in MEASURED_PEAKS.json)"}
     else:
         nbytes = model["trisolve_bytes"] if dom == "trisolve" else model["symv_bytes"]

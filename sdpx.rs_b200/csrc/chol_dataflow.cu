@@ -13,10 +13,15 @@
 //    rows, left-looking, in registers (the tile is read and written once, its operands stream
 //    through a two-stage shared-memory ring), then FULL(i, j > i+1): U(i, j) = U_ii^-T (...), or
 //    PRE(i, i) and PRE(i, i+1): the sum up to what the chain adds itself;
+//  * the inverse of the factor, X = U^-1, is part of the same launch: INV(i, j) forms
+//    X(i, j) = -(sum_{i <= s < j} X(i, s) U(s, j)) X(j, j) (INV(j, j) copies X(j, j)), a few tile rows
+//    behind the factorization, on SMs that would wait for the chain.  A launch pair per level of a
+//    recursive inverse after the factorization took 390 us at m = 2000 and 1450 at m = 4000;
 //  * progress words in global memory (acquire/release at GPU scope): prog[j] counts the final
-//    tiles of tile column j from the top (a tile is final only after the one above it), one flag
-//    per PRE tile.  Every item's inputs come from earlier tickets or from chain steps whose own
-//    inputs do, and a ticket is only taken by a running CTA, so the schedule cannot deadlock;
+//    tiles of tile column j of U from the top (a tile is final only after the one above it),
+//    xprog[i] those of tile row i of X up to the column, one flag per PRE tile.  Every item's inputs
+//    come from earlier tickets or from chain steps whose own inputs do, and a ticket is only taken by
+//    a running CTA, so the schedule cannot deadlock;
 //  * every wait is bounded: past the limit the CTA sets SDPXG_ST_SYNC_TIMEOUT and the shared
 //    error word, and every CTA leaves at its next wait;
 //  * ten warps: eight work on the FP64 tensor cores (mma.sync m8n8k4 f64), warp 8 polls the
@@ -26,9 +31,10 @@
 // What bounds it: below m of about 3000 the chain (15 us a step: POTRF 9, TRSM 2, the update of the
 // next diagonal tile 2.2, stores 1), above it the tensor-pipe time of the tile sums (one 64^3
 // product is 2.1 us of an SM's FP64 pipe).  Right-looking with every tile task reloaded from L2 and
-// the inverse formed after the panels it took 27 us a step: m = 1024 457 us, 2000 864, 4000 3206; so
-// 242, 486 and 1274.  Holding U_kk^-T back to copy it out by one warp was slower (627 at m = 2000):
-// the tiles of row k wait for it.
+// the inverse of the diagonal tiles formed after the panels the factor alone took 27 us a step:
+// m = 1024 457 us, 2000 864, 4000 3206; so 242, 486 and 1274, and with the whole inverse 248, 533 and
+// 2115.  Holding U_kk^-T back to copy it out by one warp was slower (627 at m = 2000): the tiles of
+// row k wait for it.
 #include "common.cuh"
 
 #define DF_NB 64
@@ -40,7 +46,7 @@
 #define DF_WAIT_NS 20000000000ull
 #define DFS(A, i, j) (A)[(i) + (j) * DF_LD]
 
-enum : unsigned { DF_FULL = 1u, DF_PRE = 2u, DF_CHAIN = 3u };
+enum : unsigned { DF_INV = 0u, DF_FULL = 1u, DF_PRE = 2u, DF_CHAIN = 3u };
 
 namespace {
 
@@ -159,6 +165,19 @@ __device__ __forceinline__ void df_sub_atb(const double* As, const double* Bs, d
     const double b = -DFS(Bs, kk, 8 * w + r);
 #pragma unroll
     for (int R = 0; R < 8; ++R) dmma_m8n8k4(acc[R][0], acc[R][1], DFS(As, kk, 8 * R + r), b);
+  }
+}
+
+// acc (this warp's 8-column block w) -= A B over K = 64.
+__device__ __forceinline__ void df_sub_ab(const double* As, const double* Bs, double (&acc)[8][2]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int q = lane & 3, r = lane >> 2;
+#pragma unroll 4
+  for (int ks = 0; ks < DF_NB / 4; ++ks) {
+    const int kk = ks * 4 + q;
+    const double b = -DFS(Bs, kk, 8 * w + r);
+#pragma unroll
+    for (int R = 0; R < 8; ++R) dmma_m8n8k4(acc[R][0], acc[R][1], DFS(As, 8 * R + r, kk), b);
   }
 }
 
@@ -536,13 +555,16 @@ __device__ void df_chain(double* __restrict__ F, long ld, int m, int nt, int* pr
 
 // items[t] = type << 30 | k << 20 | i << 10 | j (topological order, built on the host):
 //   FULL (k = i): U(i, j) = U_ii^-T (H(i, j) - sum_{s < i} U(s, i)' U(s, j));
-//   PRE: H(i, j) -= sum_{s < k} U(s, i)' U(s, j), for j = i (k = i - 1) and j = i + 1 (k = i).
-// F: n x n with the even leading dimension ld.  sync = {ticket, error, prog[nt], pre_o[nt],
-// pre_d[nt]}, zero at launch.
+//   PRE: H(i, j) -= sum_{s < k} U(s, i)' U(s, j), for j = i (k = i - 1) and j = i + 1 (k = i);
+//   INV: X(i, j) into Uinv and, transposed, UinvT (n x n, leading dimension m), and into Xr, from
+//   which later INV items read it.
+// F and Xr: even leading dimensions ld and ldx (Xr may be Uinv when m is even).
+// sync = {ticket, error, prog[nt], pre_o[nt], pre_d[nt], xprog[nt]}, zero at launch.
 extern "C" __global__ void __launch_bounds__(DF_THREADS, 1)
 k_chol_dataflow(double* __restrict__ F, long ld, int m, int nt, const unsigned* __restrict__ items, int nitems,
                 int* __restrict__ sync, double eps, double delta, int dynamic, const double* __restrict__ diag0,
-                double* __restrict__ Dinv, uint32_t* __restrict__ status) {
+                double* __restrict__ Dinv, double* Xr, long ldx, double* Uinv, double* UinvT,
+                uint32_t* __restrict__ status) {
   extern __shared__ __align__(16) double df_sm[];
   __shared__ DfShared sh;
   double* T = df_sm;                  // four tiles: two ring stages of two operands
@@ -552,6 +574,7 @@ k_chol_dataflow(double* __restrict__ F, long ld, int m, int nt, const unsigned* 
   int* prog = sync + 2;
   int* pre_o = prog + nt;
   int* pre_d = pre_o + nt;
+  int* xprog = pre_d + nt;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, q = lane & 3, r = lane >> 2;
   unsigned cnt = 0;  // ring stages used so far
   bool ring = false;
@@ -562,7 +585,7 @@ k_chol_dataflow(double* __restrict__ F, long ld, int m, int nt, const unsigned* 
     const int t = sh.item;
     if (t >= nitems) break;
     const unsigned code = items[t];
-    const int type = (int)(code >> 30), k = (int)((code >> 20) & 1023u);
+    const int type = (int)(code >> 30);
     const int i = (int)((code >> 10) & 1023u), j = (int)(code & 1023u);
     if (!ring) {  // the chain's tiles are released by one thread, the ring's by the eight warps
       if (threadIdx.x == 0) {
@@ -587,18 +610,22 @@ k_chol_dataflow(double* __restrict__ F, long ld, int m, int nt, const unsigned* 
     }
     const int i0 = i * DF_NB, j0 = j * DF_NB;
     const int ni = min(DF_NB, m - i0), nc = min(DF_NB, m - j0);
-    const bool full = type == (int)DF_FULL;
+    const bool full = type == (int)DF_FULL, inv = type == (int)DF_INV;
+    // tile rows s0 .. s1-1 of the sum, then one more stage with the tile U_dd^-T (d = i or j)
+    const int s0 = inv ? i : 0, s1 = inv ? j : (int)((code >> 20) & 1023u);
+    const bool close = full || inv;
+    const int d = full ? i : j;
     if (w == 8) {  // operands
-      int pi = 0, pj = 0;
-      for (int s = 0; s < k + (full ? 1 : 0); ++s) {
+      int pa = 0, pj = 0;
+      for (int s = s0; s < s1 + (close ? 1 : 0); ++s) {
         int ok = 1;
         if (lane == 0) {
-          if (s < k) {
-            if (pi <= s) pi = df_wait(prog + i, s + 1, err, status);
-            if (pi > 0 && pj <= s) pj = df_wait(prog + j, s + 1, err, status);
-            ok = pi > 0 && pj > 0;
+          if (s < s1) {
+            if (pa <= s) pa = df_wait(inv ? xprog + i : prog + i, s + 1, err, status);
+            if (pa > 0 && pj <= s) pj = df_wait(prog + j, s + 1, err, status);
+            ok = pa > 0 && pj > 0;
           } else {
-            ok = df_wait(prog + i, i + 1, err, status) > 0;  // U_ii^-T
+            ok = df_wait(prog + d, d + 1, err, status) > 0;
           }
           if (!ok) *(volatile int*)&sh.abort = 1;
         }
@@ -607,11 +634,12 @@ k_chol_dataflow(double* __restrict__ F, long ld, int m, int nt, const unsigned* 
         const unsigned x = cnt & 1;
         if (!ok || !df_bar_wait(&sh.empty[x], ((cnt >> 1) & 1) ^ 1, &sh)) break;
         double* As = T + 2 * x * DF_TILE;
-        if (s < k) {
-          df_stream_tile(As, F + s * DF_NB + (long)i0 * ld, ld, DF_NB, ni);
-          if (i != j) df_stream_tile(As + DF_TILE, F + s * DF_NB + (long)j0 * ld, ld, DF_NB, nc);
+        if (s == s1) {
+          df_stream_tile(As, Dinv + (long)d * DF_NB * DF_NB, DF_NB, DF_NB, DF_NB);
         } else {
-          df_stream_tile(As, Dinv + (long)i * DF_NB * DF_NB, DF_NB, DF_NB, DF_NB);
+          if (inv) df_stream_tile(As, Xr + i0 + (long)s * DF_NB * ldx, ldx, DF_NB, DF_NB);
+          else df_stream_tile(As, F + s * DF_NB + (long)i0 * ld, ld, DF_NB, ni);
+          if (inv || i != j) df_stream_tile(As + DF_TILE, F + s * DF_NB + (long)j0 * ld, ld, DF_NB, nc);
         }
         df_stream_done(&sh.full[x]);
         ++cnt;
@@ -623,32 +651,35 @@ k_chol_dataflow(double* __restrict__ F, long ld, int m, int nt, const unsigned* 
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int row = 8 * R + r, col = 8 * w + 2 * q + e;
-          acc[R][e] = (row < ni && col < nc) ? __ldcg(F + (i0 + row) + (long)(j0 + col) * ld) : 0.0;
+          acc[R][e] = (!inv && row < ni && col < nc) ? __ldcg(F + (i0 + row) + (long)(j0 + col) * ld) : 0.0;
         }
       bool ok = true;
-      for (int s = 0; s < k && ok; ++s) {
+      for (int s = s0; s < s1; ++s) {
         const unsigned x = cnt & 1;
         ok = df_bar_wait(&sh.full[x], (cnt >> 1) & 1, &sh);
         if (!ok) break;
         const double* As = T + 2 * x * DF_TILE;
-        df_sub_atb(As, i == j ? As : As + DF_TILE, acc);
+        if (inv) df_sub_ab(As, As + DF_TILE, acc);
+        else df_sub_atb(As, i == j ? As : As + DF_TILE, acc);
         __syncwarp();
         if (lane == 0) df_bar_arrive(&sh.empty[x]);
         ++cnt;
       }
-      if (ok && full) {  // U(i, j) = U_ii^-T acc, this warp's columns through the stage's second tile
+      if (close) {
         const unsigned x = cnt & 1;
-        ok = df_bar_wait(&sh.full[x], (cnt >> 1) & 1, &sh);
-        if (ok) {
-          const double* Ys = T + 2 * x * DF_TILE;
-          double* Bs = T + (2 * x + 1) * DF_TILE;
+        const double* Ys = T + 2 * x * DF_TILE;  // U_dd^-T
+        double* Bs = T + (2 * x + 1) * DF_TILE;
+        ok = df_all(ok && df_bar_wait(&sh.full[x], (cnt >> 1) & 1, &sh));
+        if (ok && (full || i != j)) {
 #pragma unroll
           for (int R = 0; R < 8; ++R)
 #pragma unroll
             for (int e = 0; e < 2; ++e) DFS(Bs, 8 * R + r, 8 * w + 2 * q + e) = acc[R][e];
-          __syncwarp();
 #pragma unroll
           for (int R = 0; R < 8; ++R) acc[R][0] = acc[R][1] = 0.0;
+        }
+        if (ok && full) {  // U(i, j) = U_ii^-T acc: this warp's columns alone
+          __syncwarp();
 #pragma unroll
           for (int ks = 0; ks < DF_NB / 4; ++ks) {
             const int kk = ks * 4 + q;
@@ -657,10 +688,23 @@ k_chol_dataflow(double* __restrict__ F, long ld, int m, int nt, const unsigned* 
             for (int R = 0; R < 8; ++R)
               if (R >= ks / 2) dmma_m8n8k4(acc[R][0], acc[R][1], DFS(Ys, 8 * R + r, kk), b);
           }
-          __syncwarp();
-          if (lane == 0) df_bar_arrive(&sh.empty[x]);
-          ++cnt;
+        } else if (ok && i != j) {  // X(i, j) = acc X(j, j), X(j, j)(k, c) = U_jj^-T(c, k)
+          df_sync<BAR_MMA, DF_MMA>();
+          for (int ks = 0; ks < 2 * w + 2; ++ks) {
+            const int kk = ks * 4 + q;
+            const double b = DFS(Ys, 8 * w + r, kk);
+#pragma unroll
+            for (int R = 0; R < 8; ++R) dmma_m8n8k4(acc[R][0], acc[R][1], DFS(Bs, 8 * R + r, kk), b);
+          }
+        } else if (ok) {  // X(j, j)
+#pragma unroll
+          for (int R = 0; R < 8; ++R)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) acc[R][e] = DFS(Ys, 8 * w + 2 * q + e, 8 * R + r);
         }
+        __syncwarp();
+        if (ok && lane == 0) df_bar_arrive(&sh.empty[x]);
+        ++cnt;
       }
       if (ok) {
 #pragma unroll
@@ -668,13 +712,21 @@ k_chol_dataflow(double* __restrict__ F, long ld, int m, int nt, const unsigned* 
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int row = 8 * R + r, col = 8 * w + 2 * q + e;
-            if (row < ni && col < nc) F[(i0 + row) + (long)(j0 + col) * ld] = acc[R][e];
+            if (row >= ni || col >= nc) continue;
+            if (inv) {
+              Uinv[(i0 + row) + (long)(j0 + col) * m] = acc[R][e];
+              UinvT[(j0 + col) + (long)(i0 + row) * m] = acc[R][e];
+              if (Xr != Uinv) Xr[(i0 + row) + (long)(j0 + col) * ldx] = acc[R][e];
+            } else {
+              F[(i0 + row) + (long)(j0 + col) * ld] = acc[R][e];
+            }
           }
       }
       df_sync<BAR_MMA, DF_MMA>();
       if (threadIdx.x == 0 && ok) {
         __threadfence();
-        if (full) df_st_release(prog + j, i + 1);
+        if (inv) df_st_release(xprog + i, j + 1);
+        else if (full) df_st_release(prog + j, i + 1);
         else df_st_release((i == j ? pre_d : pre_o) + i, 1);
       }
     }

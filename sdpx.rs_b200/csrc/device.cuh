@@ -234,7 +234,7 @@ __global__ void k_gram_forward(const BlockDesc*, const int*, const int*, const i
 __global__ void k_gram_adjoint(const BlockDesc*, const int*, const int*, const int*, const int*,
                                const long*, const double*, const double*, const double*, double*);
 __global__ void k_chol_dataflow(double*, long, int, int, const unsigned*, int, int*, double, double, int,
-                                const double*, double*, uint32_t*);
+                                const double*, double*, double*, long, double*, double*, uint32_t*);
 __global__ void k_syrk_update(double*, long, int, int);
 __global__ void k_trtri_diag(int, const double*, double*, double*);
 __global__ void k_trinv_level(const double*, long, double*, double*, double*, int, int, int);

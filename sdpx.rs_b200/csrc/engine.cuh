@@ -94,21 +94,31 @@ inline bool rank_one_column(const double* v, int n, double* u, double* sigma) {
 // (ticket 0: every POTRF(k), TRSM(k, k+1) and the update of tile (k+1, k+1) by row k):
 //   PRE(i, i) (i >= 2): the sums of rows < i - 1 of the diagonal tile; PRE(i, i+1) (i >= 1): the sums
 //   of rows < i of the tile right of it; FULL(i, j >= i + 2): the whole tile U(i, j).
-// The PRE items of a row come first: the chain waits for them.
-// Encoded type << 30 | k << 20 | i << 10 | j with k the number of rows an item sums over.
-enum : unsigned { kCholFull = 1u, kCholPre = 2u, kCholChain = 3u };
-inline std::vector<unsigned> chol_schedule(int nt) {
+// The PRE items of a row come first: the chain waits for them.  `lag` rows behind, the inverse
+// X = U^-1: INV(i, j), i <= j, of tile column j after the items of row j + lag.  Any lag is valid;
+// measured with lags 1, 4, 8 and 16 at m = 1024: 248, 246, 248, 248 us; 2000: 537, 529, 533, 545;
+// 3000: 1183, 1045, 1020, 1032; 4000: 2385, 2115, 2115, 2112.  Too close, and the inverse takes SMs
+// from the tiles that the chain waits for.
+// Encoded type << 30 | k << 20 | i << 10 | j with k the number of rows of U above row i that an item
+// waits for (0 for the diagonal tiles of X).
+enum : unsigned { kCholInv = 0u, kCholFull = 1u, kCholPre = 2u, kCholChain = 3u };
+inline std::vector<unsigned> chol_schedule(int nt, int lag = 8) {
   auto code = [](unsigned type, int k, int i, int j) {
     return (type << 30) | ((unsigned)k << 20) | ((unsigned)i << 10) | (unsigned)j;
   };
   std::vector<unsigned> it;
   if (nt <= 0) return it;
   it.push_back(code(kCholChain, 0, 0, 0));
+  auto inverse = [&](int j) {
+    for (int i = j; i >= 0; --i) it.push_back(code(kCholInv, i == j ? 0 : i, i, j));
+  };
   for (int i = 0; i < nt; ++i) {
     if (i >= 2) it.push_back(code(kCholPre, i - 1, i, i));
     if (i >= 1 && i + 1 < nt) it.push_back(code(kCholPre, i, i, i + 1));
     for (int j = i + 2; j < nt; ++j) it.push_back(code(kCholFull, i, i, j));
+    if (i >= lag) inverse(i - lag);
   }
+  for (int j = std::max(nt - lag, 0); j < nt; ++j) inverse(j);
   return it;
 }
 
@@ -117,7 +127,7 @@ inline std::vector<unsigned> chol_schedule(int nt) {
 // which k_chol_dataflow cannot deadlock (the chain, ticket 0, only waits on items that precede
 // every item waiting on it) -- and that every tile ends factored.  False on any violation.
 inline bool chol_schedule_valid(const std::vector<unsigned>& it, int nt) {
-  std::vector<int> prog(nt, 0), pre_d(nt, 0), pre_o(nt, 0);  // the kernel's progress words
+  std::vector<int> prog(nt, 0), pre_d(nt, 0), pre_o(nt, 0), xprog(nt, 0);  // the kernel's progress words
   bool chain = false;
   int step = 0;            // next chain step
   bool diag_done = false;  // the chain's POTRF of `step` is done, its TRSM is pending
@@ -150,6 +160,11 @@ inline bool chol_schedule_valid(const std::vector<unsigned>& it, int nt) {
       continue;
     }
     advance();
+    if (type == kCholInv) {  // X(i, j): the row of X before it, the column of U and X(j, j)
+      if (i > j || k != (i == j ? 0 : i) || prog[j] != j + 1 || xprog[i] != (i == j ? 0 : j)) return false;
+      xprog[i] = j + 1;
+      continue;
+    }
     if (prog[i] < k || prog[j] < k) return false;  // the rows an item sums over are final
     if (type == kCholFull) {
       if (k != i || j < i + 2 || prog[i] != i + 1 || prog[j] != i) return false;
@@ -167,7 +182,7 @@ inline bool chol_schedule_valid(const std::vector<unsigned>& it, int nt) {
   advance();
   if (!chain || step != nt) return false;
   for (int j = 0; j < nt; ++j)
-    if (prog[j] != j + 1) return false;
+    if (prog[j] != j + 1 || xprog[j] != nt) return false;
   return true;
 }
 constexpr int kNB = 64;
@@ -776,7 +791,7 @@ class Engine {
     check(cudaMemsetAsync(gv_cnt_.p, 0, gv_cnt_.n * sizeof(unsigned), st), "gemv counters");
     Uinv_.alloc((size_t)n * n);
     UinvT_.alloc((size_t)n * n);
-    Tmp_.alloc((size_t)n * n);
+    Tmp_.alloc((size_t)factor_ld(n) * n);
     make_schedule(nchol, df_list_, df_sync_, &df_items_, &df_grid_);
     if (split_active()) prepare_split();
     step_out_.alloc(2 * (nblk + 1));
@@ -1101,7 +1116,7 @@ class Engine {
     if (!chol_schedule_valid(items, nt)) throw CudaError("invalid Cholesky work list");
     list.alloc(items.size());
     list.upload(items.data(), items.size(), st);
-    sync.alloc(2 + 3 * (size_t)nt);
+    sync.alloc(2 + 4 * (size_t)nt);
     int sms = 0;
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "SM count");
     // one CTA per SM: the chain CTA (the critical path) then has its SM to itself; the
@@ -1127,7 +1142,7 @@ class Engine {
     s.diag0.alloc(ns);
     s.Uinv.alloc((size_t)ns * ns);
     s.UinvT.alloc((size_t)ns * ns);
-    s.Tmp.alloc((size_t)ns * ns);
+    s.Tmp.alloc((size_t)factor_ld(ns) * ns);
     s.b = FactorBufs();
     s.b.n = ns;
     s.b.nchol = nt;
@@ -1152,11 +1167,11 @@ class Engine {
     if (diag_src)
       ++g_launches, k_strided_diag<<<(b.n + 255) / 256, 256, 0, st>>>(diag_src, diag_stride, b.n, eps, b.diag0);
     if (b.df_items > 0) {  // one persistent launch over the whole tile schedule
-      check(cudaMemsetAsync(b.df_sync, 0, (2 + 3 * (size_t)b.nchol) * sizeof(int), st),
+      check(cudaMemsetAsync(b.df_sync, 0, (2 + 4 * (size_t)b.nchol) * sizeof(int), st),
             "dataflow sync reset");
       ++g_launches, k_chol_dataflow<<<b.df_grid, kDfThreads, kSmemDf, st>>>(
           b.F, b.ldf, b.n, b.nchol, b.df_list, b.df_items, b.df_sync, dyn_eps, dyn_delta, dynamic ? 1 : 0, b.diag0,
-          b.Dinv, status_);
+          b.Dinv, b.ldf == b.n ? b.Uinv : b.Tmp, b.ldf, b.Uinv, b.UinvT, status_);
     }
     for (int kb = 0; b.df_items == 0 && kb < b.nchol; ++kb) {
       ++g_launches, k_potrf_diag<<<1, 1024, kSmemTrtri, st>>>(b.F, b.ldf, b.n, kb, dyn_eps, dyn_delta, dynamic ? 1 : 0,
@@ -1169,8 +1184,10 @@ class Engine {
     }
     launched("factor");
   }
-  // X = U^-1 of one factorisation: diagonal tiles, then one batched GEMM pair per level.
+  // X = U^-1 of one factorisation beyond the dataflow launch's tile limit (that launch forms X
+  // itself): diagonal tiles, then one batched GEMM pair per level.
   void launch_trinv(const FactorBufs& b) {
+    if (b.df_items > 0) return;
     ++g_launches, k_trtri_diag<<<b.nchol, SDPXG_THREADS, 0, st>>>(b.n, b.Dinv, b.Uinv, b.UinvT);
     for (int level = 1; (1 << (level - 1)) < b.nchol; ++level) {
       const int g = 1 << level, h = g >> 1;
@@ -1225,15 +1242,15 @@ class Engine {
     check(cudaMemsetAsync(oz_status_word(), 0, sizeof(uint32_t), st), "memset");
     // phase timers: the dataflow launches under KT_FACTOR, the diagonal-block inverses under
     // KT_TRINV, the split-precision products and the assembly under KT_SPLIT
+    // the inverse kernels write the upper triangles only; the split-precision products read
+    // X11 and X22 whole, so their lower triangles must be zeros, not a recycled block's contents
+    check(cudaMemsetAsync(sub1_.Uinv.p, 0, (size_t)n1 * n1 * sizeof(double), st), "memset");
+    check(cudaMemsetAsync(sub2_.Uinv.p, 0, (size_t)n2 * n2 * sizeof(double), st), "memset");
     copy_block(sub1_.H, n1, Hsave_, ldn, n1, n1);
     copy_block(sub2_.H, n2, Hsave_ + (long)n1 * ldn + n1, ldn, n2, n2);
     tbegin(KT_FACTOR);
     launch_chol(sub1_.b, eps, dynamic, dyn_eps, dyn_delta);
     tend(KT_FACTOR);
-    // the inverse kernels write the upper triangles only; the split-precision products read
-    // X11 and X22 whole, so their lower triangles must be zeros, not a recycled block's contents
-    check(cudaMemsetAsync(sub1_.Uinv.p, 0, (size_t)n1 * n1 * sizeof(double), st), "memset");
-    check(cudaMemsetAsync(sub2_.Uinv.p, 0, (size_t)n2 * n2 * sizeof(double), st), "memset");
     tbegin(KT_TRINV);
     launch_trinv(sub1_.b);
     tend(KT_TRINV);
