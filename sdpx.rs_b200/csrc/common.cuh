@@ -19,9 +19,11 @@
 #define SDPXG_THREADS 256         // dense tile kernels (their thread maps assume 256)
 #define SDPXG_CONE_THREADS 1024   // one CTA per PSD block
 #define SDPXG_NT_SVD_THREADS 512  // the NT scaling's Jacobi launch (8 warps iterate, 128 registers)
+#define SDPXG_EIG_THREADS 256     // step length and margins (tridiagonalisation in 4 warps' registers)
+#define SDPXG_TRIDIAG_WORK 544    // doubles of shared scratch for cta_tridiagonalize
+#define SDPXG_STURM_WORK (2 * SDPXG_NMAX)  // and for cta_eig_min / cta_eig_all
 #define SDPXG_RSQRT2 0.70710678118654752440
 #define SDPXG_SQRT2 1.41421356237309504880
-#define SDPXG_CHOL_SCRATCH (3 * SDPXG_NMAX)  // doubles of shared scratch for cta_cholesky_lower
 
 // Device status bits reported by the kernels (read back by the host after each phase).
 enum SdpxgStatus : uint32_t {
@@ -143,19 +145,30 @@ __device__ __forceinline__ void cta_zero_mat(double* M) {
 // M = smat(v): symmetric matrix from an svec (zero padded to 64 x 64).  Column j of the upper
 // triangle is contiguous in the svec (v[j(j+1)/2 + i], i <= j): one warp per column reads it
 // coalesced and writes both triangles.
+// M = smat(v), zero padded to 64 x 64: one warp a column, the loads of four columns in flight.
 __device__ __forceinline__ void cta_load_smat(double* M, const double* __restrict__ v, int n) {
-  for (int e = threadIdx.x; e < SDPXG_NMAX * SDPXG_NMAX; e += blockDim.x) {
-    const int i = e % SDPXG_NMAX, j = e / SDPXG_NMAX;
-    if (i >= n || j >= n) SM(M, i, j) = 0.0;
-  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  for (int j = warp; j < n; j += nwarps) {
-    const double* col = v + j * (j + 1) / 2;
-    for (int i = lane; i <= j; i += 32) {
-      double x = col[i];
-      if (i != j) x *= SDPXG_RSQRT2;
-      SM(M, i, j) = x;
-      SM(M, j, i) = x;
+  for (int j0 = warp; j0 < SDPXG_NMAX; j0 += 4 * nwarps) {
+    double x[4][2];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = j0 + u * nwarps;
+      const double* col = v + j * (j + 1) / 2;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) x[u][h] = (j < n && lane + 32 * h <= j) ? col[lane + 32 * h] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = j0 + u * nwarps;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h;
+        if (j < SDPXG_NMAX && i <= j) {
+          const double y = i != j ? x[u][h] * SDPXG_RSQRT2 : x[u][h];
+          SM(M, i, j) = y;
+          SM(M, j, i) = y;
+        }
+      }
     }
   }
 }
@@ -169,10 +182,20 @@ __device__ __forceinline__ void cta_store_svec(double* __restrict__ v, const dou
   }
 }
 
+// M = the n x n matrix at g, zero padded to 64 x 64, eight loads in flight per thread.
 __device__ __forceinline__ void cta_load_mat(double* M, const double* __restrict__ g, int n) {
-  for (int e = threadIdx.x; e < SDPXG_NMAX * SDPXG_NMAX; e += blockDim.x) {
-    int i = e % SDPXG_NMAX, j = e / SDPXG_NMAX;
-    SM(M, i, j) = (i < n && j < n) ? g[i + j * n] : 0.0;
+  for (int e0 = threadIdx.x; e0 < SDPXG_NMAX * SDPXG_NMAX; e0 += 8 * blockDim.x) {
+    double x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int e = e0 + u * blockDim.x, i = e % SDPXG_NMAX, j = e / SDPXG_NMAX;
+      x[u] = (i < n && j < n) ? g[i + j * n] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int e = e0 + u * blockDim.x;
+      if (e < SDPXG_NMAX * SDPXG_NMAX) SM(M, e % SDPXG_NMAX, e / SDPXG_NMAX) = x[u];
+    }
   }
 }
 
@@ -235,87 +258,16 @@ __device__ __forceinline__ void cta_gemm(double* C, const double* A, bool ta, co
   }
 }
 
-// In-place lower Cholesky A = L L' (lower triangle of A used), the shared-memory form for CTAs of
-// fewer than 256 threads.  The update is lagged so one barrier per column suffices: the trailing matrix is updated with the unscaled
-// column divided by the pivot, and columns are scaled at the end.  The thread that
-// finishes the next diagonal entry computes its reciprocal once and publishes it for the
-// next step (0 marks a pivot that is not positive and finite: the reciprocal of a finite
-// positive double is never 0).  Step k visits only the trailing (n-k-1)^2 square.
-// cta_cholesky_lower2 factors two matrices of the same order at once (one barrier per
-// column for both, the same arithmetic per entry); a failed matrix stops being updated and
-// reports false, the other one carries on.
-// `piv` is SDPXG_CHOL_SCRATCH doubles of shared memory per matrix: pivots, reciprocals, roots.
-__device__ inline void cta_cholesky_lower2_smem(double* A, double* B, int n, double* pivA,
-                                                double* pivB, bool* okA, bool* okB) {
-  double* pinvA = pivA + SDPXG_NMAX;
-  double* pinvB = pivB + SDPXG_NMAX;
-  const bool two = (B != nullptr);
-  if (threadIdx.x == 0 && n > 0) {
-    const double a = SM(A, 0, 0);
-    pivA[0] = a;
-    pinvA[0] = (a > 0.0 && isfinite(a)) ? 1.0 / a : 0.0;
-    if (two) {
-      const double b = SM(B, 0, 0);
-      pivB[0] = b;
-      pinvB[0] = (b > 0.0 && isfinite(b)) ? 1.0 / b : 0.0;
-    }
-  }
-  bool liveA = true, liveB = two;
-  for (int k = 0; k < n; ++k) {
-    __syncthreads();
-    const double dA = pinvA[k];  // written in step k - 1, not touched in step k
-    const double dB = two ? pinvB[k] : 0.0;
-    liveA = liveA && dA != 0.0;
-    liveB = liveB && dB != 0.0;
-    if (!liveA && !liveB) break;
-    const int w = n - k - 1, tot = w * w;
-    const int lim = two ? 2 * tot : tot;
-    for (int e = threadIdx.x; e < lim; e += blockDim.x) {
-      const bool second = e >= tot;
-      const int r = second ? e - tot : e;
-      const int i = k + 1 + r % w, j = k + 1 + r / w;
-      if (i < j || (second ? !liveB : !liveA)) continue;
-      double* X = second ? B : A;
-      const double v = SM(X, i, j) - SM(X, i, k) * SM(X, j, k) * (second ? dB : dA);
-      SM(X, i, j) = v;
-      if (i == k + 1 && j == k + 1) {  // the next pivot is final now
-        double* pv = second ? pivB : pivA;
-        pv[k + 1] = v;
-        pv[SDPXG_NMAX + k + 1] = (v > 0.0 && isfinite(v)) ? 1.0 / v : 0.0;
-      }
-    }
-  }
-  __syncthreads();
-  *okA = liveA;
-  *okB = liveB;
-  double* rootA = pinvA + SDPXG_NMAX;
-  double* rootB = pinvB + SDPXG_NMAX;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    if (liveA) rootA[j] = sqrt(pivA[j]);
-    if (liveB) rootB[j] = sqrt(pivB[j]);
-  }
-  __syncthreads();
-  const int lim = two ? 2 * n * n : n * n;
-  for (int e = threadIdx.x; e < lim; e += blockDim.x) {
-    const bool second = e >= n * n;
-    if (second ? !liveB : !liveA) continue;
-    const int r = second ? e - n * n : e;
-    const int i = r % n, j = r / n;
-    double* X = second ? B : A;
-    const double* root = second ? rootB : rootA;
-    if (i > j) SM(X, i, j) /= root[j];
-    else if (i == j) SM(X, i, j) = root[j];
-    else SM(X, i, j) = 0.0;
-  }
-  __syncthreads();
+// v in [2^-1000, 2^1000): an integer test on the exponent (a double comparison takes part of the FP64
+// pipe and three times as long).
+__device__ __forceinline__ bool mid_range(double v) {
+  return (unsigned)__double2hiint(v) - 0x01700000u < 0x7d000000u;
 }
 
-// 1/v for a positive v: the hardware approximation refined by two Newton-Raphson steps
+// 1/v for v in the mid range: the hardware approximation refined by two Newton-Raphson steps
 // y <- y + y (1 - v y) (each doubles the correct bits; the result is within a few units in the
-// last place of 1/v).  Outside [2^-1000, 2^1000], where the approximation flushes, the IEEE
-// division.  Used on the critical path of the blocked CTA Cholesky factorisation.
-__device__ __forceinline__ double recip_newton(double v) {
-  if (!(v >= 0x1p-1000 && v <= 0x1p1000)) return 1.0 / v;
+// last place of 1/v).
+__device__ __forceinline__ double recip_mid(double v) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
   double e = fma(-v, y, 1.0);
@@ -324,14 +276,25 @@ __device__ __forceinline__ double recip_newton(double v) {
   return fma(y, e, y);
 }
 
-// Blocked right-looking form (blockDim.x >= 256): panels of 8 columns.  Warp 0 factors A's
+// 1/sqrt(v) for v in the mid range: the hardware approximation y (about 22 bits) and one Householder
+// step of third order, y (1 + e/2 + 3 e^2 / 8) with e = 1 - v y^2.
+__device__ __forceinline__ double rsqrt_mid(double v) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
+  const double e = fma(-v * y, y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// In-place lower Cholesky A = L L' (lower triangle of A used; blockDim.x >= 256), and of B = L L' of
+// the same order next to it when B is given: panels of 8 columns, right-looking.  Warp 0 factors A's
 // panel and warp 1 B's, in registers (lane l holds panel rows kb + l and kb + 32 + l; the pivot
-// and the entries of the updating rows come by shuffles; L(r,c) = a(r,c) / sqrt(pivot), the
-// reciprocal by recip_newton); then every warp takes 8 x 8 tiles of the trailing lower triangle
-// of both matrices, A22 -= L21 L21' on the FP64 tensor cores (two m8n8k4 steps).  Two barriers
-// per panel instead of one per column.  A pivot that is not positive and finite stops that
-// matrix (false); the other carries on.  Entries above the diagonal end as zeros.
-__device__ inline void cta_cholesky_lower2_panel(double* A, double* B, int n, bool* okA, bool* okB) {
+// and the entries of the updating rows come by shuffles; L(r,c) = a(r,c) * rd, rd = pivot^-1/2, and
+// L(c,c) = pivot rd with the residual of its square corrected); then every warp takes 8 x 8 tiles of
+// the trailing lower triangle of both matrices, A22 -= L21 L21' on the FP64 tensor cores (two m8n8k4
+// steps).  Two barriers per panel.  A pivot that is not positive and finite stops that matrix
+// (false); the other carries on.  Entries above the diagonal end as zeros.  Bound by the panel's
+// chain, eight times pivot -> shuffle -> root -> shuffle -> update.
+__device__ inline void cta_cholesky_lower2(double* A, double* B, int n, bool* okA, bool* okB) {
   __shared__ int live[2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const bool two = (B != nullptr);
@@ -356,9 +319,10 @@ __device__ inline void cta_cholesky_lower2_panel(double* A, double* B, int n, bo
       for (int c = 0; c < 8; ++c) {
         if (c < w && ok) {
           const double piv = __shfl_sync(0xffffffffu, P0[c], c);
-          ok = piv > 0.0 && isfinite(piv);
+          ok = (unsigned)__double2hiint(piv) - 1u < 0x7fefffffu || (piv > 0.0 && isfinite(piv));
           if (ok) {
-            const double d = sqrt(piv), rd = recip_newton(d);
+            const double rd = mid_range(piv) ? rsqrt_mid(piv) : rsqrt(piv), d0 = piv * rd;
+            const double d = fma(0.5 * rd, fma(-d0, d0, piv), d0);
             P0[c] = lane < c ? 0.0 : (lane == c ? d : P0[c] * rd);
             P1[c] *= rd;
 #pragma unroll
@@ -419,15 +383,9 @@ __device__ inline void cta_cholesky_lower2_panel(double* A, double* B, int n, bo
   __syncthreads();
 }
 
-__device__ inline void cta_cholesky_lower2(double* A, double* B, int n, double* pivA, double* pivB,
-                                           bool* okA, bool* okB) {
-  if (blockDim.x >= 256) cta_cholesky_lower2_panel(A, B, n, okA, okB);
-  else cta_cholesky_lower2_smem(A, B, n, pivA, pivB, okA, okB);
-}
-
-__device__ inline bool cta_cholesky_lower(double* A, int n, double* piv) {
+__device__ inline bool cta_cholesky_lower(double* A, int n) {
   bool ok, unused;
-  cta_cholesky_lower2(A, nullptr, n, piv, piv, &ok, &unused);
+  cta_cholesky_lower2(A, nullptr, n, &ok, &unused);
   return ok;
 }
 

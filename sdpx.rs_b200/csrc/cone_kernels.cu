@@ -31,7 +31,7 @@ constexpr int kMat = SDPXG_LD * SDPXG_NMAX;  // doubles per shared matrix
 // threads, room for the register-resident Jacobi) reads them back and writes R, Rinv, Ginv,
 // lam and lam^-1/2.  A failed factorisation sets SDPXG_ST_CHOL_FAIL, which the second launch
 // reads to leave every block alone (the scaling is rejected as a whole).
-// Shared memory of k_nt_factor: 3 matrices + 2 Cholesky scratches; of k_nt_svd: 5 matrices +
+// Shared memory of k_nt_factor: 3 matrices; of k_nt_svd: 5 matrices +
 // 2n doubles + n ints + 1 int.
 // ---------------------------------------------------------------------------------------
 extern "C" __global__ void __launch_bounds__(SDPXG_CONE_THREADS)
@@ -44,13 +44,11 @@ k_nt_factor(const BlockDesc* __restrict__ blocks, const double* __restrict__ s,
   double* L1 = smem;
   double* L2 = L1 + kMat;
   double* M = L2 + kMat;
-  double* piv = M + kMat;
-  double* piv2 = piv + SDPXG_CHOL_SCRATCH;
   cta_zero_mat(M);
   cta_load_smat(L1, s + bd.svec_off, n);
   cta_load_smat(L2, z + bd.svec_off, n);
   bool ok1, ok2;
-  cta_cholesky_lower2(L1, L2, n, piv, piv2, &ok1, &ok2);  // chol(S), chol(Z) together
+  cta_cholesky_lower2(L1, L2, n, &ok1, &ok2);  // chol(S), chol(Z) together
   if (!ok1 || !ok2) {
     if (threadIdx.x == 0) atomicOr(status, SDPXG_ST_CHOL_FAIL);
     return;
@@ -380,7 +378,7 @@ extern "C" __global__ void k_shift_unit(const BlockDesc* __restrict__ blocks, do
 // mode 1: admission only (out = amax if admitted else 0).
 // out[2*block + side].
 // ---------------------------------------------------------------------------------------
-extern "C" __global__ void __launch_bounds__(SDPXG_CONE_THREADS)
+extern "C" __global__ void __launch_bounds__(SDPXG_EIG_THREADS)
 k_step_length(const BlockDesc* __restrict__ blocks, const double* __restrict__ R,
               const double* __restrict__ Rinv, const double* __restrict__ lisqrt,
               const double* __restrict__ dz, const double* __restrict__ ds, double amax, int mode,
@@ -393,12 +391,9 @@ k_step_length(const BlockDesc* __restrict__ blocks, const double* __restrict__ R
   double* X = B + kMat;
   double* T = X + kMat;
   double* D = T + kMat;
-  double* small = D + kMat;  // Cholesky scratch, d[n], e[n], work[2n], red[32]
-  double* piv = small;
-  double* dd = piv + SDPXG_CHOL_SCRATCH;
+  double* dd = D + kMat;  // d[n], e[n], one int
   double* ee = dd + SDPXG_NMAX;
-  double* work = ee + SDPXG_NMAX;
-  double* red = work + 2 * SDPXG_NMAX;
+  int* best = reinterpret_cast<int*>(ee + SDPXG_NMAX);
   cta_load_mat(B, (side == 0 ? R : Rinv) + bd.mat_off, n);
   cta_load_smat(X, (side == 0 ? dz : ds) + bd.svec_off, n);
   __syncthreads();
@@ -417,15 +412,15 @@ k_step_length(const BlockDesc* __restrict__ blocks, const double* __restrict__ R
     SM(T, i, j) = amax * SM(X, i, j) + (i == j ? 1.0 : 0.0);
   }
   __syncthreads();
-  bool admitted = (n <= 3 && mode == 0) ? false : cta_cholesky_lower(T, n, piv);
+  bool admitted = (n <= 3 && mode == 0) ? false : cta_cholesky_lower(T, n);
   if (mode == 1) {
     if (threadIdx.x == 0) out[2 * b + side] = admitted ? amax : 0.0;
     return;
   }
   if (!admitted) {
-    cta_tridiagonalize(X, n, dd, ee, work, red);
+    cta_tridiagonalize(X, n, dd, ee, T);
     bool ok = true;
-    double g = cta_eig_min(dd, ee, n, reinterpret_cast<int*>(red), &ok);
+    double g = cta_eig_min(dd, ee, n, reinterpret_cast<double2*>(B), best, &ok);
     if (!ok || !isfinite(g)) {
       if (threadIdx.x == 0) atomicOr(status, SDPXG_ST_EIG_FAIL);
       res = 0.0;
@@ -443,7 +438,7 @@ k_step_length(const BlockDesc* __restrict__ blocks, const double* __restrict__ R
 // min(lambda_min, 0) and out[2b+1] = 0.  A block whose Cholesky factorisation succeeds is
 // positive definite to working accuracy and gives 0 without an eigensolve; the others take the
 // tridiagonal reduction and the multisection for lambda_min alone.
-extern "C" __global__ void __launch_bounds__(SDPXG_CONE_THREADS)
+extern "C" __global__ void __launch_bounds__(SDPXG_EIG_THREADS)
 k_margins(const BlockDesc* __restrict__ blocks, const double* __restrict__ v, long ld,
           double* __restrict__ out, uint32_t* __restrict__ status, int min_only) {
   extern __shared__ double smem[];
@@ -454,22 +449,22 @@ k_margins(const BlockDesc* __restrict__ blocks, const double* __restrict__ v, lo
   double* dd = X + kMat;
   double* ee = dd + SDPXG_NMAX;
   double* work = ee + SDPXG_NMAX;
-  double* red = work + 2 * SDPXG_NMAX;
-  double* eig = red + 32;
+  double* eig = work + SDPXG_TRIDIAG_WORK;
+  int* best = reinterpret_cast<int*>(eig + SDPXG_NMAX);
   const double* vb = v + (long)blockIdx.y * ld + bd.svec_off;
   const long o = 2L * ((long)blockIdx.y * gridDim.x + b);
   cta_load_smat(X, vb, n);
   __syncthreads();
   if (min_only) {
-    if (cta_cholesky_lower(X, n, dd)) {
+    if (cta_cholesky_lower(X, n)) {
       if (threadIdx.x == 0) out[o] = out[o + 1] = 0.0;
       return;
     }
     cta_load_smat(X, vb, n);
     __syncthreads();
-    cta_tridiagonalize(X, n, dd, ee, work, red);
+    cta_tridiagonalize(X, n, dd, ee, work);
     bool ok = true;
-    const double g = cta_eig_min(dd, ee, n, reinterpret_cast<int*>(red), &ok);
+    const double g = cta_eig_min(dd, ee, n, reinterpret_cast<double2*>(work), best, &ok);
     if (threadIdx.x == 0) {
       if (!ok || !isfinite(g)) atomicOr(status, SDPXG_ST_EIG_FAIL);
       out[o] = fmin(g, 0.0);
@@ -477,8 +472,8 @@ k_margins(const BlockDesc* __restrict__ blocks, const double* __restrict__ v, lo
     }
     return;
   }
-  cta_tridiagonalize(X, n, dd, ee, work, red);
-  cta_eig_all(dd, ee, n, eig, status);
+  cta_tridiagonalize(X, n, dd, ee, work);
+  cta_eig_all(dd, ee, n, reinterpret_cast<double2*>(work), eig, status);
   __syncthreads();
   if (threadIdx.x == 0) {
     double mn = eig[0], pos = 0.0;

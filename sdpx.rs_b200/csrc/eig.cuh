@@ -6,14 +6,13 @@
 //    needs (the reference takes the SVD of L2'L1 directly instead of an eigensolve of the
 //    squared matrix, cones/psdtrianglecone.rs:378-386).
 //  * cta_tridiagonalize: Householder reduction of a symmetric matrix to tridiagonal form.
-//  * sturm_count / bisect_kth: eigenvalues of the tridiagonal by Sturm-sequence bisection
-//    (the same method the reference uses for its binary64 lambda_min bound,
+//  * sturm / cta_eig_*: eigenvalues of the tridiagonal by Sturm-sequence multisection
+//    (the reference bisects for its binary64 lambda_min bound,
 //    cones/psdtrianglecone.rs:1250-1290), every loop bounded.
 #pragma once
 #include "common.cuh"
 
 #define SDPXG_JACOBI_MAX_SWEEPS 60
-#define SDPXG_BISECT_MAX 256
 
 namespace jacobi_detail {
 
@@ -187,155 +186,294 @@ __device__ inline int cta_jacobi_left(double* M, int n, double* part, int* out) 
   return res;
 }
 
-// Householder tridiagonalisation of the symmetric A (destroyed).  d[0..n), e[0..n-1).
-// `work` is 2*n doubles of shared memory, `red` 32 doubles.  blockDim.x is a multiple of 64.
-// Step k reflects column k below the diagonal, x = A[k+1:n, k] (m <= 63 entries): warp 0 forms
-// |x|^2, the reflector's scale and v = (x - alpha e1) / |x - alpha e1| into shared memory (one
-// barrier); p = A v, one warp per row reading the row as a column (A stays exactly symmetric;
-// a barrier); warp 0 forms K = v'p and q = p - K v in place of p (a barrier); then the rank-2
-// update A -= 2 (v q' + q v'), thread t on row t % 64 of the columns t / 64 + 16 s (a barrier).
-__device__ inline void cta_tridiagonalize(double* A, int n, double* d, double* e, double* work,
-                                          double* red) {
-  double* p = work;
-  double* v = work + n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  for (int k = 0; k + 2 < n; ++k) {
-    const int m = n - k - 1;  // length of the column below the diagonal
-    const double* x = &SM(A, k + 1, k);
-    if (warp == 0) {
-      double part = 0.0;
-      for (int i = lane; i < m; i += 32) part = fma(x[i], x[i], part);
-      const double nrm2 = warp_sum(part);
-      const double x0 = x[0];
-      const double alpha = -copysign(sqrt(nrm2), x0);
-      const double vnorm2 = nrm2 - x0 * x0 + (x0 - alpha) * (x0 - alpha);
-      const bool skip = (nrm2 == 0.0 || vnorm2 == 0.0);  // column already reduced
-      const double vs = skip ? 0.0 : rsqrt(vnorm2);
-      for (int i = lane; i < m; i += 32) v[i] = (i == 0) ? (x0 - alpha) * vs : x[i] * vs;
-      if (lane == 0) {
-        d[k] = SM(A, k, k);
-        e[k] = (nrm2 == 0.0) ? 0.0 : alpha;
-        red[0] = skip ? 0.0 : 1.0;
-      }
-    }
-    __syncthreads();
-    if (red[0] == 0.0) {
-      __syncthreads();  // red[0] is read by every thread before warp 0 rewrites it
-      continue;
-    }
-    // p = A_sub v
-    for (int i = warp; i < m; i += nwarps) {
-      double acc = 0.0;
-      for (int j = lane; j < m; j += 32) acc = fma(SM(A, k + 1 + j, k + 1 + i), v[j], acc);
-      acc = warp_sum(acc);
-      if (lane == 0) p[i] = acc;
-    }
-    __syncthreads();
-    if (warp == 0) {  // K = v'p, then p <- q = p - K v in place
-      double kp = 0.0;
-      for (int i = lane; i < m; i += 32) kp = fma(v[i], p[i], kp);
-      const double K = warp_sum(kp);
-      for (int i = lane; i < m; i += 32) p[i] = p[i] - K * v[i];
-    }
-    __syncthreads();
-    // A_sub -= 2 (v q' + q v') (both triangles from the same two products)
-    const int ri = threadIdx.x & 63, cstride = blockDim.x >> 6;
-    if (ri < m) {
-      const double vi = v[ri], qi = p[ri];
-      for (int j = threadIdx.x >> 6; j < m; j += cstride) {
-        const double vj = v[j], qj = p[j];
-        const double u = __dadd_rn(__dmul_rn(vi, qj), __dmul_rn(qi, vj));
-        SM(A, k + 1 + ri, k + 1 + j) -= 2.0 * u;
-      }
-    }
-    __syncthreads();
+namespace tridiag_detail {
+
+// Shared memory of cta_tridiagonalize (SDPXG_TRIDIAG_WORK doubles): the step's column x and the next
+// one, x in column order per warp, the warps' partials of A x, and per warp p in its column order.
+constexpr int kX = 0, kY = 64, kXp = 128, kPart = 208, kPw = 464, kRow = 20;
+static_assert(kPw + 4 * kRow == SDPXG_TRIDIAG_WORK, "layout");
+
+// Position k of the padded matrix is at hand: warp k & 3 publishes its first column as x (rows above
+// k + 1 zero, and d[k]), the warp of column k + 1 that one as y.
+template <bool LOW>
+__device__ __forceinline__ void publish(int k, int off, double unscale, const double (&a0)[16],
+                                        const double (&a1)[16], double* d, double* ws) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = k >> 2;
+  if (w == (k & 3)) {
+    const double x0 = (LOW && lane > k) ? a0[0] : 0.0, x1 = lane + 32 > k ? a1[0] : 0.0;
+    ws[kX + lane] = x0;
+    ws[kX + lane + 32] = x1;
+    double* xp = ws + kXp + (lane & 3) * kRow;  // the columns that are gone leave zeros at the end
+    xp[((lane >> 2) - t) & 15] = x0;
+    xp[((lane >> 2) + 8 - t) & 15] = x1;
+    if (lane == (k & 31)) d[k - off] = ((LOW && k < 32) ? a0[0] : a1[0]) * unscale;
   }
-  if (threadIdx.x == 0) {
-    if (n >= 2) {
-      d[n - 2] = SM(A, n - 2, n - 2);
-      d[n - 1] = SM(A, n - 1, n - 1);
-      e[n - 2] = SM(A, n - 1, n - 2);
-    } else if (n == 1) {
-      d[0] = SM(A, 0, 0);
+  const int j = (k & 3) == 3;  // column k + 1 is its warp's first or, of warp 0, the second
+  if (w == ((k + 1) & 3)) {
+    if (LOW) ws[kY + lane] = j ? a0[1] : a0[0];
+    ws[kY + lane + 32] = j ? a1[1] : a1[0];
+  }
+}
+
+// Steps k0 .. k1-1 (positions of the padded matrix) with NJ columns alive per warp; LOW: rows 0 .. 31 too.
+template <int NJ, bool LOW>
+__device__ __forceinline__ void steps(int k0, int k1, int off, double unscale, double (&a0)[16], double (&a1)[16],
+                                      double* d, double* e, double* ws) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int k = k0; k < k1; ++k) {
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    const double x0 = LOW ? ws[kX + lane] : 0.0, x1 = ws[kX + lane + 32], xk = ws[kX + k + 1];
+    const double y0 = LOW ? ws[kY + lane] : 0.0, y1 = ws[kY + lane + 32];
+    double vc[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; j += 2) {
+      const double2 t = *reinterpret_cast<const double2*>(ws + kXp + w * kRow + j);
+      vc[j] = t.x;
+      vc[j + 1] = t.y;
     }
+    const double nrm2 = warp_sum(LOW ? fma(x0, x0, x1 * x1) : x1 * x1);
+    double p0 = 0.0, p1 = 0.0, s0 = 0.0, s1 = 0.0;  // A x: this warp's columns
+#pragma unroll
+    for (int j = 0; j < NJ; j += 2) {
+      if (LOW) p0 = fma(a0[j], vc[j], p0);
+      p1 = fma(a1[j], vc[j], p1);
+      if (LOW) s0 = fma(a0[j + 1], vc[j + 1], s0);
+      s1 = fma(a1[j + 1], vc[j + 1], s1);
+    }
+    if (LOW) ws[kPart + 64 * w + lane] = p0 + s0;
+    ws[kPart + 64 * w + lane + 32] = p1 + s1;
+    const bool live = __double2hiint(nrm2) >= 0x01700000;  // 2^-1000 or more
+    const double rs = live ? rsqrt_mid(nrm2) : 0.0;
+    const double alpha = -copysign(nrm2 * rs, xk), u = xk - alpha;
+    const double c = recip_mid(fma(fabs(xk), rs, 1.0));  // 2 / |v rs|^2, in [1/2, 1]
+    const double up = live ? fma(xk, rs, copysign(1.0, xk)) : 0.0;
+    const double v0 = lane == k + 1 ? up : x0 * rs, v1 = lane + 32 == k + 1 ? up : x1 * rs;
+    if (threadIdx.x == 0) e[k - off] = live ? alpha * unscale : 0.0;
+    vc[0] = w == (k & 3) + 1 ? u : vc[0];  // column k + 1
+    vc[1] = w + 3 == (k & 3) ? u : vc[1];
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (LOW) {
+      const double* b = ws + kPart + lane;
+      p0 = fma(-alpha, y0, (b[0] + b[64]) + (b[128] + b[192]));
+    }
+    {
+      const double* b = ws + kPart + lane + 32;
+      p1 = fma(-alpha, y1, (b[0] + b[64]) + (b[128] + b[192]));
+    }
+    {
+      const int j = (lane >> 2) - (k >> 2);
+      if ((lane & 3) == w) {
+        if (LOW) ws[kPw + w * kRow + (j & 15)] = j >= 0 ? p0 : 0.0;
+        ws[kPw + w * kRow + ((j + 8) & 15)] = j + 8 >= 0 ? p1 : 0.0;
+      }
+    }
+    __syncwarp();
+    p0 *= rs;
+    p1 *= rs;
+    const double S = warp_sum(LOW ? fma(v0, p0, v1 * p1) : v1 * p1);
+    const double cr = c * rs, f0 = -cr * v0, f1 = -cr * v1;
+#pragma unroll
+    for (int j = 0; j < NJ; j += 2) {
+      const double2 t = *reinterpret_cast<const double2*>(ws + kPw + w * kRow + j);
+      if (LOW) {
+        a0[j] = fma(f0, t.x, a0[j]);
+        a0[j + 1] = fma(f0, t.y, a0[j + 1]);
+      }
+      a1[j] = fma(f1, t.x, a1[j]);
+      a1[j + 1] = fma(f1, t.y, a1[j + 1]);
+    }
+    const double cs = c * S, g0 = cr * fma(cs, v0, -p0), g1 = cr * fma(cs, v1, -p1);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      if (LOW) a0[j] = fma(g0, vc[j], a0[j]);
+      a1[j] = fma(g1, vc[j], a1[j]);
+    }
+    if ((k & 3) == 3) {  // the warps' first columns are done with
+#pragma unroll
+      for (int j = 0; j + 1 < NJ; ++j) {
+        if (LOW) a0[j] = a0[j + 1];
+        a1[j] = a1[j + 1];
+      }
+      if (LOW) a0[NJ - 1] = 0.0;
+      a1[NJ - 1] = 0.0;
+    }
+    publish<LOW>(k + 1, off, unscale, a0, a1, d, ws);
+  }
+}
+
+}  // namespace tridiag_detail
+
+// Householder tridiagonalisation of the symmetric A (n <= 64, shared memory).  d[0..n), e[0..n-1).
+// `ws` is SDPXG_TRIDIAG_WORK doubles of shared memory, 16-byte aligned.  Every thread of the CTA calls
+// it (blockDim.x >= 128); warps 0..3 take part.
+// The matrix stays in registers, as the last n rows and columns of a 64 x 64 one (so that every order
+// ends with the same short steps): warp w holds the columns 4j + w, its first register the first column
+// that is still alive, lane l the rows l and l + 32.  Step k reflects column k below the diagonal, x =
+// A[k+1:, k], by v = x - alpha e1, alpha = -sign(x_1) |x|; with r = 1/|x|, c = 1/(1 + |x_1| r) and p = A v
+// = A x - alpha A e1:
+//   A <- A - c (vr) (pr)' - c (pr) (vr)' + c^2 ((vr)'(pr)) (vr) (vr)'
+// (scaled by r so that no product leaves the range that |x|^2 allows).  A x needs neither |x| nor alpha:
+// the warps' partials of it cross shared memory while |x| is summed; the terms with p' are applied while
+// (vr)'(pr) is summed.  Rows up to k carry on without being read (they see an orthogonal factor on one
+// side); from k = 32 on only the rows 32 .. 63 are kept up.
+// Bound by the step's chain -- two barriers, two warp sums (180 cycles each), a root, the published
+// column: 1140 cycles a step at n = 64.  One warp for the scalars between four CTA barriers and operands
+// in shared memory took 3200; eight warps, each summing all eight partials again, 2290.
+__device__ inline void cta_tridiagonalize(const double* A, int n, double* d, double* e, double* ws) {
+  using namespace tridiag_detail;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, off = SDPXG_NMAX - n;
+  double unscale = 1.0;
+  if (w < 4) {
+    double a0[16], a1[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int c = 4 * (j + (off >> 2)) + w - off, r = lane - off;
+      const bool in = c >= 0 && c < n;
+      a0[j] = in && r >= 0 ? SM(A, r, c) : 0.0;
+      a1[j] = in && r + 32 >= 0 ? SM(A, r + 32, c) : 0.0;
+    }
+    // entries below one in magnitude by a power of two: |x|^2 < 2^-1000 is then nothing
+    double mx = 0.0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) mx = fmax(mx, fmax(fabs(a0[j]), fabs(a1[j])));
+    mx = warp_max(mx);
+    if (lane == 0) ws[kPw + w] = mx;
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    mx = fmax(fmax(ws[kPw], ws[kPw + 1]), fmax(ws[kPw + 2], ws[kPw + 3]));
+    int ex = 0;
+    if (mx > 0.0 && isfinite(mx)) ex = max(-1000, min(1000, ilogb(mx) + 1));
+    const double scale = ldexp(1.0, -ex);
+    unscale = ldexp(1.0, ex);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      a0[j] *= scale;
+      a1[j] *= scale;
+    }
+    publish<true>(off, off, unscale, a0, a1, d, ws);
+    steps<16, true>(off, 16, off, unscale, a0, a1, d, e, ws);
+    steps<12, true>(max(off, 16), 32, off, unscale, a0, a1, d, e, ws);
+    steps<8, false>(max(off, 32), 48, off, unscale, a0, a1, d, e, ws);
+    steps<4, false>(max(off, 48), SDPXG_NMAX - 2, off, unscale, a0, a1, d, e, ws);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && n >= 2) {
+    e[n - 2] = ws[kX + SDPXG_NMAX - 1] * unscale;
+    d[n - 1] = ws[kY + SDPXG_NMAX - 1] * unscale;
   }
   __syncthreads();
 }
 
-// Number of eigenvalues of the tridiagonal (d, e) strictly below x.  The quotient of each step
-// takes the Newton-refined reciprocal (recip_newton: a few units in the last place), which
-// keeps the count that of a matrix within a few ulps of (d, e); |q| >= pivmin throughout.
-__device__ __forceinline__ int sturm_count(const double* d, const double* e, int n, double x,
-                                           double pivmin) {
-  int cnt = 0;
-  double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  cnt += (q < 0.0);
-  for (int i = 1; i < n; ++i) {
-    q = (d[i] - x) - e[i - 1] * e[i - 1] * copysign(recip_newton(fabs(q)), q);
-    if (fabs(q) < pivmin) q = -pivmin;
-    cnt += (q < 0.0);
-  }
-  return cnt;
-}
-
-__device__ __forceinline__ void gershgorin(const double* d, const double* e, int n, double* lo,
-                                           double* hi, double* pivmin) {
-  double l = 1e300, h = -1e300, emax = 0.0;
-  for (int i = 0; i < n; ++i) {
-    double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i + 1 < n ? fabs(e[i]) : 0.0);
+// The tridiagonal (d, e) made ready for the Sturm sequences: t[i] = (d_i, e_{i-1}^2) times a power of
+// two (its square) that brings the Gershgorin interval to about one, e^2 at least 2^-200 (a perturbation
+// of 2^-100 relative to the norm keeps every sequence from stopping at zero), padded to a multiple of
+// eight rows with (4, 0), which change no sign.  Returns the interval in the scaled units and, in
+// *unscale, the factor back.  `t` is 16-byte aligned shared memory, SDPXG_STURM_WORK doubles.
+__device__ inline void sturm_prepare(const double* d, const double* e, int n, double2* t, double* lo, double* hi,
+                                     double* unscale) {
+  const int lane = threadIdx.x & 31;
+  double l = 1e300, h = -1e300;
+  for (int i = lane; i < n; i += 32) {
+    const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i + 1 < n ? fabs(e[i]) : 0.0);
     l = fmin(l, d[i] - r);
     h = fmax(h, d[i] + r);
-    if (i + 1 < n) emax = fmax(emax, e[i] * e[i]);
   }
-  double span = fmax(fabs(l), fabs(h));
-  *lo = l - 2.0 * 2.220446049250313e-16 * span - 1e-300;
-  *hi = h + 2.0 * 2.220446049250313e-16 * span + 1e-300;
-  *pivmin = 2.2250738585072014e-308 * fmax(1.0, emax);
+  l = -warp_max(-l);
+  h = warp_max(h);
+  const double span = fmax(fabs(l), fabs(h));
+  l -= 2.0 * 2.220446049250313e-16 * span;
+  h += 2.0 * 2.220446049250313e-16 * span;
+  int ex = 0;
+  if (span > 0.0 && isfinite(span)) ex = max(-1000, min(1000, ilogb(span) + 1));
+  const double s = ldexp(1.0, -ex);
+  *unscale = ldexp(1.0, ex);
+  *lo = l * s - 0x1p-200;
+  *hi = h * s + 0x1p-200;
+  const int np = (n + 7) & ~7;
+  for (int i = threadIdx.x; i < np; i += blockDim.x) {
+    const double v = (i > 0 && i < n) ? e[i - 1] * s : 0.0;
+    t[i] = i < n ? make_double2(d[i] * s, fmax(v * v, 0x1p-200)) : make_double2(4.0, 0.0);
+  }
+  __syncthreads();
 }
 
-// Smallest eigenvalue of the tridiagonal (d, e) by CTA-wide multisection: each round T threads
-// evaluate one Sturm count each on an even grid over the current bracket and the bracket
-// shrinks to the first grid cell holding an eigenvalue (about T-fold per round).  T = 512: a
-// Sturm count is a chain of n dependent divisions, and with more than 16 warps per SM evaluating
-// them the rounds become bound by FP64 issue rather than by that chain, so 1024 points cost
-// twice as long per round for one more bit.
-// Uniform result; `best` is one int of shared memory.  *ok = false if the round bound is hit.
-__device__ inline double cta_eig_min(const double* d, const double* e, int n, int* best, bool* ok) {
-  double lo, hi, pivmin;
-  gershgorin(d, e, n, &lo, &hi, &pivmin);
-  const int T = min((int)blockDim.x, 512);
-  for (int round = 0; round < 16; ++round) {
-    if (!(hi - lo > 2.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + pivmin)) {
+// The leading principal minors of T - x for the tridiagonal prepared by sturm_prepare, p_i = (d_i - x)
+// p_{i-1} - e_{i-1}^2 p_{i-2}: COUNT ? the number of their sign changes, the eigenvalues below x : the
+// sign of any (at least one eigenvalue below x).  Each step perturbs d_i - x and e_{i-1}^2 by a few
+// units in the last place, as the quotient form q_i = d_i - x - e_{i-1}^2 / q_{i-1} does, but its chain
+// is one multiply-add (8 cycles) instead of a reciprocal (about 110).  Every eighth step rescales the
+// pair by a power of two (eight steps change it by at most 2^16 upwards and about 2^-800 downwards).
+template <bool COUNT>
+__device__ __forceinline__ int sturm(const double2* t, int n, double x) {
+  double p0 = 0.0, p1 = 1.0;
+  int cnt = 0;
+  double2 r[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) r[u] = t[u];
+  for (int i = 0; i < n; i += 8) {
+    double2 next[8];
+    const double2* tn = t + (i + 8 < n ? i + 8 : 0);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) next[u] = tn[u];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const double p2 = fma(r[u].x - x, p1, -(r[u].y * p0));
+      if (COUNT) cnt += (int)((unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31);
+      else cnt |= __double2hiint(p2);
+      p0 = p1;
+      p1 = p2;
+    }
+    const int m = max(__double2hiint(p0) & 0x7ff00000, __double2hiint(p1) & 0x7ff00000);
+    const double s = __hiloint2double(0x7fe00000 - min(max(m, 0x00100000), 0x7fd00000), 0);
+    p0 *= s;
+    p1 *= s;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) r[u] = next[u];
+  }
+  return COUNT ? cnt : (int)((unsigned)cnt >> 31);
+}
+
+// Smallest eigenvalue of the tridiagonal (d, e) by CTA-wide multisection: each round every thread
+// evaluates one Sturm sequence on an even grid over the current bracket and the bracket shrinks to the
+// first grid cell holding an eigenvalue.  With 256 threads a round is bound by the sequence's chain
+// and gives 8 bits; with 512 it is bound by issue and gives 9.
+// An eigenvalue is resolved relative to itself, down to 2^-200 of the norm: at most 26 rounds.
+// Uniform result; `best` is one int of shared memory, `t` SDPXG_STURM_WORK doubles.
+// *ok = false if the round bound is hit.
+__device__ inline double cta_eig_min(const double* d, const double* e, int n, double2* t, int* best, bool* ok) {
+  double lo, hi, unscale;
+  sturm_prepare(d, e, n, t, &lo, &hi, &unscale);
+  const int T = blockDim.x;
+  for (int round = 0; round < 40; ++round) {
+    if (!(hi - lo > 2.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + 0x1p-200)) {
       *ok = true;
-      return 0.5 * (lo + hi);
+      return 0.5 * (lo + hi) * unscale;
     }
     const double step = (hi - lo) / (T + 1);
     if (threadIdx.x == 0) *best = T;
     __syncthreads();
     const double x = lo + step * (threadIdx.x + 1);
-    if ((int)threadIdx.x < T && x > lo && x < hi && sturm_count(d, e, n, x, pivmin) >= 1)
-      atomicMin(best, (int)threadIdx.x);
+    const unsigned bal = __ballot_sync(0xffffffffu, x > lo && x < hi && sturm<false>(t, n, x));
+    if (bal && (threadIdx.x & 31) == 0) atomicMin(best, (int)threadIdx.x + __ffs(bal) - 1);
     __syncthreads();
-    const int t = *best;
+    const int b = *best;
     __syncthreads();
-    const double nlo = (t == 0) ? lo : lo + step * t;
-    const double nhi = (t == T) ? hi : lo + step * (t + 1);
+    const double nlo = (b == 0) ? lo : lo + step * b;
+    const double nhi = (b == T) ? hi : lo + step * (b + 1);
     lo = nlo;
     hi = nhi;
   }
   *ok = false;
-  return 0.5 * (lo + hi);
+  return 0.5 * (lo + hi) * unscale;
 }
 
 // Every eigenvalue of the tridiagonal (d, e), ascending, into eig[0..n): 16-lane groups, one
-// eigenvalue per group, multisection with 15 Sturm counts per round (the bracket shrinks
-// 16-fold per round), the same convergence test as bisect_kth; no CTA barrier inside.
+// eigenvalue per group, multisection with 15 Sturm counts per round (the bracket shrinks 16-fold per
+// round), no CTA barrier inside.  `t`: SDPXG_STURM_WORK doubles.
 // Sets the status bit SDPXG_ST_EIG_FAIL for an eigenvalue whose round bound was hit.
-__device__ inline void cta_eig_all(const double* d, const double* e, int n, double* eig,
+__device__ inline void cta_eig_all(const double* d, const double* e, int n, double2* t, double* eig,
                                    uint32_t* status) {
-  double lo0, hi0, pivmin;
-  gershgorin(d, e, n, &lo0, &hi0, &pivmin);
+  double lo0, hi0, unscale;
+  sturm_prepare(d, e, n, t, &lo0, &hi0, &unscale);
   constexpr int P = 16;
   const int grp = threadIdx.x / P, sl = threadIdx.x % P, base = threadIdx.x & 16;
   const unsigned gmask = 0xFFFFu << base;
@@ -343,13 +481,13 @@ __device__ inline void cta_eig_all(const double* d, const double* e, int n, doub
     double lo = lo0, hi = hi0;
     bool conv = false;
     for (int round = 0; round < 64; ++round) {
-      if (!(hi - lo > 2.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + pivmin)) {
+      if (!(hi - lo > 2.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + 0x1p-200)) {
         conv = true;
         break;
       }
       const double step = (hi - lo) / P;
       const double x = lo + step * (sl + 1);
-      const bool above = (sl < P - 1) && x > lo && x < hi && sturm_count(d, e, n, x, pivmin) > k;
+      const bool above = (sl < P - 1) && x > lo && x < hi && sturm<true>(t, n, x) > k;
       const unsigned bal = (__ballot_sync(gmask, above) >> base) & 0xFFFFu;
       const int c = bal ? __ffs(bal) - 1 : P - 1;  // eigenvalue k lies in cell c
       const double nlo = (c == 0) ? lo : lo + step * c;
@@ -358,27 +496,8 @@ __device__ inline void cta_eig_all(const double* d, const double* e, int n, doub
       hi = nhi;
     }
     if (sl == 0) {
-      eig[k] = 0.5 * (lo + hi);
+      eig[k] = 0.5 * (lo + hi) * unscale;
       if (!conv) atomicOr(status, SDPXG_ST_EIG_FAIL);
     }
   }
-}
-
-// k-th smallest eigenvalue (k = 0 is the minimum) by bisection; one thread.
-// Sets *ok = false when the bound on steps was hit before convergence.
-__device__ inline double bisect_kth(const double* d, const double* e, int n, int k, bool* ok) {
-  double lo, hi, pivmin;
-  gershgorin(d, e, n, &lo, &hi, &pivmin);
-  for (int it = 0; it < SDPXG_BISECT_MAX; ++it) {
-    double mid = 0.5 * (lo + hi);
-    if (!(mid > lo && mid < hi) ||
-        hi - lo <= 2.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + pivmin) {
-      *ok = true;
-      return mid;
-    }
-    if (sturm_count(d, e, n, mid, pivmin) > k) hi = mid;
-    else lo = mid;
-  }
-  *ok = false;
-  return 0.5 * (lo + hi);
 }

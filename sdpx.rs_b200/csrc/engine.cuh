@@ -30,12 +30,12 @@
 namespace sdpxg {
 
 constexpr int kMatD = SDPXG_LD * SDPXG_NMAX;
-constexpr size_t kSmemNtFactor = (3 * kMatD + 2 * SDPXG_CHOL_SCRATCH) * sizeof(double);
+constexpr size_t kSmemNtFactor = 3 * kMatD * sizeof(double);
 constexpr size_t kSmemNt = (5 * kMatD + 2 * SDPXG_NMAX) * sizeof(double) + (SDPXG_NMAX + 1) * sizeof(int);
 constexpr size_t kSmemCong = (2 * kMatD + 2 * 16 * SDPXG_LD) * sizeof(double);
 constexpr size_t kSmemCirc = 2 * kMatD * sizeof(double);
-constexpr size_t kSmemStep = (4 * kMatD + SDPXG_CHOL_SCRATCH + 4 * SDPXG_NMAX + 32) * sizeof(double);
-constexpr size_t kSmemMarg = (kMatD + 5 * SDPXG_NMAX + 32) * sizeof(double);
+constexpr size_t kSmemStep = (4 * kMatD + 2 * SDPXG_NMAX + 1) * sizeof(double);
+constexpr size_t kSmemMarg = (kMatD + 3 * SDPXG_NMAX + SDPXG_TRIDIAG_WORK + 1) * sizeof(double);
 constexpr size_t kSmemTrans = 3 * kMatD * sizeof(double);
 constexpr size_t kSmemTrsm = 2 * 64 * 65 * sizeof(double);
 constexpr size_t kSmemSyrk = 2 * 64 * 66 * sizeof(double);
@@ -919,7 +919,7 @@ class Engine {
     clear_status();
     tbegin(KT_STEP);
     if (nblk)
-      ++g_launches, k_step_length<<<dim3(nblk, 2), SDPXG_CONE_THREADS, kSmemStep, st>>>(
+      ++g_launches, k_step_length<<<dim3(nblk, 2), SDPXG_EIG_THREADS, kSmemStep, st>>>(
           blocks_, R_, Rinv_, lisqrt_, dz, ds, amax, mode, step_out_, status_);
     if (nnn_)
       ++g_launches, k_nn_step<<<1, 256, 0, st>>>(nnn_, nn_idx_, nnw_, nnlam_, dz, ds, amax, mode,
@@ -947,7 +947,7 @@ class Engine {
     if (!parts) return true;
     clear_status();
     if (nblk)
-      ++g_launches, k_margins<<<dim3(nblk, 1), SDPXG_CONE_THREADS, kSmemMarg, st>>>(blocks_, v, m, marg_out_,
+      ++g_launches, k_margins<<<dim3(nblk, 1), SDPXG_EIG_THREADS, kSmemMarg, st>>>(blocks_, v, m, marg_out_,
                                                                                     status_, min_only ? 1 : 0);
     if (nnn_) ++g_launches, k_nn_margins<<<1, 256, 0, st>>>(nnn_, nn_idx_, v, marg_out_.p + 2 * nblk);
     launched("k_margins");
