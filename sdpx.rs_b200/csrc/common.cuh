@@ -18,7 +18,7 @@
 #define SDPXG_LD 68
 #define SDPXG_THREADS 256         // dense tile kernels (their thread maps assume 256)
 #define SDPXG_CONE_THREADS 1024   // one CTA per PSD block
-#define SDPXG_NT_SVD_THREADS 512  // the NT scaling's Jacobi launch (8 warps iterate, 128 registers)
+#define SDPXG_NT_SVD_THREADS 256  // the NT scaling's Jacobi launch (4 warps iterate)
 #define SDPXG_EIG_THREADS 256     // step length and margins (tridiagonalisation in 4 warps' registers)
 #define SDPXG_TRIDIAG_WORK 544    // doubles of shared scratch for cta_tridiagonalize
 #define SDPXG_STURM_WORK (2 * SDPXG_NMAX)  // and for cta_eig_min / cta_eig_all
@@ -200,7 +200,9 @@ __device__ __forceinline__ void cta_load_mat(double* M, const double* __restrict
 }
 
 __device__ __forceinline__ void cta_store_mat(double* __restrict__ g, const double* M, int n) {
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) g[e] = SM(M, e % n, e / n);
+  const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  for (int j = threadIdx.x >> 5; j < n; j += nwarps)
+    for (int i = lane; i < n; i += 32) g[i + j * n] = SM(M, i, j);
 }
 
 // One FP64 tensor-core MMA: D(8x8) = A(8x4) B(4x8) + C.  Fragments (PTX mma.m8n8k4 .f64):
@@ -211,50 +213,55 @@ __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, do
                : "d"(a), "d"(b));
 }
 
-// C = op(A) op(B) on zero-padded shared matrices, one 8 x 8 output tile per warp at a time.
+// What is known of a product: nothing; A'B of two lower triangular matrices (only k >= max(i, j)
+// counts); op(B) is upper triangular (k <= j); the result is symmetric (tiles i <= j, mirrored).
+enum GemmForm { GEMM_FULL, GEMM_LOWER_TN, GEMM_UPPER_B, GEMM_SYMMETRIC };
+
+// C = op(A) op(B) on zero-padded shared matrices.  A warp takes 8 x 8 tiles of one tile row (NJ of them:
+// 8 with 8 warps, 2 with 32), so that one fragment of A serves NJ MMAs: with a fragment of each operand
+// per MMA the shared-memory reads take as long as the tensor pipe (16 cycles an MMA and quarter).  Warps
+// w and w + 4 of an SM quarter take tile rows w and 7 - w, equal work for every form.
 // K runs to n rounded up to 4, never further: C is written only up to n rounded up to 8, and
 // a later product that reads C as an operand must not reach its unwritten columns (another
-// kernel's leftovers there, NaN included, would enter through 0 x NaN).  Full groups of four
-// k-steps load their fragments before their four MMAs, so the shared-memory latency overlaps
-// the accumulation chain; the remaining k-steps follow one by one.  C must not alias A or B.
-template <bool TA, bool TB>
-__device__ __forceinline__ void cta_gemm_mma(double* C, const double* A, const double* B, int n) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int tiles = (n + 7) >> 3, ksteps = (n + 3) >> 2, kfull = ksteps & ~3;
+// kernel's leftovers there, NaN included, would enter through 0 x NaN).  C must not alias A or B.
+// blockDim.x is 2048 / NJ.
+template <bool TA, bool TB, int NJ, GemmForm F = GEMM_FULL>
+__device__ __forceinline__ void cta_gemm(double* C, const double* A, const double* B, int n) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tiles = (n + 7) >> 3, ksteps = (n + 3) >> 2;
   const int r = lane >> 2, q = lane & 3;
-  for (int t = warp; t < tiles * tiles; t += nwarps) {
-    const int ti = (t % tiles) << 3, tj = (t / tiles) << 3;
-    double d0 = 0.0, d1 = 0.0;
-    for (int ks0 = 0; ks0 < kfull; ks0 += 4) {
-      double a[4], b[4];
+  const int I = (warp & 4) ? 7 - (warp & 3) : (warp & 3), J0 = warp >> 3;  // tile columns J0, J0 + 8 / NJ, ...
+  if (I >= tiles) return;
+  double d[NJ][2];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int k = ((ks0 + u) << 2) + q;
-        a[u] = TA ? SM(A, k, ti + r) : SM(A, ti + r, k);
-        b[u] = TB ? SM(B, tj + r, k) : SM(B, k, tj + r);
-      }
+  for (int u = 0; u < NJ; ++u) d[u][0] = d[u][1] = 0.0;
+  for (int ks = F == GEMM_LOWER_TN ? 2 * I : 0; ks < ksteps; ++ks) {
+    const int k = (ks << 2) + q;
+    const double a = TA ? SM(A, k, 8 * I + r) : SM(A, 8 * I + r, k);
+    double b[NJ];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) dmma_m8n8k4(d0, d1, a[u], b[u]);
+    for (int u = 0; u < NJ; ++u) {
+      const int J = J0 + u * (8 / NJ);
+      b[u] = TB ? SM(B, 8 * J + r, k) : SM(B, k, 8 * J + r);
     }
-    for (int ks = kfull; ks < ksteps; ++ks) {
-      const int k = (ks << 2) + q;
-      dmma_m8n8k4(d0, d1, TA ? SM(A, k, ti + r) : SM(A, ti + r, k),
-                  TB ? SM(B, tj + r, k) : SM(B, k, tj + r));
+#pragma unroll
+    for (int u = 0; u < NJ; ++u) {
+      const int J = J0 + u * (8 / NJ);
+      if (J < tiles && (F != GEMM_LOWER_TN || ks >= 2 * J) && (F != GEMM_UPPER_B || ks < 2 * J + 2) &&
+          (F != GEMM_SYMMETRIC || J >= I))
+        dmma_m8n8k4(d[u][0], d[u][1], a, b[u]);
     }
-    SM(C, ti + r, tj + 2 * q) = d0;
-    SM(C, ti + r, tj + 2 * q + 1) = d1;
   }
-}
-
-// C = op(A) * op(B); ta/tb select the transpose.  C must not alias A or B.
-__device__ __forceinline__ void cta_gemm(double* C, const double* A, bool ta, const double* B,
-                                         bool tb, int n) {
-  if (ta) {
-    if (tb) cta_gemm_mma<true, true>(C, A, B, n);
-    else cta_gemm_mma<true, false>(C, A, B, n);
-  } else {
-    if (tb) cta_gemm_mma<false, true>(C, A, B, n);
-    else cta_gemm_mma<false, false>(C, A, B, n);
+#pragma unroll
+  for (int u = 0; u < NJ; ++u) {
+    const int J = J0 + u * (8 / NJ);
+    if (J >= tiles || (F == GEMM_SYMMETRIC && J < I)) continue;
+    SM(C, 8 * I + r, 8 * J + 2 * q) = d[u][0];
+    SM(C, 8 * I + r, 8 * J + 2 * q + 1) = d[u][1];
+    if (F == GEMM_SYMMETRIC && J != I) {
+      SM(C, 8 * J + 2 * q, 8 * I + r) = d[u][0];
+      SM(C, 8 * J + 2 * q + 1, 8 * I + r) = d[u][1];
+    }
   }
 }
 
@@ -285,151 +292,170 @@ __device__ __forceinline__ double rsqrt_mid(double v) {
   return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
-// In-place lower Cholesky A = L L' (lower triangle of A used; blockDim.x >= 256), and of B = L L' of
-// the same order next to it when B is given: panels of 8 columns, right-looking.  Warp 0 factors A's
-// panel and warp 1 B's, in registers (lane l holds panel rows kb + l and kb + 32 + l; the pivot
-// and the entries of the updating rows come by shuffles; L(r,c) = a(r,c) * rd, rd = pivot^-1/2, and
-// L(c,c) = pivot rd with the residual of its square corrected); then every warp takes 8 x 8 tiles of
-// the trailing lower triangle of both matrices, A22 -= L21 L21' on the FP64 tensor cores (two m8n8k4
-// steps).  Two barriers per panel.  A pivot that is not positive and finite stops that matrix
-// (false); the other carries on.  Entries above the diagonal end as zeros.  Bound by the panel's
-// chain, eight times pivot -> shuffle -> root -> shuffle -> update.
-__device__ inline void cta_cholesky_lower2(double* A, double* B, int n, bool* okA, bool* okB) {
-  __shared__ int live[2];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  const bool two = (B != nullptr);
-  if (threadIdx.x == 0) {
-    live[0] = 1;
-    live[1] = two ? 1 : 0;
+// One 8-column panel of cta_cholesky_lower in one warp, columns kb .. kb+w-1, any pivot: lane l holds the
+// panel's rows kb + l and kb + 32 + l, pivots and the updating rows' entries come by shuffles.  False at
+// a pivot that is not positive and finite.
+static __device__ __noinline__ bool cholesky_panel_any(double* A, int n, int kb, int w) {
+  const int lane = threadIdx.x & 31, r0 = kb + lane, r1 = kb + 32 + lane;
+  double P0[8], P1[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    P0[c] = (c < w && r0 < n) ? SM(A, r0, kb + c) : 0.0;
+    P1[c] = (c < w && r1 < n) ? SM(A, r1, kb + c) : 0.0;
   }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    if (c < w) {
+      const double piv = __shfl_sync(0xffffffffu, P0[c], c);
+      if (!(piv > 0.0 && isfinite(piv))) return false;
+      const double d = sqrt(piv), rd = 1.0 / d;
+      P0[c] = lane < c ? 0.0 : (lane == c ? d : P0[c] * rd);
+      P1[c] *= rd;
+#pragma unroll
+      for (int c2 = c + 1; c2 < 8; ++c2) {
+        const double l = __shfl_sync(0xffffffffu, P0[c], c2);  // L(kb + c2, kb + c)
+        P0[c2] = fma(-P0[c], l, P0[c2]);
+        P1[c2] = fma(-P1[c], l, P1[c2]);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    if (c < w && r0 < n) SM(A, r0, kb + c) = P0[c];
+    if (c < w && r1 < n) SM(A, r1, kb + c) = P1[c];
+  }
+  return true;
+}
+
+// In-place lower Cholesky A = L L' (lower triangle of A used, zero padded; 256 threads): panels of 8
+// columns, right-looking.  Warp 0 factors the panel: every lane has the 8 x 8 diagonal block to itself
+// and eliminates it next to its own two rows, so that the chain of a column is root -> scale -> update
+// (about 70 cycles) without a shuffle; L(r,c) = a(r,c) rd, rd = pivot^-1/2, and L(c,c) = pivot rd with
+// the residual of its square corrected.  A pivot out of [2^-1000, 2^1000) repeats the panel the slow way.
+// Then A22 -= L21 L21' on the lower 8 x 8 tiles on the FP64 tensor cores (two m8n8k4 steps), one warp a
+// tile row, rows w and 7 - w in the same quarter of the SM.  Two barriers a panel.  False when a pivot
+// is not positive and finite.  Entries above the diagonal end as zeros.
+// Order 64: 19200 cycles; with a shuffle per updating entry, a root and a reciprocal a column and the
+// tiles dealt to 32 warps, two matrices at once, 31900.
+__device__ inline bool cta_cholesky_lower(double* A, int n) {
+  __shared__ int live;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ti = (warp & 4) ? 7 - (warp & 3) : (warp & 3), r = lane >> 2, q = lane & 3;
+  if (threadIdx.x == 0) live = 1;
   __syncthreads();
   for (int kb = 0; kb < n; kb += 8) {
     const int w = min(8, n - kb);
-    if (warp < 2 && live[warp]) {  // panel of one matrix in one warp
-      double* X = warp == 0 ? A : B;
+    if (warp == 0) {
       const int r0 = kb + lane, r1 = kb + 32 + lane;
-      double P0[8], P1[8];
+      double D[36], P0[8], P1[8], dg[8];  // D: the block's lower triangle by columns
+#pragma unroll
+      for (int c = 0, e = 0; c < 8; ++c)
+#pragma unroll
+        for (int i = c; i < 8; ++i, ++e) D[e] = i < w ? SM(A, kb + i, kb + c) : (i == c ? 1.0 : 0.0);
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        P0[c] = (c < w && r0 < n) ? SM(X, r0, kb + c) : 0.0;
-        P1[c] = (c < w && r1 < n) ? SM(X, r1, kb + c) : 0.0;
+        P0[c] = (c < w && r0 < n) ? SM(A, r0, kb + c) : 0.0;
+        P1[c] = (c < w && r1 < n) ? SM(A, r1, kb + c) : 0.0;
+      }
+      bool mid = true;
+#pragma unroll
+      for (int c = 0, e = 0; c < 8; e += 8 - c, ++c) {
+        const double piv = D[e], rd = rsqrt_mid(piv), d0 = piv * rd;
+        mid = mid && mid_range(piv);
+        dg[c] = fma(0.5 * rd, fma(-d0, d0, piv), d0);
+#pragma unroll
+        for (int i = c + 1; i < 8; ++i) D[e + i - c] *= rd;
+        P0[c] *= rd;
+        P1[c] *= rd;
+#pragma unroll
+        for (int j = c + 1, f = e + 8 - c; j < 8; f += 8 - j, ++j) {
+          const double l = D[e + j - c];
+#pragma unroll
+          for (int i = j; i < 8; ++i) D[f + i - j] = fma(-D[e + i - c], l, D[f + i - j]);
+          P0[j] = fma(-P0[c], l, P0[j]);
+          P1[j] = fma(-P1[c], l, P1[j]);
+        }
       }
       bool ok = true;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        if (c < w && ok) {
-          const double piv = __shfl_sync(0xffffffffu, P0[c], c);
-          ok = (unsigned)__double2hiint(piv) - 1u < 0x7fefffffu || (piv > 0.0 && isfinite(piv));
-          if (ok) {
-            const double rd = mid_range(piv) ? rsqrt_mid(piv) : rsqrt(piv), d0 = piv * rd;
-            const double d = fma(0.5 * rd, fma(-d0, d0, piv), d0);
-            P0[c] = lane < c ? 0.0 : (lane == c ? d : P0[c] * rd);
-            P1[c] *= rd;
-#pragma unroll
-            for (int c2 = c + 1; c2 < 8; ++c2) {
-              const double l = __shfl_sync(0xffffffffu, P0[c], c2);  // L(kb + c2, kb + c)
-              P0[c2] = fma(-P0[c], l, P0[c2]);
-              P1[c2] = fma(-P1[c], l, P1[c2]);
-            }
-          }
-        }
-      }
-      if (ok) {
+      if (mid) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          if (c < w && r0 < n) SM(X, r0, kb + c) = P0[c];
-          if (c < w && r1 < n) SM(X, r1, kb + c) = P1[c];
+          const double v = lane < c ? 0.0 : (lane == c ? dg[c] : P0[c]);
+          if (c < w && r0 < n) SM(A, r0, kb + c) = v;
+          if (c < w && r1 < n) SM(A, r1, kb + c) = P1[c];
         }
-      } else if (lane == 0) {
-        live[warp] = 0;
+      } else {
+        ok = cholesky_panel_any(A, n, kb, w);
       }
+      if (!ok && lane == 0) live = 0;
     }
     __syncthreads();
-    const int t0 = kb + 8;
-    if (t0 < n) {  // trailing update of the lower tiles on DMMA
-      const int nt = (n - t0 + 7) >> 3, per = nt * (nt + 1) / 2;
-      const int r = lane >> 2, q = lane & 3;
-      for (int e = warp; e < 2 * per; e += nwarps) {
-        const int mtx = e >= per ? 1 : 0;
-        if (!live[mtx]) continue;
-        double* X = mtx ? B : A;
-        int u = mtx ? e - per : e, ti = 0;
-        while (u > ti) {  // u -> (ti, tj), tj <= ti
-          u -= ti + 1;
-          ++ti;
-        }
-        const int row = t0 + 8 * ti, col = t0 + 8 * u;
-        double d0 = SM(X, row + r, col + 2 * q), d1 = SM(X, row + r, col + 2 * q + 1);
+    if (!live) return false;
+    const int t0 = kb + 8, nt = (n - t0 + 7) >> 3;
+    if (ti < nt) {
+      const double a0 = -SM(A, t0 + 8 * ti + r, kb + q), a1 = -SM(A, t0 + 8 * ti + r, kb + 4 + q);
 #pragma unroll
-        for (int k4 = 0; k4 < 8; k4 += 4) {
-          const double a = -SM(X, row + r, kb + k4 + q), b = SM(X, col + r, kb + k4 + q);
-          dmma_m8n8k4(d0, d1, a, b);
+      for (int tj = 0; tj < 7; ++tj) {
+        if (tj <= ti) {
+          double* C = &SM(A, t0 + 8 * ti + r, t0 + 8 * tj + 2 * q);
+          double d0 = C[0], d1 = C[SDPXG_LD];
+          dmma_m8n8k4(d0, d1, a0, SM(A, t0 + 8 * tj + r, kb + q));
+          dmma_m8n8k4(d0, d1, a1, SM(A, t0 + 8 * tj + r, kb + 4 + q));
+          C[0] = d0;
+          C[SDPXG_LD] = d1;
         }
-        SM(X, row + r, col + 2 * q) = d0;
-        SM(X, row + r, col + 2 * q + 1) = d1;
       }
     }
     __syncthreads();
   }
-  *okA = live[0] != 0;
-  *okB = two && live[1] != 0;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int i = e % n, j = e / n;
-    if (i < j) {
-      if (*okA) SM(A, i, j) = 0.0;
-      if (two && *okB) SM(B, i, j) = 0.0;
-    }
-  }
+  for (int j = warp; j < n; j += 8)
+    for (int i = lane; i < j; i += 32) SM(A, i, j) = 0.0;
   __syncthreads();
+  return true;
 }
 
-__device__ inline bool cta_cholesky_lower(double* A, int n) {
-  bool ok, unused;
-  cta_cholesky_lower2(A, nullptr, n, &ok, &unused);
-  return ok;
-}
-
-// Solve L' X = B in place of B (L lower, n x n), one column per thread.
-// B := L^-T B for the lower triangular L (n x n, n <= 64): blocked back substitution, 8 rows at
-// a time from the bottom.  Each block of rows is solved against its 8 x 8 diagonal block, one
-// thread per column of B (x_i = (b_i - sum_k L(k,i) x_k) / L(i,i), the reciprocals formed first,
-// in parallel); the rows above then take B(0:ib, :) -= L(ib:ib+8, 0:ib)' X on the FP64 tensor
-// cores, one warp per 8 x 8 tile (two m8n8k4 steps).  Two barriers per block of rows.
-// blockDim.x >= 64; `rd` is n doubles of shared memory.
+// B := L^-T B for the lower triangular L (n x n, n <= 64, both zero padded), back substitution by blocks
+// of 8 rows from the bottom, left-looking: warp w has the 8 columns from 8w on to itself, so no barrier
+// of the CTA is needed between blocks.  B(I, w) -= sum_{K > I} L(K, I)' X(K, w) on the FP64 tensor cores,
+// then the 8 x 8 diagonal block, one lane a column with its eight entries in registers (x_i = (b_i -
+// sum_k L(k,i) x_k) / L(i,i), the reciprocals formed first).
+// blockDim.x >= 256; `rd` is n doubles of shared memory.
 __device__ __forceinline__ void cta_trsm_lower_t_blocked(const double* L, double* B, int n, double* rd) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) rd[i] = 1.0 / SM(L, i, i);
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int r = lane >> 2, q = lane & 3, nt = (n + 7) >> 3;
-  for (int ib = (nt - 1) * 8; ib >= 0; ib -= 8) {
-    const int ie = min(ib + 8, n);
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-      for (int i = ie - 1; i >= ib; --i) {
-        double acc = SM(B, i, j);
-        for (int k = i + 1; k < ie; ++k) acc = fma(-SM(L, k, i), SM(B, k, j), acc);
-        SM(B, i, j) = acc * rd[i];
+  const int lane = threadIdx.x & 31, J = threadIdx.x >> 5, r = lane >> 2, q = lane & 3, nt = (n + 7) >> 3;
+  for (int I = nt - 1; J < nt && I >= 0; --I) {
+    const int ib = 8 * I;
+    if (I < nt - 1) {
+      double d[2][2];
+      d[0][0] = SM(B, ib + r, 8 * J + 2 * q);
+      d[0][1] = SM(B, ib + r, 8 * J + 2 * q + 1);
+      d[1][0] = d[1][1] = 0.0;
+      for (int K = ib + 8; K < 8 * nt; K += 8) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          dmma_m8n8k4(d[u][0], d[u][1], -SM(L, K + 4 * u + q, ib + r), SM(B, K + 4 * u + q, 8 * J + r));
+      }
+      SM(B, ib + r, 8 * J + 2 * q) = d[0][0] + d[1][0];
+      SM(B, ib + r, 8 * J + 2 * q + 1) = d[0][1] + d[1][1];
+      __syncwarp();
+    }
+    if (lane < 8) {
+      const int j = 8 * J + lane;
+      double x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = ib + i < n ? SM(B, ib + i, j) : 0.0;
+#pragma unroll
+      for (int i = 7; i >= 0; --i) {
+        if (ib + i < n) {
+          x[i] *= rd[ib + i];
+          SM(B, ib + i, j) = x[i];
+#pragma unroll
+          for (int k = 0; k < i; ++k) x[k] = fma(-SM(L, ib + i, ib + k), x[i], x[k]);
+        }
       }
     }
-    __syncthreads();
-    for (int t = warp; t < (ib >> 3) * nt; t += nwarps) {  // tiles above the block
-      const int ti = (t % (ib >> 3)) << 3, tj = (t / (ib >> 3)) << 3;
-      double d0 = SM(B, ti + r, tj + 2 * q), d1 = SM(B, ti + r, tj + 2 * q + 1);
-#pragma unroll
-      for (int k4 = 0; k4 < 8; k4 += 4)
-        dmma_m8n8k4(d0, d1, -SM(L, ib + k4 + q, ti + r), SM(B, ib + k4 + q, tj + r));
-      SM(B, ti + r, tj + 2 * q) = d0;
-      SM(B, ti + r, tj + 2 * q + 1) = d1;
-    }
-    __syncthreads();
+    __syncwarp();
   }
-}
-
-__device__ __forceinline__ void cta_trsm_lower_t(const double* L, double* B, int n) {
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    for (int i = n - 1; i >= 0; --i) {
-      double acc = SM(B, i, j);
-      for (int k = i + 1; k < n; ++k) acc = fma(-SM(L, k, i), SM(B, k, j), acc);
-      SM(B, i, j) = acc / SM(L, i, i);
-    }
-  }
+  __syncthreads();
 }

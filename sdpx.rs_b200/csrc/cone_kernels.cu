@@ -26,37 +26,37 @@ constexpr int kMat = SDPXG_LD * SDPXG_NMAX;  // doubles per shared matrix
 // normalised columns that one-sided Jacobi leaves in M, so the rotations are not accumulated
 // into V.  Both forms have the same
 // normwise accuracy (a triangular solve with L1 or with L2 each).  Ginv = Rinv' Rinv.
-// Two launches: k_nt_factor (1024 threads: both Cholesky factors in the register-resident CTA
-// form, M = L2'L1) leaves M in R's slot and L2 in Rinv's slot of each block; k_nt_svd (512
-// threads, room for the register-resident Jacobi) reads them back and writes R, Rinv, Ginv,
-// lam and lam^-1/2.  A failed factorisation sets SDPXG_ST_CHOL_FAIL, which the second launch
-// reads to leave every block alone (the scaling is rejected as a whole).
-// Shared memory of k_nt_factor: 3 matrices; of k_nt_svd: 5 matrices +
-// 2n doubles + n ints + 1 int.
+// Two launches: k_nt_factor, one CTA per block and matrix, leaves L1 in R's slot and L2 in Rinv's slot
+// of each block; k_nt_svd reads them back and writes R, Rinv, Ginv, lam and lam^-1/2.  A failed
+// factorisation sets SDPXG_ST_CHOL_FAIL, which the second launch reads to leave every block alone (the
+// scaling is rejected as a whole).
+// Shared memory of k_nt_factor: 1 matrix; of k_nt_svd: 5 matrices + 5n doubles + n ints + 1 int.
+// At n = 64, k_nt_factor 31 us with both factors and M in one CTA of 1024 threads, now 22; k_nt_svd (12
+// sweeps) 357 us with eight warps on the Jacobi rounds, scalar loops over the columns and a back
+// substitution with two barriers a block of rows, now 257.
 // ---------------------------------------------------------------------------------------
-extern "C" __global__ void __launch_bounds__(SDPXG_CONE_THREADS)
+extern "C" __global__ void __launch_bounds__(SDPXG_EIG_THREADS)
 k_nt_factor(const BlockDesc* __restrict__ blocks, const double* __restrict__ s,
             const double* __restrict__ z, double* __restrict__ R, double* __restrict__ Rinv,
             uint32_t* __restrict__ status) {
   extern __shared__ double smem[];
   const BlockDesc bd = blocks[blockIdx.x];
   const int n = bd.n;
-  double* L1 = smem;
-  double* L2 = L1 + kMat;
-  double* M = L2 + kMat;
-  cta_zero_mat(M);
-  cta_load_smat(L1, s + bd.svec_off, n);
-  cta_load_smat(L2, z + bd.svec_off, n);
-  bool ok1, ok2;
-  cta_cholesky_lower2(L1, L2, n, &ok1, &ok2);  // chol(S), chol(Z) together
-  if (!ok1 || !ok2) {
+  double* L = smem;
+  cta_load_smat(L, (blockIdx.y == 0 ? s : z) + bd.svec_off, n);
+  if (!cta_cholesky_lower(L, n)) {
     if (threadIdx.x == 0) atomicOr(status, SDPXG_ST_CHOL_FAIL);
     return;
   }
-  cta_gemm(M, L2, true, L1, false, n);  // M = L2' L1
-  __syncthreads();
-  cta_store_mat(R + bd.mat_off, M, n);
-  cta_store_mat(Rinv + bd.mat_off, L2, n);
+  cta_store_mat((blockIdx.y == 0 ? R : Rinv) + bd.mat_off, L, n);
+}
+
+// a / b from y = 1 / b rounded: one residual step (a b that is no denominator of an ordinary quotient
+// divides).
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+  const double q = a * y;
+  const double q1 = fma(fma(-q, b, a), y, q);
+  return mid_range(b) && isfinite(q1) ? q1 : a / b;
 }
 
 extern "C" __global__ void __launch_bounds__(SDPXG_NT_SVD_THREADS)
@@ -74,70 +74,96 @@ k_nt_svd(const BlockDesc* __restrict__ blocks, double* __restrict__ R, double* _
   double* X = V + kMat;
   double* sig = X + kMat;
   double* lsort = sig + SDPXG_NMAX;
-  int* rank = reinterpret_cast<int*>(lsort + SDPXG_NMAX);
+  double* root = lsort + SDPXG_NMAX;
+  double* iroot = root + SDPXG_NMAX;
+  double* isig = iroot + SDPXG_NMAX;
+  int* rank = reinterpret_cast<int*>(isig + SDPXG_NMAX);
   int* flag = rank + SDPXG_NMAX;
 
   cta_zero_mat(V);  // V and X are written n x n only: keep their padding zero for the MMAs
   cta_zero_mat(X);
-  cta_load_mat(M, R + bd.mat_off, n);
+  cta_load_mat(L1, R + bd.mat_off, n);
   cta_load_mat(L2, Rinv + bd.mat_off, n);
+  __syncthreads();
+  cta_gemm<true, false, 8, GEMM_LOWER_TN>(M, L2, L1, n);  // M = L2' L1
   __syncthreads();
   int sweeps = cta_jacobi_left(M, n, L1, flag);  // M -> U diag(lam); L1 as scratch
   if (sweeps < 0) {
     if (threadIdx.x == 0) atomicOr(status, SDPXG_ST_SVD_UNCONVERGED);
     return;
   }
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+  // singular values and their ranks, eight threads a column
+  const int g8 = threadIdx.x >> 3, u8 = threadIdx.x & 7;
+  for (int j0 = 0; j0 < n; j0 += SDPXG_NT_SVD_THREADS / 8) {
+    const int j = j0 + g8;
     double acc = 0.0;
-    for (int k = 0; k < n; ++k) acc = fma(SM(M, k, j), SM(M, k, j), acc);
-    sig[j] = sqrt(acc);
-  }
-  __syncthreads();
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    int r = 0;
-    for (int k = 0; k < n; ++k) r += (sig[k] > sig[j]) || (sig[k] == sig[j] && k < j);
-    rank[j] = r;
-    lsort[r] = sig[j];
+    for (int k = u8; k < n; k += 8) acc = j < n ? fma(SM(M, k, j), SM(M, k, j), acc) : 0.0;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (u8 == 0 && j < n) sig[j] = sqrt(acc);
   }
   __syncthreads();
   bool good = true;
-  for (int j = 0; j < n; ++j) good = good && (lsort[j] > 0.0) && isfinite(lsort[j]);
-  if (!good) {
+  for (int j0 = 0; j0 < n; j0 += SDPXG_NT_SVD_THREADS / 8) {
+    const int j = j0 + g8;
+    int r = 0;
+    if (j < n)
+      for (int k = u8; k < n; k += 8) r += (sig[k] > sig[j]) || (sig[k] == sig[j] && k < j);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    if (u8 == 0 && j < n) {
+      rank[j] = r;
+      lsort[r] = sig[j];
+      root[r] = sqrt(sig[j]);
+      iroot[r] = 1.0 / sqrt(sig[j]);
+      isig[j] = 1.0 / sig[j];
+      good = sig[j] > 0.0 && isfinite(sig[j]);
+    }
+  }
+  if (!__syncthreads_and(good)) {
     if (threadIdx.x == 0) atomicOr(status, SDPXG_ST_CHOL_FAIL);
     return;
   }
   // X = U with columns in descending singular-value order; V = X as the right-hand side
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    int i = e % n, j = e / n;
-    const double u = SM(M, i, j) / sig[j];
-    SM(X, i, rank[j]) = u;
-    SM(V, i, rank[j]) = u;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  for (int j = warp; j < n; j += nwarps) {
+    const int c = rank[j];
+    for (int i = lane; i < n; i += 32) {
+      const double u = quotient(SM(M, i, j), sig[j], isig[j]);
+      SM(X, i, c) = u;
+      SM(V, i, c) = u;
+    }
   }
   __syncthreads();
   cta_trsm_lower_t_blocked(L2, V, n, sig);  // V = L2^-T U (sig is free: lsort holds lambda)
   double* Rg = R + bd.mat_off;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    int i = e % n, j = e / n;
-    Rg[e] = SM(V, i, j) * sqrt(lsort[j]);
-  }
-  cta_gemm(L1, X, true, L2, true, n);  // L1 = U' L2'
+  for (int j = warp; j < n; j += nwarps)
+    for (int i = lane; i < n; i += 32) Rg[i + j * n] = SM(V, i, j) * root[j];
+  cta_gemm<true, true, 8, GEMM_UPPER_B>(L1, X, L2, n);  // L1 = U' L2'
   __syncthreads();
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    int i = e % n, j = e / n;
-    SM(L1, i, j) /= sqrt(lsort[i]);  // Rinv = lam^-1/2 U' L2'
-  }
-  __syncthreads();
-  cta_store_mat(Rinv + bd.mat_off, L1, n);
-  cta_gemm(M, L1, true, L1, false, n);  // Ginv = Rinv' Rinv
-  __syncthreads();
-  cta_store_mat(Ginv + bd.mat_off, M, n);
+  double* Rig = Rinv + bd.mat_off;
   bool fin = true;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x)
-    fin = fin && isfinite(SM(M, e % n, e / n)) && isfinite(SM(L1, e % n, e / n));
+  for (int j = warp; j < n; j += nwarps)
+    for (int i = lane; i < n; i += 32) {
+      const double v = quotient(SM(L1, i, j), root[i], iroot[i]);  // Rinv = lam^-1/2 U' L2'
+      SM(L1, i, j) = v;
+      Rig[i + j * n] = v;
+      fin = fin && isfinite(v);
+    }
+  __syncthreads();
+  cta_gemm<true, false, 8, GEMM_SYMMETRIC>(M, L1, L1, n);  // Ginv = Rinv' Rinv
+  __syncthreads();
+  double* Gg = Ginv + bd.mat_off;
+  for (int j = warp; j < n; j += nwarps)
+    for (int i = lane; i < n; i += 32) {
+      const double v = SM(M, i, j);
+      Gg[i + j * n] = v;
+      fin = fin && isfinite(v);
+    }
   if (!fin) atomicOr(status, SDPXG_ST_NONFINITE);
   for (int j = threadIdx.x; j < n; j += blockDim.x) {
     lam[bd.vec_off + j] = lsort[j];
-    lisqrt[bd.vec_off + j] = 1.0 / sqrt(lsort[j]);
+    lisqrt[bd.vec_off + j] = iroot[j];
   }
 }
 
@@ -175,17 +201,17 @@ extern "C" __global__ void k_ginv_from_rinv(const BlockDesc* __restrict__ blocks
   }
 }
 
+// Y = B X B' (outer_t) or B' X B for a symmetric X, 256 threads.
 __device__ void cta_congruence(double* Y, double* T, const double* X, const double* B,
                                bool outer_t, int n) {
-  // outer_t: Y = B X B'  else Y = B' X B
   if (outer_t) {
-    cta_gemm(T, X, false, B, true, n);  // T = X B'
+    cta_gemm<false, true, 8>(T, X, B, n);  // T = X B'
     __syncthreads();
-    cta_gemm(Y, B, false, T, false, n);  // Y = B T
+    cta_gemm<false, false, 8, GEMM_SYMMETRIC>(Y, B, T, n);  // Y = B T
   } else {
-    cta_gemm(T, X, false, B, false, n);  // T = X B
+    cta_gemm<false, false, 8>(T, X, B, n);  // T = X B
     __syncthreads();
-    cta_gemm(Y, B, true, T, false, n);  // Y = B' T
+    cta_gemm<true, false, 8, GEMM_SYMMETRIC>(Y, B, T, n);  // Y = B' T
   }
   __syncthreads();
 }

@@ -16,34 +16,152 @@
 
 namespace jacobi_detail {
 
-// x'y over the eight rows a lane holds, as a tree (depth 4).
-__device__ __forceinline__ double dot8(const double* x, const double* y) {
-  const double p0 = fma(x[1], y[1], x[0] * y[0]), p1 = fma(x[3], y[3], x[2] * y[2]);
-  const double p2 = fma(x[5], y[5], x[4] * y[4]), p3 = fma(x[7], y[7], x[6] * y[6]);
-  return (p0 + p1) + (p2 + p3);
+// x'y over the R rows a lane holds, in four chains.
+template <int R>
+__device__ __forceinline__ double dot_rows(const double (&x)[R], const double (&y)[R]) {
+  double p[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) p[u] = x[u] * y[u];
+#pragma unroll
+  for (int k = 4; k < R; ++k) p[k & 3] = fma(x[k], y[k], p[k & 3]);
+  return (p[0] + p[1]) + (p[2] + p[3]);
 }
 
-// Sum of the eight warps' partials b[0], b[32], ..., b[224] as a tree (the same bits in every
-// warp that reads them).
-__device__ __forceinline__ double sum8(const double* b) {
-  return ((b[0] + b[32]) + (b[64] + b[96])) + ((b[128] + b[160]) + (b[192] + b[224]));
-}
+// Sum of the four warps' partials b[0], b[32], b[64], b[96] (the same bits in every warp).
+__device__ __forceinline__ double sum4(const double* b) { return (b[0] + b[32]) + (b[64] + b[96]); }
 
 // Rotation x' = c x - s y, y' = s x + c y with x'y' = 0 for a pair with ||x||^2 = a, ||y||^2 = b,
 // x'y = g, by the half-angle formulas (|theta| <= pi/4):
 //   cos 2t = |h| / r, sin 2t = sign(h) 2g / r, r = sqrt(h^2 + 4g^2), h = b - a,
 //   c = sqrt((1 + cos 2t) / 2), s = sin 2t / (2c);
 // c >= 1/sqrt 2, so nothing cancels, and c^2 + s^2 = 1 to rounding.  tg = (s / c) g, with which
-// ||x'||^2 = a - tg and ||y'||^2 = b + tg.
-__device__ __forceinline__ void rotation(double a, double b, double g, double& c, double& s, double& tg) {
-  const double h = b - a;
-  const double ir = rsqrt(fma(h, h, 4.0 * g * g));
-  const double c2 = fabs(h) * ir, s2 = (h < 0.0 ? -2.0 * g : 2.0 * g) * ir;
-  const double cc = fma(0.5, c2, 0.5);
-  const double ic = rsqrt(cc);
-  c = cc * ic;
-  s = 0.5 * s2 * ic;
-  tg = s * ic * g;
+// ||x'||^2 = a - tg and ||y'||^2 = b + tg.  No branch (an in-order warp pays for each): a pair that
+// is not `on`, or whose r^2 < 2^-1000 (next to columns of norm 2^200), gets the identity and false.
+__device__ __forceinline__ bool rotation(double a, double b, double g, bool on, double& c, double& s, double& tg) {
+  const double h = b - a, g2 = g + g, r2 = fma(g2, g2, h * h);
+  const bool rot = on && mid_range(r2);
+  const double ir = rsqrt_mid(r2), cc = fma(0.5 * fabs(h), ir, 0.5), ic = rsqrt_mid(cc);
+  const double t = (h < 0.0 ? -g : g) * ir * ic;
+  c = rot ? cc * ic : 1.0;
+  s = rot ? t : 0.0;
+  tg = rot ? t * ic * g : 0.0;
+  return rot;
+}
+
+// R rows per warp (n <= 4 R).
+template <int R>
+__device__ __forceinline__ int sweep_columns(double* M, int n, double* part) {
+  constexpr double kTol2 = 1e-30, kBig2 = 1e-20;
+  constexpr unsigned kFull = 0xffffffffu;
+  const int warp = threadIdx.x >> 5, j = threadIdx.x & 31;
+  const int N = n + (n & 1), H = N / 2;
+  int iA = j < H ? 2 * j : -1, iB = j < H ? 2 * j + 1 : -1;
+  double A[R], B[R], nA = 0.0, nB = 0.0, mx = 0.0;
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const int row = 4 * k + warp;
+    A[k] = (row < n && iA >= 0 && iA < n) ? SM(M, row, iA) : 0.0;
+    B[k] = (row < n && iB >= 0 && iB < n) ? SM(M, row, iB) : 0.0;
+    mx = fmax(mx, fmax(fabs(A[k]), fabs(B[k])));
+  }
+  // largest entry to 2^199 .. 2^200 by a power of two: the room that the norms' squares have
+  mx = warp_max(mx);
+  if (j == 0) part[warp] = mx;
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  mx = fmax(fmax(part[0], part[1]), fmax(part[2], part[3]));
+  int ex = 0;
+  if (mx > 0.0 && isfinite(mx)) ex = max(-800, min(1000, ilogb(mx) - 199));
+  const double down = ldexp(1.0, -ex), up = ldexp(1.0, ex);
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    A[k] *= down;
+    B[k] *= down;
+  }
+  int sweeps = (n < 2) ? 0 : -1;
+  int phase = 1;  // part[0..3] may still be read
+  for (int sweep = 0; n >= 2 && sweep < SDPXG_JACOBI_MAX_SWEEPS; ++sweep) {
+    bool rotated = false, big = false;
+    for (int r = 0; r < N; r += 2) {
+      {  // pairs (2j, 2j+1): both columns in this lane
+        double* buf = part + phase * 384;
+        phase ^= 1;
+        buf[warp * 32 + j] = dot_rows<R>(A, B);
+        if (r == 0) {
+          buf[128 + warp * 32 + j] = dot_rows<R>(A, A);
+          buf[256 + warp * 32 + j] = dot_rows<R>(B, B);
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (r == 0) {
+          nA = sum4(buf + 128 + j);
+          nB = sum4(buf + 256 + j);
+        }
+        const double a = nA, b = nB, ab = a * b, g = sum4(buf + j), gg = g * g;
+        double c, s, tg;
+        rotated |= rotation(a, b, g, j < H && gg > kTol2 * ab, c, s, tg);
+        big |= j < H && gg > kBig2 * ab;
+#pragma unroll
+        for (int k = 0; k < R; ++k) {  // rotate and trade places: A <- y', B <- x'
+          const double x = A[k], y = B[k];
+          A[k] = fma(s, x, c * y);
+          B[k] = fma(c, x, -s * y);
+        }
+        nA = b + tg;
+        nB = a - tg;
+        const int t = iA;
+        iA = iB;
+        iB = t;
+      }
+      {  // pairs (2j+1, 2j+2): this lane's B and lane j+1's A
+        double An[R], Bp[R];
+#pragma unroll
+        for (int k = 0; k < R; ++k) An[k] = __shfl_down_sync(kFull, A[k], 1);
+        const double nAn = __shfl_down_sync(kFull, nA, 1);
+        double* buf = part + phase * 384;
+        phase ^= 1;
+        buf[warp * 32 + j] = dot_rows<R>(B, An);
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const double* bj = buf + j;
+        const double q0 = bj[0], q1 = bj[32], q2 = bj[64], q3 = bj[96];
+#pragma unroll
+        for (int k = 0; k < R; ++k) Bp[k] = __shfl_up_sync(kFull, B[k], 1);
+        const int iAn = __shfl_down_sync(kFull, iA, 1), iBp = __shfl_up_sync(kFull, iB, 1);
+        const bool exists = j + 1 < H;  // pair (2j+1, 2j+2)
+        const double a = nB, b = nAn, ab = a * b, g = (q0 + q1) + (q2 + q3), gg = g * g;
+        double c, s, tg;
+        rotated |= rotation(a, b, g, exists && gg > kTol2 * ab, c, s, tg);
+        big |= exists && gg > kBig2 * ab;
+        const double nAl = __shfl_up_sync(kFull, a - tg, 1);
+        double cl = __shfl_up_sync(kFull, c, 1), sl = __shfl_up_sync(kFull, s, 1);
+        const bool recv = j >= 1 && j < H;  // lane j's A is the right column of pair j-1
+        c = exists ? c : 0.0;               // no pair: B stays
+        s = exists ? s : 1.0;
+        cl = recv ? cl : 0.0;
+        sl = recv ? sl : -1.0;
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+          B[k] = fma(s, B[k], c * An[k]);     // y' of pair j
+          A[k] = fma(cl, Bp[k], -sl * A[k]);  // x' of pair j-1
+        }
+        nB = exists ? b + tg : nB;
+        iB = exists ? iAn : iB;
+        nA = recv ? nAl : nA;
+        iA = recv ? iBp : iA;
+      }
+    }
+    if (!__any_sync(kFull, rotated) || !__any_sync(kFull, big)) {
+      sweeps = sweep + 1;
+      break;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const int row = 4 * k + warp;
+    if (row < n && j < H) {
+      if (iA < n) SM(M, row, iA) = A[k] * up;
+      if (iB < n) SM(M, row, iB) = B[k] * up;
+    }
+  }
+  return sweeps;
 }
 
 }  // namespace jacobi_detail
@@ -51,133 +169,34 @@ __device__ __forceinline__ void rotation(double a, double b, double g, double& c
 // One-sided (Hestenes) Jacobi on the columns of M (n x n, n <= 64, column-major shared memory
 // with leading dimension SDPXG_LD): on return M holds M V = U diag(sigma), columns in their
 // original order; V itself is not formed.  Returns the number of sweeps, or -1 when the sweep
-// bound was hit.  Every thread of the CTA calls it (blockDim.x >= 256).
+// bound was hit.  Every thread of the CTA calls it (blockDim.x >= 128).
 //
-// The matrix stays in registers for the whole iteration.  Warps 0..7 take part: warp w holds
-// rows [8w, 8w + 8), lane j the columns at positions 2j (A) and 2j+1 (B) of a line of
+// The matrix stays in registers for the whole iteration.  Warps 0..3 take part: warp w holds
+// the rows 4k + w, lane j the columns at positions 2j (A) and 2j+1 (B) of a line of
 // N = n rounded up to even positions (an odd n gets a zero column that never rotates).  The
 // pairs follow the odd-even ordering of Luk and Park: rounds alternate between the pairs
 // (2j, 2j+1), which a lane holds itself, and (2j+1, 2j+2), whose second column comes from lane
 // j+1 by a warp shuffle; after every rotation the two columns trade places, so in N rounds
 // every pair meets once (the moves are those of odd-even transposition sort on a reversed
-// line).  Only the across-lane rounds move data (two shuffles per row), and the lane that
-// computes a pair's rotation hands (c, s) to its right neighbour.  A pair's inner product is
-// the sum of the eight warps' row partials, taken in a fixed tree order, so every warp holds
-// the same bits and takes the same decisions without a broadcast; one named barrier per round
-// (the partials are double-buffered in `part`, 1536 doubles of shared memory).  Squared column
-// norms are summed exactly at the start of every sweep and carried through its rotations
+// line).  Only the across-lane rounds move data (two shuffles per row, one of them under the
+// exchange of the partials), and the lane that computes a pair's rotation hands (c, s) to its right
+// neighbour.  A pair's inner product is the sum of the four warps' row partials, taken in a fixed tree
+// order, so every warp holds the same bits and takes the same decisions without a broadcast; one named
+// barrier per round (the partials are double-buffered in `part`, 768 doubles of shared memory).
+// Squared column norms are summed exactly at the start of every sweep and carried through its rotations
 // (a - tg, b + tg).  A pair rotates while |x'y| > 1e-15 sqrt(||x||^2 ||y||^2); the sweeps stop
 // after one without a rotation, or after one in which every cosine was below 1e-10 (the
 // rotations of that sweep leave cosines of order 1e-20: one-sided Jacobi converges
 // quadratically).
+// One warp per SM quarter, not two: a round is bound by its chain (inner product, exchange, two roots,
+// rotation), every warp repeats the scalars, and half the warps read half the partials: 1110 cycles a
+// pair of rounds at n = 64 against 1600.  Of these the rotations' chains take 360, the FP64 pipe's
+// issue of inner products and rotations 400, the shuffles 140.
 __device__ inline int cta_jacobi_left(double* M, int n, double* part, int* out) {
-  using namespace jacobi_detail;
-  constexpr double kTol2 = 1e-30, kBig2 = 1e-20;
-  constexpr unsigned kFull = 0xffffffffu;
-  const int warp = threadIdx.x >> 5, j = threadIdx.x & 31;
-  if (warp < 8) {
-    const int N = n + (n & 1), H = N / 2;
-    int iA = j < H ? 2 * j : -1, iB = j < H ? 2 * j + 1 : -1;
-    double A[8], B[8], nA = 0.0, nB = 0.0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int row = 8 * warp + k;
-      A[k] = (row < n && iA >= 0 && iA < n) ? SM(M, row, iA) : 0.0;
-      B[k] = (row < n && iB >= 0 && iB < n) ? SM(M, row, iB) : 0.0;
-    }
-    int sweeps = (n < 2) ? 0 : -1;
-    int phase = 0;
-    for (int sweep = 0; n >= 2 && sweep < SDPXG_JACOBI_MAX_SWEEPS; ++sweep) {
-      bool rotated = false, big = false;
-      for (int r = 0; r < N; r += 2) {
-        {  // pairs (2j, 2j+1): both columns in this lane
-          double* buf = part + phase * 768;
-          phase ^= 1;
-          buf[warp * 32 + j] = dot8(A, B);
-          if (r == 0) {
-            buf[256 + warp * 32 + j] = dot8(A, A);
-            buf[512 + warp * 32 + j] = dot8(B, B);
-          }
-          asm volatile("bar.sync 1, 256;" ::: "memory");
-          const double g = sum8(buf + j);
-          if (r == 0) {
-            nA = sum8(buf + 256 + j);
-            nB = sum8(buf + 512 + j);
-          }
-          const double a = nA, b = nB, gg = g * g, ab = a * b;
-          const bool rot = j < H && gg > kTol2 * ab;
-          rotated |= rot;
-          big |= j < H && gg > kBig2 * ab;
-          double c = 1.0, s = 0.0, tg = 0.0;
-          if (rot) rotation(a, b, g, c, s, tg);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {  // rotate and trade places: A <- y', B <- x'
-            const double x = A[k], y = B[k];
-            A[k] = fma(s, x, c * y);
-            B[k] = fma(c, x, -s * y);
-          }
-          nA = b + tg;
-          nB = a - tg;
-          const int t = iA;
-          iA = iB;
-          iB = t;
-        }
-        {  // pairs (2j+1, 2j+2): this lane's B and lane j+1's A
-          double An[8], Bp[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            An[k] = __shfl_down_sync(kFull, A[k], 1);
-            Bp[k] = __shfl_up_sync(kFull, B[k], 1);
-          }
-          const double nAn = __shfl_down_sync(kFull, nA, 1);
-          const int iAn = __shfl_down_sync(kFull, iA, 1), iBp = __shfl_up_sync(kFull, iB, 1);
-          double* buf = part + phase * 768;
-          phase ^= 1;
-          buf[warp * 32 + j] = dot8(B, An);
-          asm volatile("bar.sync 1, 256;" ::: "memory");
-          const double g = sum8(buf + j);
-          const bool ex = j + 1 < H;  // pair (2j+1, 2j+2) exists
-          const double a = nB, b = nAn, gg = g * g, ab = a * b;
-          const bool rot = ex && gg > kTol2 * ab;
-          rotated |= rot;
-          big |= ex && gg > kBig2 * ab;
-          double c = ex ? 1.0 : 0.0, s = ex ? 0.0 : 1.0, tg = 0.0;  // no pair: B stays
-          if (rot) rotation(a, b, g, c, s, tg);
-          double cl = __shfl_up_sync(kFull, c, 1), sl = __shfl_up_sync(kFull, s, 1);
-          const double nAl = __shfl_up_sync(kFull, a - tg, 1);
-          const bool recv = j >= 1 && j < H;  // lane j's A is the right column of pair j-1
-          if (!recv) {
-            cl = 0.0;
-            sl = -1.0;
-          }
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            B[k] = fma(s, B[k], c * An[k]);   // y' of pair j
-            A[k] = fma(cl, Bp[k], -sl * A[k]);  // x' of pair j-1
-          }
-          if (ex) {
-            nB = b + tg;
-            iB = iAn;
-          }
-          if (recv) {
-            nA = nAl;
-            iA = iBp;
-          }
-        }
-      }
-      if (!__any_sync(kFull, rotated) || !__any_sync(kFull, big)) {
-        sweeps = sweep + 1;
-        break;
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int row = 8 * warp + k;
-      if (row < n && j < H) {
-        if (iA < n) SM(M, row, iA) = A[k];
-        if (iB < n) SM(M, row, iB) = B[k];
-      }
-    }
+  if (threadIdx.x < 128) {
+    const int sweeps = n <= 16 ? jacobi_detail::sweep_columns<4>(M, n, part)
+                     : n <= 32 ? jacobi_detail::sweep_columns<8>(M, n, part)
+                               : jacobi_detail::sweep_columns<16>(M, n, part);
     if (threadIdx.x == 0) *out = sweeps;
   }
   __syncthreads();

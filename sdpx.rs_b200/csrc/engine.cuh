@@ -30,8 +30,8 @@
 namespace sdpxg {
 
 constexpr int kMatD = SDPXG_LD * SDPXG_NMAX;
-constexpr size_t kSmemNtFactor = 3 * kMatD * sizeof(double);
-constexpr size_t kSmemNt = (5 * kMatD + 2 * SDPXG_NMAX) * sizeof(double) + (SDPXG_NMAX + 1) * sizeof(int);
+constexpr size_t kSmemNtFactor = kMatD * sizeof(double);
+constexpr size_t kSmemNt = (5 * kMatD + 5 * SDPXG_NMAX) * sizeof(double) + (SDPXG_NMAX + 1) * sizeof(int);
 constexpr size_t kSmemCong = (2 * kMatD + 2 * 16 * SDPXG_LD) * sizeof(double);
 constexpr size_t kSmemCirc = 2 * kMatD * sizeof(double);
 constexpr size_t kSmemStep = (4 * kMatD + 2 * SDPXG_NMAX + 1) * sizeof(double);
@@ -843,7 +843,7 @@ class Engine {
     clear_status();
     tbegin(KT_SCALE);
     if (nblk) {
-      ++g_launches, k_nt_factor<<<nblk, SDPXG_CONE_THREADS, kSmemNtFactor, st>>>(blocks_, s, z, R_, Rinv_,
+      ++g_launches, k_nt_factor<<<dim3(nblk, 2), SDPXG_EIG_THREADS, kSmemNtFactor, st>>>(blocks_, s, z, R_, Rinv_,
                                                                                   status_);
       ++g_launches, k_nt_svd<<<nblk, SDPXG_NT_SVD_THREADS, kSmemNt, st>>>(blocks_, R_, Rinv_, Ginv_, lam_,
                                                                            lisqrt_, status_);

@@ -35,9 +35,9 @@ k_schur_transform(const BlockDesc* __restrict__ blocks, const int* __restrict__ 
   const long off = acol_off[j] + (long)t * tn;
   cta_load_smat(X, Acol + off, n);
   __syncthreads();
-  cta_gemm(Y, G, false, X, false, n);  // Y = Ginv A
+  cta_gemm<false, false, 2>(Y, G, X, n);  // Y = Ginv A
   __syncthreads();
-  cta_gemm(X, Y, false, G, false, n);  // X = Ginv A Ginv
+  cta_gemm<false, false, 2, GEMM_SYMMETRIC>(X, Y, G, n);  // X = Ginv A Ginv
   __syncthreads();
   cta_store_svec(Tcol + off, X, n);
 }
