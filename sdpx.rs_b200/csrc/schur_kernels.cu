@@ -11,6 +11,8 @@
 // computed as T = svec(Ginv A Ginv) per column (k_schur_transform), one grouped GEMM
 // S_j = Acol_j' T_j per block (k_schur_block_gemm), and a deterministic cone-order gather
 // into the dense m x m matrix (k_schur_gather).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace {
@@ -43,89 +45,149 @@ k_schur_transform(const BlockDesc* __restrict__ blocks, const int* __restrict__ 
 }
 
 // Grouped GEMM S_j = Acol_j' * Tcol_j (k_j x k_j, inner tri(n_j)) on the FP64 tensor cores.
-// Tile list entries (block, tile row, tile col) of 32 x 32 output tiles; a 32-row K chunk of both
-// operands is staged in shared memory, and each of the 8 warps owns two 8 x 8 output subtiles
-// accumulated by mma.sync m8n8k4 (lane (r, q): A fragment A'(row r, k q), B fragment T(k q,
-// column r); results C(r, 2q) and C(r, 2q + 1)).
+// Tile list entries (block, tile row, tile col) of 32 x 32 output tiles; the inner rows of a tile are dealt
+// in 32-row chunks to the CTAs of one cluster (its size is the launch's), whose sums meet through
+// distributed shared memory in rank order.  A four-stage ring of chunks (cp.async, 8 bytes: a column
+// starts anywhere) feeds the 8 warps, each with two 8 x 8 output subtiles accumulated by mma.sync m8n8k4
+// (lane (r, q): A fragment A'(row r, k q), B fragment T(k q, column r); results C(r, 2q) and C(r, 2q + 1)).
+// Chunk columns are 36 doubles apart (4 mod 16: the fragment reads of a half-warp hit distinct banks).
+// Bound by the latency of the chunks while the tiles are few: 49 tiles of 1275 inner rows (order 50, 200
+// constraints) took 117 us with one CTA a tile and plain loads, 27.5 with the ring, 17 with it in clusters.
 #define SCHUR_TILE 32
 #define SCHUR_KC 32
+#define SCHUR_LD 36
+#define SCHUR_STAGES 4
+static_assert(kSchurSmem == SCHUR_STAGES * 2 * SCHUR_TILE * SCHUR_LD * sizeof(double), "ring");
+
+namespace {
+
+__device__ __forceinline__ void schur_copy8(double* dst, const double* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 8 : 0)
+               : "memory");
+}
+
+}  // namespace
+
 extern "C" __global__ void __launch_bounds__(SDPXG_THREADS)
 k_schur_block_gemm(const BlockDesc* __restrict__ blocks, const int* __restrict__ tiles,
                    const int* __restrict__ kcount, const long* __restrict__ acol_off,
                    const long* __restrict__ s_off, const double* __restrict__ Acol,
                    const double* __restrict__ Tcol, double* __restrict__ S) {
-  __shared__ double As[SCHUR_KC][SCHUR_TILE + 1];
-  __shared__ double Ts[SCHUR_KC][SCHUR_TILE + 1];
-  const int j = tiles[3 * blockIdx.x], ti = tiles[3 * blockIdx.x + 1],
-            tj = tiles[3 * blockIdx.x + 2];
+  namespace cg = cooperative_groups;
+  extern __shared__ double smem[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int split = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int* tile = tiles + 3 * (blockIdx.x / split);
+  const int j = tile[0], ti = tile[1], tj = tile[2];
   const int n = blocks[j].n;
   const int tn = n * (n + 1) / 2;
   const int k = kcount[j];
   const double* A = Acol + acol_off[j];
   const double* T = Tcol + acol_off[j];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = lane >> 2, q = lane & 3;
-  // subtiles w and w + 8 of the 4 x 4 grid of 8 x 8 subtiles
-  const int I0 = w >> 2, J0 = w & 3, I1 = (w + 8) >> 2, J1 = (w + 8) & 3;
-  double c00 = 0, c01 = 0, c10 = 0, c11 = 0;
-  for (int r0 = 0; r0 < tn; r0 += SCHUR_KC) {
-    for (int e = threadIdx.x; e < SCHUR_KC * SCHUR_TILE; e += blockDim.x) {
-      int rr = e % SCHUR_KC, cc = e / SCHUR_KC;
-      int rw = r0 + rr;
-      int ca = ti * SCHUR_TILE + cc, cb = tj * SCHUR_TILE + cc;
-      As[rr][cc] = (rw < tn && ca < k) ? A[(long)ca * tn + rw] : 0.0;
-      Ts[rr][cc] = (rw < tn && cb < k) ? T[(long)cb * tn + rw] : 0.0;
+  const int chunks = (tn + SCHUR_KC - 1) / SCHUR_KC, c_end = (int)((long)chunks * (rank + 1) / split);
+  int next = (int)((long)chunks * rank / split);
+  auto load = [&](int c, int stage) {  // a lane: one row; a warp: columns w, w + 8, ...
+    if (c < c_end) {
+      double* As = smem + stage * 2 * SCHUR_TILE * SCHUR_LD;
+      double* Ts = As + SCHUR_TILE * SCHUR_LD;
+      const int row = c * SCHUR_KC + lane;
+#pragma unroll
+      for (int u = 0; u < SCHUR_TILE / 8; ++u) {
+        const int cc = w + 8 * u, ca = ti * SCHUR_TILE + cc, cb = tj * SCHUR_TILE + cc;
+        const bool ia = row < tn && ca < k, ib = row < tn && cb < k;
+        schur_copy8(As + cc * SCHUR_LD + lane, ia ? A + (long)ca * tn + row : A, ia);
+        schur_copy8(Ts + cc * SCHUR_LD + lane, ib ? T + (long)cb * tn + row : T, ib);
+      }
     }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  // subtiles w and w + 8 of the 4 x 4 grid of 8 x 8 subtiles
+  const int I0 = w >> 2, J = w & 3, I1 = I0 + 2;
+  double c[2][2] = {};
+  const int first = next;
+  for (int s = 0; s < SCHUR_STAGES - 1; ++s) load(next + s, s);
+  for (; next < c_end; ++next) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(SCHUR_STAGES - 2) : "memory");
     __syncthreads();
+    load(next + SCHUR_STAGES - 1, (next - first + SCHUR_STAGES - 1) % SCHUR_STAGES);
+    const double* As = smem + (next - first) % SCHUR_STAGES * 2 * SCHUR_TILE * SCHUR_LD;
+    const double* Ts = As + SCHUR_TILE * SCHUR_LD;
 #pragma unroll
     for (int ks = 0; ks < SCHUR_KC / 4; ++ks) {
       const int kk = 4 * ks + q;
-      dmma_m8n8k4(c00, c01, As[kk][8 * I0 + r], Ts[kk][8 * J0 + r]);
-      dmma_m8n8k4(c10, c11, As[kk][8 * I1 + r], Ts[kk][8 * J1 + r]);
+      const double b = Ts[(8 * J + r) * SCHUR_LD + kk];
+      dmma_m8n8k4(c[0][0], c[0][1], As[(8 * I0 + r) * SCHUR_LD + kk], b);
+      dmma_m8n8k4(c[1][0], c[1][1], As[(8 * I1 + r) * SCHUR_LD + kk], b);
     }
-    __syncthreads();
   }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  double* sum = smem;  // 32 x 32, columns SCHUR_LD apart
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    double* o = sum + 8 * (I0 + 2 * h) + r + (8 * J + 2 * q) * SCHUR_LD;
+    o[0] = c[h][0];
+    o[SCHUR_LD] = c[h][1];
+  }
+  cluster.sync();
   double* out = S + s_off[j];
-  const int a0 = ti * SCHUR_TILE + 8 * I0 + r, b0 = tj * SCHUR_TILE + 8 * J0 + 2 * q;
-  const int a1 = ti * SCHUR_TILE + 8 * I1 + r, b1 = tj * SCHUR_TILE + 8 * J1 + 2 * q;
-  if (a0 < k && b0 < k) out[a0 + (long)b0 * k] = c00;
-  if (a0 < k && b0 + 1 < k) out[a0 + (long)(b0 + 1) * k] = c01;
-  if (a1 < k && b1 < k) out[a1 + (long)b1 * k] = c10;
-  if (a1 < k && b1 + 1 < k) out[a1 + (long)(b1 + 1) * k] = c11;
+  for (int e = threadIdx.x + rank * blockDim.x; e < SCHUR_TILE * SCHUR_TILE; e += split * blockDim.x) {
+    const int i = e & 31, cc = e >> 5, a0 = ti * SCHUR_TILE + i, b0 = tj * SCHUR_TILE + cc;
+    if (a0 >= k || b0 >= k) continue;
+    double v = 0.0;
+    for (int p = 0; p < split; ++p) v += cluster.map_shared_rank(sum, p)[i + cc * SCHUR_LD];
+    out[a0 + (long)b0 * k] = v;
+  }
+  cluster.sync();  // nobody leaves while its sums are read
 }
 
 // H (m x m, full, column-major) = sum over shared blocks of S_j[la, lb], in cone order.
-// One thread per (a, b) with a <= b; both triangles written (symmetrised by construction).
-extern "C" __global__ void k_schur_gather(int m, const int* __restrict__ c2b_ptr,
-                                          const int* __restrict__ c2b_blk,
-                                          const int* __restrict__ c2b_loc,
-                                          const int* __restrict__ kcount,
-                                          const long* __restrict__ s_off,
-                                          const double* __restrict__ S, double* __restrict__ H) {
-  long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  long total = (long)m * m;
-  if (idx >= total) return;
-  int a = (int)(idx % m), b = (int)(idx / m);
-  if (a > b) return;
-  int pa = c2b_ptr[a], ea = c2b_ptr[a + 1], pb = c2b_ptr[b], eb = c2b_ptr[b + 1];
-  double acc = 0.0;
-  while (pa < ea && pb < eb) {
-    int ja = c2b_blk[pa], jb = c2b_blk[pb];
-    if (ja < jb) {
-      ++pa;
-    } else if (jb < ja) {
-      ++pb;
-    } else {
-      const int k = kcount[ja];
-      const double* Sj = S + s_off[ja];
-      int la = c2b_loc[pa], lb = c2b_loc[pb];
-      // symmetric in exact arithmetic: average the two computed halves
-      acc += 0.5 * (Sj[la + (long)lb * k] + Sj[lb + (long)la * k]);
-      ++pa;
-      ++pb;
+// One CTA per 32 x 32 tile on or above the diagonal (grid.x numbers them by columns); both triangles are
+// written (symmetrised by construction), the mirrored tile through shared memory so that its stores are
+// whole lines too (m = 4000: 143 us, 164 with one thread an entry and stores a column apart).
+extern "C" __global__ void __launch_bounds__(1024)
+k_schur_gather(int m, const int* __restrict__ c2b_ptr, const int* __restrict__ c2b_blk,
+               const int* __restrict__ c2b_loc, const int* __restrict__ kcount,
+               const long* __restrict__ s_off, const double* __restrict__ S, double* __restrict__ H) {
+  __shared__ double mirror[32][33];
+  int tj = (int)((sqrtf(8.0f * blockIdx.x + 1.0f) - 1.0f) * 0.5f);
+  while ((long)tj * (tj + 1) / 2 > blockIdx.x) --tj;
+  while ((long)(tj + 1) * (tj + 2) / 2 <= blockIdx.x) ++tj;
+  const int ti = (int)(blockIdx.x - (long)tj * (tj + 1) / 2);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int a = 32 * ti + lane;
+  {
+    const int b = 32 * tj + w;
+    if (a <= b && b < m) {
+      int pa = c2b_ptr[a], pb = c2b_ptr[b];
+      const int ea = c2b_ptr[a + 1], eb = c2b_ptr[b + 1];
+      double acc = 0.0;
+      while (pa < ea && pb < eb) {
+        int ja = c2b_blk[pa], jb = c2b_blk[pb];
+        if (ja < jb) {
+          ++pa;
+        } else if (jb < ja) {
+          ++pb;
+        } else {
+          const int k = kcount[ja];
+          const double* Sj = S + s_off[ja];
+          int la = c2b_loc[pa], lb = c2b_loc[pb];
+          // symmetric in exact arithmetic: average the two computed halves
+          acc += 0.5 * (Sj[la + (long)lb * k] + Sj[lb + (long)la * k]);
+          ++pa;
+          ++pb;
+        }
+      }
+      H[a + (long)b * m] = acc;
+      mirror[lane][w] = acc;
     }
   }
-  H[a + (long)b * m] = acc;
-  H[b + (long)a * m] = acc;
+  __syncthreads();
+  const int b = 32 * tj + lane;
+  const int col = 32 * ti + w;
+  if (col < b && b < m) H[b + (long)col * m] = mirror[w][lane];
 }
 
 // H += sym(P) for P given as an upper-triangular CSC (n x n).
