@@ -387,104 +387,79 @@ k_trinv_level(const double* __restrict__ F, long ldf, double* __restrict__ Uinv,
     }
 }
 
-// out[c] = sum over the stored triangle of column c of A (n x n): rows 0..c (upper) or c..n-1
-// (lower), times v.  One warp per column: coalesced column reads.
-extern "C" __global__ void k_tri_colgemv(const double* __restrict__ A, int n, int lower,
-                                         const double* __restrict__ v, double* __restrict__ out) {
-  // one warp per column, eight independent partial sums per lane so that each lane keeps eight
-  // loads in flight (the matrix streams from HBM/L2 once per solve)
-  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (c >= n) return;
-  const int r0 = lower ? c : 0, r1 = lower ? n : c + 1;
-  const double* col = A + (long)c * n;
-  double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int r = r0 + lane;
-  for (; r + 7 * 32 < r1; r += 8 * 32) {
-#pragma unroll
-    for (int u = 0; u < 8; ++u) acc[u] = fma(__ldg(col + r + 32 * u), __ldg(v + r + 32 * u), acc[u]);
-  }
-  for (; r < r1; r += 32) acc[0] = fma(col[r], v[r], acc[0]);
-  double t = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
-  t = warp_sum(t);
-  if (lane == 0) out[c] = t;
-}
-
 // out[c] = rbase[c] + alpha * (column c of A) . v for a dense column-major n x n A restricted to
-// a triangle (tri 0: all rows, 1: rows <= c, 2: rows >= c; other entries are never read).  One
-// warp per (column, 256-row segment), eight loads in flight per lane, so every warp finishes in
-// one memory round trip whatever the column length; the segment sums go to partial[seg][c] and
-// the warp that finishes a column last (a ticket per column, reset for the next use) adds them
-// in increasing segment order -- the result does not depend on the order the warps ran in.
-#define CD_SEG 256
-__device__ __forceinline__ void cd_seg_range(int tri, int c, int n, int& s0, int& s1) {
-  const int nseg = (n + CD_SEG - 1) / CD_SEG;
-  s0 = 0;
-  s1 = nseg;
-  if (tri == 1) s1 = c / CD_SEG + 1;  // rows 0..c
-  if (tri == 2) s0 = c / CD_SEG;      // rows c..n-1
+// a triangle (tri 0: all rows, 1: rows <= c, 2: rows >= c; other entries are never read).  W warps of one
+// CTA share a pair of adjacent columns (they read v once for both), 16 matrix loads in flight a lane;
+// their sums meet in shared memory in warp order.  The longest columns of a triangle come first.
+// Bound by L2 (the matrices of a few thousand rows stay there) and, below that, by one memory round trip
+// and the launch.  W: as many warps as leave a lane at most 16 rows (one round of loads), and no more
+// than 4.  Two triangles and the full matrix in three launches, W = 1 / 2 / 4 / 8: n = 1000 12.5 / 12.6 /
+// 12.5 / 12.6 us, 2000 19.7 / 18.4 / 18.5 / 19.1, 3000 43 / 35 / 35 / 41, 4000 61 / 56 / 54 / 55; segments of
+// 256 rows as work units, combined through global memory by a ticket per column, took 18.7, 32, 64 and 100.
+template <int W>
+__global__ void __launch_bounds__(256)
+k_coldot(const double* __restrict__ A, int n, int tri, const double* __restrict__ v,
+         const double* __restrict__ rbase, double alpha, double* __restrict__ out) {
+  __shared__ double part[8][2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wi = warp % W;
+  const int pairs = (n + 1) / 2, idx = blockIdx.x * (8 / W) + warp / W;
+  const int c0 = 2 * (tri == 1 ? pairs - 1 - idx : idx), c1 = c0 + 1;
+  const bool in = idx < pairs;
+  double s0 = 0.0, s1 = 0.0;
+  if (in) {
+    const int r0 = tri == 2 ? c0 : 0, r1 = tri == 1 ? min(c1 + 1, n) : n;
+    const int e0 = tri == 1 ? c0 + 1 : n, b1 = tri == 2 ? c1 : 0, e1 = c1 < n ? r1 : 0;  // rows of each column
+    const double* col = A + (long)c0 * n;
+    double acc[4][2] = {};
+    for (int r = r0 + 32 * wi + lane; r < r1; r += 8 * 32 * W) {
+      double x[8], y0[8], y1[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int k = r + 32 * W * u;
+        x[u] = k < r1 ? __ldg(v + k) : 0.0;
+        y0[u] = k < e0 && k < r1 ? __ldg(col + k) : 0.0;
+        y1[u] = k >= b1 && k < e1 ? __ldg(col + n + k) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        acc[u & 3][0] = fma(y0[u], x[u], acc[u & 3][0]);
+        acc[u & 3][1] = fma(y1[u], x[u], acc[u & 3][1]);
+      }
+    }
+    s0 = warp_sum((acc[0][0] + acc[1][0]) + (acc[2][0] + acc[3][0]));
+    s1 = warp_sum((acc[0][1] + acc[1][1]) + (acc[2][1] + acc[3][1]));
+  }
+  if (W > 1) {
+    if (lane == 0) {
+      part[warp][0] = s0;
+      part[warp][1] = s1;
+    }
+    __syncthreads();
+    if (wi == 0) {
+#pragma unroll
+      for (int k = 1; k < W; ++k) {
+        s0 += part[warp + k][0];
+        s1 += part[warp + k][1];
+      }
+    }
+  }
+  if (!in || wi != 0 || lane > 1 || c0 + lane >= n) return;
+  const double t = lane ? s1 : s0;
+  out[c0 + lane] = (rbase ? rbase[c0 + lane] : 0.0) + alpha * t;
 }
 
-extern "C" __global__ void __launch_bounds__(256)
-k_coldot_seg(const double* __restrict__ A, int n, int tri, const double* __restrict__ v,
-             const double* __restrict__ rbase, double alpha, double* __restrict__ out,
-             double* __restrict__ partial, unsigned* __restrict__ counters) {
-  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31, sg = blockIdx.y;
-  if (c >= n) return;
-  int s0, s1;
-  cd_seg_range(tri, c, n, s0, s1);
-  if (sg < s0 || sg >= s1) return;
-  int r0 = sg * CD_SEG, r1 = min(n, r0 + CD_SEG);
-  if (tri == 1) r1 = min(r1, c + 1);
-  if (tri == 2) r0 = max(r0, c);
-  const double* col = A + (long)c * n;
-  double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const int r = r0 + lane + 32 * u;
-    if (r < r1) acc[u] = __ldg(col + r) * __ldg(v + r);
-  }
-  double t = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
-  t = warp_sum(t);
-  if (s1 - s0 == 1) {  // one segment: nothing to combine
-    if (lane == 0) out[c] = (rbase ? rbase[c] : 0.0) + alpha * t;
-    return;
-  }
-  unsigned ticket = 0;
-  if (lane == 0) {
-    partial[(long)sg * n + c] = t;
-    __threadfence();
-    ticket = atomicAdd(counters + c, 1u);
-  }
-  ticket = __shfl_sync(0xffffffffu, ticket, 0);
-  if (ticket != (unsigned)(s1 - s0 - 1)) return;
-  if (lane == 0) {
-    __threadfence();
-    double sum = 0.0;
-    for (int k = s0; k < s1; ++k) sum += __ldcg(partial + (long)k * n + c);
-    out[c] = (rbase ? rbase[c] : 0.0) + alpha * sum;
-    counters[c] = 0u;
-  }
+namespace sdpxg {
+
+void launch_coldot(const double* A, int n, int tri, const double* v, const double* rbase, double alpha, double* out,
+                   cudaStream_t st) {
+  if (n <= 0) return;
+  const int pairs = (n + 1) / 2;
+  auto go = [&](auto kernel, int w) {
+    kernel<<<(pairs * w + 7) / 8, 256, 0, st>>>(A, n, tri, v, rbase, alpha, out);
+  };
+  if (n <= 512) go(k_coldot<1>, 1);
+  else if (n <= 1024) go(k_coldot<2>, 2);
+  else go(k_coldot<4>, 4);
 }
 
-// e = r - H x for the symmetric H (both triangles stored): e_i = r_i - (column i of H) . x, one
-// warp per column, coalesced, eight partial sums per lane (one launch, no partial buffer).
-extern "C" __global__ void k_symv_cols(const double* __restrict__ H, int m,
-                                       const double* __restrict__ x, const double* __restrict__ r,
-                                       double* __restrict__ e) {
-  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (c >= m) return;
-  const double* col = H + (long)c * m;
-  double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int k = lane;
-  for (; k + 7 * 32 < m; k += 8 * 32) {
-#pragma unroll
-    for (int u = 0; u < 8; ++u) acc[u] = fma(__ldg(col + k + 32 * u), __ldg(x + k + 32 * u), acc[u]);
-  }
-  for (; k < m; k += 32) acc[0] = fma(col[k], x[k], acc[0]);
-  double t = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
-  t = warp_sum(t);
-  if (lane == 0) e[c] = r[c] - t;
-}
+}  // namespace sdpxg

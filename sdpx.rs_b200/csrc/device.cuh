@@ -191,6 +191,9 @@ struct PinnedBuf {
 };
 
 // Kernel declarations (defined in the *_kernels.cu translation units of this library).
+// k_coldot (dense_kernels.cu): out = rbase + alpha * (column dots of A, or of a triangle of it, with v).
+void launch_coldot(const double* A, int n, int tri, const double* v, const double* rbase, double alpha, double* out,
+                   cudaStream_t st);
 extern "C" {
 __global__ void k_nt_factor(const BlockDesc*, const double*, const double*, double*, double*,
                             uint32_t*);
@@ -238,13 +241,9 @@ __global__ void k_chol_dataflow(double*, long, int, int, const unsigned*, int, i
 __global__ void k_syrk_update(double*, long, int, int);
 __global__ void k_trtri_diag(int, const double*, double*, double*);
 __global__ void k_trinv_level(const double*, long, double*, double*, double*, int, int, int);
-__global__ void k_tri_colgemv(const double*, int, int, const double*, double*);
 __global__ void k_shifted_copy(const double*, double*, long, int, double, double*);
 __global__ void k_strided_diag(const double*, long, int, double, double*);
 __global__ void k_transpose_block(const double*, long, int, int, double*, long);
-__global__ void k_symv_cols(const double*, int, const double*, const double*, double*);
-__global__ void k_coldot_seg(const double*, int, int, const double*, const double*, double, double*,
-                             double*, unsigned*);
 __global__ void k_lincomb(long, double, const double*, double, const double*, double,
                           const double*, double*);
 __global__ void k_reduce_partial(int, long, const double*, const double*, double*);

@@ -129,13 +129,12 @@ extern "C" int32_t sdpxg_solve_noalloc(sdpxg_ctx* ctx, const double* d_rhs, doub
     double* slots = red + 3 * SDPXG_NOALLOC_RED_BLOCKS;
     cudaStream_t st = E.st;
     const Settings cfg;  // binary64 refinement defaults, as in sdpxg_solve_many
-    const int grid = (n + 7) / 8;
     auto trisolve = [&](const double* r, double* x) {
-      ++g_launches, k_tri_colgemv<<<grid, 256, 0, st>>>(E.uinv(), n, 0, r, tri);
-      ++g_launches, k_tri_colgemv<<<grid, 256, 0, st>>>(E.uinvT(), n, 1, tri, x);
+      ++g_launches, launch_coldot(E.uinv(), n, 1, r, nullptr, 1.0, tri, st);
+      ++g_launches, launch_coldot(E.uinvT(), n, 2, tri, nullptr, 1.0, x, st);
     };
     auto residual = [&](const double* r, const double* x, double* e) {
-      ++g_launches, k_symv_cols<<<(n + 7) / 8, 256, 0, st>>>(E.Hsave(), n, x, r, e);
+      ++g_launches, launch_coldot(E.Hsave(), n, 0, x, r, -1.0, e, st);
     };
     auto fetch = [&](int count, double* host) {
       check(cudaMemcpyAsync(host, slots, count * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
