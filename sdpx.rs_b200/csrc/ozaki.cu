@@ -21,38 +21,47 @@ constexpr int kModuli[kOzMod] = {oz_mod(0),  oz_mod(1),  oz_mod(2),  oz_mod(3), 
                                  oz_mod(6),  oz_mod(7),  oz_mod(8),  oz_mod(9),  oz_mod(10), oz_mod(11),
                                  oz_mod(12), oz_mod(13), oz_mod(14), oz_mod(15)};
 
-// Garner tables, passed by value: inv[t] = (p_0 ... p_{t-1})^-1 mod p_t, pre[s][t] =
-// (p_0 ... p_{s-1}) mod p_t.
+constexpr int kOzTriples = (kOzMod + 2) / 3;  // moduli 3g, 3g + 1, 3g + 2
+// Tables of the residue and reconstruction kernels, in constant memory (every index is a literal after
+// unrolling).  With P the product of the moduli and W_t = P / p_t:
 struct OzTables {
-  int p[kOzMod];
-  int inv[kOzMod];
-  short pre[kOzMod][kOzMod];
+  uint32_t wlo[kOzMod], whi[kOzMod];  // 256^k mod p for the bytes k of a 64-bit integer
+  uint32_t init[kOzMod];              // floor(p / 2) - 2^62 mod p
+  uint32_t magic[kOzMod];             // ceil(2^32 / p): floor(x / p) = x magic >> 32 for x < 2^24
+  uint32_t inv[kOzMod];               // W_t^-1 mod p
+  uint32_t div[kOzMod];               // floor(2^22 / p)
+  uint32_t co[kOzMod];                // product of the other moduli of the triple of p
+  uint32_t W[kOzTriples][4], P[4];    // P / (a triple's product) and P in 32-bit limbs
 };
-
-const OzTables& tables() {
-  static OzTables T;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    for (int t = 0; t < kOzMod; ++t) {
-      const int p = kModuli[t];
-      T.p[t] = p;
-      long prod = 1;
-      for (int s = 0; s < kOzMod; ++s) {
-        T.pre[s][t] = (short)(s <= t ? prod : 0);
-        if (s < t) prod = prod * (kModuli[s] % p) % p;
-      }
-      // prod = (p_0 ... p_{t-1}) mod p; its inverse by search (p <= 256)
-      int inv = 1;
-      for (int x = 1; x < p; ++x)
-        if ((long)x * prod % p == 1) {
-          inv = x;
-          break;
-        }
-      T.inv[t] = t == 0 ? 1 : inv;
+constexpr OzTables oz_tables() {
+  OzTables T{};
+  unsigned __int128 P = 1;
+  for (int t = 0; t < kOzMod; ++t) P *= (unsigned)oz_mod(t);
+  for (int l = 0; l < 4; ++l) T.P[l] = (uint32_t)(P >> (32 * l));
+  for (int t = 0; t < kOzMod; ++t) {
+    const uint32_t p = (uint32_t)oz_mod(t);
+    uint32_t w = 1;
+    for (int k = 0; k < 8; ++k) {
+      (k < 4 ? T.wlo[t] : T.whi[t]) |= w << (8 * (k & 3));
+      w = w * 256u % p;
     }
-  });
+    T.init[t] = p / 2 + (p - (uint32_t)((1ull << 62) % p)) % p;
+    T.magic[t] = (uint32_t)(((1ull << 32) + p - 1) / p);
+    T.div[t] = (1u << 22) / p;
+    uint32_t triple = p;
+    for (int u = t / 3 * 3; u < kOzMod && u < t / 3 * 3 + 3; ++u)
+      if (u != t) triple *= (uint32_t)oz_mod(u);
+    T.co[t] = triple / p;
+    for (int l = 0; l < 4; ++l) T.W[t / 3][l] = (uint32_t)(P / triple >> (32 * l));
+    const unsigned __int128 W = P / p;
+    const uint32_t wm = (uint32_t)(W % p);
+    for (uint32_t x = 1; x < p; ++x)  // the inverse by search (p <= 256)
+      if (wm * x % p == 1) T.inv[t] = x;
+  }
   return T;
 }
+__constant__ OzTables kOz = oz_tables();
+constexpr float kOzLead = 1.0f / (float)oz_tables().P[3];  // 2^96 / P to 2^-24 and the limb's 2^-30
 
 double log2_product() {
   double s = 0;
@@ -112,45 +121,69 @@ __global__ void k_oz_amax(const double* __restrict__ X, int rows, int K, long sr
 // Shift of a line with maximum `bits`: b - 1 - floor(log2 max) puts the line below 2^b; 0 for a
 // zero or non-finite line.
 __device__ __forceinline__ int oz_shift(unsigned long long bits, int b) {
-  const double m = __longlong_as_double((long long)bits);
-  return (m > 0.0 && isfinite(m)) ? b - 1 - ilogb(m) : 0;
+  const int e = (int)(bits >> 52);
+  if (e == 0) return bits ? b - 1 - ilogb(__longlong_as_double((long long)bits)) : 0;
+  return e == 2047 ? 0 : b - 1 - (e - 1023);
 }
 
-// Symmetric residue in [-(p-1)/2, p/2] of the integer (neg ? -1 : 1) (hi 2^32 + lo), hi < 2^30:
-// 32-bit reductions by the literal modulus p (the caller's loop is unrolled).
-__device__ __forceinline__ int oz_sym_residue(uint32_t hi, uint32_t lo, bool neg, const int p) {
-  const uint32_t c = (uint32_t)((1ull << 32) % (unsigned)p);
-  int r = (int)(((hi % (unsigned)p) * c + lo % (unsigned)p) % (unsigned)p);
-  if (neg && r) r = p - r;
-  if (r > p / 2) r -= p;
-  return r;
-}
+__device__ __forceinline__ double oz_pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }  // |e| <= 1022
 
 // Residues of the quantised lines as signed-byte planes: out[(l * Rpad + x) * Kld + k] =
 // rint(X(x, k) 2^shift[x]) mod p_l (symmetric), zeros in the padding.  One CTA per tile of
 // 32 lines x 128 k, staged in shared memory so that both the reads (along whichever index is
 // contiguous) and the 16-byte plane writes are coalesced.
+// A thread has four consecutive k of a line, so that a modulus costs one 4-byte store for the four.  A
+// residue is a dot product of the integer's bytes with 256^k mod p (two dp4a; 2^62 added first makes it
+// non-negative) and one reduction by a multiply-high: 24 instructions for four residues, where a byte
+// at a time with three reductions each had 60.  Bound by instruction issue: 4.2e6 entries took 92 us
+// and take 33.
 constexpr int kResPitch = 144;  // bytes per staged line (128 + 16: 16-byte aligned rows)
 __global__ void __launch_bounds__(256) k_oz_residues(const double* __restrict__ X, int rows, int K, long sr, long sk,
                                                      const unsigned long long* __restrict__ amax, int b,
                                                      int8_t* __restrict__ out, int Rpad, int Kld) {
   extern __shared__ int8_t tile[];  // [kOzMod][32][kResPitch]
+  __shared__ double scale[32][2];   // 2^shift of a line as two factors: the exponent may exceed 1023
   const int r0 = blockIdx.y * 32, k0 = blockIdx.x * 128;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < 32) {
+    const int sh = r0 + lane < rows ? oz_shift(amax[r0 + lane], b) : 0, h = sh / 2;
+    scale[lane][0] = oz_pow2(h);
+    scale[lane][1] = oz_pow2(sh - h);
+  }
+  __syncthreads();
   const bool along_k = (sk == 1);
-  for (int e = threadIdx.x; e < 32 * 128; e += 256) {
-    const int rr = along_k ? e / 128 : e % 32;
-    const int kk = along_k ? e % 128 : e / 32;
-    const int x = r0 + rr, k = k0 + kk;
-    long long q = 0;
-    if (x < rows && k < K) {
-      const double v = X[(long)x * sr + (long)k * sk];
-      if (isfinite(v)) q = llrint(ldexp(v, oz_shift(amax[x], b)));
-    }
-    const unsigned long long u = (unsigned long long)(q < 0 ? -q : q);
-    const uint32_t hi = (uint32_t)(u >> 32), lo = (uint32_t)u;
+#pragma unroll 1
+  for (int pass = 0; pass < 4; ++pass) {
+    // a warp: one line of 128 k, or 8 lines x 16 k where the lines are contiguous
+    const int task = pass * 8 + warp;
+    const int rr = along_k ? task : 8 * (task & 3) + (lane & 7);
+    const int kk = along_k ? 4 * lane : 16 * (task >> 2) + 4 * (lane >> 3);
+    const int x = r0 + rr;
+    const double s0 = scale[rr][0], s1 = scale[rr][1];
+    double v[4];
 #pragma unroll
-    for (int l = 0; l < kOzMod; ++l)
-      tile[(l * 32 + rr) * kResPitch + kk] = (int8_t)oz_sym_residue(hi, lo, q < 0, oz_mod(l));
+    for (int u = 0; u < 4; ++u) v[u] = x < rows && k0 + kk + u < K ? X[(long)x * sr + (long)(k0 + kk + u) * sk] : 0.0;
+    uint32_t lo[4], hi[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long q = isfinite(v[u]) ? __double2ll_rn(v[u] * s0 * s1) : 0;
+      const unsigned long long w = (unsigned long long)q + (1ull << 62);
+      lo[u] = (uint32_t)w;
+      hi[u] = (uint32_t)(w >> 32);
+    }
+#pragma unroll
+    for (int l = 0; l < kOzMod; ++l) {
+      uint32_t r[4];  // residue + floor(p / 2), non-negative
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t y = __dp4a(hi[u], kOz.whi[l], __dp4a(lo[u], kOz.wlo[l], kOz.init[l]));
+        r[u] = y - __umulhi(y, kOz.magic[l]) * (uint32_t)oz_mod(l);
+      }
+      const uint32_t w = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+      const uint32_t h = (uint32_t)(oz_mod(l) / 2) * 0x01010101u, top = 0x80808080u;
+      *reinterpret_cast<uint32_t*>(tile + (l * 32 + rr) * kResPitch + kk) =
+          ((w | top) - (h & ~top)) ^ ((w ^ ~h) & top);  // bytewise w - h
+    }
   }
   __syncthreads();
   const int rr = threadIdx.x >> 3, c = threadIdx.x & 7;
@@ -161,48 +194,85 @@ __global__ void __launch_bounds__(256) k_oz_residues(const double* __restrict__ 
   }
 }
 
-// C(i, j) = alpha * 2^-(sL_i + sR_j) * X_ij + beta * C(i, j), X_ij the integer product rebuilt
-// from its residues by Garner's algorithm with symmetric digits v_t in [-p_t/2, p_t/2]
-// (X = v_0 + p_0 (v_1 + p_1 (v_2 + ...)), exact for |X| < P/2) and evaluated by Horner's rule
-// in double-double arithmetic (error-free FMA product and two-sum per step: about 2^-100
-// relative), so the FP64 value of X is its correct rounding except within 2^-100 of a tie.
-__global__ void k_oz_garner(const int8_t* __restrict__ PC, long plane, int M, int N,
-                            const unsigned long long* __restrict__ aL, const unsigned long long* __restrict__ aR,
-                            int b, OzTables T, double alpha, double beta, double* __restrict__ C, long ldc,
-                            int upper_only) {
-  const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long)M * N) return;
-  const int i = (int)(idx % M), j = (int)(idx / M);
-  if (upper_only && i > j) return;
-  int v[kOzMod];
+// C(i, j) = alpha * 2^-(sL_i + sR_j) * X_ij + beta * C(i, j), X_ij the integer product rebuilt from its
+// residues: X = sum_t y_t W_t - k P with y_t = x_t W_t^-1 mod p_t (in [0, 2 p_t)), three moduli at a time
+// (y_0 p_1 p_2 + y_1 p_0 p_2 + y_2 p_0 p_1) P / (p_0 p_1 p_2), exact in 32-bit limbs, and k = round(sum / P)
+// from the leading bits (|X| <= P / 4 leaves the quotient a quarter from a tie); rounded to FP64 once.  A
+// thread has four consecutive entries of the planes (one 4-byte load a modulus).
+// Bound by instruction issue; mixed-radix digits (a triangle of 120 products and three reductions a
+// digit) and a double-double Horner evaluation took 167 us for 4.2e6 entries, one modulus at a time in
+// limbs 84, this 62.
+__global__ void __launch_bounds__(256) k_oz_crt(const int8_t* __restrict__ PC, long plane, int M, int N,
+                                                const unsigned long long* __restrict__ aL,
+                                                const unsigned long long* __restrict__ aR, int b, double alpha,
+                                                double beta, double* __restrict__ C, long ldc, int upper_only) {
+  const long total = (long)M * N, idx0 = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x);
+  if (idx0 >= total) return;
+  int j = (int)(idx0 / M), i = (int)(idx0 - (long)j * M);
+  if (upper_only && i > j && i + 3 < M) return;  // four entries of a column below the diagonal
+  uint32_t word[kOzMod];
+  const bool whole = idx0 + 4 <= total && (plane & 3) == 0;
 #pragma unroll
   for (int t = 0; t < kOzMod; ++t) {
-    const int p = oz_mod(t);
-    int r = (int)PC[t * plane + idx] % p;
-    if (r < 0) r += p;
-    int u = 0;
-#pragma unroll
-    for (int s = 0; s < t; ++s) u += v[s] * (int)T.pre[s][t];
-    int d = (r - u) % p;
-    if (d < 0) d += p;
-    d = d * T.inv[t] % p;
-    if (d > p / 2) d -= p;
-    v[t] = d;
+    if (whole) {
+      word[t] = __ldg(reinterpret_cast<const uint32_t*>(PC + t * plane + idx0));
+    } else {
+      word[t] = 0;
+      for (int u = 0; u < 4; ++u)
+        if (idx0 + u < total) word[t] |= (uint32_t)(uint8_t)PC[t * plane + idx0 + u] << (8 * u);
+    }
   }
-  double h = (double)v[kOzMod - 1], lo = 0.0;
+#pragma unroll 1
+  for (int u = 0; u < 4; ++u, ++i) {
+    if (i == M) {
+      i = 0;
+      ++j;
+    }
+    if (j >= N) return;
+    unsigned long long s0 = 0, s1 = 0, s2 = 0, s3 = 0;
 #pragma unroll
-  for (int t = kOzMod - 2; t >= 0; --t) {
-    const double p = (double)oz_mod(t), vt = (double)v[t];
-    const double ph = h * p, pe = fma(h, p, -ph);  // h p = ph + pe exactly
-    const double s = ph + vt, bb = s - ph;
-    const double se = (ph - (s - bb)) + (vt - bb);  // ph + vt = s + se exactly
-    const double tt = se + pe + lo * p;
-    h = s + tt;
-    lo = tt - (h - s);
+    for (int g = 0; g < kOzTriples; ++g) {
+      uint32_t z = 0;  // below 2^27
+#pragma unroll
+      for (int t = 3 * g; t < kOzMod && t < 3 * g + 3; ++t) {
+        const int p = oz_mod(t), r = (int)(int8_t)(uint8_t)word[t];
+        word[t] >>= 8;
+        const uint32_t x = (uint32_t)(r + p) * kOz.inv[t];             // r >= -128 > -p; below 2^17
+        z += (x - (x * kOz.div[t] >> 22) * (uint32_t)p) * kOz.co[t];  // the quotient is at most one short
+      }
+      s0 += (unsigned long long)z * kOz.W[g][0];
+      s1 += (unsigned long long)z * kOz.W[g][1];
+      s2 += (unsigned long long)z * kOz.W[g][2];
+      s3 += (unsigned long long)z * kOz.W[g][3];
+    }
+    if (upper_only && i > j) continue;
+    const float lead = (float)(s3 + (s2 >> 32));  // sum / 2^96, below 2^36
+    const uint32_t k = (uint32_t)(lead * kOzLead + 0.5f);
+    // differences of less than 2^62 in each limb; arithmetic carries
+    const long long d0 = (long long)(s0 - (unsigned long long)k * kOz.P[0]);
+    const long long d1 = (long long)(s1 - (unsigned long long)k * kOz.P[1]) + (d0 >> 32);
+    const long long d2 = (long long)(s2 - (unsigned long long)k * kOz.P[2]) + (d1 >> 32);
+    const long long d3 = (long long)(s3 - (unsigned long long)k * kOz.P[3]) + (d2 >> 32);
+    unsigned long long hi = (unsigned long long)d3 << 32 | (uint32_t)d2, lo = (unsigned long long)(uint32_t)d1 << 32 | (uint32_t)d0;
+    const bool neg = d3 < 0;
+    if (neg) {
+      lo = ~lo + 1;
+      hi = ~hi + (lo == 0);
+    }
+    int e = 0;
+    if (hi) {  // the top 64 bits, the rest as a sticky bit: one rounding
+      const int z = __clzll((long long)hi);  // at least 1: |X| < 2^127
+      e = 64 - z;
+      const unsigned long long rest = lo << z;
+      lo = hi << z | lo >> (64 - z) | (rest != 0);
+    }
+    double x = __ull2double_rn(lo);
+    if (neg) x = -x;
+    e -= oz_shift(aL[i], b) + oz_shift(aR[j], b);
+    x = e >= -1022 && e <= 1023 ? x * oz_pow2(e) : ldexp(x, e);
+    double* c = C + i + (long)j * ldc;
+    *c = beta == 0.0 ? alpha * x : fma(alpha, x, beta * *c);
   }
-  double x = ldexp(h + lo, -(oz_shift(aL[i], b) + oz_shift(aR[j], b)));
-  double* c = C + i + (long)j * ldc;
-  *c = beta == 0.0 ? alpha * x : fma(alpha, x, beta * *c);
 }
 
 template <typename T>
@@ -238,7 +308,6 @@ void ozaki_gemm(OzakiWorkspace& ws, cudaStream_t st, int M, int N, int K, const 
   if (M <= 0 || N <= 0) return;
   if (K <= 0 || K > (1 << 16)) throw std::invalid_argument("split GEMM: K must be in 1..65536");
   if (!L || !R || !C) throw std::invalid_argument("split GEMM: null operand");
-  const OzTables& T = tables();
   if (!ws.init) {
     grow(ws.moduli, kOzMod);
     ws.moduli.upload(kModuli, kOzMod, st);
@@ -272,8 +341,8 @@ void ozaki_gemm(OzakiWorkspace& ws, cudaStream_t st, int M, int N, int K, const 
   ga.m = M; ga.n = N; ga.L = kOzMod; ga.moduli = ws.moduli; ga.upper_only = upper_only;
   ga.out = ws.PC.p; ga.plane = (long)M * N; ga.err = ws.err.p;
   launch_i8_gemm(1, ws.PL, ws.PR, ga, st);
-  ++g_launches, k_oz_garner<<<(unsigned)(((long)M * N + 255) / 256), 256, 0, st>>>(
-      ws.PC, (long)M * N, M, N, ws.amaxL, ws.amaxR, b, T, alpha, beta, C, ldc, upper_only);
+  ++g_launches, k_oz_crt<<<(unsigned)(((long)M * N + 1023) / 1024), 256, 0, st>>>(
+      ws.PC, (long)M * N, M, N, ws.amaxL, ws.amaxR, b, alpha, beta, C, ldc, upper_only);
   check(cudaGetLastError(), "split GEMM launch");
 }
 

@@ -8,9 +8,9 @@
 //      signed bytes, written K-major;
 //   3. per modulus one INT8 tensor-core GEMM (k_i8_mod_gemm, digits 1) gives
 //      (q_L q_R^T) mod p_l exactly;
-//   4. a symmetric-digit Garner CRT rebuilds the integer product (|.| < P/2 because
-//      b = floor((log2 P - 2 - ceil(log2 K)) / 2)) and Horner-evaluates it in FP64 (exact below
-//      2^53, a few ulps above), scaled back by 2^-(s_i + t_j).
+//   4. the CRT rebuilds the integer product exactly (|.| <= P/4 because
+//      b = floor((log2 P - 2 - ceil(log2 K)) / 2)), rounds it to FP64 and scales it back by
+//      2^-(s_i + t_j).
 // Accuracy: the quantisation error of an entry is at most 2^-b-1 of its row's largest entry,
 // b = 56 at K = 2048 and 55 at K = 4096 -- finer than binary64's own rounding of that entry.
 // FP64 stays for the scaling, the residues and the reconstruction; the products are INT8.
