@@ -81,25 +81,30 @@ __device__ __forceinline__ void give_up(volatile int* abort, int* err) {
   if (err) atomicOr(err, 1);
 }
 
-// Symmetric residue of v modulo p (|v| < 2^31, 2 <= p <= 256) in [-(p-1)/2, p/2]: the quotient
-// rounded from an FP64 product (v and v/p are exact to far below 1/2 in FP64, so it is the
-// nearest integer to v/p up to a tie), the remainder in 32-bit integers (exact modulo 2^32, and
-// the true remainder is small), then at most one correction each way.
-__device__ __forceinline__ int sym_mod_small(int v, int p, double pinv) {
-  const int q = __double2int_rn((double)v * pinv);
-  int r = v - q * p;
-  if (r > p / 2) r -= p;
-  if (r < -((p - 1) / 2)) r += p;
-  return r;
+// Residues modulo p (2 <= p < 2^15) of the accumulators, in 32-bit integers: the epilogue of a tile waits
+// for its MMAs and, with one CTA per SM, the tensor cores wait for the epilogue.
+struct Mod {
+  uint32_t p, m, c;  // m = floor((2^32 - 1) / p), c the largest multiple of p up to 2^31
+  __device__ explicit Mod(int modulus) : p((uint32_t)modulus), m(0xffffffffu / p), c(0x80000000u / p * p) {}
+  // x mod p or that plus p: the quotient x m >> 32 is at most one short.
+  __device__ __forceinline__ uint32_t lazy(uint32_t x) const { return x - __umulhi(x, m) * p; }
+  __device__ __forceinline__ uint32_t full(uint32_t x) const {  // in [0, p)
+    const uint32_t r = lazy(x);
+    return min(r, r - p);
+  }
+};
+// Symmetric residue in [-(p-1)/2, p/2] of an accumulator, |v| <= 2^31 - 2^15: 2^17 products of bytes up to
+// 127 (a power of two as p allows any v).  With two digits a call has 2^16 products of a low (128) and a
+// high digit (64), twice.
+__device__ __forceinline__ int sym_mod(int v, const Mod& M) {
+  const uint32_t h = (M.p - 1) / 2;
+  return (int)(M.full((uint32_t)v + M.c + h) - h);
 }
-// Residue of v modulo p in [0, p) for |v| < 2^50, p < 2^15: FP64 quotient as above (v exact in
-// FP64), remainder in 64-bit integers, one correction.
-__device__ __forceinline__ int mod_wide(long long v, int p, double pinv) {
-  const long long q = __double2ll_rn((double)v * pinv);
-  long long r = v - q * p;
-  if (r < 0) r += p;
-  if (r >= p) r -= p;
-  return (int)r;
+// (v0 + 2^8 v1 + 2^16 v2 + add) mod p in [0, p), add < 2^15; m8 = 2^8 mod p, m16 = 2^16 mod p.
+__device__ __forceinline__ uint32_t mod_digits(int v0, int v1, int v2, uint32_t add, uint32_t m8, uint32_t m16,
+                                               const Mod& M) {
+  const uint32_t r0 = M.lazy((uint32_t)v0 + M.c), r1 = M.lazy((uint32_t)v1 + M.c), r2 = M.full((uint32_t)v2 + M.c);
+  return M.full(r0 + r1 * m8 + r2 * m16 + add);  // below 2^16 + 2^24 + 2^30 + 2^15
 }
 
 template <int DIGITS, int VAR>
@@ -165,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<DIGITS, VAR>::CTAS)
       issued = it + 1;
     }
   } else if (warp == 5 && lane == 0) {  // ---- MMA issuer ----
-    constexpr uint32_t idesc = tc05::idesc_i8(kBM, BN);
+    constexpr uint32_t idesc = tc05::idesc_i8(kBM, BN), idesc2 = tc05::idesc_i8(kBM, DIGITS * BN);
     int it = 0;
     for (; it < nk; ++it) {
       const int s = it % STAGES, r = it / STAGES;
@@ -187,10 +192,16 @@ __global__ void __launch_bounds__(kThreads, Cfg<DIGITS, VAR>::CTAS)
           const uint64_t a1 = tc05::sdesc_k_sw128(st + A_TILE) + 2 * kk;
           const uint64_t b0 = tc05::sdesc_k_sw128(st + 2 * A_TILE) + 2 * kk;
           const uint64_t b1 = tc05::sdesc_k_sw128(st + 2 * A_TILE + B_TILE) + 2 * kk;
-          tc05::mma_i8(tmem, a0, b0, idesc, first);               // D0 += lo lo
-          tc05::mma_i8(tmem + BN, a0, b1, idesc, first);          // D1 += lo hi
-          tc05::mma_i8(tmem + BN, a1, b0, idesc, 1u);             // D1 += hi lo
-          tc05::mma_i8(tmem + 2 * BN, a1, b1, idesc, first);      // D2 += hi hi
+          // The two digits of B lie one after the other in shared memory and the sums D0, D1, D2 in
+          // TMEM, so one MMA of twice the width serves a digit of A: half the reads of A, without which
+          // shared memory (48 cycles an MMA of 64 columns) and not the tensor pipe (32) sets the pace.
+          tc05::mma_i8(tmem, a0, b0, idesc2, first);              // D0 += lo lo, D1 += lo hi
+          if (first) {
+            tc05::mma_i8(tmem + BN, a1, b0, idesc2, 1u);          // D1 += hi lo, D2 += hi hi
+          } else {
+            tc05::mma_i8(tmem + BN, a1, b0, idesc, 1u);           // D1 += hi lo
+            tc05::mma_i8(tmem + 2 * BN, a1, b1, idesc, 0u);       // D2 = hi hi
+          }
         }
       }
       tc05::mma_commit(&empty[s]);
@@ -206,8 +217,8 @@ __global__ void __launch_bounds__(kThreads, Cfg<DIGITS, VAR>::CTAS)
     if (go) {
       const int row = warp * 32 + lane;
       const int i = tm * kBM + row;
-      const int p = a.moduli[l];
-      const double pinv = 1.0 / (double)p;
+      const Mod M(a.moduli[l]);
+      const uint32_t m8 = 256u % M.p, m16 = 65536u % M.p;
       const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
@@ -223,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<DIGITS, VAR>::CTAS)
             for (int q = 0; q < 32; ++q) {
               const int j = j0 + q;
               if (j < a.n) {
-                out[(long)j * a.m + i] = (int8_t)sym_mod_small((int)acc[0][q], p, pinv);
+                out[(long)j * a.m + i] = (int8_t)sym_mod((int)acc[0][q], M);
               }
             }
           } else {
@@ -232,14 +243,9 @@ __global__ void __launch_bounds__(kThreads, Cfg<DIGITS, VAR>::CTAS)
             for (int q = 0; q < 32; ++q) {
               const int j = j0 + q;
               if (j < a.n) {
-                long long v = (long long)(int)acc[0][q] + ((long long)(int)acc[NACC > 1 ? 1 : 0][q] << 8) +
-                              ((long long)(int)acc[NACC > 2 ? 2 : 0][q] << 16);
-                long long r = mod_wide(v, p, pinv);
-                if (a.accumulate) {
-                  r += out[(long)j * a.m + i];
-                  if (r >= p) r -= p;
-                }
-                out[(long)j * a.m + i] = (int)r;
+                const uint32_t add = a.accumulate ? (uint32_t)out[(long)j * a.m + i] : 0u;
+                out[(long)j * a.m + i] = (int)mod_digits((int)acc[0][q], (int)acc[NACC > 1 ? 1 : 0][q],
+                                                         (int)acc[NACC > 2 ? 2 : 0][q], add, m8, m16, M);
               }
             }
           }
