@@ -1,20 +1,24 @@
-// Modular INT8 tensor-core GEMM on sm_100a: one CTA per (128-row tile, tile_n-column tile,
-// modulus).  Warp-specialised, non-persistent:
+// Modular INT8 tensor-core GEMM on sm_100a, persistent: a CTA takes the tiles (128 rows, tile_n columns, a
+// modulus) blockIdx.x, blockIdx.x + gridDim.x, ...  Warp-specialised:
 //   warp 4 (one lane)  TMA producer: K-blocks of 128 bytes of every digit plane of A and B into a
 //                      ring of shared-memory stages (128-byte swizzle), completion counted in
-//                      bytes on the stage's `full` mbarrier;
-//   warp 5 (one lane)  MMA issuer: 4 x tcgen05.mma.kind::i8 (K = 32 bytes each) per digit pair and
+//                      bytes on the stage's `full` mbarrier; it runs ahead into the next tile;
+//   warp 5 (one lane)  MMA issuer: 4 x tcgen05.mma.kind::i8 (K = 32 bytes each) per digit of A and
 //                      stage into TMEM accumulators (one per digit sum), tcgen05.commit frees the
-//                      stage; a last commit signals the epilogue;
+//                      stage, a commit per tile hands the accumulators to the epilogue;
 //   warps 0-3          epilogue: tcgen05.ld of the accumulators (warp w reads TMEM lanes
 //                      32w..32w+31 = output rows), reduction modulo the tile's modulus, coalesced
-//                      stores (consecutive lanes = consecutive rows of a column-major plane).
+//                      stores (consecutive lanes = consecutive rows of a column-major plane), while
+//                      the next tile's MMAs run into the other set of accumulators where TMEM has two.
 // Every wait is bounded; a wait that gives up sets bit 0 of args.err, the other roles stop at
-// their next wait, outstanding TMA copies are drained (bounded) and TMEM is released before exit.
+// their next wait, outstanding TMA copies are drained and the MMAs issued waited for (both bounded) and
+// TMEM is released before exit.
 #include <cuda.h>
 
+#include <algorithm>
 #include <array>
 #include <atomic>
+#include <climits>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -34,34 +38,38 @@ constexpr int kKB = 128;     // K bytes per stage (one 128-byte swizzle row)
 constexpr int kThreads = 192;
 
 // Tile configurations: variant 0 (the default), variant 1 (half the tile width, deeper stage
-// ring) and variant 2 (two CTAs per SM: a two-stage ring each, so that one CTA's epilogue overlaps
-// the other's main loop); the autotuner picks per shape class.  Every variant gives the same bits.
+// ring) and variant 2 (two CTAs per SM: a two-stage ring each); the autotuner picks per shape class.
+// Every variant gives the same bits.  NBUF: sets of accumulators in TMEM.
+// Persistent CTAs keep the ring full across tiles and, with two sets, store one tile under the MMAs of
+// the next: 16 products of 2048^3 one tile per CTA 236 / 318 / 169 us (variants 0 / 1 / 2), persistent 145 / 187 /
+// 156; 37 primes of 2000^3 in two digits 1350 / 1870 / 1268 and 1234 / 1253 / 1197.  256 x 256 tiles for one
+// digit (one set of accumulators) were no faster than variant 2 with one tile per CTA (168).
 constexpr int kVariants = 3;
 template <int DIGITS, int VAR>
 struct Cfg;
 template <>
 struct Cfg<1, 0> {
-  static constexpr int BN = 256, STAGES = 4, NACC = 1, TMEM_COLS = 256, CTAS = 1;
+  static constexpr int BN = 256, STAGES = 4, NACC = 1, NBUF = 2, TMEM_COLS = 512, CTAS = 1;
 };
 template <>
 struct Cfg<1, 1> {
-  static constexpr int BN = 128, STAGES = 6, NACC = 1, TMEM_COLS = 128, CTAS = 1;
+  static constexpr int BN = 128, STAGES = 6, NACC = 1, NBUF = 2, TMEM_COLS = 256, CTAS = 1;
 };
 template <>
 struct Cfg<1, 2> {
-  static constexpr int BN = 256, STAGES = 2, NACC = 1, TMEM_COLS = 256, CTAS = 2;
+  static constexpr int BN = 256, STAGES = 2, NACC = 1, NBUF = 1, TMEM_COLS = 256, CTAS = 2;
 };
 template <>
 struct Cfg<2, 0> {
-  static constexpr int BN = 128, STAGES = 3, NACC = 3, TMEM_COLS = 512, CTAS = 1;
+  static constexpr int BN = 128, STAGES = 3, NACC = 3, NBUF = 1, TMEM_COLS = 512, CTAS = 1;
 };
 template <>
 struct Cfg<2, 1> {
-  static constexpr int BN = 64, STAGES = 4, NACC = 3, TMEM_COLS = 256, CTAS = 1;
+  static constexpr int BN = 64, STAGES = 4, NACC = 3, NBUF = 2, TMEM_COLS = 512, CTAS = 1;
 };
 template <>
 struct Cfg<2, 2> {
-  static constexpr int BN = 64, STAGES = 2, NACC = 3, TMEM_COLS = 256, CTAS = 2;
+  static constexpr int BN = 64, STAGES = 2, NACC = 3, NBUF = 1, TMEM_COLS = 256, CTAS = 2;
 };
 
 template <int DIGITS, int VAR>
@@ -70,9 +78,9 @@ constexpr int stage_bytes() {
 }
 template <int DIGITS, int VAR>
 constexpr size_t smem_bytes() {
-  // stages, then 2 * STAGES + 1 mbarriers, the TMEM address, the abort flag and the consumed
+  // stages, then 2 * STAGES + 5 mbarriers, the TMEM address, the abort flag and the consumed
   // count, plus 1024 bytes to align the stage ring to the swizzle atom
-  return (size_t)Cfg<DIGITS, VAR>::STAGES * stage_bytes<DIGITS, VAR>() + (2 * Cfg<DIGITS, VAR>::STAGES + 1) * 8 + 16 +
+  return (size_t)Cfg<DIGITS, VAR>::STAGES * stage_bytes<DIGITS, VAR>() + (2 * Cfg<DIGITS, VAR>::STAGES + 5) * 8 + 16 +
          1024;
 }
 
@@ -111,18 +119,33 @@ template <int DIGITS, int VAR>
 __global__ void __launch_bounds__(kThreads, Cfg<DIGITS, VAR>::CTAS)
     k_i8_mod_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, I8GemmArgs a) {
   constexpr int BN = Cfg<DIGITS, VAR>::BN, STAGES = Cfg<DIGITS, VAR>::STAGES, NACC = Cfg<DIGITS, VAR>::NACC;
-  constexpr int TCOLS = Cfg<DIGITS, VAR>::TMEM_COLS;
+  constexpr int TCOLS = Cfg<DIGITS, VAR>::TMEM_COLS, NBUF = Cfg<DIGITS, VAR>::NBUF;
   constexpr int SB = stage_bytes<DIGITS, VAR>();
   constexpr int A_TILE = kBM * kKB, B_TILE = BN * kKB;
-  const int tm = blockIdx.x, tn = blockIdx.y, l = blockIdx.z;
-  if (a.upper_only && tm * kBM > tn * BN + BN - 1) return;  // every entry of the tile has i > j
+  const int nm = a.Mpad / kBM, nn = a.Npad / BN, tiles = nm * nn * a.L;
+  // every role walks the same tiles: tile t is (t % nm, t / nm % nn, t / (nm nn)); with upper_only those
+  // whose every entry has i > j are left out
+  struct Tile {
+    int tm, tn, l;
+    bool skip;
+  };
+  auto tile = [&](int t) {
+    Tile x;
+    x.tm = t % nm;
+    x.tn = t / nm % nn;
+    x.l = t / (nm * nn);
+    x.skip = a.upper_only && x.tm * kBM > x.tn * BN + BN - 1;
+    return x;
+  };
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)STAGES * SB);
   uint64_t* empty = full + STAGES;
-  uint64_t* done = empty + STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  uint64_t* acc_full = empty + STAGES;  // a set of accumulators is complete / has been read
+  uint64_t* acc_empty = acc_full + 2;
+  uint64_t* drain = acc_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* consumed = reinterpret_cast<int*>(tmem_slot + 2);
 
@@ -132,7 +155,11 @@ __global__ void __launch_bounds__(kThreads, Cfg<DIGITS, VAR>::CTAS)
       tc05::mbar_init(&full[s], 1);
       tc05::mbar_init(&empty[s], 1);
     }
-    tc05::mbar_init(done, 1);
+    for (int q = 0; q < 2; ++q) {
+      tc05::mbar_init(&acc_full[q], 1);
+      tc05::mbar_init(&acc_empty[q], 4);  // one arrival per epilogue warp
+    }
+    tc05::mbar_init(drain, 1);
     *abort = 0;
     *consumed = 0;
     tc05::fence_barrier_init();
@@ -152,84 +179,110 @@ __global__ void __launch_bounds__(kThreads, Cfg<DIGITS, VAR>::CTAS)
   if (warp == 4 && lane == 0) {  // ---- TMA producer ----
     tc05::tma_prefetch_map(&tA);
     tc05::tma_prefetch_map(&tB);
-    for (int it = 0; it < nk; ++it) {
-      const int s = it % STAGES, r = it / STAGES;
-      if (r > 0 && !tc05::mbar_wait(&empty[s], (r - 1) & 1, abort)) {
-        give_up(abort, a.err);
-        break;
-      }
-      tc05::mbar_arrive_expect_tx(&full[s], SB);
-      uint8_t* st = smem + (size_t)s * SB;
-      const int x = a.k0 + it * kKB;
+    int it = 0;
+    bool go = true;
+    for (int t = blockIdx.x; go && t < tiles; t += gridDim.x) {
+      const Tile x = tile(t);
+      if (x.skip) continue;
+      for (int kb = 0; kb < nk; ++kb, ++it) {
+        const int s = it % STAGES, r = it / STAGES;
+        if (r > 0 && !tc05::mbar_wait(&empty[s], (r - 1) & 1, abort)) {
+          give_up(abort, a.err);
+          go = false;
+          break;
+        }
+        tc05::mbar_arrive_expect_tx(&full[s], SB);
+        uint8_t* st = smem + (size_t)s * SB;
+        const int c = a.k0 + kb * kKB;
 #pragma unroll
-      for (int d = 0; d < DIGITS; ++d) {
-        tc05::tma_load_2d(st + d * A_TILE, &tA, &full[s], x, (l * DIGITS + d) * a.Mpad + tm * kBM);
-        tc05::tma_load_2d(st + DIGITS * A_TILE + d * B_TILE, &tB, &full[s], x,
-                          (l * DIGITS + d) * a.Npad + tn * BN);
+        for (int d = 0; d < DIGITS; ++d) {
+          tc05::tma_load_2d(st + d * A_TILE, &tA, &full[s], c, (x.l * DIGITS + d) * a.Mpad + x.tm * kBM);
+          tc05::tma_load_2d(st + DIGITS * A_TILE + d * B_TILE, &tB, &full[s], c,
+                            (x.l * DIGITS + d) * a.Npad + x.tn * BN);
+        }
+        issued = it + 1;
       }
-      issued = it + 1;
     }
   } else if (warp == 5 && lane == 0) {  // ---- MMA issuer ----
     constexpr uint32_t idesc = tc05::idesc_i8(kBM, BN), idesc2 = tc05::idesc_i8(kBM, DIGITS * BN);
-    int it = 0;
-    for (; it < nk; ++it) {
-      const int s = it % STAGES, r = it / STAGES;
-      if (!tc05::mbar_wait(&full[s], r & 1, abort)) {
+    int it = 0, n = 0;  // K-blocks and tiles so far
+    bool go = true;
+    for (int t = blockIdx.x; go && t < tiles; t += gridDim.x) {
+      if (tile(t).skip) continue;
+      const int buf = n % NBUF, round = n / NBUF;
+      if (round > 0 && !tc05::mbar_wait(&acc_empty[buf], (round - 1) & 1, abort)) {
         give_up(abort, a.err);
         break;
       }
       tc05::tc_fence_after();
-      const uint32_t st = tc05::smem_u32(smem + (size_t)s * SB);
+      const uint32_t acc = tmem + buf * (NACC * BN);
+      for (int kb = 0; kb < nk; ++kb, ++it) {
+        const int s = it % STAGES, r = it / STAGES;
+        if (!tc05::mbar_wait(&full[s], r & 1, abort)) {
+          give_up(abort, a.err);
+          go = false;
+          break;
+        }
+        tc05::tc_fence_after();
+        const uint32_t st = tc05::smem_u32(smem + (size_t)s * SB);
 #pragma unroll
-      for (int kk = 0; kk < kKB / 32; ++kk) {
-        const uint32_t first = (it == 0 && kk == 0) ? 0u : 1u;
-        if (DIGITS == 1) {
-          const uint64_t ad = tc05::sdesc_k_sw128(st) + 2 * kk;
-          const uint64_t bd = tc05::sdesc_k_sw128(st + A_TILE) + 2 * kk;
-          tc05::mma_i8(tmem, ad, bd, idesc, first);
-        } else {
-          const uint64_t a0 = tc05::sdesc_k_sw128(st) + 2 * kk;
-          const uint64_t a1 = tc05::sdesc_k_sw128(st + A_TILE) + 2 * kk;
-          const uint64_t b0 = tc05::sdesc_k_sw128(st + 2 * A_TILE) + 2 * kk;
-          const uint64_t b1 = tc05::sdesc_k_sw128(st + 2 * A_TILE + B_TILE) + 2 * kk;
-          // The two digits of B lie one after the other in shared memory and the sums D0, D1, D2 in
-          // TMEM, so one MMA of twice the width serves a digit of A: half the reads of A, without which
-          // shared memory (48 cycles an MMA of 64 columns) and not the tensor pipe (32) sets the pace.
-          tc05::mma_i8(tmem, a0, b0, idesc2, first);              // D0 += lo lo, D1 += lo hi
-          if (first) {
-            tc05::mma_i8(tmem + BN, a1, b0, idesc2, 1u);          // D1 += hi lo, D2 += hi hi
+        for (int kk = 0; kk < kKB / 32; ++kk) {
+          const uint32_t first = (kb == 0 && kk == 0) ? 0u : 1u;
+          if (DIGITS == 1) {
+            const uint64_t ad = tc05::sdesc_k_sw128(st) + 2 * kk;
+            const uint64_t bd = tc05::sdesc_k_sw128(st + A_TILE) + 2 * kk;
+            tc05::mma_i8(acc, ad, bd, idesc, first);
           } else {
-            tc05::mma_i8(tmem + BN, a1, b0, idesc, 1u);           // D1 += hi lo
-            tc05::mma_i8(tmem + 2 * BN, a1, b1, idesc, 0u);       // D2 = hi hi
+            const uint64_t a0 = tc05::sdesc_k_sw128(st) + 2 * kk;
+            const uint64_t a1 = tc05::sdesc_k_sw128(st + A_TILE) + 2 * kk;
+            const uint64_t b0 = tc05::sdesc_k_sw128(st + 2 * A_TILE) + 2 * kk;
+            const uint64_t b1 = tc05::sdesc_k_sw128(st + 2 * A_TILE + B_TILE) + 2 * kk;
+            // The two digits of B lie one after the other in shared memory and the sums D0, D1, D2 in
+            // TMEM, so one MMA of twice the width serves a digit of A: half the reads of A, without which
+            // shared memory (48 cycles an MMA of 64 columns) and not the tensor pipe (32) sets the pace.
+            tc05::mma_i8(acc, a0, b0, idesc2, first);              // D0 += lo lo, D1 += lo hi
+            if (first) {
+              tc05::mma_i8(acc + BN, a1, b0, idesc2, 1u);          // D1 += hi lo, D2 += hi hi
+            } else {
+              tc05::mma_i8(acc + BN, a1, b0, idesc, 1u);           // D1 += hi lo
+              tc05::mma_i8(acc + 2 * BN, a1, b1, idesc, 0u);       // D2 = hi hi
+            }
           }
         }
+        tc05::mma_commit(&empty[s]);
       }
-      tc05::mma_commit(&empty[s]);
+      tc05::mma_commit(&acc_full[buf]);  // completes once every MMA issued above has
+      ++n;
     }
     *consumed = it;
-    tc05::mma_commit(done);  // completes once every MMA issued above has
+    tc05::mma_commit(drain);
+    tc05::mbar_wait(drain, 0, nullptr);  // TMEM is released below
   } else if (warp < 4) {  // ---- epilogue ----
-    const bool waited = tc05::mbar_wait(done, 0, abort);
-    if (!waited) give_up(abort, a.err);
-    // warp-uniform decision: tcgen05.ld is .sync.aligned
-    const bool go = __all_sync(0xffffffffu, waited && !*abort);
-    tc05::tc_fence_after();
-    if (go) {
-      const int row = warp * 32 + lane;
-      const int i = tm * kBM + row;
-      const Mod M(a.moduli[l]);
+    int n = 0;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+      const Tile x = tile(t);
+      if (x.skip) continue;
+      const int buf = n % NBUF;
+      const bool waited = tc05::mbar_wait(&acc_full[buf], (n / NBUF) & 1, abort);
+      if (!waited) give_up(abort, a.err);
+      // warp-uniform decision: tcgen05.ld is .sync.aligned
+      if (!__all_sync(0xffffffffu, waited && !*abort)) break;
+      tc05::tc_fence_after();
+      const int i = x.tm * kBM + warp * 32 + lane;
+      const Mod M(a.moduli[x.l]);
       const uint32_t m8 = 256u % M.p, m16 = 65536u % M.p;
-      const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
+      const uint32_t acc0 = tmem + buf * (NACC * BN) + ((uint32_t)(warp * 32) << 16);
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
+        __syncwarp();  // tcgen05.ld is .sync.aligned
         uint32_t acc[NACC][32];
 #pragma unroll
-        for (int q = 0; q < NACC; ++q) tc05::tmem_ld32(lane_base + q * BN + c0, acc[q]);
+        for (int q = 0; q < NACC; ++q) tc05::tmem_ld32(acc0 + q * BN + c0, acc[q]);
         tc05::tmem_ld_wait();
-        const int j0 = tn * BN + c0;
+        const int j0 = x.tn * BN + c0;
         if (i < a.m) {
           if (DIGITS == 1) {
-            int8_t* out = static_cast<int8_t*>(a.out) + (long)l * a.plane;
+            int8_t* out = static_cast<int8_t*>(a.out) + (long)x.l * a.plane;
 #pragma unroll
             for (int q = 0; q < 32; ++q) {
               const int j = j0 + q;
@@ -238,7 +291,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<DIGITS, VAR>::CTAS)
               }
             }
           } else {
-            int* out = static_cast<int*>(a.out) + (long)l * a.plane;
+            int* out = static_cast<int*>(a.out) + (long)x.l * a.plane;
 #pragma unroll
             for (int q = 0; q < 32; ++q) {
               const int j = j0 + q;
@@ -251,6 +304,10 @@ __global__ void __launch_bounds__(kThreads, Cfg<DIGITS, VAR>::CTAS)
           }
         }
       }
+      tc05::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc05::mbar_arrive(&acc_empty[buf]);
+      ++n;
     }
   }
   __syncthreads();
@@ -307,6 +364,14 @@ std::mutex g_i8_mu;
 double g_i8_ms = 0.0, g_i8_ops = 0.0, g_i8_alg_ops = 0.0;
 uint64_t g_i8_count = 0;
 
+// SMs of the current device.
+int sm_count() {
+  int dev = 0, n = 0;
+  check(cudaGetDevice(&dev), "cudaGetDevice");
+  check(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev), "SM count");
+  return n;
+}
+
 // One launch of variant VAR (returns after queueing; with timing on, after the event).
 template <int DIGITS, int VAR>
 void launch_variant(const int8_t* A, const int8_t* B, const I8GemmArgs& a, cudaStream_t st, float* ms_out) {
@@ -319,7 +384,9 @@ void launch_variant(const int8_t* A, const int8_t* B, const I8GemmArgs& a, cudaS
   });
   const CUtensorMap ta = byte_map(A, (long)a.L * DIGITS * a.Mpad, a.Kld, kBM);
   const CUtensorMap tb = byte_map(B, (long)a.L * DIGITS * a.Npad, a.Kld, BN);
-  const dim3 grid(a.Mpad / kBM, a.Npad / BN, a.L);
+  const long tiles_all = (long)(a.Mpad / kBM) * (a.Npad / BN) * a.L;
+  if (tiles_all > INT_MAX) throw std::invalid_argument("i8 GEMM: too many tiles");
+  const int grid = (int)std::min<long>(tiles_all, (long)sm_count() * Cfg<DIGITS, VAR>::CTAS);
   const bool timed = ms_out != nullptr || g_i8_timing.load() != 0;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (timed) {
