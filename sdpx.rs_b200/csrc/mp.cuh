@@ -508,8 +508,8 @@ MPD_FN Val<N> from_double(double f, long long e) {
 
 // 1 / x and 1 / sqrt(x) by Newton's iteration from an FP64 seed (quadratic convergence: four
 // steps carry 53 bits past 512): accurate to a few units in the last place, not correctly
-// rounded -- the Jacobi rotation parameters, whose orthogonality they bound, and the estimates
-// that the correctly rounded operations correct.
+// rounded -- the Jacobi rotation parameters, whose orthogonality they bound, and the estimate
+// that the correctly rounded root corrects.
 template <int N>
 MPD_CALL Val<N> recip_approx(Val<N> x) {
   long long e;
@@ -564,23 +564,67 @@ MPD_FN void sub_product(uint32_t* R, const uint32_t* Q, const uint32_t* M) {
   sub_words<2 * N + 2>(R, T);
 }
 
-// Step Q until R = X - Q M lies in [0, M) (R 2N + 2 words, two's complement).
+// Q (2N + 1 words) = floor(R 2^(64N + 2) / M), for a positive R (2N + 1 words) below 2^(64N + 1) and not
+// above 2 M, M (2N words) with its top bit set; returns whether the division leaves a remainder.
+// Long division with signed digits: one of 2 bits (at most 8), then 2N of 32 bits, each the nearest
+// integer to the leading three words of the remainder over the leading two of M in FP64 (off by less than
+// 2^-18), so that |R| stays below 0.51 M.  A digit is one row of products and an FP64 estimate, about a
+// hundred cycles at four limbs; Newton steps of full-width products took 7600 for the quotient.
 template <int N>
-MPD_FN void fix_quotient(uint32_t* Q, uint32_t* R, const uint32_t* M) {
-  uint32_t D[2 * N + 2];
+MPD_FN bool long_division(uint32_t* R, const uint32_t* M, uint32_t* Q) {
+  constexpr int W = 2 * N + 1;
+  const double m = (double)M[2 * N - 1] * 0x1p32 + (double)M[2 * N - 2];
+  const double y = 1.0 / m;
 #pragma unroll
-  for (int i = 0; i < 2 * N + 2; ++i) D[i] = i < 2 * N ? M[i < 2 * N ? i : 0] : 0u;
+  for (int i = 0; i < W; ++i) Q[i] = 0u;
 #pragma unroll 1
-  for (int it = 0; it < 4096 && (R[2 * N + 1] >> 31); ++it) {
-    uint32_t one[2 * N + 1] = {1u};
-    sub_words<2 * N + 1>(Q, one);
-    add_words<2 * N + 2>(R, D, 0u);
+  for (int k = 0; k <= 2 * N; ++k) {
+    const double r = (double)(int32_t)R[W - 1] * 0x1p64 + ((double)R[W - 2] * 0x1p32 + (double)R[W - 3]);
+    const long long q = (long long)rint(r * (k == 0 ? 4.0 * y : 0x1p32 * y));
+    const uint32_t b = (uint32_t)(q < 0 ? -q : q), mask = q < 0 ? 0u : 0xffffffffu;
+    if (k == 0) {  // R 4, R 2^32 after it
+#pragma unroll
+      for (int i = W - 1; i > 0; --i) R[i] = funnel_l(R[i - 1], R[i], 2);
+      R[0] <<= 2;
+    } else {
+#pragma unroll
+      for (int i = W - 1; i > 0; --i) R[i] = R[i - 1];
+      R[0] = 0u;
+    }
+    uint32_t P[W + 1], O[W + 1];  // b M: even and odd words' products apart
+#pragma unroll
+    for (int i = 0; i < 2 * N; i += 2) {
+      const uint64_t e = (uint64_t)M[i] * b, o = (uint64_t)M[i + 1] * b;
+      P[i] = (uint32_t)e;
+      P[i + 1] = (uint32_t)(e >> 32);
+      O[i + 1] = (uint32_t)o;
+      O[i + 2] = (uint32_t)(o >> 32);
+    }
+    P[W - 1] = O[0] = 0u;
+    add_words<W>(P, O, 0u);
+#pragma unroll
+    for (int i = 0; i < W; ++i) P[i] ^= mask;  // R - q M
+    add_words<W>(R, P, mask & 1u);
+    if (k > 0) {  // Q = Q 2^32 + q
+#pragma unroll
+      for (int i = W - 1; i > 0; --i) Q[i] = Q[i - 1];
+      Q[0] = 0u;
+    }
+    const uint32_t up = q < 0 ? 0xffffffffu : 0u;
+#pragma unroll
+    for (int i = 1; i < W; ++i) O[i] = up;
+    O[0] = (uint32_t)q;
+    add_words<W>(Q, O, 0u);
   }
-#pragma unroll 1
-  for (int it = 0; it < 4096 && cmp_words<2 * N + 2>(R, D) >= 0; ++it) {
-    add_word<2 * N + 1>(Q, 1u);
-    sub_words<2 * N + 2>(R, D);
+  if (R[W - 1] >> 31) {
+    uint32_t D[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) D[i] = i < 2 * N ? M[i < 2 * N ? i : 0] : 0u;
+    add_words<W>(R, D, 0u);
+    uint32_t one[W] = {1u};
+    sub_words<W>(Q, one);
   }
+  return !is_zero<W>(R);
 }
 // (Q + sticky) 2^scale rounded, sticky below Q's last bit.
 template <int N>
@@ -597,38 +641,24 @@ MPD_FN Val<N> round_quotient(const uint32_t* Q, bool sticky, bool neg, long long
 // 1 / d: Q = floor(2^K / M_d), K = 128N + 2, remainder sticky.
 template <int N>
 MPD_CALL Val<N> recip(Val<N> d) {
-  constexpr long long K = 128LL * N + 2;
-  Val<N> m = d;  // M_d 2^-64N in [1/2, 1)
-  m.neg = false;
-  m.s = -64LL * N;
-  const Val<N> y = recip_approx<N>(m);  // ~ 2^64N / M_d
-  uint32_t Q[2 * N + 1], R[2 * N + 2];
-  to_words<N>(y, K - 64LL * N, Q);  // ~ 2^K / M_d
+  uint32_t Q[2 * N + 1], R[2 * N + 1];
 #pragma unroll
-  for (int i = 0; i < 2 * N + 2; ++i) R[i] = 0u;  // 2^K vanishes modulo 2^(64N + 64)
-  sub_product<N>(R, Q, d.m);
-  fix_quotient<N>(Q, R, d.m);
-  return round_quotient<N>(Q, !is_zero<2 * N + 2>(R), d.neg, -K - d.s);
+  for (int i = 0; i < 2 * N; ++i) R[i] = 0u;
+  R[2 * N] = 1u;
+  const bool sticky = long_division<N>(R, d.m, Q);
+  return round_quotient<N>(Q, sticky, d.neg, -(128LL * N + 2) - d.s);
 }
 
 // a / b: Q = floor(M_a 2^K / M_b), K = 64N + 2, remainder sticky.  b must be nonzero.
 template <int N>
 MPD_CALL Val<N> divide(Val<N> a, Val<N> b) {
   if (a.zero) return zero_val<N>();
-  constexpr long long K = 64LL * N + 2;
-  Val<N> an = a, bn = b;
-  an.neg = bn.neg = false;
-  an.s = bn.s = -64LL * N;
-  const Val<N> q = mul<N>(an, recip_approx<N>(bn));  // ~ M_a / M_b
-  uint32_t Q[2 * N + 1], R[2 * N + 2];
-  to_words<N>(q, K, Q);
+  uint32_t Q[2 * N + 1], R[2 * N + 1];
 #pragma unroll
-  for (int i = 0; i < 2 * N; ++i) R[i] = 0u;  // M_a 2^K modulo 2^(64N + 64)
-  R[2 * N] = a.m[0] << 2;
-  R[2 * N + 1] = funnel_l(a.m[0], a.m[1], 2);
-  sub_product<N>(R, Q, b.m);
-  fix_quotient<N>(Q, R, b.m);
-  return round_quotient<N>(Q, !is_zero<2 * N + 2>(R), a.neg != b.neg, a.s - b.s - K);
+  for (int i = 0; i < 2 * N; ++i) R[i] = a.m[i];
+  R[2 * N] = 0u;
+  const bool sticky = long_division<N>(R, b.m, Q);
+  return round_quotient<N>(Q, sticky, a.neg != b.neg, a.s - b.s - (64LL * N + 2));
 }
 
 // sqrt(a), a >= 0: Y = floor(sqrt(M 2^e)), the radicand 2 (64N + 2) bits wide (e even with s - e),

@@ -1,4 +1,6 @@
 // MPFR dense LDL' kernels on MpFloat<N> arrays (see mp_ldl.cuh and mp.cuh).
+#include <cooperative_groups.h>
+
 #include <stdexcept>
 
 #include "device.cuh"
@@ -23,40 +25,46 @@ __device__ __forceinline__ const unsigned char* el(const unsigned char* A, long 
 // d_j = a_jj - dot(r_j, w_j) (the exact difference rounded once when that rounds to zero), the
 // pivot rule, D^-1; then every later row i: r_ij = (a_ij - dot(r_i, w_j)) * d_j^-1,
 // w_ij = r_ij d_j.  Dots are exact and rounded once; the other operations round once each.
-// One CTA, bound by the chain of its columns: the pivot (dot, difference, reciprocal) and the
-// column's dots are independent once the column before is done, so warp 0 forms the pivot while
-// the other warps take the dots, eight lanes a row (four rows a warp at once, three butterfly steps
-// instead of five); then one thread a row finishes its two products.  The block's lower triangle is
-// copied into a row-major scratch R (W is row-major too), w_j is staged in shared memory.
+// One cluster of four CTAs, bound by the chain of its columns: the pivot (dot, difference, reciprocal)
+// and the column's dots are independent once the column before is done, so warp 0 of every CTA forms
+// the pivot (the same one: cheaper than handing it round) while the other warps take the dots of the
+// CTA's rows (i mod 4), 16 lanes a row; then one thread a row finishes its two products.  A barrier of the
+// cluster closes a column.  The block's lower triangle is copied into a row-major scratch R (W is row-major
+// too), w_j is staged in shared memory.
 // Up to 4 limbs 512 threads leave 128 registers for the accumulator, operands and product of a
-// dot; above, 256 threads.  LDL' of order 1000 at 256 bits (eight leaves of 125): 217 ms with a warp a
-// row and run-time limb loops in local memory, 28.1 ms so.
+// dot; above, 256 threads and 8 lanes a row.  LDL' of order 1000 at 256 bits (eight leaves of 125): 217 ms
+// with a warp a row and run-time limb loops in local memory, 26 ms with one CTA (33000 cycles a column: dots
+// 28000, or dot 9100, reciprocal 13900 of the pivot; 8300 for the products, on four warps), 19.1 with four and the long division.
 // Scratch: 2 size^2 elements (W, then R).
+constexpr int kLeafCtas = 4;
 template <int N>
 constexpr int kLeafThreads = N <= 4 ? 512 : 256;
 template <int N>
-__global__ void __launch_bounds__(kLeafThreads<N>) k_mp_ldl_dots(unsigned char* A, long lda, int off, int size,
-                                                                 unsigned char* Wsc, unsigned char* dinv,
-                                                                 const unsigned char* reg, uint32_t* status) {
-  constexpr int esz = 8 * N + 8, G = 8;
+__global__ void __cluster_dims__(kLeafCtas, 1, 1) __launch_bounds__(kLeafThreads<N>)
+    k_mp_ldl_dots(unsigned char* A, long lda, int off, int size, unsigned char* Wsc, unsigned char* dinv,
+                  const unsigned char* reg, uint32_t* status) {
+  namespace cg = cooperative_groups;
+  constexpr int esz = 8 * N + 8, G = N <= 4 ? 16 : 8, C = kLeafCtas;
   __shared__ __align__(8) unsigned char srow[kMpRecBase * esz];  // w_j
   __shared__ __align__(8) unsigned char sdot[kMpRecBase * esz];  // dot(r_i, w_j), i > j
   __shared__ __align__(8) unsigned char sd[2 * esz];             // d_j, d_j^-1
   __shared__ int s_fail;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), tid = rank * (int)blockDim.x + (int)threadIdx.x;
   unsigned char* B = A + ((long)off + (long)off * lda) * esz;
   unsigned char* W = Wsc;                            // row-major: (i, c) at i * size + c
   unsigned char* R = Wsc + (long)size * size * esz;  // row-major copy of the lower triangle
   auto rm = [&](unsigned char* M, int i, int c) { return M + ((long)i * size + c) * esz; };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) s_fail = 0;
-  for (long wd = threadIdx.x; wd < (long)size * size * (N + 1); wd += blockDim.x) {  // R(i, c) = B(i, c)
+  for (long wd = tid; wd < (long)size * size * (N + 1); wd += C * blockDim.x) {  // R(i, c) = B(i, c)
     const long e = wd / (N + 1), o = wd % (N + 1) * 8;
     const int i = (int)(e / size), c = (int)(e % size);
     if (c <= i)
       *reinterpret_cast<unsigned long long*>(rm(R, i, c) + o) =
           *reinterpret_cast<const unsigned long long*>(el<N>(B, i, c, lda) + o);
   }
-  __syncthreads();
+  cluster.sync();
   for (int j = 0; j < size; ++j) {
     for (int wd = threadIdx.x; wd < j * (N + 1); wd += blockDim.x)
       reinterpret_cast<unsigned long long*>(srow)[wd] = reinterpret_cast<const unsigned long long*>(rm(W, j, 0))[wd];
@@ -79,36 +87,38 @@ __global__ void __launch_bounds__(kLeafThreads<N>) k_mp_ldl_dots(unsigned char* 
           const Val<N> di = mpd::recip<N>(d);
           mpd::store<N>(sd, d, status);
           mpd::store<N>(sd + esz, di, status);
-          mpd::store<N>(dinv + (long)j * esz, di, status);
+          if (rank == 0) mpd::store<N>(dinv + (long)j * esz, di, status);
         }
       }
     } else {
       const int sub = lane & (G - 1);
-      for (int i = j + 1 + (threadIdx.x - 32) / G; i < size; i += (blockDim.x - 32) / G) {  // group-uniform
+      // the rows i > j with i mod C = rank, group-uniform
+      for (int i = j + 1 + ((rank - j - 1) & (C - 1)) + C * ((threadIdx.x - 32) / G); i < size;
+           i += C * ((blockDim.x - 32) / G)) {
         const Val<N> dot = mpd::dot<N, G>(nullptr, rm(R, i, 0), 1, srow, 1, j, &ok);
         if (sub == 0) mpd::store<N>(sdot + i * esz, dot, status);
       }
     }
     if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
     __syncthreads();
-    if (s_fail) return;
-    for (int i = j + 1 + threadIdx.x; i < size; i += blockDim.x) {
+    if (s_fail) return;  // in every CTA: the pivots are the same
+    for (int i = j + 1 + ((rank - j - 1) & (C - 1)) + C * (int)threadIdx.x; i < size; i += C * blockDim.x) {
       const Val<N> d = mpd::load<N>(sd), di = mpd::load<N>(sd + esz);
       const Val<N> t = mpd::addsub<N>(mpd::load<N>(rm(R, i, j)), mpd::load<N>(sdot + i * esz), -1);
       const Val<N> v = mpd::mul<N>(t, di);
       mpd::store<N>(rm(R, i, j), v, status);
       mpd::store<N>(rm(W, i, j), mpd::mul<N>(v, d), status);
     }
-    __syncthreads();
+    cluster.sync();  // row j + 1 of R and W is there for every CTA
   }
-  for (long wd = threadIdx.x; wd < (long)size * size * (N + 1); wd += blockDim.x) {  // B(i, c) = R(i, c), c < i
+  for (long wd = tid; wd < (long)size * size * (N + 1); wd += C * blockDim.x) {  // B(i, c) = R(i, c), c < i
     const long e = wd / (N + 1), o = wd % (N + 1) * 8;
     const int i = (int)(e / size), c = (int)(e % size);
     if (c < i)
       *reinterpret_cast<unsigned long long*>(el<N>(B, i, c, lda) + o) =
           *reinterpret_cast<const unsigned long long*>(rm(R, i, c) + o);
   }
-  for (int j = threadIdx.x; j < size; j += blockDim.x)  // unit diagonal
+  for (int j = tid; j < size; j += C * blockDim.x)  // unit diagonal
     mpd::store<N>(el<N>(B, j, j, lda), mpd::one_val<N>(), status);
 }
 
@@ -240,7 +250,7 @@ void mp_launch_ldl_dots(unsigned char* A, long lda, int off, int size, int N, un
   if (size <= 0) return;
   if (size > kMpRecBase) throw std::invalid_argument("MPFR LDL: leaf above the recursion base");
   mpd::by_limbs(N, [&](auto n) {
-    ++g_launches, k_mp_ldl_dots<n()><<<1, kLeafThreads<n()>, 0, st>>>(A, lda, off, size, W, dinv, reg, status);
+    ++g_launches, k_mp_ldl_dots<n()><<<kLeafCtas, kLeafThreads<n()>, 0, st>>>(A, lda, off, size, W, dinv, reg, status);
   });
   check(cudaGetLastError(), "k_mp_ldl_dots");
 }
