@@ -214,7 +214,7 @@ __global__ void k_schur_transform(const BlockDesc*, const int*, const int*, cons
 __global__ void k_schur_block_gemm(const BlockDesc*, const int*, const int*, const long*,
                                    const long*, const double*, const double*, double*);
 __global__ void k_schur_gather(int, const int*, const int*, const int*, const int*, const long*,
-                               const double*, double*);
+                               const double*, double*, uint32_t*);
 __global__ void k_add_upper_csc(int, const int*, const int*, const double*, double*);
 __global__ void k_op_forward(const BlockDesc*, const int*, const int*, const int*, const long*,
                              const double*, const int*, const int*, const double*, long, double,

@@ -1037,6 +1037,7 @@ class Engine {
   // ---- Schur complement ----
   bool assemble() {
     factor_ok_ = false;  // the factor no longer matches the Schur complement being rebuilt
+    clear_status();
     tbegin(KT_ASSEMBLE);
     if (nwork_) {
       ++g_launches, k_schur_transform<<<nwork_, SDPXG_CONE_THREADS, kSmemTrans, st>>>(blocks_, wblk_, wloc_, acol_off_,
@@ -1083,7 +1084,7 @@ class Engine {
     if (tot) {
       const long gt = (n + 31) / 32;
       ++g_launches, k_schur_gather<<<(unsigned)(gt * (gt + 1) / 2), 1024, 0, st>>>(n, c2b_ptr_, c2b_blk_, c2b_loc_,
-                                                                  kcount_, s_off_, S_, Hsave_);
+                                                                  kcount_, s_off_, S_, Hsave_, status_);
       launched("k_schur_gather");
     }
     if (pup_nnz_) {
@@ -1095,6 +1096,7 @@ class Engine {
       launched("k_nn_schur");
     }
     tend(KT_ASSEMBLE);
+    if (!pup_nnz_ && !nnn_) return (read_status() & SDPXG_ST_NONFINITE) == 0;  // the gather has looked at every entry
     int s = red.add(st, RED_FINITE, tot, Hsave_, nullptr);
     return red.fetch(st)[s] == 1.0;
   }

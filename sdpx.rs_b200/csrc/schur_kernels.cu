@@ -146,11 +146,14 @@ k_schur_block_gemm(const BlockDesc* __restrict__ blocks, const int* __restrict__
 // H (m x m, full, column-major) = sum over shared blocks of S_j[la, lb], in cone order.
 // One CTA per 32 x 32 tile on or above the diagonal (grid.x numbers them by columns); both triangles are
 // written (symmetrised by construction), the mirrored tile through shared memory so that its stores are
-// whole lines too (m = 4000: 143 us, 164 with one thread an entry and stores a column apart).
+// whole lines too.  A non-finite entry sets SDPXG_ST_NONFINITE (`status`), which saves another pass over H
+// (74 us at m = 4000).  m = 4000, four of 64 blocks a row: 143 us, 164 with one thread an entry and stores a
+// column apart, 157 with the tile's block lists in shared memory.
 extern "C" __global__ void __launch_bounds__(1024)
 k_schur_gather(int m, const int* __restrict__ c2b_ptr, const int* __restrict__ c2b_blk,
                const int* __restrict__ c2b_loc, const int* __restrict__ kcount,
-               const long* __restrict__ s_off, const double* __restrict__ S, double* __restrict__ H) {
+               const long* __restrict__ s_off, const double* __restrict__ S, double* __restrict__ H,
+               uint32_t* __restrict__ status) {
   __shared__ double mirror[32][33];
   int tj = (int)((sqrtf(8.0f * blockIdx.x + 1.0f) - 1.0f) * 0.5f);
   while ((long)tj * (tj + 1) / 2 > blockIdx.x) --tj;
@@ -158,6 +161,7 @@ k_schur_gather(int m, const int* __restrict__ c2b_ptr, const int* __restrict__ c
   const int ti = (int)(blockIdx.x - (long)tj * (tj + 1) / 2);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int a = 32 * ti + lane;
+  bool bad = false;
   {
     const int b = 32 * tj + w;
     if (a <= b && b < m) {
@@ -182,9 +186,10 @@ k_schur_gather(int m, const int* __restrict__ c2b_ptr, const int* __restrict__ c
       }
       H[a + (long)b * m] = acc;
       mirror[lane][w] = acc;
+      bad = !isfinite(acc);
     }
   }
-  __syncthreads();
+  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(status, SDPXG_ST_NONFINITE);
   const int b = 32 * tj + lane;
   const int col = 32 * ti + w;
   if (col < b && b < m) H[b + (long)col * m] = mirror[w][lane];

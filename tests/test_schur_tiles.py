@@ -33,3 +33,19 @@ def test_schur_of_one_dense_block(n, k):
     bound = 4 * (t + 2 * n) * EPS * np.linalg.norm(G) ** 2 * np.outer(*2 * (np.linalg.norm(A, axis=0),))
     assert np.all(np.abs(H - want) <= bound)
     assert np.array_equal(H, H.T)
+
+
+@pytest.mark.parametrize("k,bad", [(1, 0), (33, 32), (64, 0), (70, 69), (70, 31)])
+def test_one_non_finite_entry_is_found(k, bad):
+    """Column `bad` overflows only against itself: one infinite entry, on the diagonal, in any tile."""
+    A = np.random.default_rng(k).standard_normal((10, k))
+    A[:, bad] *= 1e200
+    ctx = KernelContext()
+    ctx.upload(sp.csc_matrix(A), [4])
+    ctx.identity_scaling()
+    with pytest.raises(Exception, match="non-finite"):
+        ctx.schur()
+    A[:, bad] /= 1e200
+    ctx.upload(sp.csc_matrix(A), [4])
+    ctx.identity_scaling()
+    assert np.all(np.isfinite(ctx.schur()))
