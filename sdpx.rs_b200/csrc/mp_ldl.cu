@@ -124,28 +124,44 @@ __global__ void __cluster_dims__(kLeafCtas, 1, 1) __launch_bounds__(kLeafThreads
 
 // arrow.rs:437-447: each row of B solves x L' = b by exact dots, x_j = b_j - dot(x_<j, L(j, <j)).
 // One warp per row, four rows per CTA: bound by the chain of the row's k dots, each over the 32
-// lanes with the row's solved entries in shared memory.
+// lanes with the row's solved entries and the row of L in shared memory (the next one on its way in
+// registers meanwhile): k = 125 at 256 bits 473 us, 597 with L read from global memory by every dot.
 constexpr int kSolveRows = 4;
 template <int N>
 __global__ void __launch_bounds__(32 * kSolveRows) k_mp_solve_lt(const unsigned char* L, long ldl, int k,
                                                                  unsigned char* B, long ldb, int m,
                                                                  uint32_t* status) {
   constexpr int esz = 8 * N + 8;
+  static_assert(32 * kSolveRows == kMpRecBase, "a thread has N + 1 words of a row of L");
   __shared__ __align__(8) unsigned char sx[kSolveRows][kMpRecBase * esz];
+  __shared__ __align__(8) unsigned char sl[kMpRecBase * esz];  // L(j, c), c < j
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * kSolveRows + warp;
-  if (i >= m) return;  // warp-uniform
   for (int j = 0; j < k; ++j) {
-    bool ok = true;
-    const Val<N> b = mpd::load<N>(el<N>(B, i, j, ldb));
-    const Val<N> dot = mpd::dot<N, 32>(nullptr, sx[warp], 1, el<N>(L, j, 0, ldl), ldl, j, &ok);
-    const Val<N> x = mpd::addsub<N>(b, dot, -1);
-    if (lane == 0) {
-      if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
-      mpd::store<N>(sx[warp] + j * esz, x, status);
-      mpd::store<N>(el<N>(B, i, j, ldb), x, status);
+    unsigned long long next[N + 1];  // words threadIdx.x + 128 u of L(j + 1, 0 .. j)
+#pragma unroll
+    for (int u = 0; u <= N; ++u) {
+      const int wd = (int)threadIdx.x + 32 * kSolveRows * u, c = wd / (N + 1);
+      next[u] = j + 1 < k && c <= j
+                    ? reinterpret_cast<const unsigned long long*>(el<N>(L, j + 1, c, ldl))[wd % (N + 1)]
+                    : 0ull;
     }
-    __syncwarp();  // x_j visible to the lanes' next dot
+    if (i < m) {  // warp-uniform
+      bool ok = true;
+      const Val<N> b = mpd::load<N>(el<N>(B, i, j, ldb));
+      const Val<N> dot = mpd::dot<N, 32>(nullptr, sx[warp], 1, sl, 1, j, &ok);
+      const Val<N> x = mpd::addsub<N>(b, dot, -1);
+      if (lane == 0) {
+        if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
+        mpd::store<N>(sx[warp] + j * esz, x, status);
+        mpd::store<N>(el<N>(B, i, j, ldb), x, status);
+      }
+    }
+    __syncthreads();  // x_j visible to the lanes' next dot, nobody reads row j of L any more
+#pragma unroll
+    for (int u = 0; u <= N; ++u)
+      reinterpret_cast<unsigned long long*>(sl)[threadIdx.x + 32 * kSolveRows * u] = next[u];
+    __syncthreads();
   }
 }
 
