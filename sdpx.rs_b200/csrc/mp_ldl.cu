@@ -34,9 +34,13 @@ __device__ __forceinline__ const unsigned char* el(const unsigned char* A, long 
 // Up to 4 limbs 512 threads leave 128 registers for the accumulator, operands and product of a
 // dot; above, 256 threads and 8 lanes a row.  LDL' of order 1000 at 256 bits (eight leaves of 125): 217 ms
 // with a warp a row and run-time limb loops in local memory, 26 ms with one CTA (33000 cycles a column: dots
-// 28000, or dot 9100, reciprocal 13900 of the pivot; 8300 for the products, on four warps), 19.1 with four and the long division.
+// 28000, or dot 9100, reciprocal 13900 of the pivot; 8300 for the products, on four warps), 19.1 with four and the long division; a
+// leaf 1348 us with R in global memory, 1211 with the CTAs' rows and the pivot's in shared memory.
 // Scratch: 2 size^2 elements (W, then R).
 constexpr int kLeafCtas = 4;
+// The rows of a CTA stay in shared memory, where they fit next to the rest (32 rows of 128 entries).
+template <int N>
+constexpr bool kLeafRows = N <= 5;
 template <int N>
 constexpr int kLeafThreads = N <= 4 ? 512 : 256;
 template <int N>
@@ -45,7 +49,10 @@ __global__ void __cluster_dims__(kLeafCtas, 1, 1) __launch_bounds__(kLeafThreads
                   const unsigned char* reg, uint32_t* status) {
   namespace cg = cooperative_groups;
   constexpr int esz = 8 * N + 8, G = N <= 4 ? 16 : 8, C = kLeafCtas;
+  constexpr bool kRows = kLeafRows<N>;
+  extern __shared__ __align__(8) unsigned char sr[];             // the CTA's rows of R (kRows)
   __shared__ __align__(8) unsigned char srow[kMpRecBase * esz];  // w_j
+  __shared__ __align__(8) unsigned char sprow[kMpRecBase * esz]; // r_j
   __shared__ __align__(8) unsigned char sdot[kMpRecBase * esz];  // dot(r_i, w_j), i > j
   __shared__ __align__(8) unsigned char sd[2 * esz];             // d_j, d_j^-1
   __shared__ int s_fail;
@@ -55,9 +62,17 @@ __global__ void __cluster_dims__(kLeafCtas, 1, 1) __launch_bounds__(kLeafThreads
   unsigned char* W = Wsc;                            // row-major: (i, c) at i * size + c
   unsigned char* R = Wsc + (long)size * size * esz;  // row-major copy of the lower triangle
   auto rm = [&](unsigned char* M, int i, int c) { return M + ((long)i * size + c) * esz; };
+  auto own = [&](int i, int c) { return kRows ? sr + ((i / C) * size + c) * esz : rm(R, i, c); };  // i mod C = rank
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) s_fail = 0;
-  for (long wd = tid; wd < (long)size * size * (N + 1); wd += C * blockDim.x) {  // R(i, c) = B(i, c)
+  for (long wd = threadIdx.x; kRows && wd < (long)(size + C - 1) / C * size * (N + 1); wd += blockDim.x) {
+    const long e = wd / (N + 1), o = wd % (N + 1) * 8;
+    const int i = (int)(e / size) * C + rank, c = (int)(e % size);
+    if (i < size && c <= i)
+      *reinterpret_cast<unsigned long long*>(own(i, c) + o) =
+          *reinterpret_cast<const unsigned long long*>(el<N>(B, i, c, lda) + o);
+  }
+  for (long wd = tid; !kRows && wd < (long)size * size * (N + 1); wd += C * blockDim.x) {  // R(i, c) = B(i, c)
     const long e = wd / (N + 1), o = wd % (N + 1) * 8;
     const int i = (int)(e / size), c = (int)(e % size);
     if (c <= i)
@@ -66,15 +81,17 @@ __global__ void __cluster_dims__(kLeafCtas, 1, 1) __launch_bounds__(kLeafThreads
   }
   cluster.sync();
   for (int j = 0; j < size; ++j) {
-    for (int wd = threadIdx.x; wd < j * (N + 1); wd += blockDim.x)
+    for (int wd = threadIdx.x; wd < j * (N + 1); wd += blockDim.x) {
       reinterpret_cast<unsigned long long*>(srow)[wd] = reinterpret_cast<const unsigned long long*>(rm(W, j, 0))[wd];
+      reinterpret_cast<unsigned long long*>(sprow)[wd] = reinterpret_cast<const unsigned long long*>(rm(R, j, 0))[wd];
+    }
     __syncthreads();
     bool ok = true;
     if (warp == 0) {  // the pivot: the dot over the lanes, the rest on lane 0
-      const Val<N> a = mpd::load<N>(rm(R, j, j));
-      const Val<N> dot = mpd::dot<N, 32>(nullptr, rm(R, j, 0), 1, srow, 1, j, &ok);
+      const Val<N> a = mpd::load<N>(el<N>(B, j, j, lda));  // B is written after the last column
+      const Val<N> dot = mpd::dot<N, 32>(nullptr, sprow, 1, srow, 1, j, &ok);
       Val<N> d = mpd::addsub<N>(a, dot, -1);
-      if (d.zero && j > 0) d = mpd::dot<N, 32>(&a, rm(R, j, 0), 1, srow, 1, j, &ok);
+      if (d.zero && j > 0) d = mpd::dot<N, 32>(&a, sprow, 1, srow, 1, j, &ok);
       if (lane == 0) {
         if (reg) {  // DenseLeaf::pivot (arrow.rs:618-632), sign +1
           const Val<N> eps = mpd::load<N>(reg), delta = mpd::load<N>(reg + esz);
@@ -95,7 +112,7 @@ __global__ void __cluster_dims__(kLeafCtas, 1, 1) __launch_bounds__(kLeafThreads
       // the rows i > j with i mod C = rank, group-uniform
       for (int i = j + 1 + ((rank - j - 1) & (C - 1)) + C * ((threadIdx.x - 32) / G); i < size;
            i += C * ((blockDim.x - 32) / G)) {
-        const Val<N> dot = mpd::dot<N, G>(nullptr, rm(R, i, 0), 1, srow, 1, j, &ok);
+        const Val<N> dot = mpd::dot<N, G>(nullptr, own(i, 0), 1, srow, 1, j, &ok);
         if (sub == 0) mpd::store<N>(sdot + i * esz, dot, status);
       }
     }
@@ -104,9 +121,10 @@ __global__ void __cluster_dims__(kLeafCtas, 1, 1) __launch_bounds__(kLeafThreads
     if (s_fail) return;  // in every CTA: the pivots are the same
     for (int i = j + 1 + ((rank - j - 1) & (C - 1)) + C * (int)threadIdx.x; i < size; i += C * blockDim.x) {
       const Val<N> d = mpd::load<N>(sd), di = mpd::load<N>(sd + esz);
-      const Val<N> t = mpd::addsub<N>(mpd::load<N>(rm(R, i, j)), mpd::load<N>(sdot + i * esz), -1);
+      const Val<N> t = mpd::addsub<N>(mpd::load<N>(own(i, j)), mpd::load<N>(sdot + i * esz), -1);
       const Val<N> v = mpd::mul<N>(t, di);
       mpd::store<N>(rm(R, i, j), v, status);
+      if (kRows) mpd::store<N>(own(i, j), v, status);
       mpd::store<N>(rm(W, i, j), mpd::mul<N>(v, d), status);
     }
     cluster.sync();  // row j + 1 of R and W is there for every CTA
@@ -266,7 +284,13 @@ void mp_launch_ldl_dots(unsigned char* A, long lda, int off, int size, int N, un
   if (size <= 0) return;
   if (size > kMpRecBase) throw std::invalid_argument("MPFR LDL: leaf above the recursion base");
   mpd::by_limbs(N, [&](auto n) {
-    ++g_launches, k_mp_ldl_dots<n()><<<kLeafCtas, kLeafThreads<n()>, 0, st>>>(A, lda, off, size, W, dinv, reg, status);
+    constexpr size_t esz = 8 * n() + 8;
+    const size_t rows = kLeafRows<n()> ? (size + kLeafCtas - 1) / kLeafCtas * size * esz : 0;
+    if (rows)  // per device
+      check(cudaFuncSetAttribute(k_mp_ldl_dots<n()>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows),
+            "LDL leaf smem attribute");
+    ++g_launches, k_mp_ldl_dots<n()><<<kLeafCtas, kLeafThreads<n()>, rows, st>>>(A, lda, off, size, W, dinv, reg,
+                                                                                status);
   });
   check(cudaGetLastError(), "k_mp_ldl_dots");
 }

@@ -13,8 +13,11 @@ import make_ldl_fixtures as F  # noqa: E402
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 6, 33])
-@pytest.mark.parametrize("limbs", range(1, 9))
+CASES = [(limbs, n) for limbs in range(1, 9) for n in (1, 2, 3, 4, 5, 6, 33)]
+CASES += [(1, 127), (4, 128), (5, 128), (6, 126)]  # whole leaves, with rows in shared memory up to 5 limbs
+
+
+@pytest.mark.parametrize("limbs,n", CASES)
 def test_mp_leaf_bitwise(limbs, n):
     from sdpx_b200.solver import KernelContext
     A = F.matrix(limbs, n, 20, 7 * limbs + n)
