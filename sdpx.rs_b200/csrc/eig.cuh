@@ -356,9 +356,12 @@ __device__ inline void cta_tridiagonalize(const double* A, int n, double* d, dou
 #pragma unroll
     for (int j = 0; j < 16; ++j) mx = fmax(mx, fmax(fabs(a0[j]), fabs(a1[j])));
     mx = warp_max(mx);
-    if (lane == 0) ws[kPw + w] = mx;
+    if (lane == 0) ws[kPart + w] = mx;
+    // the steps from row 32 on write half of a warp's row of p and read all of it, gone columns too: those
+    // have to be numbers, since a gone column's zero in x does not silence a NaN
+    if (lane < kRow) ws[kPw + w * kRow + lane] = 0.0;
     asm volatile("bar.sync 1, 128;" ::: "memory");
-    mx = fmax(fmax(ws[kPw], ws[kPw + 1]), fmax(ws[kPw + 2], ws[kPw + 3]));
+    mx = fmax(fmax(ws[kPart], ws[kPart + 1]), fmax(ws[kPart + 2], ws[kPart + 3]));
     int ex = 0;
     if (mx > 0.0 && isfinite(mx)) ex = max(-1000, min(1000, ilogb(mx) + 1));
     const double scale = ldexp(1.0, -ex);
@@ -387,15 +390,20 @@ __device__ inline void cta_tridiagonalize(const double* A, int n, double* d, dou
 // of 2^-100 relative to the norm keeps every sequence from stopping at zero), padded to a multiple of
 // eight rows with (4, 0), which change no sign.  Returns the interval in the scaled units and, in
 // *unscale, the factor back.  `t` is 16-byte aligned shared memory, SDPXG_STURM_WORK doubles.
-__device__ inline void sturm_prepare(const double* d, const double* e, int n, double2* t, double* lo, double* hi,
+// False (in every thread) for a (d, e) with a NaN or an infinity, which minima, maxima and sign tests
+// would pass over.
+__device__ inline bool sturm_prepare(const double* d, const double* e, int n, double2* t, double* lo, double* hi,
                                      double* unscale) {
   const int lane = threadIdx.x & 31;
   double l = 1e300, h = -1e300;
+  bool fin = true;
   for (int i = lane; i < n; i += 32) {
     const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i + 1 < n ? fabs(e[i]) : 0.0);
+    fin = fin && isfinite(d[i]) && isfinite(r);
     l = fmin(l, d[i] - r);
     h = fmax(h, d[i] + r);
   }
+  fin = __all_sync(0xffffffffu, fin);
   l = -warp_max(-l);
   h = warp_max(h);
   const double span = fmax(fabs(l), fabs(h));
@@ -413,6 +421,7 @@ __device__ inline void sturm_prepare(const double* d, const double* e, int n, do
     t[i] = i < n ? make_double2(d[i] * s, fmax(v * v, 0x1p-200)) : make_double2(4.0, 0.0);
   }
   __syncthreads();
+  return fin;
 }
 
 // The leading principal minors of T - x for the tridiagonal prepared by sturm_prepare, p_i = (d_i - x)
@@ -457,10 +466,11 @@ __device__ __forceinline__ int sturm(const double2* t, int n, double x) {
 // and gives 8 bits; with 512 it is bound by issue and gives 9.
 // An eigenvalue is resolved relative to itself, down to 2^-200 of the norm: at most 26 rounds.
 // Uniform result; `best` is one int of shared memory, `t` SDPXG_STURM_WORK doubles.
-// *ok = false if the round bound is hit.
+// *ok = false if the round bound is hit or (d, e) is not finite.
 __device__ inline double cta_eig_min(const double* d, const double* e, int n, double2* t, int* best, bool* ok) {
   double lo, hi, unscale;
-  sturm_prepare(d, e, n, t, &lo, &hi, &unscale);
+  *ok = false;
+  if (!sturm_prepare(d, e, n, t, &lo, &hi, &unscale)) return 0.0;
   const int T = blockDim.x;
   for (int round = 0; round < 40; ++round) {
     if (!(hi - lo > 2.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + 0x1p-200)) {
@@ -481,18 +491,18 @@ __device__ inline double cta_eig_min(const double* d, const double* e, int n, do
     lo = nlo;
     hi = nhi;
   }
-  *ok = false;
   return 0.5 * (lo + hi) * unscale;
 }
 
 // Every eigenvalue of the tridiagonal (d, e), ascending, into eig[0..n): 16-lane groups, one
 // eigenvalue per group, multisection with 15 Sturm counts per round (the bracket shrinks 16-fold per
 // round), no CTA barrier inside.  `t`: SDPXG_STURM_WORK doubles.
-// Sets the status bit SDPXG_ST_EIG_FAIL for an eigenvalue whose round bound was hit.
+// Sets the status bit SDPXG_ST_EIG_FAIL for an eigenvalue whose round bound was hit and for a (d, e) that
+// is not finite.
 __device__ inline void cta_eig_all(const double* d, const double* e, int n, double2* t, double* eig,
                                    uint32_t* status) {
   double lo0, hi0, unscale;
-  sturm_prepare(d, e, n, t, &lo0, &hi0, &unscale);
+  if (!sturm_prepare(d, e, n, t, &lo0, &hi0, &unscale) && threadIdx.x == 0) atomicOr(status, SDPXG_ST_EIG_FAIL);
   constexpr int P = 16;
   const int grp = threadIdx.x / P, sl = threadIdx.x % P, base = threadIdx.x & 16;
   const unsigned gmask = 0xFFFFu << base;
