@@ -35,6 +35,7 @@
 // m = 1024 457 us, 2000 864, 4000 3206; so 242, 486 and 1274, and with the whole inverse 248, 533 and
 // 2115.  Holding U_kk^-T back to copy it out by one warp was slower (627 at m = 2000): the tiles of
 // row k wait for it.
+#include "chol_publish.cuh"
 #include "common.cuh"
 
 #define DF_NB 64
@@ -52,7 +53,7 @@ namespace {
 
 struct DfShared {
   uint64_t full[2], empty[2];  // ring stages (chain: 0 the tile (k, k+1), 1 the tile (k+1, k+1))
-  uint64_t pub[2];             // chain: the eight warps' stores of U_kk^-T and of U(k, k+1) are issued
+  uint64_t pub[chol_publish::kSlots];  // chain: the eight warps' stores of a publication are issued
   int item, abort, fail;
 };
 
@@ -446,7 +447,7 @@ __device__ void df_chain(double* __restrict__ F, long ld, int m, int nt, int* pr
     if (lane != 0) return;
     for (int t = 0; t + 1 < 2 * nt; ++t) {
       const int k = t >> 1;
-      if (!df_bar_wait(&sh->pub[t & 1], k & 1, sh)) return;
+      if (!df_bar_wait(&sh->pub[chol_publish::slot(t)], chol_publish::parity(t), sh)) return;
       __threadfence();
       if (t & 1) df_st_release(prog + k + 1, k + 1);
       else df_st_release(prog + k, k + 1);
@@ -483,7 +484,7 @@ __device__ void df_chain(double* __restrict__ F, long ld, int m, int nt, int* pr
       }
     }
     __syncwarp();
-    if (lane == 0) df_bar_arrive(&sh->pub[0]);
+    if (lane == 0) df_bar_arrive(&sh->pub[chol_publish::slot(2 * k)]);
     if (k + 1 >= nt) return;
     const int j0 = k0 + DF_NB, nc = min(DF_NB, m - j0);
     if (!df_all(df_bar_wait(&sh->full[0], k & 1, sh))) return;
@@ -507,7 +508,7 @@ __device__ void df_chain(double* __restrict__ F, long ld, int m, int nt, int* pr
         if (col < nc) F[(k0 + row) + (long)(j0 + col) * ld] = v;
       }
     __syncwarp();
-    if (lane == 0) df_bar_arrive(&sh->pub[1]);
+    if (lane == 0) df_bar_arrive(&sh->pub[chol_publish::slot(2 * k + 1)]);
     df_sync<BAR_MMA, DF_MMA>();
     if (!df_all(df_bar_wait(&sh->full[1], k & 1, sh))) return;
     {  // upper 8 x 8 blocks (R, J), numbers w, w + 8, ... of 36: up to five at once
@@ -592,8 +593,8 @@ k_chol_dataflow(double* __restrict__ F, long ld, int m, int nt, const unsigned* 
         for (int x = 0; x < 2; ++x) {
           df_bar_init(&sh.full[x], 32);
           df_bar_init(&sh.empty[x], type == (int)DF_CHAIN ? 1 : 8);
-          df_bar_init(&sh.pub[x], 8);
         }
+        for (int x = 0; x < chol_publish::kSlots; ++x) df_bar_init(&sh.pub[x], 8);
         sh.abort = sh.fail = 0;
       }
       __syncthreads();
@@ -739,4 +740,5 @@ k_chol_dataflow(double* __restrict__ F, long ld, int m, int nt, const unsigned* 
       break;
     }
   }
+  if (w == 8) asm volatile("cp.async.wait_all;\n" ::: "memory");  // copies of an item that was given up
 }
