@@ -112,6 +112,18 @@ __device__ __forceinline__ int tri_idx(int i, int j) {  // i <= j
   return j * (j + 1) / 2 + i;
 }
 
+// The larger of two magnitudes, NaN when either is one (fmax and std::max lose one): a residual of NaNs is
+// no small residual.  Magnitudes order like their bits as unsigned integers, NaNs of either sign (fabs
+// may leave one negative) above infinity.
+__host__ __device__ __forceinline__ double max_nan(double a, double b) {
+#if defined(__CUDA_ARCH__)
+  return __longlong_as_double((long long)max((unsigned long long)__double_as_longlong(a),
+                                             (unsigned long long)__double_as_longlong(b)));
+#else
+  return (b <= a || a != a) ? a : b;
+#endif
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -385,8 +385,8 @@ inline bool HsdSolver::kkt_solve(const double* bx, const double* bz, double* x, 
   });
   bool ok = true;
   auto& h = E.red.fetch(st());
-  const double normb = std::max(h[0], h[1]);
-  double norme = std::max(h[2], h[3]);
+  const double normb = max_nan(h[0], h[1]);
+  double norme = max_nan(h[2], h[3]);
   if (!std::isfinite(norme)) {
     ok = false;
   } else {
@@ -412,7 +412,7 @@ inline bool HsdSolver::kkt_solve(const double* bx, const double* bz, double* x, 
         E.red.add_batch(st(), {{RED_MAXABS, n, ex2_, nullptr}, {RED_MAXABS, m, ez2_, nullptr}});
       });
       auto& hh = E.red.fetch(st());
-      norme = std::max(hh[0], hh[1]);
+      norme = max_nan(hh[0], hh[1]);
       if (!std::isfinite(norme)) { ok = false; break; }
       double ratio = previous / norme;
       if (ratio < st_.ir_stop_ratio) {

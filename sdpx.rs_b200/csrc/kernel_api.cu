@@ -322,7 +322,7 @@ int32_t sdpxg_residual(sdpxg_ctx* ctx, const double* bx, const double* bz, const
     int s0 = E.red.add(E.st, RED_MAXABS, E.n, ctx->e, nullptr);
     int s1 = E.red.add(E.st, RED_MAXABS, E.m, ctx->f, nullptr);
     auto& h = E.red.fetch(E.st);
-    if (norm) *norm = std::max(h[s0], h[s1]);
+    if (norm) *norm = max_nan(h[s0], h[s1]);
     if (ex) to_host(ex, ctx->e, E.n, E.st);
     if (ez) to_host(ez, ctx->f, E.m, E.st);
     return 0;

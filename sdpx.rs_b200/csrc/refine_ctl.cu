@@ -10,9 +10,6 @@
 // results equal the host-driven refinement's bit for bit.
 #include "common.cuh"
 
-// std::max(a, b) of the host driver: (a < b) ? b : a (a NaN in b is ignored, one in a is kept)
-__device__ __forceinline__ double host_max(double a, double b) { return (a < b) ? b : a; }
-
 __device__ __forceinline__ void ctl_set(cudaGraphConditionalHandle h, bool go) {
   cudaGraphSetConditional(h, go ? 1u : 0u);
 }
@@ -70,8 +67,8 @@ __device__ void refine_step(double e, RefineCtl* c, const RefineParams& p, cudaG
 // After recover + full residual: |bx|, |bz|, |ex|, |ez|.
 __device__ void refine_outer_init(const double* v, RefineCtl* c, const RefineParams& p,
                                   cudaGraphConditionalHandle h) {
-  c->onormb = host_max(v[0], v[1]);
-  const double e = host_max(v[2], v[3]);
+  c->onormb = max_nan(v[0], v[1]);
+  const double e = max_nan(v[2], v[3]);
   c->onorme = e;
   c->oit = 0;
   c->oaccept = c->ocont = 0;
@@ -93,7 +90,7 @@ __device__ void refine_outer_step(const double* v, RefineCtl* c, const RefinePar
   bool go = false;
   int acc = 0;
   if (c->ok) {  // the correction's own solve passed its checks
-    const double e = host_max(v[0], v[1]);
+    const double e = max_nan(v[0], v[1]);
     if (!isfinite(e)) {
       c->ok = 0;
     } else {
@@ -118,7 +115,7 @@ __device__ void refine_outer_step(const double* v, RefineCtl* c, const RefinePar
 }
 
 // The norms of one control point and the control itself in one launch: grid row r is request r
-// (largest magnitude or all finite, both independent of the order of combination), the block that
+// (largest magnitude, NaN kept, or all finite, both independent of the order of combination), the block that
 // arrives last folds every row, one thread of it applies the stopping rule and sets the loop's
 // condition, and after an inner step the block keeps the candidate and its residual (n entries).
 // A graph node costs about 3 us here whatever it computes, and a refined solve of a small system is
@@ -135,16 +132,16 @@ k_refine(RedBatch b, double* __restrict__ partial, unsigned* __restrict__ ticket
   double acc = fin ? 1.0 : 0.0;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < q.n; i += (long)gridDim.x * blockDim.x) {
     const double v = q.x[i];
-    acc = fin ? fmin(acc, isfinite(v) ? 1.0 : 0.0) : fmax(acc, fabs(v));
+    acc = fin ? fmin(acc, isfinite(v) ? 1.0 : 0.0) : max_nan(acc, fabs(v));
   }
   for (int o = 16; o > 0; o >>= 1) {
     const double v = __shfl_xor_sync(0xffffffffu, acc, o);
-    acc = fin ? fmin(acc, v) : fmax(acc, v);
+    acc = fin ? fmin(acc, v) : max_nan(acc, v);
   }
   if (lane == 0) red[warp] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) acc = fin ? fmin(acc, red[w]) : fmax(acc, red[w]);
+    for (int w = 1; w < 8; ++w) acc = fin ? fmin(acc, red[w]) : max_nan(acc, red[w]);
     partial[blockIdx.y * pitch + blockIdx.x] = acc;
     __threadfence();
     last = atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1;
@@ -157,11 +154,11 @@ k_refine(RedBatch b, double* __restrict__ partial, unsigned* __restrict__ ticket
     double v = f ? 1.0 : 0.0;
     for (int k = lane; k < (int)gridDim.x; k += 32) {
       const double u = __ldcg(partial + r * pitch + k);
-      v = f ? fmin(v, u) : fmax(v, u);
+      v = f ? fmin(v, u) : max_nan(v, u);
     }
     for (int o = 16; o > 0; o >>= 1) {
       const double u = __shfl_xor_sync(0xffffffffu, v, o);
-      v = f ? fmin(v, u) : fmax(v, u);
+      v = f ? fmin(v, u) : max_nan(v, u);
     }
     if (lane == 0) val[r] = v;
   }

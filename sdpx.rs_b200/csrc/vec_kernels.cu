@@ -33,8 +33,8 @@ extern "C" __global__ void k_lincomb_batch(LinBatch bt) {
 }
 
 // op 0: sum x*y;  op 1: sum (x*y)^2 (scaled 2-norm squared, y = scales or null);
-// op 2: max |x*y|;  op 3: all finite (1.0 / 0.0) of x;  op 4: max(0, max -x*y) (y >= 0: a
-// nonnegative scale, or a mask that selects rows)
+// op 2: max |x*y|, NaN when an entry is one;  op 3: all finite (1.0 / 0.0) of x;  op 4: max(0, max -x*y)
+// (y >= 0: a nonnegative scale, or a mask that selects rows)
 __device__ __forceinline__ double red_elem(int op, const double* x, const double* y, long i) {
   double xv = x[i];
   double yv = y ? y[i] : 1.0;
@@ -48,7 +48,8 @@ __device__ __forceinline__ double red_elem(int op, const double* x, const double
 }
 
 __device__ __forceinline__ double red_combine(int op, double a, double b) {
-  if (op == 2 || op == 4) return fmax(a, b);
+  if (op == 2) return max_nan(a, b);
+  if (op == 4) return fmax(a, b);
   if (op == 3) return fmin(a, b);
   return a + b;
 }
