@@ -378,6 +378,31 @@ MPD_FN void store(unsigned char* p, const Val<N>& v, uint32_t* status) {
   l[N] = ((unsigned long long)(z ? 0u : (uint32_t)(int)ex) << 32) | kind;
 }
 
+// An intermediate for another thread of the CTA, 8N + 8 bytes: the value as it is in registers, its scale
+// not held to the range of a stored element (the dot that an entry is reduced by may lie outside where
+// the entry does not).
+template <int N>
+MPD_FN void stage(unsigned char* p, const Val<N>& v) {
+  unsigned long long* l = reinterpret_cast<unsigned long long*>(p);
+#pragma unroll
+  for (int q = 0; q < N; ++q) l[q] = ((unsigned long long)v.m[2 * q + 1] << 32) | (unsigned long long)v.m[2 * q];
+  l[N] = (unsigned long long)v.s << 2 | (v.neg ? 2u : 0u) | (v.zero ? 1u : 0u);
+}
+template <int N>
+MPD_FN Val<N> unstage(const unsigned char* p) {
+  Val<N> v;
+  const unsigned long long* l = reinterpret_cast<const unsigned long long*>(p);
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    v.m[2 * q] = (uint32_t)l[q];
+    v.m[2 * q + 1] = (uint32_t)(l[q] >> 32);
+  }
+  v.s = (long long)l[N] >> 2;
+  v.neg = l[N] & 2u;
+  v.zero = l[N] & 1u;
+  return v;
+}
+
 // ---- sums and products ----
 
 // B >>= d bits over K words (d <= 32 K); bits shifted out are or-ed into the result's last bit.

@@ -113,7 +113,7 @@ __global__ void __cluster_dims__(kLeafCtas, 1, 1) __launch_bounds__(kLeafThreads
       for (int i = j + 1 + ((rank - j - 1) & (C - 1)) + C * ((threadIdx.x - 32) / G); i < size;
            i += C * ((blockDim.x - 32) / G)) {
         const Val<N> dot = mpd::dot<N, G>(nullptr, own(i, 0), 1, srow, 1, j, &ok);
-        if (sub == 0) mpd::store<N>(sdot + i * esz, dot, status);
+        if (sub == 0) mpd::stage<N>(sdot + i * esz, dot);
       }
     }
     if (!ok) atomicOr(status, SDPXG_ST_EXACT_SPREAD);
@@ -121,7 +121,7 @@ __global__ void __cluster_dims__(kLeafCtas, 1, 1) __launch_bounds__(kLeafThreads
     if (s_fail) return;  // in every CTA: the pivots are the same
     for (int i = j + 1 + ((rank - j - 1) & (C - 1)) + C * (int)threadIdx.x; i < size; i += C * blockDim.x) {
       const Val<N> d = mpd::load<N>(sd), di = mpd::load<N>(sd + esz);
-      const Val<N> t = mpd::addsub<N>(mpd::load<N>(own(i, j)), mpd::load<N>(sdot + i * esz), -1);
+      const Val<N> t = mpd::addsub<N>(mpd::load<N>(own(i, j)), mpd::unstage<N>(sdot + i * esz), -1);
       const Val<N> v = mpd::mul<N>(t, di);
       mpd::store<N>(rm(R, i, j), v, status);
       if (kRows) mpd::store<N>(own(i, j), v, status);

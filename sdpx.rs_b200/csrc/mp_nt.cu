@@ -68,14 +68,14 @@ __device__ void chol_group(unsigned char* L, int n, int t, int nt, int bar, unsi
     } else {
       for (int i = j + 1 + (t - 32) / G; i < n; i += (nt - 32) / G) {  // group-uniform
         const Val<N> dot = mpd::dot<N, G>(nullptr, at(i, 0), n, at(j, 0), n, j, &ok);
-        if ((t & (G - 1)) == 0) mpd::store<N>(sdot + i * esz, dot, status);
+        if ((t & (G - 1)) == 0) mpd::stage<N>(sdot + i * esz, dot);
       }
     }
     named_sync(bar, nt);
     if (*fail) break;
     if (t < n - 1 - j) {
       const int i = j + 1 + t;
-      const Val<N> d = mpd::addsub<N>(mpd::load<N>(at(i, j)), mpd::load<N>(sdot + i * esz), -1);
+      const Val<N> d = mpd::addsub<N>(mpd::load<N>(at(i, j)), mpd::unstage<N>(sdot + i * esz), -1);
       mpd::store<N>(at(i, j), mpd::divide<N>(d, mpd::load<N>(sd)), status);
     }
     named_sync(bar, nt);
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kNtThreads<N>) k_mp_nt_scale(const MpNtBlock* 
     for (int e = t; e < P * n; e += nt) {
       const int k = e / n, i = e % n, p = spair[buf][2 * k], q = spair[buf][2 * k + 1];
       if (p < 0) continue;
-      const Val<N> c = mpd::load<N>(srot[buf] + 2 * k * esz), sn = mpd::load<N>(srot[buf] + (2 * k + 1) * esz);
+      const Val<N> c = mpd::unstage<N>(srot[buf] + 2 * k * esz), sn = mpd::unstage<N>(srot[buf] + (2 * k + 1) * esz);
       unsigned char* xp = el(M2, i + (long)p * n);
       unsigned char* xq = el(M2, i + (long)q * n);
       const Val<N> vp = mpd::load<N>(xp), vq = mpd::load<N>(xq);
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kNtThreads<N>) k_mp_nt_scale(const MpNtBlock* 
         if (!round_pair(d / 3, r, mm, n, &p, &q)) continue;
         const int x = d % 3 == 1 ? q : p, y = d % 3 == 0 ? p : q;  // (p, p), (q, q), (p, q)
         const Val<N> v = mpd::dot<N, LG>(nullptr, el(A, (long)x * n), 1, el(A, (long)y * n), 1, n, &ok);
-        if ((tid & (LG - 1)) == 0) mpd::store<N>(ssum + d * esz, v, status);
+        if ((tid & (LG - 1)) == 0) mpd::stage<N>(ssum + d * esz, v);
       }
       __syncthreads();
       if (tid < 32) {
@@ -257,13 +257,13 @@ __global__ void __launch_bounds__(kNtThreads<N>) k_mp_nt_scale(const MpNtBlock* 
           Val<N> c, sn;
           bool rot = round_pair(tid, r, mm, n, &p, &q);
           if (rot)
-            rot = rotation<N>(mpd::load<N>(ssum + 3 * tid * esz), mpd::load<N>(ssum + (3 * tid + 1) * esz),
-                              mpd::load<N>(ssum + (3 * tid + 2) * esz), c, sn);
+            rot = rotation<N>(mpd::unstage<N>(ssum + 3 * tid * esz), mpd::unstage<N>(ssum + (3 * tid + 1) * esz),
+                              mpd::unstage<N>(ssum + (3 * tid + 2) * esz), c, sn);
           spair[cur][2 * tid] = rot ? p : -1;
           spair[cur][2 * tid + 1] = q;
           if (rot) {
-            mpd::store<N>(srot[cur] + 2 * tid * esz, c, status);
-            mpd::store<N>(srot[cur] + (2 * tid + 1) * esz, sn, status);
+            mpd::stage<N>(srot[cur] + 2 * tid * esz, c);
+            mpd::stage<N>(srot[cur] + (2 * tid + 1) * esz, sn);
             atomicAdd(&rotated, 1);
           }
         }
