@@ -387,13 +387,16 @@ __device__ inline void cta_tridiagonalize(const double* A, int n, double* d, dou
 
 // The tridiagonal (d, e) made ready for the Sturm sequences: t[i] = (d_i, e_{i-1}^2) times a power of
 // two (its square) that brings the Gershgorin interval to about one, e^2 at least 2^-200 (a perturbation
-// of 2^-100 relative to the norm keeps every sequence from stopping at zero), padded to a multiple of
-// eight rows with (4, 0), which change no sign.  Returns the interval in the scaled units and, in
-// *unscale, the factor back.  `t` is 16-byte aligned shared memory, SDPXG_STURM_WORK doubles.
-// False (in every thread) for a (d, e) with a NaN or an infinity, which minima, maxima and sign tests
-// would pass over.
-__device__ inline bool sturm_prepare(const double* d, const double* e, int n, double2* t, double* lo, double* hi,
-                                     double* unscale) {
+// of 2^-100 relative to the norm keeps every sequence from stopping at zero; `raised` when there is one),
+// padded to a multiple of eight rows with (4, 0), which change no sign.  lo and hi: the interval in the
+// scaled units.  `t` is 16-byte aligned shared memory, SDPXG_STURM_WORK doubles.  The same in every thread.
+// `finite` is false for a (d, e) with a NaN or an infinity, which minima, maxima and sign tests would pass
+// over.
+struct SturmRange {
+  double lo, hi, scale, unscale;
+  bool finite, raised;
+};
+__device__ inline SturmRange sturm_prepare(const double* d, const double* e, int n, double2* t) {
   const int lane = threadIdx.x & 31;
   double l = 1e300, h = -1e300;
   bool fin = true;
@@ -403,7 +406,6 @@ __device__ inline bool sturm_prepare(const double* d, const double* e, int n, do
     l = fmin(l, d[i] - r);
     h = fmax(h, d[i] + r);
   }
-  fin = __all_sync(0xffffffffu, fin);
   l = -warp_max(-l);
   h = warp_max(h);
   const double span = fmax(fabs(l), fabs(h));
@@ -411,17 +413,41 @@ __device__ inline bool sturm_prepare(const double* d, const double* e, int n, do
   h += 2.0 * 2.220446049250313e-16 * span;
   int ex = 0;
   if (span > 0.0 && isfinite(span)) ex = max(-1000, min(1000, ilogb(span) + 1));
-  const double s = ldexp(1.0, -ex);
-  *unscale = ldexp(1.0, ex);
-  *lo = l * s - 0x1p-200;
-  *hi = h * s + 0x1p-200;
+  SturmRange r;
+  r.scale = ldexp(1.0, -ex);
+  r.unscale = ldexp(1.0, ex);
+  r.lo = l * r.scale - 0x1p-200;
+  r.hi = h * r.scale + 0x1p-200;
+  bool small = false;
+  for (int i = lane; i + 1 < n; i += 32) small = small || fabs(e[i]) * r.scale < 0x1p-100;
+  r.finite = __all_sync(0xffffffffu, fin);
+  r.raised = __any_sync(0xffffffffu, small);
   const int np = (n + 7) & ~7;
   for (int i = threadIdx.x; i < np; i += blockDim.x) {
-    const double v = (i > 0 && i < n) ? e[i - 1] * s : 0.0;
-    t[i] = i < n ? make_double2(d[i] * s, fmax(v * v, 0x1p-200)) : make_double2(4.0, 0.0);
+    const double v = (i > 0 && i < n) ? e[i - 1] * r.scale : 0.0;
+    t[i] = i < n ? make_double2(d[i] * r.scale, fmax(v * v, 0x1p-200)) : make_double2(4.0, 0.0);
   }
   __syncthreads();
-  return fin;
+  return r;
+}
+
+// An eigenvalue x (scaled units) that the raised e^2 may have moved by more than a rounding: they move it
+// by up to 2^-99.  It is found again by quotients, from e^2 as it is, and to kSturmFine.
+constexpr double kSturmCoarse = 0x1p-200, kSturmFine = 0x1p-250;  // brackets of an eigenvalue zero end here
+__device__ __forceinline__ bool sturm_again(const SturmRange& r, double x) { return r.raised && fabs(x) < 0x1p-46; }
+
+// Eigenvalues of the tridiagonal below x / s by the quotients q_i = d_i - x - e_{i-1}^2 / q_{i-1}, |q_i| at
+// least the smallest normal number.
+static __device__ __noinline__ int sturm_quotients(const double* d, const double* e, int n, double s, double x) {
+  int cnt = 0;
+  double q = 1.0;
+  for (int i = 0; i < n; ++i) {
+    const double v = i > 0 ? e[i - 1] * s : 0.0;
+    q = (d[i] * s - x) - v * v / q;
+    if (fabs(q) < 0x1p-1022) q = -0x1p-1022;
+    cnt += q < 0.0;
+  }
+  return cnt;
 }
 
 // The leading principal minors of T - x for the tridiagonal prepared by sturm_prepare, p_i = (d_i - x)
@@ -460,28 +486,26 @@ __device__ __forceinline__ int sturm(const double2* t, int n, double x) {
   return COUNT ? cnt : (int)((unsigned)cnt >> 31);
 }
 
-// Smallest eigenvalue of the tridiagonal (d, e) by CTA-wide multisection: each round every thread
-// evaluates one Sturm sequence on an even grid over the current bracket and the bracket shrinks to the
-// first grid cell holding an eigenvalue.  With 256 threads a round is bound by the sequence's chain
-// and gives 8 bits; with 512 it is bound by issue and gives 9.
-// An eigenvalue is resolved relative to itself, down to 2^-200 of the norm: at most 26 rounds.
-// Uniform result; `best` is one int of shared memory, `t` SDPXG_STURM_WORK doubles.
-// *ok = false if the round bound is hit or (d, e) is not finite.
-__device__ inline double cta_eig_min(const double* d, const double* e, int n, double2* t, int* best, bool* ok) {
-  double lo, hi, unscale;
-  *ok = false;
-  if (!sturm_prepare(d, e, n, t, &lo, &hi, &unscale)) return 0.0;
+// Smallest eigenvalue in scaled units by CTA-wide multisection: each round every thread evaluates one
+// Sturm sequence on an even grid over the current bracket and the bracket shrinks to the first grid cell
+// holding an eigenvalue.  With 256 threads a round is bound by the sequence's chain and gives 8 bits; with
+// 512 it is bound by issue and gives 9.  *ok = false if the round bound is hit.
+template <bool QUOTIENTS>
+__device__ __forceinline__ double multisect_min(const double* d, const double* e, int n, const double2* t,
+                                                const SturmRange& r, int* best, bool* ok) {
   const int T = blockDim.x;
+  double lo = r.lo, hi = r.hi;
   for (int round = 0; round < 40; ++round) {
-    if (!(hi - lo > 2.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + 0x1p-200)) {
+    if (!(hi - lo > 2.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + (QUOTIENTS ? kSturmFine : kSturmCoarse))) {
       *ok = true;
-      return 0.5 * (lo + hi) * unscale;
+      return 0.5 * (lo + hi);
     }
     const double step = (hi - lo) / (T + 1);
     if (threadIdx.x == 0) *best = T;
     __syncthreads();
     const double x = lo + step * (threadIdx.x + 1);
-    const unsigned bal = __ballot_sync(0xffffffffu, x > lo && x < hi && sturm<false>(t, n, x));
+    const unsigned bal = __ballot_sync(0xffffffffu, x > lo && x < hi &&
+                                       (QUOTIENTS ? sturm_quotients(d, e, n, r.scale, x) : sturm<false>(t, n, x)));
     if (bal && (threadIdx.x & 31) == 0) atomicMin(best, (int)threadIdx.x + __ffs(bal) - 1);
     __syncthreads();
     const int b = *best;
@@ -491,42 +515,74 @@ __device__ inline double cta_eig_min(const double* d, const double* e, int n, do
     lo = nlo;
     hi = nhi;
   }
-  return 0.5 * (lo + hi) * unscale;
+  *ok = false;
+  return 0.5 * (lo + hi);
+}
+static __device__ __noinline__ double multisect_min_again(const double* d, const double* e, int n, SturmRange r,
+                                                          int* best, bool* ok) {
+  return multisect_min<true>(d, e, n, nullptr, r, best, ok);
+}
+
+// Smallest eigenvalue of the tridiagonal (d, e), resolved relative to itself down to about 2^-200 of the
+// norm: at most 26 rounds, and 32 more by quotients.  Uniform result; `best` is one int of shared memory, `t`
+// SDPXG_STURM_WORK doubles.  *ok = false if the round bound is hit or (d, e) is not finite.
+__device__ inline double cta_eig_min(const double* d, const double* e, int n, double2* t, int* best, bool* ok) {
+  const SturmRange r = sturm_prepare(d, e, n, t);
+  *ok = false;
+  if (!r.finite) return 0.0;
+  double x = multisect_min<false>(d, e, n, t, r, best, ok);
+  if (*ok && sturm_again(r, x)) x = multisect_min_again(d, e, n, r, best, ok);
+  return x * r.unscale;
+}
+
+// Eigenvalue k in scaled units by the 16 lanes of a group (lane sl, the warp's lanes from `base` on):
+// multisection with 15 Sturm counts per round (the bracket shrinks 16-fold per round).
+template <bool QUOTIENTS>
+__device__ __forceinline__ double multisect_kth(const double* d, const double* e, int n, const double2* t,
+                                                const SturmRange& r, int k, bool* ok) {
+  constexpr int P = 16;
+  const int sl = threadIdx.x % P, base = threadIdx.x & 16;
+  const unsigned gmask = 0xFFFFu << base;
+  double lo = r.lo, hi = r.hi;
+  for (int round = 0; round < 64; ++round) {
+    if (!(hi - lo > 2.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + (QUOTIENTS ? kSturmFine : kSturmCoarse))) {
+      *ok = true;
+      return 0.5 * (lo + hi);
+    }
+    const double step = (hi - lo) / P;
+    const double x = lo + step * (sl + 1);
+    const bool above = (sl < P - 1) && x > lo && x < hi &&
+                       (QUOTIENTS ? sturm_quotients(d, e, n, r.scale, x) : sturm<true>(t, n, x)) > k;
+    const unsigned bal = (__ballot_sync(gmask, above) >> base) & 0xFFFFu;
+    const int c = bal ? __ffs(bal) - 1 : P - 1;  // eigenvalue k lies in cell c
+    const double nlo = (c == 0) ? lo : lo + step * c;
+    const double nhi = (c == P - 1) ? hi : lo + step * (c + 1);
+    lo = nlo;
+    hi = nhi;
+  }
+  *ok = false;
+  return 0.5 * (lo + hi);
+}
+static __device__ __noinline__ double multisect_kth_again(const double* d, const double* e, int n, SturmRange r, int k,
+                                                          bool* ok) {
+  return multisect_kth<true>(d, e, n, nullptr, r, k, ok);
 }
 
 // Every eigenvalue of the tridiagonal (d, e), ascending, into eig[0..n): 16-lane groups, one
-// eigenvalue per group, multisection with 15 Sturm counts per round (the bracket shrinks 16-fold per
-// round), no CTA barrier inside.  `t`: SDPXG_STURM_WORK doubles.
+// eigenvalue per group, no CTA barrier inside.  `t`: SDPXG_STURM_WORK doubles.
 // Sets the status bit SDPXG_ST_EIG_FAIL for an eigenvalue whose round bound was hit and for a (d, e) that
 // is not finite.
 __device__ inline void cta_eig_all(const double* d, const double* e, int n, double2* t, double* eig,
                                    uint32_t* status) {
-  double lo0, hi0, unscale;
-  if (!sturm_prepare(d, e, n, t, &lo0, &hi0, &unscale) && threadIdx.x == 0) atomicOr(status, SDPXG_ST_EIG_FAIL);
-  constexpr int P = 16;
-  const int grp = threadIdx.x / P, sl = threadIdx.x % P, base = threadIdx.x & 16;
-  const unsigned gmask = 0xFFFFu << base;
-  for (int k = grp; k < n; k += blockDim.x / P) {
-    double lo = lo0, hi = hi0;
-    bool conv = false;
-    for (int round = 0; round < 64; ++round) {
-      if (!(hi - lo > 2.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + 0x1p-200)) {
-        conv = true;
-        break;
-      }
-      const double step = (hi - lo) / P;
-      const double x = lo + step * (sl + 1);
-      const bool above = (sl < P - 1) && x > lo && x < hi && sturm<true>(t, n, x) > k;
-      const unsigned bal = (__ballot_sync(gmask, above) >> base) & 0xFFFFu;
-      const int c = bal ? __ffs(bal) - 1 : P - 1;  // eigenvalue k lies in cell c
-      const double nlo = (c == 0) ? lo : lo + step * c;
-      const double nhi = (c == P - 1) ? hi : lo + step * (c + 1);
-      lo = nlo;
-      hi = nhi;
-    }
-    if (sl == 0) {
-      eig[k] = 0.5 * (lo + hi) * unscale;
-      if (!conv) atomicOr(status, SDPXG_ST_EIG_FAIL);
+  const SturmRange r = sturm_prepare(d, e, n, t);
+  if (!r.finite && threadIdx.x == 0) atomicOr(status, SDPXG_ST_EIG_FAIL);
+  for (int k = threadIdx.x / 16; k < n; k += blockDim.x / 16) {
+    bool ok;
+    double x = multisect_kth<false>(d, e, n, t, r, k, &ok);
+    if (ok && sturm_again(r, x)) x = multisect_kth_again(d, e, n, r, k, &ok);
+    if (threadIdx.x % 16 == 0) {
+      eig[k] = x * r.unscale;
+      if (!ok) atomicOr(status, SDPXG_ST_EIG_FAIL);
     }
   }
 }

@@ -104,3 +104,28 @@ def test_a_matrix_that_is_not_finite_is_reported(device, n, value):
     X[n - 1, n // 2] = X[n // 2, n - 1] = value
     _, _, ok, st = run(device, X)
     assert not ok and st != 0
+
+
+@pytest.mark.parametrize("n", [2, 3, 4, 9, 17, 33, 64])
+@pytest.mark.parametrize("size", [1e-18, 1e-30, 1e-40, 1e-55])
+@pytest.mark.parametrize("kind", ["diagonal", "block"])
+def test_eigenvalues_far_below_the_norm(device, kind, size, n):
+    """A small block beside a large entry, without coupling: its eigenvalues are found to their own rounding
+    (8 n eps of the block's norm), wherever the block stands."""
+    rng = np.random.default_rng(n)
+    B = np.diag(np.r_[1.0, 1.0, rng.uniform(1.0, 2.0, n)][:n - 1])
+    if kind == "block":
+        B = rng.standard_normal((n - 1, n - 1))
+        B = B @ B.T + np.eye(n - 1)
+    for at in (0, n - 1):
+        for sign in (1.0, -1.0):
+            X = np.zeros((n, n))
+            X[at, at] = 1.0
+            keep = np.arange(n) != at
+            X[np.ix_(keep, keep)] = sign * size * B
+            w = sign * size * np.linalg.eigvalsh(B)
+            rows, low, ok, st = run(device, X)
+            assert ok and st == 0
+            got = np.sort(rows[2, :n])[:-1]
+            bound = 8 * n * EPS * size * np.linalg.norm(B, 2)
+            assert np.max(np.abs(got - np.sort(w))) <= bound and abs(low - np.min(w)) <= bound
