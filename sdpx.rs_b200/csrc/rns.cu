@@ -48,6 +48,7 @@
 #include <vector>
 
 #include "../../include/sdpx_b200.h"
+#include "crt_widths.cuh"
 #include "engine.cuh"
 #include "i8_gemm.cuh"
 #include "mp.cuh"
@@ -63,7 +64,7 @@ std::shared_ptr<void>* ctx_rns_slot(sdpxg_ctx* c);
 
 #define RNS_MAXN 16    // limbs: up to 1024-bit values
 #define RNS_MAXL 256   // primes (products of four 768-bit factors need about 220 of 15 bits)
-#define RNS_MAXW 64    // 64-bit words of the reconstructed integer
+#define RNS_MAXW sdpxg::kCrtMaxWords  // 64-bit words of the reconstructed integer
 #define RNS_KC 8192    // exact FP64 terms between two reductions modulo the prime
 #define MP_ZERO 2
 #define MP_REGULAR 3
@@ -559,12 +560,16 @@ void launch_crt_f64(unsigned blocks, cudaStream_t st, const double* RC, long pla
                     const uint32_t* primes, const uint32_t* wt, const double* pinv, const unsigned long long* mu,
                     const unsigned long long* MT, const unsigned long long* Mbig, const int* loA, const int* loB,
                     int N, int upper_only, unsigned char* C, uint32_t* status) {
-  if (WW <= 16)
-    k_rns_crt_f64<16><<<blocks, 128, 0, st>>>(RC, planeC, m, n, L, WW, primes, wt, pinv, mu, MT, Mbig, loA, loB, N,
-                                              upper_only, C, status);
-  else
-    k_rns_crt_f64<RNS_MAXW><<<blocks, 128, 0, st>>>(RC, planeC, m, n, L, WW, primes, wt, pinv, mu, MT, Mbig, loA, loB,
-                                                    N, upper_only, C, status);
+  auto go = [&](auto kernel) {
+    kernel<<<blocks, 128, 0, st>>>(RC, planeC, m, n, L, WW, primes, wt, pinv, mu, MT, Mbig, loA, loB, N, upper_only, C,
+                                   status);
+  };
+  switch (crt_f64_words(WW)) {
+    case 8: go(k_rns_crt_f64<8>); break;
+    case 16: go(k_rns_crt_f64<16>); break;
+    case 32: go(k_rns_crt_f64<32>); break;
+    default: go(k_rns_crt_f64<RNS_MAXW>);
+  }
 }
 
 // INT8 form: one entry of a pair's table row.  Primes are taken two at a time:
