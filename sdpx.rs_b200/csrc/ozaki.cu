@@ -61,7 +61,7 @@ constexpr OzTables oz_tables() {
   return T;
 }
 __constant__ OzTables kOz = oz_tables();
-constexpr float kOzLead = 1.0f / (float)oz_tables().P[3];  // 2^96 / P to 2^-24 and the limb's 2^-30
+constexpr double kOzLead = 1.0 / ((double)oz_tables().P[3] + (double)oz_tables().P[2] * 0x1p-32);  // 2^96 / P
 
 double log2_product() {
   double s = 0;
@@ -246,8 +246,9 @@ __global__ void __launch_bounds__(256) k_oz_crt(const int8_t* __restrict__ PC, l
       s3 += (unsigned long long)z * kOz.W[g][3];
     }
     if (upper_only && i > j) continue;
-    const float lead = (float)(s3 + (s2 >> 32));  // sum / 2^96, below 2^36
-    const uint32_t k = (uint32_t)(lead * kOzLead + 0.5f);
+    const unsigned long long top = s3 + (s2 >> 32);  // sum / 2^96, below 2^36; its double without a conversion
+    const double lead = __hiloint2double(0x43300000 | (int)(top >> 32), (int)top) - 0x1p52;
+    const uint32_t k = (uint32_t)__double2loint(fma(lead, kOzLead, 0x1.8p52));  // rounded to the nearest
     // differences of less than 2^62 in each limb; arithmetic carries
     const long long d0 = (long long)(s0 - (unsigned long long)k * kOz.P[0]);
     const long long d1 = (long long)(s1 - (unsigned long long)k * kOz.P[1]) + (d0 >> 32);

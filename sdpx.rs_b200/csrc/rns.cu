@@ -404,8 +404,8 @@ __device__ __forceinline__ unsigned long long word_at(const unsigned long long (
 // With M = prod p_t, M_t = M / p_t and w_t = M_t^-1 mod p_t: c_t = r_t w_t mod p_t,
 // S = sum_t c_t M_t (exact), f = sum_t c_t / p_t, and the signed integer is X = S - rint(f) M.  The
 // prime set covers more than twice the largest |X| plus a margin (|X| < M / 4), so S / M = f
-// sits within 1/4 of an integer and the error of f in floating point (below L^2 2^-24 in FP32)
-// cannot move rint(f); X is then exact.
+// sits within 1/4 of an integer and FP64's error in f (below L^2 2^-53) cannot move rint(f); X is
+// then exact.
 //
 // FP64 form (exact integers |r| < 2^53 of either sign, primes below 2^21): S in 32-bit digits, one
 // 64-bit accumulator each (c < 2^21 times a 32-bit digit is below 2^53, so up to 2^11 primes sum
@@ -579,9 +579,8 @@ void launch_crt_f64(unsigned blocks, cudaStream_t st, const double* RC, long pla
 constexpr int kCrtBits = 26;
 struct CrtPair {
   uint32_t p1, p2;  // an odd set's last prime has p2 = 1 and no second residue
-  float inv;        // 1 / (p1 p2)
+  double inv;       // 1 / (p1 p2)
   uint32_t w1, w2;  // CRT weights, for residues that do not carry them
-  uint32_t pad;
   unsigned long long mu1, mu2;  // Barrett constants of p1, p2
 };
 
@@ -614,7 +613,7 @@ __global__ void __launch_bounds__(128) k_rns_crt(const int* __restrict__ RC, lon
   unsigned long long acc[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) acc[d] = 0ull;
-  float f = 0.f;
+  double f = 0.0;
   const int np = (L + 1) >> 1;
 #pragma unroll 1
   for (int t = 0; t < np; ++t) {
@@ -626,7 +625,7 @@ __global__ void __launch_bounds__(128) k_rns_crt(const int* __restrict__ RC, lon
       if (c2) c2 = modb((unsigned long long)c2 * pr.w2, pr.p2, pr.mu2);
     }
     const uint32_t c = c1 * pr.p2 + c2 * pr.p1;
-    f = fmaf((float)c, pr.inv, f);
+    f = fma(__hiloint2double(0x43300000, (int)c) - 0x1p52, pr.inv, f);  // (double)c without a conversion
     const uint4* row = reinterpret_cast<const uint4*>(rows + (size_t)t * D);
 #pragma unroll
     for (int d = 0; d < D; d += 4) {
@@ -653,7 +652,7 @@ __global__ void __launch_bounds__(128) k_rns_crt(const int* __restrict__ RC, lon
     }
   }
   {  // S -= k M (two's complement over K words; |X| < M / 4 fits with room for the sign)
-    const uint32_t k = (uint32_t)__float2int_rn(f);
+    const uint32_t k = (uint32_t)__double2int_rn(f);
     long long carry = 0;
 #pragma unroll
     for (int w = 0; w < K; ++w) {
@@ -950,10 +949,9 @@ PrimeTables make_tables(const std::vector<uint32_t>& ps, int L) {
     const int t1 = 2 * j, t2 = 2 * j + 1;
     c.p1 = T.primes[t1];
     c.p2 = t2 < L ? T.primes[t2] : 1u;
-    c.inv = (float)(1.0 / ((double)c.p1 * c.p2));
+    c.inv = 1.0 / ((double)c.p1 * c.p2);
     c.w1 = T.wt[t1];
     c.w2 = t2 < L ? T.wt[t2] : 0u;
-    c.pad = 0;
     c.mu1 = T.mu[t1];
     c.mu2 = t2 < L ? T.mu[t2] : 0ull;
     std::vector<unsigned long long> x(T.MT.begin() + (size_t)t1 * T.WW, T.MT.begin() + (size_t)(t1 + 1) * T.WW);
