@@ -182,15 +182,6 @@ __device__ __forceinline__ void df_sub_ab(const double* As, const double* Bs, do
   }
 }
 
-// 1/sqrt(d) for d in [2^-1000, 2^1000]: the hardware approximation y (about 2^-22 off) and one
-// Householder step of third order, y (1 + e/2 + 3 e^2 / 8) with e = 1 - d y^2: within an ulp or two.
-__device__ __forceinline__ double df_rsqrt(double d) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double e = fma(-d * y, y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
 // The packed upper triangle u of an 8 x 8 block factored in place, v <- U^-T v.  Returns false (u
 // and v then unusable) when a pivot does not lie in (floor, 2^1000].
 __device__ __forceinline__ bool df_factor8(double (&u)[36], double (&v)[8], double floor) {
@@ -199,7 +190,7 @@ __device__ __forceinline__ bool df_factor8(double (&u)[36], double (&v)[8], doub
   for (int kk = 0; kk < 8; ++kk) {
     const double d = u[kk * (kk + 3) / 2];
     ok = ok && d > floor && d <= 0x1p1000;
-    const double ri = df_rsqrt(d);
+    const double ri = rsqrt_mid(d);
     u[kk * (kk + 3) / 2] = d * ri;
 #pragma unroll
     for (int j = kk + 1; j < 8; ++j) u[j * (j + 1) / 2 + kk] *= ri;  // row kk of U

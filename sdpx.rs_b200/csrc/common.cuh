@@ -285,8 +285,8 @@ __device__ __forceinline__ bool mid_range(double v) {
 }
 
 // 1/v for v in the mid range: the hardware approximation refined by two Newton-Raphson steps
-// y <- y + y (1 - v y) (each doubles the correct bits; the result is within a few units in the
-// last place of 1/v).
+// y <- y + y (1 - v y) (each doubles the correct bits; the error left is the last step's rounding, 2^-53
+// relative).
 __device__ __forceinline__ double recip_mid(double v) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
@@ -296,8 +296,9 @@ __device__ __forceinline__ double recip_mid(double v) {
   return fma(y, e, y);
 }
 
-// 1/sqrt(v) for v in the mid range: the hardware approximation y (about 22 bits) and one Householder
-// step of third order, y (1 + e/2 + 3 e^2 / 8) with e = 1 - v y^2.
+// 1/sqrt(v) for v in the mid range (and 2^1000): the hardware approximation y (about 22 bits) and one
+// Householder step of third order, y (1 + e/2 + 3 e^2 / 8) with e = 1 - v y^2.  The step leaves e^3; the rounding
+// of v y moves the result by half of 2^-53, that of the last operation by 2^-53.
 __device__ __forceinline__ double rsqrt_mid(double v) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(v));
