@@ -120,29 +120,31 @@ __device__ void refine_outer_step(const double* v, RefineCtl* c, const RefinePar
 // condition, and after an inner step the block keeps the candidate and its residual (n entries).
 // A graph node costs about 3 us here whatever it computes, and a refined solve of a small system is
 // little else: norms, control and copy were three nodes each time.
+// Both kinds of request are a maximum of unsigned integers: a magnitude's bits (max_nan), or 1 for an entry
+// that is not finite.  The copy has eight loads of each vector in flight a thread: 2048 entries a memory round
+// trip, so that one block is enough beside the matrix products of a step.
 extern "C" __global__ void __launch_bounds__(256)
 k_refine(RedBatch b, double* __restrict__ partial, unsigned* __restrict__ ticket, int pitch, RefineOp op,
          RefineCtl* c, RefineParams p, cudaGraphConditionalHandle h) {
-  __shared__ double red[8];
+  typedef unsigned long long u64;
+  __shared__ u64 red[8];
   __shared__ double val[kRedBatchMax];
   __shared__ int last, keep[2];
   const RedReq q = b.r[blockIdx.y];
   const bool fin = q.op == 3;  // RED_FINITE, else RED_MAXABS
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double acc = fin ? 1.0 : 0.0;
+  u64* part = reinterpret_cast<u64*>(partial);
+  u64 acc = 0;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < q.n; i += (long)gridDim.x * blockDim.x) {
-    const double v = q.x[i];
-    acc = fin ? fmin(acc, isfinite(v) ? 1.0 : 0.0) : max_nan(acc, fabs(v));
+    const u64 v = (u64)__double_as_longlong(q.x[i]) & ~(1ull << 63);
+    acc = max(acc, fin ? (u64)(v >= 0x7ff0000000000000ull) : v);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double v = __shfl_xor_sync(0xffffffffu, acc, o);
-    acc = fin ? fmin(acc, v) : max_nan(acc, v);
-  }
+  for (int o = 16; o > 0; o >>= 1) acc = max(acc, __shfl_xor_sync(0xffffffffu, acc, o));
   if (lane == 0) red[warp] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) acc = fin ? fmin(acc, red[w]) : max_nan(acc, red[w]);
-    partial[blockIdx.y * pitch + blockIdx.x] = acc;
+    for (int w = 1; w < 8; ++w) acc = max(acc, red[w]);
+    part[blockIdx.y * pitch + blockIdx.x] = acc;
     __threadfence();
     last = atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1;
   }
@@ -150,17 +152,10 @@ k_refine(RedBatch b, double* __restrict__ partial, unsigned* __restrict__ ticket
   if (!last) return;
   __threadfence();
   for (int r = warp; r < op.rows; r += 8) {
-    const bool f = b.r[r].op == 3;
-    double v = f ? 1.0 : 0.0;
-    for (int k = lane; k < (int)gridDim.x; k += 32) {
-      const double u = __ldcg(partial + r * pitch + k);
-      v = f ? fmin(v, u) : max_nan(v, u);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const double u = __shfl_xor_sync(0xffffffffu, v, o);
-      v = f ? fmin(v, u) : max_nan(v, u);
-    }
-    if (lane == 0) val[r] = v;
+    u64 v = 0;
+    for (int k = lane; k < (int)gridDim.x; k += 32) v = max(v, __ldcg(part + r * pitch + k));
+    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (lane == 0) val[r] = b.r[r].op == 3 ? (v ? 0.0 : 1.0) : __longlong_as_double((long long)v);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -173,10 +168,23 @@ k_refine(RedBatch b, double* __restrict__ partial, unsigned* __restrict__ ticket
     keep[1] = op.kind == REFINE_STEP && c->cont;
   }
   __syncthreads();
-  if (keep[0])
-    for (long i = threadIdx.x; i < op.n; i += blockDim.x) op.x[i] = op.cand[i];
-  if (keep[1])
-    for (long i = threadIdx.x; i < op.n; i += blockDim.x) op.e[i] = op.e2[i];
+  const bool k0 = keep[0], k1 = keep[1];
+  if (!k0 && !k1) return;
+  for (long i0 = threadIdx.x; i0 < op.n; i0 += 8 * 256) {
+    double y[8], f[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const bool in = i0 + 256 * u < op.n;
+      y[u] = in && k0 ? op.cand[i0 + 256 * u] : 0.0;
+      f[u] = in && k1 ? op.e2[i0 + 256 * u] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const bool in = i0 + 256 * u < op.n;
+      if (in && k0) op.x[i0 + 256 * u] = y[u];
+      if (in && k1) op.e[i0 + 256 * u] = f[u];
+    }
+  }
 }
 
 // After an outer step: x1 <- y1 (n entries) and x2 <- y2 (m) when the candidate is kept, e1 <- f1 and
