@@ -44,7 +44,11 @@ constexpr size_t kSmemTrinv = 4 * 64 * 68 * sizeof(double);  // k_trinv_level: 2
 constexpr size_t kSmemDf = (4 * 64 * 68 + 2 * 64) * sizeof(double);  // k_chol_dataflow
 constexpr size_t kSmemGram = 3 * kMatD * sizeof(double);                 // k_gram_basis/adjoint
 constexpr int kDfThreads = 320;    // k_chol_dataflow: 8 MMA warps, one loading, one publishing
-constexpr int kDfMaxTiles = 256;  // dataflow schedule up to m = 16384 (nt^3/6 items)
+// Dataflow launch up to m = 16384 (about nt^2 items); SDPX_B200_DATAFLOW_TILES at prepare moves the line, 0
+// takes every factorisation through the launches per tile row.  The line is where sizes in use end, not
+// where the launch loses: factor and inverse, dataflow / launches per row, m = 4000 2.1 / 8.7 ms, 8001 15.2 /
+// 36.0, 16384 121 / 227, 16449 125 / 230.
+constexpr int kDfMaxTiles = 256;
 
 // Rank-one test of one PSD column block: svec v (upper, column order, off-diagonal x sqrt2) of
 // an n x n matrix M.  On success M = sigma u u' entrywise to a few ulps (32 eps relative to
@@ -273,6 +277,7 @@ class Engine {
   int nchol = 0;  // Schur tiles per side
   int factor_form = kFormPlain;  // SDPX_B200_FORM=split or sdpx_b200_set_form
   OzakiWorkspace oz;             // split-precision GEMM scratch
+  int df_max_tiles = kDfMaxTiles;
   bool split_active() const { return factor_form == kFormSplit && n >= kSplitMin; }
   bool gram_enabled = true;  // rank-one blocks use the Gram form (SDPX_B200_GRAM=0 disables)
   int gram_blocks() const { return ngram_; }
@@ -449,6 +454,8 @@ class Engine {
       graphs_enabled = !(c && c[0] == '0');
       const char* f = std::getenv("SDPX_B200_FORM");  // "split": split-precision factorisation
       factor_form = (f && std::string(f) == "split") ? kFormSplit : kFormPlain;
+      const char* d = std::getenv("SDPX_B200_DATAFLOW_TILES");  // a work list numbers 1023 tiles
+      if (d) df_max_tiles = std::max(0, std::min(1023, std::atoi(d)));
     }
     red.init();
     status_.alloc(1);
@@ -1131,7 +1138,7 @@ class Engine {
   void make_schedule(int nt, DevBuf<unsigned>& list, DevBuf<int>& sync, int* items_out, int* grid_out) {
     *items_out = 0;
     *grid_out = 0;
-    if (nt <= 0 || nt > kDfMaxTiles) return;
+    if (nt <= 0 || nt > df_max_tiles) return;
     std::vector<unsigned> items = chol_schedule(nt);
     if (!chol_schedule_valid(items, nt)) throw CudaError("invalid Cholesky work list");
     list.alloc(items.size());
