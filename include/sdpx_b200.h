@@ -249,7 +249,7 @@ int32_t sdpxg_set_factor_form(sdpxg_ctx *ctx, uint32_t form);
 /* C = alpha op(A) op(B) + beta C in binary64 through split-precision products on the INT8 tensor
  * cores (Ozaki scheme II: rows of op(A) and columns of op(B) scaled by powers of two to integers
  * of b = 55..57 bits, residues modulo 16 coprime moduli <= 256, one tcgen05 kind::i8 GEMM per
- * modulus, Garner reconstruction in FP64).  DEVICE pointers, column-major, k <= 65536; returns
+ * modulus, reconstruction in 32-bit limbs, rounded to FP64 once).  DEVICE pointers, column-major, k <= 65536; returns
  * when C is complete; *status = SDPXG_ST_NONFINITE bit for non-finite inputs.  Replaces the f64
  * dgemm of the reference's BLAS provider on the dense factorisation's trailing updates
  * (algebra/dense/blas/traits.rs XgemmScalar, used by kkt/ldl/dense_block.rs:515-594). */

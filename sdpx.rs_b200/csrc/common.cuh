@@ -157,8 +157,7 @@ __device__ __forceinline__ void cta_zero_mat(double* M) {
 
 // M = smat(v): symmetric matrix from an svec (zero padded to 64 x 64).  Column j of the upper
 // triangle is contiguous in the svec (v[j(j+1)/2 + i], i <= j): one warp per column reads it
-// coalesced and writes both triangles.
-// M = smat(v), zero padded to 64 x 64: one warp a column, the loads of four columns in flight.
+// coalesced, the loads of four columns in flight, and writes both triangles.
 __device__ __forceinline__ void cta_load_smat(double* M, const double* __restrict__ v, int n) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   for (int j0 = warp; j0 < SDPXG_NMAX; j0 += 4 * nwarps) {

@@ -391,9 +391,9 @@ k_trinv_level(const double* __restrict__ F, long ldf, double* __restrict__ Uinv,
 // a triangle (tri 0: all rows, 1: rows <= c, 2: rows >= c; other entries are never read).  W warps of one
 // CTA share a pair of adjacent columns (they read v once for both), 16 matrix loads in flight a lane;
 // their sums meet in shared memory in warp order.  The longest columns of a triangle come first.
-// Bound by L2 (the matrices of a few thousand rows stay there) and, below that, by one memory round trip
-// and the launch.  W: as many warps as leave a lane at most 16 rows (one round of loads), and no more
-// than 4.  Two triangles and the full matrix in three launches, W = 1 / 2 / 4 / 8: n = 1000 12.5 / 12.6 /
+// Bound by L2 (the matrices of a few thousand rows stay there) and, below that, by two memory round trips
+// and the launch.  A round is eight rows of each column a lane.  W: as many warps as leave a lane at most 16
+// rows (two rounds), and no more than 4 (from n = 2049 on a lane has more rounds).  Two triangles and the full matrix in three launches, W = 1 / 2 / 4 / 8: n = 1000 12.5 / 12.6 /
 // 12.5 / 12.6 us, 2000 19.7 / 18.4 / 18.5 / 19.1, 3000 43 / 35 / 35 / 41, 4000 61 / 56 / 54 / 55; segments of
 // 256 rows as work units, combined through global memory by a ticket per column, took 18.7, 32, 64 and 100.
 template <int W>

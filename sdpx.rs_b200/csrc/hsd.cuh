@@ -87,7 +87,7 @@ class HsdSolver {
     auto vn = [&](DevBuf<double>& b) { b.alloc(std::max(n, 1)); };
     auto vm = [&](DevBuf<double>& b) { b.alloc(std::max(m, 1)); };
     for (auto* b : {&x_, &px_, &bx_, &rx_, &rxinf_, &Px_, &x2_, &dx_, &ax_, &tx_, &prevx_, &bestx_,
-                    &rhsx_, &x1_, &xhat_, &en_, &dxn_, &candn_, &e2n_, &ex_, &cx_, &candx_, &ex2_,
+                    &rhsx_, &x1_, &xhat_, &en_, &candn_, &e2n_, &ex_, &cx_, &candx_, &ex2_,
                     &negq_, &q_, &d_, &dinv_, &wn_})
       vn(*b);
     for (auto* b : {&s_, &z_, &ps_, &pz_, &rz_, &rzinf_, &z2_, &ds_, &dz_, &as_, &az_, &ts_, &tz_,
@@ -206,7 +206,7 @@ class HsdSolver {
   PinnedBuf<RefineCtl> hctl_;
   bool program_failed_ = false;  // building the device-driven solve failed once: host-driven
   DevBuf<double> x_, px_, bx_, rx_, rxinf_, Px_, x2_, dx_, ax_, tx_, prevx_, bestx_, rhsx_, x1_,
-      xhat_, en_, dxn_, candn_, e2n_, ex_, cx_, candx_, ex2_, negq_, q_, d_, dinv_, wn_;
+      xhat_, en_, candn_, e2n_, ex_, cx_, candx_, ex2_, negq_, q_, d_, dinv_, wn_;
   DevBuf<double> s_, z_, ps_, pz_, rz_, rzinf_, z2_, ds_, dz_, as_, az_, ts_, tz_, prevs_, prevz_,
       bests_, bestz_, rhsz_, rhss_, cvec_, workz_, z1_, tm_, ez_, cz_, candz_, ez2_, wm1_, wm2_, wm3_,
       b_, e_, einv_, nn_e_, nn_einv_;
