@@ -135,8 +135,9 @@ __device__ __forceinline__ double oz_pow2(int e) { return __hiloint2double((1023
 // A thread has four consecutive k of a line, so that a modulus costs one 4-byte store for the four.  A
 // residue is a dot product of the integer's bytes with 256^k mod p (two dp4a; 2^62 added first makes it
 // non-negative) and one reduction by a multiply-high: 24 instructions for four residues, where a byte
-// at a time with three reductions each had 60.  Bound by instruction issue: 4.2e6 entries took 92 us
-// and take 33.
+// at a time with three reductions each had 60.  4.2e6 entries took 92 us and take 33, with half of the issue
+// slots used: the staged planes leave three blocks an SM, whose warps wait for their lines and for the integer
+// pipes about equally.
 constexpr int kResPitch = 144;  // bytes per staged line (128 + 16: 16-byte aligned rows)
 __global__ void __launch_bounds__(256) k_oz_residues(const double* __restrict__ X, int rows, int K, long sr, long sk,
                                                      const unsigned long long* __restrict__ amax, int b,
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(256) k_oz_residues(const double* __restrict__ 
 // (y_0 p_1 p_2 + y_1 p_0 p_2 + y_2 p_0 p_1) P / (p_0 p_1 p_2), exact in 32-bit limbs, and k = round(sum / P)
 // from the leading bits (|X| <= P / 4 leaves the quotient a quarter from a tie); rounded to FP64 once.  A
 // thread has four consecutive entries of the planes (one 4-byte load a modulus).
-// Bound by instruction issue; mixed-radix digits (a triangle of 120 products and three reductions a
+// Bound by instruction issue (71 % of the slots, the integer pipes ahead); mixed-radix digits (a triangle of 120 products and three reductions a
 // digit) and a double-double Horner evaluation took 167 us for 4.2e6 entries, one modulus at a time in
 // limbs 84, this 62.
 __global__ void __launch_bounds__(256) k_oz_crt(const int8_t* __restrict__ PC, long plane, int M, int N,

@@ -584,12 +584,14 @@ struct CrtPair {
   unsigned long long mu1, mu2;  // Barrett constants of p1, p2
 };
 
-// The INT8 form's CRT: residues in [0, p) per output, already times w_t unless `weights`.  Bound by
-// the multiply-adds of the coefficients with the table rows (D a pair, one thread an output), D the
-// number of digits rounded up to the instantiated widths (launch_crt).  Then the carried words,
+// The INT8 form's CRT: residues in [0, p) per output, already times w_t unless `weights`.  A pair's
+// coefficient times its table row is D multiply-adds (one thread an output), D the number of digits rounded
+// up to the instantiated widths (launch_crt).  Bound by the latency of a pair's loads (two residues and the
+// row): 96 registers leave five blocks an SM, ten of fifteen waiting warps wait for loads and 31 % of the
+// issue slots are used.  Then the carried words,
 // S - rint(f) M, its magnitude shifted up to the top of the K words, and one rounding at the bit
 // below the N leading limbs.  2000 x 2000 outputs of 256 bits: 2166 us with one prime a step in 32-bit
-// digits, 803 us so.
+// digits, 805 us so.
 template <int D>
 __global__ void __launch_bounds__(128) k_rns_crt(const int* __restrict__ RC, long planeC, int m, int n, int L,
                                                  const CrtPair* __restrict__ pairs, const uint32_t* __restrict__ rows,
