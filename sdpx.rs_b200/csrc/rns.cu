@@ -737,10 +737,12 @@ void launch_crt(cudaStream_t st, int digits, const int* RC, long planeC, int m, 
 // svec_quadratic, 4175-4277 symmetric_bilinear) ----
 // Residues in [0, p_t) of a flat array of MpFloat<N> aligned at one exponent lo (the class's
 // lowest set bit): entry e is (-1)^s M_e 2^(exp_e - 64N - lo); out[t * count + e].  absval drops
-// the signs.  The residue is computed as in k_rns8_residues (residue_words).
-extern "C" __global__ void k_rns_class_residues(const unsigned char* __restrict__ X, int N, int count, int lo,
-                                                int absval, int L, const ResiduePrime* __restrict__ rp,
-                                                const uint32_t* __restrict__ factor, int S, int* __restrict__ out) {
+// the signs.  The residue is computed as in k_rns8_residues (residue_words; NW: words of the mantissa,
+// rounded up).
+template <int NW>
+__global__ void k_rns_class_residues(const unsigned char* __restrict__ X, int N, int count, int lo, int absval, int L,
+                                     const ResiduePrime* __restrict__ rp, const uint32_t* __restrict__ factor, int S,
+                                     int* __restrict__ out) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= count) return;
   const unsigned char* x = X + (size_t)e * (8 * N + 8);
@@ -752,12 +754,12 @@ extern "C" __global__ void k_rns_class_residues(const unsigned char* __restrict_
   const bool neg = kind < 0 && !absval;
   const int shift = elem_exp(x, N) - 64 * N - lo;
   const uint32_t* lp = reinterpret_cast<const uint32_t*>(x);
-  uint32_t w[2 * RNS_MAXN];
+  uint32_t w[NW];
 #pragma unroll
-  for (int q = 0; q < 2 * RNS_MAXN; ++q) w[q] = q < 2 * N ? lp[q] : 0u;
+  for (int q = 0; q < NW; ++q) w[q] = q < 2 * N ? lp[q] : 0u;
   for (int t = 0; t < L; ++t) {
     const int p = (int)rp[t].p;
-    int r = residue_words<2 * RNS_MAXN>(w, rp[t].c, rp[t].p, rp[t].ninv, factor[(size_t)t * S + shift]);
+    int r = residue_words<NW>(w, rp[t].c, rp[t].p, rp[t].ninv, factor[(size_t)t * S + shift]);
     if (neg && r) r = p - r;
     out[(size_t)t * count + e] = r;
   }
@@ -1331,10 +1333,16 @@ void class_residues(RnsWorkspace& ws, cudaStream_t st, DevTables& DT, int N, int
   }
   grow(ws.cres, total * L);
   DT.factors(maxbits - 64 * N + 1, st);
-  for (int c = 0; c < n; ++c)
-    if (count[c])
-      ++g_launches, k_rns_class_residues<<<(unsigned)((count[c] + 127) / 128), 128, 0, st>>>(
-          arr[c], N, count[c], lo[c], absval[c], L, DT.rp, DT.fac, DT.S, ws.cres.p + off[c] * L);
+  auto launch = [&](auto kernel) {
+    for (int c = 0; c < n; ++c)
+      if (count[c])
+        ++g_launches, kernel<<<(unsigned)((count[c] + 127) / 128), 128, 0, st>>>(
+            arr[c], N, count[c], lo[c], absval[c], L, DT.rp, DT.fac, DT.S, ws.cres.p + off[c] * L);
+  };
+  if (N <= 2) launch(k_rns_class_residues<4>);
+  else if (N <= 4) launch(k_rns_class_residues<8>);
+  else if (N <= 8) launch(k_rns_class_residues<16>);
+  else launch(k_rns_class_residues<32>);
 }
 
 // v[k] = sum_{i <= j} c_ij x_tri(j)+i q_ik q_jk (c_ii = 1, c_ij = sqrt2), k < kmax, each rounded
