@@ -19,7 +19,8 @@
 #define SDPXG_THREADS 256         // dense tile kernels (their thread maps assume 256)
 #define SDPXG_CONE_THREADS 1024   // one CTA per PSD block
 #define SDPXG_NT_SVD_THREADS 256  // the NT scaling's Jacobi launch (4 warps iterate)
-constexpr size_t kSchurSmem = 4 * 2 * 32 * 36 * sizeof(double);  // the chunk ring of k_schur_block_gemm
+constexpr size_t kSchurSmem = 2 * 2 * 32 * 36 * sizeof(double);  // the chunk ring of k_schur_block_gemm
+constexpr int kSchurGatherTile = 8;                              // rows and columns of a CTA of k_schur_gather
 #define SDPXG_EIG_THREADS 256     // step length and margins (tridiagonalisation in 4 warps' registers)
 #define SDPXG_TRIDIAG_WORK 544    // doubles of shared scratch for cta_tridiagonalize
 #define SDPXG_STURM_WORK (2 * SDPXG_NMAX)  // and for cta_eig_min / cta_eig_all

@@ -1052,7 +1052,7 @@ class Engine {
       launched("k_schur_transform");
       // CTAs that share the inner rows of a tile: up to eight (a portable cluster) while that does not
       // give an SM more than three CTAs nor a CTA less than two 32-row chunks of the longest block.  At 49
-      // tiles of 1275 rows 1 / 2 / 4 / 8 CTAs take 27.5 / 17.7 / 16.7 / 17.7 us.
+      // tiles of 1275 rows (a ring of four stages) 1 / 2 / 4 / 8 CTAs take 27.5 / 17.7 / 16.7 / 17.7 us.
       int split = 1;
       while (split < 8 && 2L * ntiles_ * split <= 3 * 148 && tn_max_ >= 2 * split * 64) split *= 2;
       cudaLaunchAttribute at{};
@@ -1089,9 +1089,9 @@ class Engine {
     }
     long tot = (long)n * n;
     if (tot) {
-      const long gt = (n + 31) / 32;
-      ++g_launches, k_schur_gather<<<(unsigned)(gt * (gt + 1) / 2), 1024, 0, st>>>(n, c2b_ptr_, c2b_blk_, c2b_loc_,
-                                                                  kcount_, s_off_, S_, Hsave_, status_);
+      const long gt = (n + kSchurGatherTile - 1) / kSchurGatherTile;
+      ++g_launches, k_schur_gather<<<(unsigned)(gt * (gt + 1) / 2), kSchurGatherTile * kSchurGatherTile, 0, st>>>(
+                        n, c2b_ptr_, c2b_blk_, c2b_loc_, kcount_, s_off_, S_, Hsave_, status_);
       launched("k_schur_gather");
     }
     if (pup_nnz_) {

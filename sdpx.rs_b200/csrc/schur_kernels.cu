@@ -47,16 +47,19 @@ k_schur_transform(const BlockDesc* __restrict__ blocks, const int* __restrict__ 
 // Grouped GEMM S_j = Acol_j' * Tcol_j (k_j x k_j, inner tri(n_j)) on the FP64 tensor cores.
 // Tile list entries (block, tile row, tile col) of 32 x 32 output tiles; the inner rows of a tile are dealt
 // in 32-row chunks to the CTAs of one cluster (its size is the launch's), whose sums meet through
-// distributed shared memory in rank order.  A four-stage ring of chunks (cp.async, 8 bytes: a column
+// distributed shared memory in rank order.  A two-stage ring of chunks (cp.async, 8 bytes: a column
 // starts anywhere) feeds the 8 warps, each with two 8 x 8 output subtiles accumulated by mma.sync m8n8k4
 // (lane (r, q): A fragment A'(row r, k q), B fragment T(k q, column r); results C(r, 2q) and C(r, 2q + 1)).
 // Chunk columns are 36 doubles apart (4 mod 16: the fragment reads of a half-warp hit distinct banks).
 // Bound by the latency of the chunks while the tiles are few: 49 tiles of 1275 inner rows (order 50, 200
-// constraints) took 117 us with one CTA a tile and plain loads, 27.5 with the ring, 17 with it in clusters.
+// constraints) took 117 us with one CTA a tile and plain loads, 27.5 with a ring, 17 with it in clusters.  Two
+// stages leave room for six CTAs an SM; with four stages and three CTAs an SM 16.3 us against 14.4 here, 59.6
+// against 57.5 (256 tiles of 2080 rows), 720 against 654 (4000 tiles of 2080 rows), 611 against 444 (50000 tiles of
+// 36 rows).
 #define SCHUR_TILE 32
 #define SCHUR_KC 32
 #define SCHUR_LD 36
-#define SCHUR_STAGES 4
+#define SCHUR_STAGES 2
 static_assert(kSchurSmem == SCHUR_STAGES * 2 * SCHUR_TILE * SCHUR_LD * sizeof(double), "ring");
 
 namespace {
@@ -144,26 +147,28 @@ k_schur_block_gemm(const BlockDesc* __restrict__ blocks, const int* __restrict__
 }
 
 // H (m x m, full, column-major) = sum over shared blocks of S_j[la, lb], in cone order.
-// One CTA per 32 x 32 tile on or above the diagonal (grid.x numbers them by columns); both triangles are
+// One CTA per 8 x 8 tile on or above the diagonal (grid.x numbers them by columns); both triangles are
 // written (symmetrised by construction), the mirrored tile through shared memory so that its stores are
-// whole lines too.  A non-finite entry sets SDPXG_ST_NONFINITE (`status`), which saves another pass over H
-// (74 us at m = 4000).  m = 4000, four of 64 blocks a row: 143 us, 164 with one thread an entry and stores a
-// column apart, 157 with the tile's block lists in shared memory.
-extern "C" __global__ void __launch_bounds__(1024)
+// whole sectors too.  A non-finite entry sets SDPXG_ST_NONFINITE (`status`), which saves another pass over H
+// (74 us at m = 4000).  A thread's chain of loads bounds it, so small CTAs on all SMs: m = 4000, four of 64
+// blocks a row, 129 us (131 with 16 x 16, 145 with 32 x 32 tiles; 164 with one thread an entry and stores a
+// column apart); m = 100, all of 200 blocks a row, 76 us (80, 174); m = 1500, 40 blocks 184 (209, 264).
+#define SCHUR_GT kSchurGatherTile
+extern "C" __global__ void __launch_bounds__(SCHUR_GT * SCHUR_GT)
 k_schur_gather(int m, const int* __restrict__ c2b_ptr, const int* __restrict__ c2b_blk,
                const int* __restrict__ c2b_loc, const int* __restrict__ kcount,
                const long* __restrict__ s_off, const double* __restrict__ S, double* __restrict__ H,
                uint32_t* __restrict__ status) {
-  __shared__ double mirror[32][33];
+  __shared__ double mirror[SCHUR_GT][SCHUR_GT + 1];
   int tj = (int)((sqrtf(8.0f * blockIdx.x + 1.0f) - 1.0f) * 0.5f);
   while ((long)tj * (tj + 1) / 2 > blockIdx.x) --tj;
   while ((long)(tj + 1) * (tj + 2) / 2 <= blockIdx.x) ++tj;
   const int ti = (int)(blockIdx.x - (long)tj * (tj + 1) / 2);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int a = 32 * ti + lane;
+  const int lane = threadIdx.x % SCHUR_GT, w = threadIdx.x / SCHUR_GT;
+  const int a = SCHUR_GT * ti + lane;
   bool bad = false;
   {
-    const int b = 32 * tj + w;
+    const int b = SCHUR_GT * tj + w;
     if (a <= b && b < m) {
       int pa = c2b_ptr[a], pb = c2b_ptr[b];
       const int ea = c2b_ptr[a + 1], eb = c2b_ptr[b + 1];
@@ -190,8 +195,8 @@ k_schur_gather(int m, const int* __restrict__ c2b_ptr, const int* __restrict__ c
     }
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(status, SDPXG_ST_NONFINITE);
-  const int b = 32 * tj + lane;
-  const int col = 32 * ti + w;
+  const int b = SCHUR_GT * tj + lane;
+  const int col = SCHUR_GT * ti + w;
   if (col < b && b < m) H[b + (long)col * m] = mirror[w][lane];
 }
 
