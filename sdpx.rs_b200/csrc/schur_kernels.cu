@@ -280,9 +280,15 @@ extern "C" __global__ void k_op_adjoint_partial(const BlockDesc* __restrict__ bl
   for (; r + 7 * 32 < tn; r += 8 * 32)
 #pragma unroll
     for (int u = 0; u < 8; ++u) a8[u] = fma(A[r + 32 * u], zc[r + 32 * u], a8[u]);
+  if (tn - (r - lane) > 64) {
 #pragma unroll
-  for (int u = 0; u < 7; ++u)
-    if (r + 32 * u < tn) a8[u] = fma(A[r + 32 * u], zc[r + 32 * u], a8[u]);
+    for (int u = 0; u < 7; ++u)
+      if (r + 32 * u < tn) a8[u] = fma(A[r + 32 * u], zc[r + 32 * u], a8[u]);
+  } else {  // a short column, or a long one's end
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (r + 32 * u < tn) a8[u] = fma(A[r + 32 * u], zc[r + 32 * u], a8[u]);
+  }
   double acc = ((a8[0] + a8[1]) + (a8[2] + a8[3])) + ((a8[4] + a8[5]) + (a8[6] + a8[7]));
   acc = warp_sum(acc);
   if (lane == 0) p[(long)blockIdx.y * ldp + col_ptr[j] + t] = acc;
