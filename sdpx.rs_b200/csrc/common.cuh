@@ -149,34 +149,35 @@ __device__ __forceinline__ double warp_min(double v) {
 // ------------------------------------------------------------------------------------
 #define SM(A, i, j) (A)[(i) + (j) * SDPXG_LD]
 
-// Shared matrices are 64 x 64 (leading dimension SDPXG_LD) whatever the block order n; the
-// entries outside n x n are kept at zero so the tensor-core products below can run on whole
-// 8 x 8 x 4 fragments.  Loads write the zero padding; products of padded inputs keep it.
-__device__ __forceinline__ void cta_zero_mat(double* M) {
-  for (int e = threadIdx.x; e < SDPXG_LD * SDPXG_NMAX; e += blockDim.x) M[e] = 0.0;
-}
+// Shared matrices are 64 x 64 (leading dimension SDPXG_LD) whatever the block order n; the entries outside
+// n x n up to the next multiple of eight are zero, so that the tensor-core products below can run on whole
+// 8 x 8 x 4 fragments.  Loads write that padding (`pad`: to another size); products of padded inputs keep
+// it.  What lies beyond is not read into a result.
+__device__ __forceinline__ int pad8(int n) { return (n + 7) & ~7; }
 
-// M = smat(v): symmetric matrix from an svec (zero padded to 64 x 64).  Column j of the upper
-// triangle is contiguous in the svec (v[j(j+1)/2 + i], i <= j): one warp per column reads it
-// coalesced, the loads of four columns in flight, and writes both triangles.
-__device__ __forceinline__ void cta_load_smat(double* M, const double* __restrict__ v, int n) {
+// M = smat(v): symmetric matrix from an svec.  Column j of the upper triangle is contiguous in the svec
+// (v[j(j+1)/2 + i], i <= j): one warp per column reads it coalesced, the loads of U columns in flight, and
+// writes both triangles.  U = 64 / warps, at most 4.
+template <int U = 4>
+__device__ __forceinline__ void cta_load_smat(double* M, const double* __restrict__ v, int n,
+                                              int pad = SDPXG_NMAX) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  for (int j0 = warp; j0 < SDPXG_NMAX; j0 += 4 * nwarps) {
-    double x[4][2];
+  for (int j0 = warp; j0 < pad; j0 += U * nwarps) {
+    double x[U][2];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < U; ++u) {
       const int j = j0 + u * nwarps;
       const double* col = v + j * (j + 1) / 2;
 #pragma unroll
       for (int h = 0; h < 2; ++h) x[u][h] = (j < n && lane + 32 * h <= j) ? col[lane + 32 * h] : 0.0;
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < U; ++u) {
       const int j = j0 + u * nwarps;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int i = lane + 32 * h;
-        if (j < SDPXG_NMAX && i <= j) {
+        if (j < pad && i <= j) {
           const double y = i != j ? x[u][h] * SDPXG_RSQRT2 : x[u][h];
           SM(M, i, j) = y;
           SM(M, j, i) = y;
@@ -195,20 +196,27 @@ __device__ __forceinline__ void cta_store_svec(double* __restrict__ v, const dou
   }
 }
 
-// M = the n x n matrix at g, zero padded to 64 x 64, eight loads in flight per thread.
-__device__ __forceinline__ void cta_load_mat(double* M, const double* __restrict__ g, int n) {
-  for (int e0 = threadIdx.x; e0 < SDPXG_NMAX * SDPXG_NMAX; e0 += 8 * blockDim.x) {
-    double x[8];
+// M = the n x n matrix at g, one warp a column, the loads of U columns in flight.
+template <int U = 4>
+__device__ __forceinline__ void cta_load_mat(double* M, const double* __restrict__ g, int n,
+                                             int pad = SDPXG_NMAX) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  for (int j0 = warp; j0 < pad; j0 += U * nwarps) {
+    double x[U][2];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int e = e0 + u * blockDim.x, i = e % SDPXG_NMAX, j = e / SDPXG_NMAX;
-      x[u] = (i < n && j < n) ? g[i + j * n] : 0.0;
-    }
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int e = e0 + u * blockDim.x;
-      if (e < SDPXG_NMAX * SDPXG_NMAX) SM(M, e % SDPXG_NMAX, e / SDPXG_NMAX) = x[u];
-    }
+      for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h, j = j0 + u * nwarps;
+        x[u][h] = (i < n && j < n) ? g[i + j * n] : 0.0;
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h, j = j0 + u * nwarps;
+        if (i < pad && j < pad) SM(M, i, j) = x[u][h];
+      }
   }
 }
 

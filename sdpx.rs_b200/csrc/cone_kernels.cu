@@ -43,7 +43,7 @@ k_nt_factor(const BlockDesc* __restrict__ blocks, const double* __restrict__ s,
   const BlockDesc bd = blocks[blockIdx.x];
   const int n = bd.n;
   double* L = smem;
-  cta_load_smat(L, (blockIdx.y == 0 ? s : z) + bd.svec_off, n);
+  cta_load_smat(L, (blockIdx.y == 0 ? s : z) + bd.svec_off, n, pad8(n));
   if (!cta_cholesky_lower(L, n)) {
     if (threadIdx.x == 0) atomicOr(status, SDPXG_ST_CHOL_FAIL);
     return;
@@ -80,10 +80,11 @@ k_nt_svd(const BlockDesc* __restrict__ blocks, double* __restrict__ R, double* _
   int* rank = reinterpret_cast<int*>(isig + SDPXG_NMAX);
   int* flag = rank + SDPXG_NMAX;
 
-  cta_zero_mat(V);  // V and X are written n x n only: keep their padding zero for the MMAs
-  cta_zero_mat(X);
-  cta_load_mat(L1, R + bd.mat_off, n);
-  cta_load_mat(L2, Rinv + bd.mat_off, n);
+  for (int j = threadIdx.x >> 5; j < pad8(n); j += SDPXG_NT_SVD_THREADS / 32)  // V and X are written n x n
+    for (int i = threadIdx.x & 31; i < pad8(n); i += 32)                       // only: zeros for the MMAs
+      if (i >= n || j >= n) SM(V, i, j) = SM(X, i, j) = 0.0;
+  cta_load_mat(L1, R + bd.mat_off, n, pad8(n));
+  cta_load_mat(L2, Rinv + bd.mat_off, n, pad8(n));
   __syncthreads();
   cta_gemm<true, false, 8, GEMM_LOWER_TN>(M, L2, L1, n);  // M = L2' L1
   __syncthreads();
@@ -302,8 +303,8 @@ k_congruence(const BlockDesc* __restrict__ blocks, int mode, const double* __res
   double* T = X + kMat;
   double* Y = T + 16 * SDPXG_LD;
   const bool use_r = (mode == 0 || mode == 1 || mode == 4);
-  cta_load_mat(B, (use_r ? R : Rinv) + bd.mat_off, n);
-  cta_load_smat(X, x + off, n);
+  cta_load_mat(B, (use_r ? R : Rinv) + bd.mat_off, n, pad8(n));
+  cta_load_smat(X, x + off, n, pad8(n));
   __syncthreads();
   // W x (R' X R) first for Hs, Winv' x (Rinv X Rinv') first for Hs^-1
   bool outer_t = mode == 1 || mode == 3 || mode == 5;
@@ -347,8 +348,8 @@ k_circ_op(const BlockDesc* __restrict__ blocks, const double* __restrict__ yv,
   const int n = bd.n;
   double* Y = smem;
   double* Z = Y + kMat;
-  cta_load_smat(Y, yv + bd.svec_off, n);
-  cta_load_smat(Z, zv + bd.svec_off, n);
+  cta_load_smat<2>(Y, yv + bd.svec_off, n, n);
+  cta_load_smat<2>(Z, zv + bd.svec_off, n, n);
   __syncthreads();
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
     int i = e % n, j = e / n;
@@ -420,8 +421,8 @@ k_step_length(const BlockDesc* __restrict__ blocks, const double* __restrict__ R
   double* dd = D + kMat;  // d[n], e[n], one int
   double* ee = dd + SDPXG_NMAX;
   int* best = reinterpret_cast<int*>(ee + SDPXG_NMAX);
-  cta_load_mat(B, (side == 0 ? R : Rinv) + bd.mat_off, n);
-  cta_load_smat(X, (side == 0 ? dz : ds) + bd.svec_off, n);
+  cta_load_mat(B, (side == 0 ? R : Rinv) + bd.mat_off, n, pad8(n));
+  cta_load_smat(X, (side == 0 ? dz : ds) + bd.svec_off, n, pad8(n));
   __syncthreads();
   cta_congruence(D, T, X, B, side == 1, n);
   const double* ls = lisqrt + bd.vec_off;
@@ -479,14 +480,14 @@ k_margins(const BlockDesc* __restrict__ blocks, const double* __restrict__ v, lo
   int* best = reinterpret_cast<int*>(eig + SDPXG_NMAX);
   const double* vb = v + (long)blockIdx.y * ld + bd.svec_off;
   const long o = 2L * ((long)blockIdx.y * gridDim.x + b);
-  cta_load_smat(X, vb, n);
+  cta_load_smat(X, vb, n, pad8(n));
   __syncthreads();
   if (min_only) {
     if (cta_cholesky_lower(X, n)) {
       if (threadIdx.x == 0) out[o] = out[o + 1] = 0.0;
       return;
     }
-    cta_load_smat(X, vb, n);
+    cta_load_smat(X, vb, n, pad8(n));
     __syncthreads();
     cta_tridiagonalize(X, n, dd, ee, work);
     bool ok = true;

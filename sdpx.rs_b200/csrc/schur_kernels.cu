@@ -33,9 +33,9 @@ k_schur_transform(const BlockDesc* __restrict__ blocks, const int* __restrict__ 
   double* G = smem;
   double* X = G + kMat;
   double* Y = X + kMat;
-  cta_load_mat(G, Ginv + bd.mat_off, n);
+  cta_load_mat<2>(G, Ginv + bd.mat_off, n, pad8(n));
   const long off = acol_off[j] + (long)t * tn;
-  cta_load_smat(X, Acol + off, n);
+  cta_load_smat<2>(X, Acol + off, n, pad8(n));
   __syncthreads();
   cta_gemm<false, false, 2>(Y, G, X, n);  // Y = Ginv A
   __syncthreads();
