@@ -202,6 +202,8 @@ __global__ void k_identity_scaling(const BlockDesc*, double*, double*, double*, 
 __global__ void k_ginv_from_rinv(const BlockDesc*, const double*, double*);
 __global__ void k_congruence(const BlockDesc*, int, const double*, const double*, const double*, const double*,
                              double*, long);
+__global__ void k_congruence_one(const BlockDesc*, int, const double*, const double*, const double*, const double*,
+                                 double*, long, int);
 __global__ void k_circ_op(const BlockDesc*, const double*, const double*, double*);
 __global__ void k_lam_inv_circ(const BlockDesc*, const double*, const double*, double*);
 __global__ void k_affine_ds(const BlockDesc*, const double*, double*);

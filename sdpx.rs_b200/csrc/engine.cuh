@@ -33,6 +33,13 @@ constexpr int kMatD = SDPXG_LD * SDPXG_NMAX;
 constexpr size_t kSmemNtFactor = kMatD * sizeof(double);
 constexpr size_t kSmemNt = (5 * kMatD + 5 * SDPXG_NMAX) * sizeof(double) + (SDPXG_NMAX + 1) * sizeof(int);
 constexpr size_t kSmemCong = (2 * kMatD + 2 * 16 * SDPXG_LD) * sizeof(double);
+// k_congruence_one, four matrices of the largest order's columns rounded up to eight, instead of a cluster
+// of four CTAs a block: up to order 16, and up to kCongOneMax once there are more clusters than run at once
+// (two CTAs an SM).  Cluster / one CTA, us, two congruences: order 16 1 block 6.2 / 6.2, 500 blocks 35 / 8.3; order
+// 32 32 blocks 8.3 / 9.4, 100 14.4 / 10.3, 500 47 / 18.5; order 48 32 blocks 12.4 / 17.4, 100 22.6 / 17.5, 500 78 / 39;
+// order 64 100 blocks 27.8 / 30.8, 500 102 / 117.
+constexpr int kCongOneMax = 48, kCongClusters = 2 * 148 / 4;
+inline size_t smem_cong_one(int cols) { return 4 * (size_t)SDPXG_LD * cols * sizeof(double); }
 constexpr size_t kSmemCirc = 2 * kMatD * sizeof(double);
 constexpr size_t kSmemStep = (4 * kMatD + 2 * SDPXG_NMAX + 1) * sizeof(double);
 constexpr size_t kSmemMarg = (kMatD + 3 * SDPXG_NMAX + SDPXG_TRIDIAG_WORK + 1) * sizeof(double);
@@ -435,6 +442,7 @@ class Engine {
     set_smem(reinterpret_cast<const void*>(k_nt_factor), kSmemNtFactor);
     set_smem(reinterpret_cast<const void*>(k_nt_svd), kSmemNt);
     set_smem(reinterpret_cast<const void*>(k_congruence), kSmemCong);
+    set_smem(reinterpret_cast<const void*>(k_congruence_one), smem_cong_one(kCongOneMax));
     set_smem(reinterpret_cast<const void*>(k_circ_op), kSmemCirc);
     set_smem(reinterpret_cast<const void*>(k_step_length), kSmemStep);
     set_smem(reinterpret_cast<const void*>(k_margins), kSmemMarg);
@@ -504,6 +512,8 @@ class Engine {
       veclen_ = vec;
     }
     nblk = (int)hblocks.size();
+    nmax_ = 0;
+    for (const BlockDesc& d : hblocks) nmax_ = std::max(nmax_, d.n);
     nnn_ = (int)nn_rows.size();
     // per-block dense column storage of A.  Columns of A are independent: the block memberships,
     // the dense columns and the rank-one tests run on the host threads (rows within a column are
@@ -883,9 +893,14 @@ class Engine {
     need(y, "cone_apply y");
     if (!nblk && !nnn_) return;
     tbegin(KT_CONE);
-    if (nblk)
+    if (nblk && (nmax_ <= 16 || (nmax_ <= kCongOneMax && (long)nblk * ncols > kCongClusters))) {
+      const int cols = (nmax_ + 7) & ~7;
+      ++g_launches, k_congruence_one<<<dim3(nblk, ncols), 256, smem_cong_one(cols), st>>>(
+          blocks_, mode, R_, Rinv_, x, base, y, ld ? ld : m, cols);
+    } else if (nblk) {
       ++g_launches, k_congruence<<<dim3(4 * nblk, ncols), 256, kSmemCong, st>>>(blocks_, mode, R_, Rinv_, x, base, y,
                                                                                ld ? ld : m);
+    }
     if (nnn_)
       ++g_launches, k_nn_cone<<<dim3((nnn_ + 255) / 256, ncols), 256, 0, st>>>(nnn_, nn_idx_, mode, nnw_, x,
                                                                                base, y, ld ? ld : m);
@@ -1397,6 +1412,7 @@ class Engine {
   void launched(const char* what) { check(cudaGetLastError(), what); }
 
   double up_t_[3] = {0, 0, 0};
+  int nmax_ = 0;  // largest block order
   int matlen_ = 0, veclen_ = 0, nwork_ = 0, ntiles_ = 0, tn_max_ = 0, p_nnz_ = 0, pup_nnz_ = 0;
   bool factor_ok_ = false;
   DevBuf<BlockDesc> blocks_;
