@@ -339,17 +339,18 @@ k_congruence(const BlockDesc* __restrict__ blocks, int mode, const double* __res
   }
 }
 
-// The same operators with one CTA a block, for problems whose blocks are small: four CTAs a block would
-// mostly load the operands four times.  The same chains of products, so the same bits.  Shared memory: four
-// matrices of `cols` columns, the largest order rounded up to eight.
-extern "C" __global__ void __launch_bounds__(kCongThreads)
+// The same operators with one CTA a block, for problems of small blocks or of many: four CTAs a block load
+// the operands four times, and past one wave of clusters that is what takes the time.  The same chains of
+// products, so the same bits.  Shared memory: four matrices of `cols` columns, the largest order rounded up to
+// eight.
+extern "C" __global__ void __launch_bounds__(1024)
 k_congruence_one(const BlockDesc* __restrict__ blocks, int mode, const double* __restrict__ R,
                  const double* __restrict__ Rinv, const double* __restrict__ x, const double* __restrict__ base,
                  double* __restrict__ y, long ld, int cols) {
   extern __shared__ double smem[];
   const BlockDesc bd = blocks[blockIdx.x];
   const int n = bd.n, nt = (n + 7) >> 3, ks = (n + 3) >> 2;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = lane >> 2, q = lane & 3;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5, r = lane >> 2, q = lane & 3;
   const long off = (long)blockIdx.y * ld + bd.svec_off;
   double* B = smem;
   double* X = B + cols * SDPXG_LD;
@@ -359,32 +360,39 @@ k_congruence_one(const BlockDesc* __restrict__ blocks, int mode, const double* _
   cta_load_mat(B, (use_r ? R : Rinv) + bd.mat_off, n, 8 * nt);
   cta_load_smat(X, x + off, n, 8 * nt);
   __syncthreads();
+  auto products = [&](auto a, auto b, auto c) {  // fragments of four steps of the inner index at once
+    int k0 = 0;
+    for (; k0 + 4 <= ks; k0 += 4) {
+      double x[4], y4[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        x[u] = a(((k0 + u) << 2) + q);
+        y4[u] = b(((k0 + u) << 2) + q);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) dmma_m8n8k4(c(u)[0], c(u)[1], x[u], y4[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+      if (k0 + u < ks) dmma_m8n8k4(c(u)[0], c(u)[1], a(((k0 + u) << 2) + q), b(((k0 + u) << 2) + q));
+  };
   auto congruence = [&](bool outer_t) {  // Y (upper tiles) = op(B)' X op(B), as slab_times and slab_close
-    for (int t = w; t < nt * nt; t += kCongThreads / 32) {
+    for (int t = w; t < nt * nt; t += warps) {
       const int I = t % nt, J = t / nt;
       double c[2][2] = {};
-      for (int k0 = 0; k0 < ks; k0 += 2)
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int k = ((k0 + u) << 2) + q;
-          if (k0 + u < ks)
-            dmma_m8n8k4(c[u][0], c[u][1], SM(X, 8 * I + r, k), outer_t ? SM(B, 8 * J + r, k) : SM(B, k, 8 * J + r));
-        }
+      products([&](int k) { return SM(X, 8 * I + r, k); },
+               [&](int k) { return outer_t ? SM(B, 8 * J + r, k) : SM(B, k, 8 * J + r); },
+               [&](int u) -> double(&)[2] { return c[u & 1]; });
       SM(T, 8 * I + r, 8 * J + 2 * q) = c[0][0] + c[1][0];
       SM(T, 8 * I + r, 8 * J + 2 * q + 1) = c[0][1] + c[1][1];
     }
     __syncthreads();
-    for (int t = w; t < nt * (nt + 1) / 2; t += kCongThreads / 32) {
+    for (int t = w; t < nt * (nt + 1) / 2; t += warps) {
       int I = t, J = 0;
       while (I > J) I -= ++J;
       double c[4][2] = {};
-      for (int k0 = 0; k0 < ks; k0 += 4)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int k = ((k0 + u) << 2) + q;
-          if (k0 + u < ks)
-            dmma_m8n8k4(c[u][0], c[u][1], outer_t ? SM(B, 8 * I + r, k) : SM(B, k, 8 * I + r), SM(T, k, 8 * J + r));
-        }
+      products([&](int k) { return outer_t ? SM(B, 8 * I + r, k) : SM(B, k, 8 * I + r); },
+               [&](int k) { return SM(T, k, 8 * J + r); }, [&](int u) -> double(&)[2] { return c[u]; });
       SM(Y, 8 * I + r, 8 * J + 2 * q) = (c[0][0] + c[1][0]) + (c[2][0] + c[3][0]);
       SM(Y, 8 * I + r, 8 * J + 2 * q + 1) = (c[0][1] + c[1][1]) + (c[2][1] + c[3][1]);
     }
@@ -393,12 +401,12 @@ k_congruence_one(const BlockDesc* __restrict__ blocks, int mode, const double* _
   const bool outer_t = mode == 1 || mode == 3 || mode == 5;
   congruence(outer_t);
   if (mode >= 4) {
-    for (int j = w; j < n; j += kCongThreads / 32)
+    for (int j = w; j < n; j += warps)
       for (int i = lane; i <= j; i += 32) SM(X, i, j) = SM(X, j, i) = SM(Y, i, j);
     __syncthreads();
     congruence(!outer_t);
   }
-  for (int j = w; j < n; j += kCongThreads / 32)
+  for (int j = w; j < n; j += warps)
     for (int i = lane; i <= j; i += 32) {
       const double v = (i == j) ? SM(Y, i, j) : SM(Y, i, j) * SDPXG_SQRT2;
       const long o = off + tri_idx(i, j);

@@ -33,12 +33,12 @@ constexpr int kMatD = SDPXG_LD * SDPXG_NMAX;
 constexpr size_t kSmemNtFactor = kMatD * sizeof(double);
 constexpr size_t kSmemNt = (5 * kMatD + 5 * SDPXG_NMAX) * sizeof(double) + (SDPXG_NMAX + 1) * sizeof(int);
 constexpr size_t kSmemCong = (2 * kMatD + 2 * 16 * SDPXG_LD) * sizeof(double);
-// k_congruence_one, four matrices of the largest order's columns rounded up to eight, instead of a cluster
-// of four CTAs a block: up to order 16, and up to kCongOneMax once there are more clusters than run at once
-// (two CTAs an SM).  Cluster / one CTA, us, two congruences: order 16 1 block 6.2 / 6.2, 500 blocks 35 / 8.3; order
-// 32 32 blocks 8.3 / 9.4, 100 14.4 / 10.3, 500 47 / 18.5; order 48 32 blocks 12.4 / 17.4, 100 22.6 / 17.5, 500 78 / 39;
-// order 64 100 blocks 27.8 / 30.8, 500 102 / 117.
-constexpr int kCongOneMax = 48, kCongClusters = 2 * 148 / 4;
+// k_congruence_one (four matrices of the largest order's columns rounded up to eight) instead of a cluster of
+// four CTAs a block: up to order 16, and above kCongClusters blocks, where the clusters do not run at once.  Its
+// threads: 256 up to order 24, 512 up to 48, 1024.  Cluster / one CTA, us, two congruences: order 16 1 block 6.2 /
+// 6.2, 500 blocks 35 / 8.3; order 32 32 blocks 8.3 / 8.3, 100 14.4 / 8.3; order 48 32 blocks 12.4 / 12.4, 100 22.6 /
+// 12.4; order 64 64 blocks 16.4 / 18.5, 100 27.7 / 18.5, 2000 409 / 226.
+constexpr int kCongClusters = 64;
 inline size_t smem_cong_one(int cols) { return 4 * (size_t)SDPXG_LD * cols * sizeof(double); }
 constexpr size_t kSmemCirc = 2 * kMatD * sizeof(double);
 constexpr size_t kSmemStep = (4 * kMatD + 2 * SDPXG_NMAX + 1) * sizeof(double);
@@ -442,7 +442,7 @@ class Engine {
     set_smem(reinterpret_cast<const void*>(k_nt_factor), kSmemNtFactor);
     set_smem(reinterpret_cast<const void*>(k_nt_svd), kSmemNt);
     set_smem(reinterpret_cast<const void*>(k_congruence), kSmemCong);
-    set_smem(reinterpret_cast<const void*>(k_congruence_one), smem_cong_one(kCongOneMax));
+    set_smem(reinterpret_cast<const void*>(k_congruence_one), smem_cong_one(SDPXG_NMAX));
     set_smem(reinterpret_cast<const void*>(k_circ_op), kSmemCirc);
     set_smem(reinterpret_cast<const void*>(k_step_length), kSmemStep);
     set_smem(reinterpret_cast<const void*>(k_margins), kSmemMarg);
@@ -893,9 +893,9 @@ class Engine {
     need(y, "cone_apply y");
     if (!nblk && !nnn_) return;
     tbegin(KT_CONE);
-    if (nblk && (nmax_ <= 16 || (nmax_ <= kCongOneMax && (long)nblk * ncols > kCongClusters))) {
-      const int cols = (nmax_ + 7) & ~7;
-      ++g_launches, k_congruence_one<<<dim3(nblk, ncols), 256, smem_cong_one(cols), st>>>(
+    if (nblk && (nmax_ <= 16 || (long)nblk * ncols > kCongClusters)) {
+      const int cols = (nmax_ + 7) & ~7, threads = nmax_ <= 24 ? 256 : nmax_ <= 48 ? 512 : 1024;
+      ++g_launches, k_congruence_one<<<dim3(nblk, ncols), threads, smem_cong_one(cols), st>>>(
           blocks_, mode, R_, Rinv_, x, base, y, ld ? ld : m, cols);
     } else if (nblk) {
       ++g_launches, k_congruence<<<dim3(4 * nblk, ncols), 256, kSmemCong, st>>>(blocks_, mode, R_, Rinv_, x, base, y,

@@ -36,22 +36,23 @@ def _interior(orders, rng):
     return tuple(np.concatenate([P.svec(spd(n)) for n in orders]) for _ in range(2))
 
 
-@pytest.mark.parametrize("orders", [list(range(1, 17)), [16] * 3, [1] * 90, [n for n in range(1, 49)] * 2, [48] * 75],
-                         ids=["1-16", "16", "1s", "1-48", "48s"])
+@pytest.mark.parametrize("orders", [list(range(1, 17)), [16] * 3, [1] * 90, [n for n in range(1, 49)] * 2, [48] * 75,
+                                    [64, 57, 3] * 25], ids=["1-16", "16", "1s", "1-48", "48s", "64s"])
 def test_congruences_do_not_depend_on_the_launch(orders):
-    """The same blocks alone (one CTA each) and before a block of order 64 (clusters)."""
+    """The same blocks together (one CTA each) and in groups with a block of order 64 (clusters, at most 64)."""
     rng = np.random.default_rng(len(orders))
     R = [rng.standard_normal((n, n)) for n in orders]
     Ri = [rng.standard_normal((n, n)) for n in orders]
-    t = sum(_tri(n) for n in orders)
-    x = rng.standard_normal(t + _tri(64))
-    out = []
-    for extra in (0, 1):
-        o = orders + [64] * extra
-        ctx, _ = _context(o, 1, rng)
-        ctx.set_scaling(R + [np.eye(64)] * extra, Ri + [np.eye(64)] * extra)
-        out.append([ctx.cone_apply(op, x[:t + extra * _tri(64)])[:t] for op in range(6)])
-    for a, b in zip(*out):
+    x = [rng.standard_normal(_tri(n)) for n in orders]
+
+    def apply(part, extra):
+        ctx, _ = _context([orders[j] for j in part] + [64] * extra, 1, rng)
+        ctx.set_scaling([R[j] for j in part] + [np.eye(64)] * extra, [Ri[j] for j in part] + [np.eye(64)] * extra)
+        v = np.concatenate([x[j] for j in part] + [np.zeros(_tri(64))] * extra)
+        return [ctx.cone_apply(op, v)[:sum(_tri(orders[j]) for j in part)] for op in range(6)]
+    groups = [range(k, min(k + 60, len(orders))) for k in range(0, len(orders), 60)]
+    want = [np.concatenate(parts) for parts in zip(*(apply(g, 1) for g in groups))]
+    for a, b in zip(apply(range(len(orders)), 0), want):
         assert np.all(np.isfinite(a)) and np.array_equal(a, b)
 
 
