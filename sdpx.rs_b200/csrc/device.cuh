@@ -192,6 +192,9 @@ struct PinnedBuf {
 
 // Kernel declarations (defined in the *_kernels.cu translation units of this library).
 // k_coldot (dense_kernels.cu): out = rbase + alpha * (column dots of A, or of a triangle of it, with v).
+void launch_op_forward(int tiles, const BlockDesc* blocks, const int* kcount, const int* col_ptr, const int* col_idx,
+                       const long* acol_off, const double* Acol, const int* ftile_blk, const int* ftile_r0,
+                       const double* x, double alpha, double beta, const double* base, double* y, cudaStream_t st);
 void launch_coldot(const double* A, int n, int tri, const double* v, const double* rbase, double alpha, double* out,
                    cudaStream_t st);
 extern "C" {
@@ -218,9 +221,6 @@ __global__ void k_schur_block_gemm(const BlockDesc*, const int*, const int*, con
 __global__ void k_schur_gather(int, const int*, const int*, const int*, const int*, const long*,
                                const double*, double*, uint32_t*);
 __global__ void k_add_upper_csc(int, const int*, const int*, const double*, double*);
-__global__ void k_op_forward(const BlockDesc*, const int*, const int*, const int*, const long*,
-                             const double*, const int*, const int*, const double*, long, double,
-                             double, const double*, double*, long);
 __global__ void k_op_adjoint_partial(const BlockDesc*, const int*, const int*, const int*,
                                      const long*, const double*, const double*, long, double*,
                                      long, int);

@@ -993,9 +993,8 @@ class Engine {
     }
     if (!nblk) return;
     if (nftile_) {
-      ++g_launches, k_op_forward<<<dim3(nftile_, 1), 512, 0, st>>>(
-          blocks_, kcount_, col_ptr_, col_idx_, acol_off_, acol_, ftile_blk_, ftile_r0_, x, n, alpha,
-          beta, base, y, m);
+      ++g_launches, launch_op_forward(nftile_, blocks_, kcount_, col_ptr_, col_idx_, acol_off_, acol_, ftile_blk_,
+                                      ftile_r0_, x, alpha, beta, base, y, st);
       launched("k_op_forward");
     }
     if (nms_) {

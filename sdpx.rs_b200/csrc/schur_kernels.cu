@@ -215,47 +215,97 @@ extern "C" __global__ void k_add_upper_csc(int n, const int* __restrict__ colptr
 }
 
 // y[rows of block j] = alpha * Acol_j x[cols_j] + beta * base.  One CTA per 32-row tile of a block
-// (tile list ftile_blk / ftile_r0): one row a lane, the columns dealt to 16 warps, four loads in
-// flight a thread; the partial sums are combined in a fixed order (deterministic).  Bound by the
-// memory round trips of a thread's columns: at 200 columns 13 of them (64 rows and four column
-// groups a CTA had 50).
-#define FWD_GROUPS 16
-extern "C" __global__ void __launch_bounds__(32 * FWD_GROUPS)
+// (tile list ftile_blk / ftile_r0): one row a lane, the columns dealt to GROUPS warps; the partial sums are
+// combined in a fixed order (deterministic).  Bound by the memory round trips of a thread's columns while the
+// tiles are few (then sixteen warps and eight loads in flight a thread), by the warps themselves when they are
+// many (four).
+namespace {
+
+template <int GROUPS>
+__global__ void __launch_bounds__(32 * GROUPS)
 k_op_forward(const BlockDesc* __restrict__ blocks, const int* __restrict__ kcount,
              const int* __restrict__ col_ptr, const int* __restrict__ col_idx,
              const long* __restrict__ acol_off, const double* __restrict__ Acol,
              const int* __restrict__ ftile_blk, const int* __restrict__ ftile_r0,
-             const double* __restrict__ x, long ldx, double alpha, double beta, const double* base,
-             double* y, long ldy) {
-  __shared__ double part[FWD_GROUPS][32];
+             const double* __restrict__ x, double alpha, double beta, const double* base, double* y) {
+  __shared__ double part[GROUPS][32];
   const int j = ftile_blk[blockIdx.x], r0 = ftile_r0[blockIdx.x];
   const BlockDesc bd = blocks[j];
   const int tn = bd.n * (bd.n + 1) / 2;
   const int k = kcount[j];
   const double* A = Acol + acol_off[j];
   const int* cols = col_idx + col_ptr[j];
-  const double* xc = x + (long)blockIdx.y * ldx;
   const int rr = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int r = r0 + rr;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   if (r < tn) {
-    int t = g;
-    for (; t + 3 * FWD_GROUPS < k; t += 4 * FWD_GROUPS)
+    if (GROUPS == 4) {
+      for (int t = g; t < k; t += GROUPS) acc[0] = fma(A[(long)t * tn + r], x[cols[t]], acc[0]);
+    } else {  // steps t, t + GROUPS, ...: whole fours into the four sums, the rest into the first
+      int t = g;
+      for (; t + 7 * GROUPS < k; t += 8 * GROUPS) {
+        int c[8];
+        double a[8], v[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        acc[u] = fma(A[(long)(t + u * FWD_GROUPS) * tn + r], xc[cols[t + u * FWD_GROUPS]], acc[u]);
-    for (; t < k; t += FWD_GROUPS) acc[0] = fma(A[(long)t * tn + r], xc[cols[t]], acc[0]);
+        for (int u = 0; u < 8; ++u) {
+          c[u] = __ldg(cols + t + u * GROUPS);
+          a[u] = __ldg(A + (long)(t + u * GROUPS) * tn + r);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = __ldg(x + c[u]);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc[u & 3] = fma(a[u], v[u], acc[u & 3]);
+      }
+      if (t < k) {  // the last ones at once too
+        int c[7];
+        double a[7], v[7];
+#pragma unroll
+        for (int u = 0; u < 7; ++u) {
+          const bool in = t + u * GROUPS < k;
+          c[u] = in ? __ldg(cols + t + u * GROUPS) : -1;
+          a[u] = in ? __ldg(A + (long)(t + u * GROUPS) * tn + r) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 7; ++u) v[u] = c[u] >= 0 ? __ldg(x + c[u]) : 0.0;
+        const bool four = t + 3 * GROUPS < k;
+#pragma unroll
+        for (int u = 0; u < 7; ++u) {
+          if (t + u * GROUPS >= k) continue;
+          if (u > 0 && u < 4 && four) acc[u] = fma(a[u], v[u], acc[u]);
+          else acc[0] = fma(a[u], v[u], acc[0]);
+        }
+      }
+    }
   }
   part[g][rr] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
   __syncthreads();
   if (g == 0 && r < tn) {
     double s = 0.0;
 #pragma unroll
-    for (int u = 0; u < FWD_GROUPS; ++u) s += part[u][rr];
-    const long o = (long)blockIdx.y * ldy + bd.svec_off + r;
+    for (int u = 0; u < GROUPS; ++u) s += part[u][rr];
+    const long o = bd.svec_off + r;
     y[o] = alpha * s + ((beta == 0.0) ? 0.0 : beta * base[o]);
   }
 }
+
+}  // namespace
+
+namespace sdpxg {
+
+// Sixteen warps a tile up to four CTAs an SM, four above.  Sixteen / four, us: 40 tiles of 200 columns 5.7 / 9.2, 150
+// of 3000 37 / 190, 65 of 500 6.2 / 16.4; 1000 of 300 16.4 / 12.3, 3500 of 10 22.6 / 6.2, 13000 of 50 141 / 45.
+void launch_op_forward(int tiles, const BlockDesc* blocks, const int* kcount, const int* col_ptr, const int* col_idx,
+                       const long* acol_off, const double* Acol, const int* ftile_blk, const int* ftile_r0,
+                       const double* x, double alpha, double beta, const double* base, double* y, cudaStream_t st) {
+  auto go = [&](auto kernel, int groups) {
+    kernel<<<tiles, 32 * groups, 0, st>>>(blocks, kcount, col_ptr, col_idx, acol_off, Acol, ftile_blk, ftile_r0, x,
+                                          alpha, beta, base, y);
+  };
+  if (tiles <= 4 * 148) go(k_op_forward<16>, 16);
+  else go(k_op_forward<4>, 4);
+}
+
+}  // namespace sdpxg
 
 // Per-block partial adjoint p[acol column] = Acol_j[:, t] . z_j  (one warp per column, eight loads
 // in flight a lane)

@@ -77,6 +77,20 @@ def test_schur_of_small_blocks(orders, m):
     assert np.max(np.abs(H - A.T @ T)) <= 4 * A.shape[0] * EPS * (a * g) ** 2
 
 
+@pytest.mark.parametrize("orders,m", [([50], k) for k in (1, 15, 16, 17, 63, 64, 65, 112, 127, 128, 129, 191, 250)]
+                         + [([33] * 35, 7), ([8] * 400, 33), ([1] * 700, 5)])
+def test_constraint_products(orders, m):
+    """A x and A' z through the residual with zero right-hand sides and the identity scaling: columns at the
+    edges of the forward product's rounds of loads, and more tiles than its sixteen-warp form takes."""
+    rng = np.random.default_rng(m)
+    ctx, A = _context(orders, m, rng)
+    ctx.identity_scaling()
+    x, z = rng.standard_normal(m), rng.standard_normal(A.shape[0])
+    ex, ez, _ = ctx.residual(np.zeros(m), np.zeros(A.shape[0]), x, z)
+    assert np.all(np.abs(-ex - A.T @ z) <= 4 * A.shape[0] * EPS * (np.abs(A.T) @ np.abs(z)))
+    assert np.all(np.abs(ez - (z - A @ x)) <= 4 * (m + 8) * EPS * (np.abs(A) @ np.abs(x) + 2 * np.abs(z).max()))
+
+
 POISON = r"""
 #include <cuda_runtime.h>
 __global__ void k_poison(int words) {
