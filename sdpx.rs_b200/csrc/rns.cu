@@ -322,6 +322,14 @@ __global__ void __launch_bounds__(256) k_rns8_residues(const unsigned char* __re
     }
   }
   const int per_t = (L + gridDim.y - 1) / gridDim.y, t0 = blockIdx.y * per_t, t1 = min(L, t0 + per_t);
+  if (x >= nlines || y >= len) {  // the padding
+    int8_t* d = o + (size_t)(2 * t0) * plane;
+    for (int t = 2 * t0; t < 2 * t1; ++t, d += plane) {
+      if (E == 4) *reinterpret_cast<uint32_t*>(d) = 0u;
+      else *reinterpret_cast<uint16_t*>(d) = 0u;
+    }
+    return;
+  }
 #pragma unroll 1
   for (int t = t0; t < t1; ++t) {
     uint32_t c[NW];
