@@ -527,6 +527,10 @@ static __device__ __noinline__ double multisect_min_again(const double* d, const
 // norm: at most 26 rounds, and 32 more by quotients.  Uniform result; `best` is one int of shared memory, `t`
 // SDPXG_STURM_WORK doubles.  *ok = false if the round bound is hit or (d, e) is not finite.
 __device__ inline double cta_eig_min(const double* d, const double* e, int n, double2* t, int* best, bool* ok) {
+  if (n == 1) {  // orthant rows come as such blocks, thousands at a time
+    *ok = isfinite(d[0]);
+    return d[0];
+  }
   const SturmRange r = sturm_prepare(d, e, n, t);
   *ok = false;
   if (!r.finite) return 0.0;
