@@ -16,8 +16,9 @@
 
 #define GR_LD SDPXG_LD  // the layout of cta_load_mat / cta_load_smat
 
-// C (64 x nc, padded) = A (64 x 64, padded) B (64 x nc, padded) on the FP64 tensor cores,
-// one 8 x 8 output tile per warp at a time; K = 64 (zero padding makes the tail exact).
+// C (nr x nc) = A (nr x nr) B (nr x nc) on the FP64 tensor cores, one 8 x 8 output tile per warp at a time; the
+// inner index runs to gr_pad(nr), where both operands are zero past nr.
+__device__ __forceinline__ int gr_pad(int n) { return (n + 15) & ~15; }
 __device__ __forceinline__ void gr_gemm_nn(double* C, const double* A, const double* B, int nr,
                                            int nc) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -26,8 +27,7 @@ __device__ __forceinline__ void gr_gemm_nn(double* C, const double* A, const dou
   for (int t = warp; t < rt * ct; t += nwarps) {
     const int ti = (t % rt) << 3, tj = (t / rt) << 3;
     double d0 = 0.0, d1 = 0.0;
-#pragma unroll
-    for (int kg = 0; kg < 4; ++kg) {
+    for (int kg = 0; kg < gr_pad(nr) / 16; ++kg) {
       double a[4], b[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -66,7 +66,7 @@ k_gram_basis(const BlockDesc* __restrict__ blocks, const int* __restrict__ item_
   const BlockDesc bd = blocks[j];
   const int n = bd.n, k = kcount[j];
   const int nc = min(64, k - c0);
-  cta_load_mat(Rs, Rinv + bd.mat_off, n);
+  cta_load_mat(Rs, Rinv + bd.mat_off, n, gr_pad(n));
   gr_load_chunk(Us, U + gu_off[j], n, k, c0);
   __syncthreads();
   gr_gemm_nn(Cs, Rs, Us, n, nc);
@@ -207,7 +207,7 @@ k_gram_adjoint(const BlockDesc* __restrict__ blocks, const int* __restrict__ ite
   const BlockDesc bd = blocks[j];
   const int n = bd.n, k = kcount[j];
   const int nc = min(64, k - c0);
-  cta_load_smat(Zs, z + bd.svec_off, n);
+  cta_load_smat(Zs, z + bd.svec_off, n, gr_pad(n));
   gr_load_chunk(Us, U + gu_off[j], n, k, c0);
   __syncthreads();
   gr_gemm_nn(Ws, Zs, Us, n, nc);  // W = Z U_chunk
